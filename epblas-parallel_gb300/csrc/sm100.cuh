@@ -33,6 +33,18 @@ __device__ __forceinline__ uint64_t globaltimer_ns()
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// Records a wait that gave up: `code` in the device word (first writer wins),
+// which the kernels' own waits poll, and in the host's mirror of it, whose
+// mapped address lies behind the device word (runtime.cu), so that the host
+// learns of it at its stream synchronisation without a copy.
+__device__ __forceinline__ void report_timeout(int *status, int code)
+{
+    if (atomicCAS(status, 0, code) != 0) return;
+    int *host = *(int *volatile *)(status + 2);
+    *(volatile int *)host = code;
+    __threadfence_system();
+}
+
 // ---- mbarrier ---------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
@@ -85,7 +97,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *s
             if (mbar_try_wait(bar, parity)) return true;
         if (status && *(volatile int *)status != 0) return false;
         if (globaltimer_ns() - t0 > limit) {
-            if (status) atomicCAS(status, 0, code);
+            if (status) report_timeout(status, code);
             return false;
         }
     }
@@ -283,7 +295,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
             if (mbar_try_wait_cluster(bar, parity)) return true;
         if (status && *(volatile int *)status != 0) return false;
         if (globaltimer_ns() - t0 > limit) {
-            if (status) atomicCAS(status, 0, code);
+            if (status) report_timeout(status, code);
             return false;
         }
     }
