@@ -3,26 +3,22 @@
 // beta pre-pass first (mf_kernels.h:63-68: beta == 0 zeroes y, beta == 1
 // leaves it), then nothing more when alpha == 0, as in the reference.
 //
-// NoTrans: thread per row, the columns split into chunks over grid.y so the
-// whole GPU streams A once; per-chunk partial sums go to scratch and a second
-// kernel folds them in a fixed order and applies y += alpha*s.
-// Trans: block per column (A's columns are contiguous), warp-shuffle and
-// shared-memory reduction, then y_j += alpha*s (mgemv.cpp:229-233).
-// mgemv_ accumulates the products in per-thread integer fixed point
-// (fixacc.cuh): x is first split once into 24-bit digit sets (32 bytes per
-// entry; it is small and stays in L2), each A(i,j) is decoded from its bits
-// and its digits multiplied into the thread's exact column sums; partial sums
-// combine as extended floats in a fixed order, and y := y + alpha*s is
+// mgemv_ forms the products of base-256 limbs on the tensor cores
+// (k_gemv_limb below; limbmma.cuh), exact sums per output and chunk of the
+// reduction, combined as extended floats in a fixed order; y := y + alpha*s is
 // rounded once to double-double. The FP64 pipe, which would bound a
 // double-double multiply-add at a fraction of HBM speed, is not used in the
 // loop.
 // mgemv_n_noalloc keeps the FP64 accumulation (TwoProduct + TwoSum into a
 // (sum, error) pair, renormalised every 32 terms, the lo*lo product dropped as
 // in mdot.cpp:60-64) so that its partial sums fit its fixed scratch array.
+#include <cuda_fp16.h>
+
 #include <mutex>
 
 #include "dd.cuh"
 #include "fixacc.cuh"
+#include "limbmma.cuh"
 #include "level3.h"
 #include "runtime.h"
 
@@ -86,58 +82,58 @@ __global__ void k_gemv_n_final(int64_t m, int nchunks, const double2 *part, dd::
     }
 }
 
-// ---- fixed-point kernels (mgemv_) ------------------------------------------------------
+// ---- byte-limb kernel (mgemv_) ----------------------------------------------------------
+//
+// One kernel for both directions: output r = 0..rows-1, reduction index
+// c = 0..len-1, element (r, c) at A[r * rs + c * cs]. A warp takes 32 outputs
+// in two MMA tiles; lane (g, t) = (lane / 4, lane % 4) owns the elements of
+// outputs g, g + 8, g + 16, g + 24 at every fourth reduction index, and their
+// aligned limbs (limbmma.cuh) are directly its share of the MMA operand A: the
+// K slots of lane t in MMA u are limbs 4u..4u+3 of its element. Operand B holds
+// the limbs of x as a Toeplitz band: slot (t, q) of result column s is limb
+// s - q of x at t's index, so column s collects every product of weight
+// 2^(8s), s = 7..30 in three N tiles (lower ones are below 2^-160 of the
+// block). 10 of the 12 (u, tile) products are not identically zero. A lane's
+// six distinct B pairs are 24 consecutive limbs of x from an offset that
+// depends only on g: they are laid out once per window of 32 indices in shared
+// memory and read with three 16-byte loads.
+//
+// Exactness: x's limbs are balanced (|.| <= 128), A's are bytes, 15 limbs
+// each, so a column grows by at most 15 * 255 * 128 per index and stays below
+// 2^24 units for a window's 32; then it moves to an int32 (at most 64 windows
+// per block). Each output keeps a block exponent: a product of exponent ep is
+// aligned by B - ep >= 2 bits; one above that folds the sums into an extended
+// float in shared memory and moves B up (rare after the first group).
+//
+// Bound: HBM (16 B per element) in principle, instruction issue in practice:
+// about 80 per element, where the 24-bit digit form with 19 IMAD.WIDE per
+// product and a thread per row (N) or a block per column (T) took 151.
+// Measured on one GB300, whole call: 16384^2 N 1.67 -> 1.01 ms (2.57 ->
+// 4.27 TB/s), T 1.01 ms (2.12 -> 4.26 TB/s), 7001 x 5003 T 0.45 -> 0.19 ms;
+// without the decode and alignment the same loads take 0.69 ms. Also measured
+// at 16384^2 N: one 16-output tile per warp with two or three blocks per SM
+// 1.11 ms (more shared-memory reads and set-up per element), loads into
+// registers one group ahead in place of the cp.async ring 1.29 ms.
 
-__global__ void k_dig_convert(int64_t n, const double2 *x, int64_t incx, fx::Dig *out)
-{
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
-        out[j] = fx::to_dig(fx::decode(x[vidx(j, n, incx)]));
-}
+constexpr int kWin = 32;                  // reduction indices per window
+constexpr int kMaxChunk = 64 * kWin;      // per block: int32 column sums stay below 2^30
+constexpr int kColWords = 104;            // B entry of one index: 8 x 12 words, its exponent, pad (8 mod 32 words:
+                                          // the 8 lanes of a 16-byte phase read distinct banks)
+constexpr int kR = 2, kE = 2 * kR;        // 16-output tiles per warp, elements per lane and group
+constexpr int kStages = 4;                // groups of four indices in flight per thread (cp.async)
+constexpr int kZeroE = -(1 << 20), kBadE = 1 << 20;   // exponent marks: zero (or past the end), non-finite
+constexpr int kNoBlock = -(1 << 22);                  // an output that has seen no nonzero product yet
 
-// NoTrans partial sums: row per thread, columns [j0, j1) of chunk blockIdx.y
-// (at most fx::kMaxAdds columns per chunk).
-__global__ void __launch_bounds__(256, 4) k_gemv_n_fx(int64_t m, int64_t n, const double2 *__restrict__ A,
-                                                     int64_t lda, const fx::Dig *__restrict__ xo, int64_t chunk,
-                                                     fx::XFPod *__restrict__ part)
-{
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const int64_t j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-    fx::Acc acc;
-    acc.reset();
-    const double2 *a = A + i;
-    int64_t j = j0;
-    // four columns in flight; carries propagated after each 2048 columns
-    while (j + 4 <= j1) {
-        const int64_t jend = min(j1, j + 2048);
-        for (; j + 4 <= jend; j += 4) {
-            const double2 a0 = __ldcs(a + j * lda), a1 = __ldcs(a + (j + 1) * lda);
-            const double2 a2 = __ldcs(a + (j + 2) * lda), a3 = __ldcs(a + (j + 3) * lda);
-            const fx::Dig x0 = xo[j], x1 = xo[j + 1], x2 = xo[j + 2], x3 = xo[j + 3];
-            if (fx::decode_is_fast(a0) && fx::decode_is_fast(a1) && fx::decode_is_fast(a2) && fx::decode_is_fast(a3) &&
-                ((x0.flags | x1.flags | x2.flags | x3.flags) & (fx::kZero | fx::kBad)) == 0) {
-                // normal operands (the common case): no per-product flag
-                // tests, one block-exponent test per four products
-                const fx::Op o0 = fx::decode_fast(a0), o1 = fx::decode_fast(a1);
-                const fx::Op o2 = fx::decode_fast(a2), o3 = fx::decode_fast(a3);
-                const int e0 = o0.e + x0.e, e1 = o1.e + x1.e, e2 = o2.e + x2.e, e3 = o3.e + x3.e;
-                acc.admit(max(max(e0, e1), max(e2, e3)));
-                acc.mul_fast(o0, x0, acc.B - e0);
-                acc.mul_fast(o1, x1, acc.B - e1);
-                acc.mul_fast(o2, x2, acc.B - e2);
-                acc.mul_fast(o3, x3, acc.B - e3);
-            } else {
-                acc.add_core(fx::decode(a0), x0);
-                acc.add_core(fx::decode(a1), x1);
-                acc.add_core(fx::decode(a2), x2);
-                acc.add_core(fx::decode(a3), x3);
-            }
-        }
-        acc.normalize();
-    }
-    for (; j < j1; ++j) acc.add_dig(fx::decode(a[j * lda]), xo[j]);
-    part[blockIdx.y * m + i] = fx::to_pod(acc.finish(), acc.bad);
-}
+struct GemvArgs {
+    const double2 *A;
+    const double2 *x;
+    double2 *y;
+    fx::XFPod *part;      // [chunk][output]; null: one chunk, y updated here
+    int64_t rows, len, rs, cs, incx, incy;
+    int64_t rowblocks, chunk;
+    dd::real alpha, beta;
+    int beta_kind;
+};
 
 // y(i) := y(i) + alpha * sum_c part(c, i), one rounding to double-double.
 __device__ __forceinline__ void fx_update_y(double2 *py, const xfp::XF &xa, xfp::XF s, bool bad)
@@ -160,91 +156,300 @@ __device__ __forceinline__ void fx_update_y(double2 *py, const xfp::XF &xa, xfp:
     *py = make_double2(h, l);
 }
 
-__global__ void k_gemv_n_fx_final(int64_t m, int nchunks, const fx::XFPod *part, dd::real alpha, double2 *y,
-                                  int64_t incy)
+// y := beta * y, then y := y + alpha * s
+__device__ __forceinline__ void gemv_store(const GemvArgs &g, int64_t r, const xfp::XF &xa, const xfp::XF &s, bool bad)
 {
-    const xfp::XF xa = xfp::xf_from_dd(alpha.hi, alpha.lo);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        xfp::XF s;
-        s.zero = true; s.neg = false; s.m = 0; s.e = 0;
-        bool bad = false;
-        for (int c = 0; c < nchunks; ++c) {
-            const fx::XFPod p = part[(int64_t)c * m + i];
-            bad |= (p.flags & 4) != 0;
-            s = xfp::xf_add(s, fx::from_pod(p));
+    double2 *py = g.y + vidx(r, g.rows, g.incy);
+    if (g.beta_kind == 0) *py = make_double2(0.0, 0.0);
+    else if (g.beta_kind == 2) dd::store(py, dd::mul_exact(g.beta, dd::load(py)));
+    fx_update_y(py, xa, s, bad);
+}
+
+__global__ void __launch_bounds__(256, 2) k_gemv_limb(const GemvArgs g)
+{
+    __shared__ __align__(16) uint32_t s_b[2][kWin * kColWords];
+    __shared__ __align__(16) uint32_t s_x[2][kWin][36];   // limbs in descending order, two alignments
+    __shared__ int s_e[2][kWin];
+    __shared__ fx::XFPod s_tot[8][16 * kR];
+    extern __shared__ __align__(16) unsigned char s_stage[];   // [stage][element][thread] 16 bytes
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lg = lane >> 2, lt = lane & 3;
+    const int64_t rb = blockIdx.x % g.rowblocks, ch = blockIdx.x / g.rowblocks;
+    const int64_t k0 = ch * g.chunk;
+    const int kn = (int)min(g.chunk, g.len - k0);
+    const int nwin = (kn + kWin - 1) / kWin;
+    const int64_t r0 = (rb * nw + wid) * (16 * kR);
+
+    for (int i = threadIdx.x; i < 2 * kWin * 36; i += blockDim.x) (&s_x[0][0][0])[i] = 0u;
+    if (lane < 16 * kR) s_tot[wid][lane] = fx::XFPod{0ull, 0ull, 0, 2};
+
+    // x: lane per index of a window, windows dealt to the warps in turn
+    const double2 *xbase = g.x;
+    auto load_x = [&](int win) {
+        const int c = win * kWin + lane;
+        return c < kn ? xbase[vidx(k0 + c, g.len, g.incx)] : make_double2(0.0, 0.0);
+    };
+    double2 xnext = load_x(wid);
+    auto split_x = [&](int win) {
+        const fx::Op o = fx::decode(xnext);
+        xnext = load_x(win + nw);
+        // balanced base-256 digits of W: the bytes of W + 0x80..80, less 128 each
+        uint32_t w[4];
+        asm("add.cc.u32 %0, %4, 0x80808080;\n\t"
+            "addc.cc.u32 %1, %5, 0x80808080;\n\t"
+            "addc.cc.u32 %2, %6, 0x80808080;\n\t"
+            "addc.u32 %3, %7, 0x80808080;"
+            : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+            : "r"(o.w[0]), "r"(o.w[1]), "r"(o.w[2]), "r"(o.w[3]));
+        const __half2 sg = __float2half2_rn((o.flags & fx::kNeg) ? -1.0f : 1.0f);
+        const __half2 off = __float2half2_rn((o.flags & fx::kNeg) ? 1152.0f : -1152.0f);
+        // limbs q (high half) and q + 1 (low half): 1024 + byte, times the sign, minus 1152
+        uint32_t ev[8], od[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            const uint32_t raw = __byte_perm(w[p >> 1], 0x64646464u, (p & 1) ? 0x4243 : 0x4041);
+            const __half2 h = __hfma2(*reinterpret_cast<const __half2 *>(&raw), sg, off);
+            ev[p] = *reinterpret_cast<const uint32_t *>(&h);
         }
-        fx_update_y(y + vidx(i, m, incy), xa, s, bad);
+#pragma unroll
+        for (int p = 0; p < 8; ++p)   // limbs 2p - 1 (high half) and 2p (low half)
+            od[p] = __byte_perm(ev[p], p ? ev[p > 0 ? p - 1 : 0] : 0u, 0x5432);
+        // limb q at position 22 - q: pairs from even positions in words 0.., from odd ones in words 17..
+        uint32_t *sx = s_x[win & 1][lane];
+#pragma unroll
+        for (int p = 0; p < 8; p += 4) {
+            *reinterpret_cast<uint4 *>(sx + 8 - p) = make_uint4(od[p + 3], od[p + 2], od[p + 1], od[p]);
+            *reinterpret_cast<uint4 *>(sx + 24 - p) = make_uint4(ev[p + 3], ev[p + 2], ev[p + 1], ev[p]);
+        }
+        s_e[win & 1][lane] = (o.flags & fx::kBad) ? kBadE : ((o.flags & fx::kZero) ? kZeroE : o.e - lmb::kExpBias);
+    };
+    auto expand = [&](int win) {
+        const int buf = win & 1;
+        for (int idx = threadIdx.x; idx < kWin * 8; idx += blockDim.x) {
+            const int c = idx >> 3, q = idx & 7;
+            const uint32_t *src = &s_x[buf][c][((q & 1) ? 0 : 17) + ((7 - q) >> 1)];
+            uint32_t *dst = &s_b[buf][c * kColWords + q * 12];
+#pragma unroll
+            for (int v = 0; v < 3; ++v)
+                *reinterpret_cast<uint4 *>(dst + 4 * v) =
+                    make_uint4(src[4 * v], src[4 * v + 1], src[4 * v + 2], src[4 * v + 3]);
+            if (q == 0) s_b[buf][c * kColWords + 96] = (uint32_t)s_e[buf][c];
+        }
+    };
+    __syncthreads();
+    for (int w = 0; w < 2 && w < nwin; ++w)
+        if (wid == w % nw) split_x(w);
+    __syncthreads();
+    expand(0);
+    __syncthreads();
+
+    const bool active = r0 < g.rows;
+    // lane (g, t): outputs r0 + g + 8e, e = 0..3 (past the last one its
+    // elements again, their sums are not stored), indices t, t + 4, ..
+    const int64_t row0 = min(r0 + lg, g.rows - 1);
+    const double2 *pn = g.A + row0 * g.rs + (k0 + lt) * g.cs;
+    int64_t dr[kE - 1];
+#pragma unroll
+    for (int e = 0; e < kE - 1; ++e) dr[e] = (min(r0 + lg + 8 * (e + 1), g.rows - 1) - row0) * g.rs;
+    const int64_t step = 4 * g.cs;
+    // a lane's slot in its warp's 512 bytes: what is contiguous in memory (over
+    // t for A^T, over g else) stays contiguous, as cp.async writes 32-byte
+    // sectors; g is xored with 2t so that the reads are free of bank conflicts
+    const uint32_t slot = wid * 512u + (g.cs == 1 ? lane * 16u : lt * 128u + ((lg ^ (2 * lt)) * 16u));
+    const uint32_t st0 = (uint32_t)__cvta_generic_to_shared(s_stage) + slot, st_e = blockDim.x * 16u;
+    const int nit = (kn + 3) >> 2;
+    // the four elements of group it into its stage of the thread's own ring
+    auto load_a = [&](int it) {
+        if (it < nit) {
+            const double2 *q = pn;
+            const int past = 4 * it + lt - (kn - 1);
+            if (past > 0) q -= past * g.cs;   // past the end: the last index again (its limbs of x are zero there)
+            const uint32_t d = st0 + (uint32_t)(it & (kStages - 1)) * kE * st_e;
+            lmb::cp_async16(d, q);
+#pragma unroll
+            for (int e = 0; e < kE - 1; ++e) lmb::cp_async16(d + (e + 1) * st_e, q + dr[e]);
+            pn += step;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int blk[kE];
+    uint32_t bad = 0;
+    float acc[kR][3][4];
+    int sum[kR][3][4];
+#pragma unroll
+    for (int h = 0; h < kR; ++h)
+#pragma unroll
+        for (int v = 0; v < 3; ++v)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                blk[i % kE] = kNoBlock;
+                acc[h][v][i] = 0.0f;
+                sum[h][v][i] = 0;
+            }
+    auto flush = [&]() {
+#pragma unroll
+        for (int h = 0; h < kR; ++h)
+#pragma unroll
+            for (int v = 0; v < 3; ++v)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    sum[h][v][i] += __float2int_rn(acc[h][v][i] * 16777216.0f);
+                    acc[h][v][i] = 0.0f;
+                }
+    };
+    // the column sums into the outputs' extended floats (all outputs of the warp)
+    auto fold = [&]() {
+        flush();
+#pragma unroll
+        for (int e = 0; e < kE; ++e) {
+            uint64_t W[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int v = 0; v < 3; ++v) {
+                int *c = &sum[e >> 1][v][2 * (e & 1)];
+                lmb::add_at(W, (int64_t)c[0] + ((int64_t)c[1] << 8), 64 * v + 16 * lt);
+                c[0] = c[1] = 0;
+            }
+            lmb::lane_sum256(W, 4);
+            if (lt == 0 && blk[e] != kNoBlock) {
+                fx::XFPod *tot = &s_tot[wid][lg + 8 * e];
+                *tot = fx::to_pod(xfp::xf_add(fx::from_pod(*tot), fx::w256_to_xf(W, 56 + blk[e])), false);
+            }
+        }
+        __syncwarp();
+    };
+
+    if (active)
+        for (int it = 0; it < kStages - 1; ++it) load_a(it);
+    for (int win = 0; win < nwin; ++win) {
+        if (win + 1 < nwin) expand(win + 1);
+        if (win + 2 < nwin && wid == (win + 2) % nw) split_x(win + 2);
+        if (active) {
+            const uint32_t *sb = s_b[win & 1] + lt * kColWords;
+            const int it1 = min(8 * win + 8, nit);
+#pragma unroll 1
+            for (int it = 8 * win; it < it1; ++it, sb += 4 * kColWords) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+                const unsigned char *cur = s_stage + slot + (size_t)(it & (kStages - 1)) * kE * st_e;
+                uint32_t w[kE][4], sgn[kE];
+                int sh[kE];
+                const int xe = (int)sb[96];
+                bool fast = true;
+#pragma unroll
+                for (int e = 0; e < kE; ++e) {
+                    const double2 v = *reinterpret_cast<const double2 *>(cur + e * st_e);
+                    int eh;
+                    const bool ok = lmb::split_fast(v, w[e], eh);
+                    sh[e] = blk[e] - xe - eh;
+                    fast = fast && ok && (uint32_t)(sh[e] - 2) < 30u;
+                    sgn[e] = (uint32_t)__double2hiint(v.x) & 0x80000000u;
+                }
+                if (__all_sync(0xffffffffu, fast)) {
+#pragma unroll
+                    for (int e = 0; e < kE; ++e) lmb::shr_short(w[e], sh[e]);
+                } else {
+                    // zeros, operands off the straight-line path, long alignments, a larger block
+                    int ep[kE], top[kE];
+                    bool raise = false;
+#pragma unroll
+                    for (int e = 0; e < kE; ++e) {
+                        const fx::Op o = fx::decode(*reinterpret_cast<const double2 *>(cur + e * st_e));
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) w[e][i] = o.w[i];
+                        const bool no = xe == kBadE || (o.flags & fx::kBad);
+                        if (no) bad |= 1u << e;
+                        ep[e] = (no || xe == kZeroE || (o.flags & fx::kZero)) ? kNoBlock : o.e + lmb::kExpBias + xe;
+                        top[e] = max(ep[e], __shfl_xor_sync(0xffffffffu, ep[e], 1));
+                        top[e] = max(top[e], __shfl_xor_sync(0xffffffffu, top[e], 2));
+                        raise = raise || (top[e] != kNoBlock && top[e] > blk[e] - 2);
+                    }
+                    if (__any_sync(0xffffffffu, raise)) {
+                        int seen = blk[0];
+#pragma unroll
+                        for (int e = 1; e < kE; ++e) seen = max(seen, blk[e]);
+                        if (__any_sync(0xffffffffu, seen != kNoBlock)) fold();
+#pragma unroll
+                        for (int e = 0; e < kE; ++e)
+                            if (top[e] != kNoBlock && top[e] > blk[e] - 2) blk[e] = top[e] + 4;
+                    }
+#pragma unroll
+                    for (int e = 0; e < kE; ++e) {
+                        const int d = ep[e] == kNoBlock ? 127 : min(blk[e] - ep[e], 127);
+                        uint32_t sv[4];
+                        fx::shr128(w[e], d, sv);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) w[e][i] = ep[e] == kNoBlock ? 0u : sv[i];
+                    }
+                }
+                load_a(it + kStages - 1);   // into the stage read in the previous turn
+                uint32_t f[12];
+#pragma unroll
+                for (int v = 0; v < 3; ++v) {
+                    const uint4 q = *reinterpret_cast<const uint4 *>(sb + lg * 12 + 4 * v);
+                    f[4 * v] = q.x; f[4 * v + 1] = q.y; f[4 * v + 2] = q.z; f[4 * v + 3] = q.w;
+                }
+#pragma unroll
+                for (int h = 0; h < kR; ++h)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const uint32_t a0 = lmb::limbs_lo(w[2 * h][u], sgn[2 * h]);
+                        const uint32_t a1 = lmb::limbs_lo(w[2 * h + 1][u], sgn[2 * h + 1]);
+                        const uint32_t a2 = lmb::limbs_hi(w[2 * h][u], sgn[2 * h]);
+                        const uint32_t a3 = lmb::limbs_hi(w[2 * h + 1][u], sgn[2 * h + 1]);
+#pragma unroll
+                        for (int v = 0; v < 3; ++v) {
+                            if (v == 2 && u < 2) continue;        // limbs 16 and up of x: zero
+                            const int b = 2 * (2 - (2 * v - u));   // pair of window 2v - u
+                            lmb::mma16816(acc[h][v], a0, a1, a2, a3, f[b], f[b + 1]);
+                        }
+                    }
+            }
+            flush();
+        }
+        __syncthreads();
+    }
+    if (!active) return;
+    fold();
+    uint32_t mine = 0;   // lane r: whether output r saw a non-finite operand
+#pragma unroll
+    for (int e = 0; e < kE; ++e) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (bad >> e) & 1u);
+        if ((lane >> 3) == e) mine = (m >> (4 * (lane & 7))) & 15u;
+    }
+    const int64_t r = r0 + lane;
+    if (lane < 16 * kR && r < g.rows) {
+        fx::XFPod p = s_tot[wid][lane];
+        if (g.part) {
+            if (mine) p.flags |= 4;
+            g.part[ch * g.rows + r] = p;
+        } else {
+            gemv_store(g, r, xfp::xf_from_dd(g.alpha.hi, g.alpha.lo), fx::from_pod(p), mine != 0);
+        }
     }
 }
 
-// Trans: block per column j of A (contiguous), threads over rows; every
-// fx::kMaxAdds products a thread's accumulator is folded into an extended float.
-__global__ void __launch_bounds__(256, 3) k_gemv_t_fx(int64_t m, int64_t n, const double2 *__restrict__ A,
-                                                     int64_t lda, const fx::Dig *__restrict__ xo, dd::real alpha,
-                                                     double2 *y, int64_t incy)
+// The chunks' sums of each output, LANES lanes per output in a fixed order,
+// then the update of y.
+template <int LANES>
+__global__ void __launch_bounds__(256) k_gemv_fold(const GemvArgs g, int nchunks)
 {
-    __shared__ fx::XFPod sh[8];
-    const int64_t j = blockIdx.x;
-    const double2 *col = A + j * lda;
-    fx::Acc acc;
-    acc.reset();
-    xfp::XF total;
-    total.zero = true; total.neg = false; total.m = 0; total.e = 0;
+    const xfp::XF xa = xfp::xf_from_dd(g.alpha.hi, g.alpha.lo);
+    const int sub = threadIdx.x % LANES;
+    const int64_t r = (int64_t)blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
+    xfp::XF s;
+    s.zero = true; s.neg = false; s.m = 0; s.e = 0;
     bool bad = false;
-    int cnt = 0;
-    auto fold = [&]() {
-        bad |= acc.bad;
-        total = xfp::xf_add(total, acc.finish());
-        acc.reset();
-        cnt = 0;
-    };
-    // four rows in flight per thread (GEMV N's flag-free groups of four);
-    // carries propagated after each run of 2048 products
-    const int64_t bs = blockDim.x;
-    int64_t i = threadIdx.x;
-    while (i + 3 * bs < m) {
-        const int64_t iend = i + 4 * bs * 512;
-        for (; i + 3 * bs < m && i < iend; i += 4 * bs) {
-            const double2 a0 = __ldcs(col + i), a1 = __ldcs(col + i + bs);
-            const double2 a2 = __ldcs(col + i + 2 * bs), a3 = __ldcs(col + i + 3 * bs);
-            const fx::Dig x0 = xo[i], x1 = xo[i + bs], x2 = xo[i + 2 * bs], x3 = xo[i + 3 * bs];
-            if (fx::decode_is_fast(a0) && fx::decode_is_fast(a1) && fx::decode_is_fast(a2) && fx::decode_is_fast(a3) &&
-                ((x0.flags | x1.flags | x2.flags | x3.flags) & (fx::kZero | fx::kBad)) == 0) {
-                const fx::Op o0 = fx::decode_fast(a0), o1 = fx::decode_fast(a1);
-                const fx::Op o2 = fx::decode_fast(a2), o3 = fx::decode_fast(a3);
-                const int e0 = o0.e + x0.e, e1 = o1.e + x1.e, e2 = o2.e + x2.e, e3 = o3.e + x3.e;
-                acc.admit(max(max(e0, e1), max(e2, e3)));
-                acc.mul_fast(o0, x0, acc.B - e0);
-                acc.mul_fast(o1, x1, acc.B - e1);
-                acc.mul_fast(o2, x2, acc.B - e2);
-                acc.mul_fast(o3, x3, acc.B - e3);
-            } else {
-                acc.add_core(fx::decode(a0), x0);
-                acc.add_core(fx::decode(a1), x1);
-                acc.add_core(fx::decode(a2), x2);
-                acc.add_core(fx::decode(a3), x3);
-            }
+    if (r < g.rows) {
+        for (int c = sub; c < nchunks; c += LANES) {
+            const fx::XFPod p = g.part[(int64_t)c * g.rows + r];
+            bad |= (p.flags & 4) != 0;
+            s = xfp::xf_add(s, fx::from_pod(p));
         }
-        acc.normalize();
-        if ((cnt += 2048) >= fx::kMaxAdds) fold();
     }
-    for (; i < m; i += bs) {
-        acc.add_dig(fx::decode(__ldcs(col + i)), xo[i]);
-        if (++cnt >= fx::kMaxAdds) fold();
+    for (int off = LANES / 2; off > 0; off >>= 1) {
+        s = xfp::xf_add(s, fx::xf_shfl_down(s, off));
+        bad |= __shfl_down_sync(0xffffffffu, bad ? 1 : 0, off) != 0;
     }
-    bad |= acc.bad;
-    total = xfp::xf_add(total, acc.finish());
-    bad = __syncthreads_or(bad ? 1 : 0) != 0;
-    xfp::XF v = fx::xf_warp_sum(total);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = fx::to_pod(v, false);
-    __syncthreads();
-    if (wid == 0) {
-        if (lane < (int)(blockDim.x >> 5)) v = fx::from_pod(sh[lane]);
-        else { v.zero = true; v.neg = false; v.m = 0; v.e = 0; }
-        v = fx::xf_warp_sum(v);
-        if (lane == 0) fx_update_y(y + vidx(j, n, incy), xfp::xf_from_dd(alpha.hi, alpha.lo), v, bad);
-    }
+    if (sub == 0 && r < g.rows) gemv_store(g, r, xa, s, bad);
 }
 
 }  // namespace
@@ -252,56 +457,74 @@ __global__ void __launch_bounds__(256, 3) k_gemv_t_fx(int64_t m, int64_t n, cons
 bool gemv_device(bool trans, int64_t m, int64_t n, dd_host alpha, const void *A, int64_t lda, const void *x,
                  int64_t incx, dd_host beta, int beta_kind, void *y, int64_t incy, const char *routine)
 {
-    int64_t leny = trans ? n : m;
-    int sms = device_sm_count();
-    if (beta_kind != 1) {
-        int64_t blocks = (leny + 255) / 256;
-        if (blocks > sms * 8) blocks = sms * 8;
-        k_scale_vec<<<(unsigned)blocks, 256, 0, stream()>>>(leny, dd::make(beta.hi, beta.lo), beta_kind, (double2 *)y,
-                                                            incy);
-        count_launch();
-    }
-    if (alpha.hi == 0.0 && alpha.lo == 0.0) return true;
-    dd::real al = dd::make(alpha.hi, alpha.lo);
-    const int64_t lenx = trans ? m : n;
-    // x as digit sets (lenx * 32 bytes), then the partial sums
-    const size_t xf_bytes = ((size_t)lenx * sizeof(fx::Dig) + 255) / 256 * 256;
-    if (!trans) {
-        int64_t rowblocks = (m + 255) / 256;
-        int64_t want = 8 * (int64_t)sms;
-        int64_t nchunks = (want + rowblocks - 1) / rowblocks;
-        if (nchunks < (n + fx::kMaxAdds - 1) / fx::kMaxAdds) nchunks = (n + fx::kMaxAdds - 1) / fx::kMaxAdds;
-        if (nchunks > n) nchunks = n;
-        if (nchunks < 1) nchunks = 1;
-        int64_t chunk = (n + nchunks - 1) / nchunks;
-        nchunks = (n + chunk - 1) / chunk;
-        if (nchunks > 65535) {
-            set_error(routine, MWBLAS_ERR_UNSUPPORTED, "n too large for the no-transpose GEMV grid");
-            return false;
+    const int64_t rows = trans ? n : m, len = trans ? m : n;
+    const int sms = device_sm_count();
+    const dd::real be = dd::make(beta.hi, beta.lo);
+    if ((alpha.hi == 0.0 && alpha.lo == 0.0) || len <= 0) {
+        if (beta_kind != 1) {
+            int64_t blocks = (rows + 255) / 256;
+            if (blocks > sms * 8) blocks = sms * 8;
+            k_scale_vec<<<(unsigned)blocks, 256, 0, stream()>>>(rows, be, beta_kind, (double2 *)y, incy);
+            count_launch();
         }
-        char *buf = (char *)dev_alloc(xf_bytes + sizeof(fx::XFPod) * (size_t)(nchunks * m), routine);
-        if (!buf) return false;
-        fx::Dig *xf = (fx::Dig *)buf;
-        fx::XFPod *part = (fx::XFPod *)(buf + xf_bytes);
-        int64_t cb = (n + 255) / 256;
-        if (cb > sms * 8) cb = sms * 8;
-        k_dig_convert<<<(unsigned)cb, 256, 0, stream()>>>(n, (const double2 *)x, incx, xf);
-        dim3 grid((unsigned)rowblocks, (unsigned)nchunks);
-        k_gemv_n_fx<<<grid, 256, 0, stream()>>>(m, n, (const double2 *)A, lda, xf, chunk, part);
-        int64_t fb = (m + 255) / 256;
-        if (fb > sms * 8) fb = sms * 8;
-        k_gemv_n_fx_final<<<(unsigned)fb, 256, 0, stream()>>>(m, (int)nchunks, part, al, (double2 *)y, incy);
-        count_launch(3);
-        dev_free(buf);
-    } else {
-        fx::Dig *xf = (fx::Dig *)dev_alloc(xf_bytes, routine);
-        if (!xf) return false;
-        int64_t cb = (m + 255) / 256;
-        if (cb > sms * 8) cb = sms * 8;
-        k_dig_convert<<<(unsigned)cb, 256, 0, stream()>>>(m, (const double2 *)x, incx, xf);
-        k_gemv_t_fx<<<(unsigned)n, 256, 0, stream()>>>(m, n, (const double2 *)A, lda, xf, al, (double2 *)y, incy);
-        count_launch(2);
-        dev_free(xf);
+        return true;
+    }
+    GemvArgs g;
+    g.A = (const double2 *)A;
+    g.x = (const double2 *)x;
+    g.y = (double2 *)y;
+    g.rows = rows;
+    g.len = len;
+    g.rs = trans ? lda : 1;
+    g.cs = trans ? 1 : lda;
+    g.incx = incx;
+    g.incy = incy;
+    g.alpha = dd::make(alpha.hi, alpha.lo);
+    g.beta = be;
+    g.beta_kind = beta_kind;
+    // 16 kR outputs per warp, up to eight warps per block: fewer where eight
+    // would leave SMs without a block (a small product is bound by the latency
+    // of its windows in turn, about 2 us each), and four where the last block
+    // would hold mostly idle warps (268 outputs in 3 x 128, not 2 x 256:
+    // 268 x 16000 N 107 -> 92 us)
+    const int64_t units = ((rows + 16 * kR - 1) / (16 * kR)) * ((len + 2 * kWin - 1) / (2 * kWin));
+    int nw = rows > 64 * kR ? 8 : (rows > 32 * kR ? 4 : (rows > 16 * kR ? 2 : 1));
+    if (nw == 8 && (rows + 127) / 128 * 128 * 8 <= (rows + 255) / 256 * 256 * 7) nw = 4;
+    while (nw > 1 && units < (int64_t)nw * sms) nw >>= 1;
+    g.rowblocks = (rows + 16 * kR * nw - 1) / (16 * kR * nw);
+    // the reduction in chunks of whole windows, in whole waves of the
+    // resident blocks (two of eight warps per SM, three of fewer), at about
+    // 640 indices (a block's set-up and final sums cost about 60)
+    const int64_t wave = (nw == 8 ? 2ll : 3ll) * sms;
+    int64_t waves = (len * g.rowblocks + 640 * wave - 1) / (640 * wave);
+    int64_t nchunks = waves * wave / g.rowblocks;
+    if (nchunks < 1) nchunks = 1;
+    int64_t chunk = (len + nchunks - 1) / nchunks;
+    chunk = (chunk + kWin - 1) / kWin * kWin;
+    if (chunk > kMaxChunk) chunk = kMaxChunk;
+    nchunks = (len + chunk - 1) / chunk;
+    g.chunk = chunk;
+    if (nchunks * g.rowblocks > INT32_MAX) {
+        set_error(routine, MWBLAS_ERR_UNSUPPORTED, "matrix too large for the GEMV grid");
+        return false;
+    }
+    fx::XFPod *part = nullptr;
+    if (nchunks > 1) {
+        part = (fx::XFPod *)dev_alloc(sizeof(fx::XFPod) * (size_t)(nchunks * rows), routine);
+        if (!part) return false;
+    }
+    g.part = part;
+    const size_t smem = (size_t)kStages * kE * 16 * 32 * nw;
+    cudaFuncSetAttribute(k_gemv_limb, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kE * 16 * 256);
+    k_gemv_limb<<<(unsigned)(nchunks * g.rowblocks), 32 * nw, smem, stream()>>>(g);
+    count_launch();
+    if (part) {
+        // eight lanes per output (27 chunks of 16384 outputs: 15 us, a warp each 31),
+        // a warp for many chunks (a few outputs, a long reduction)
+        if (nchunks <= 64) k_gemv_fold<8><<<(unsigned)((rows + 31) / 32), 256, 0, stream()>>>(g, (int)nchunks);
+        else k_gemv_fold<32><<<(unsigned)((rows + 7) / 8), 256, 0, stream()>>>(g, (int)nchunks);
+        count_launch();
+        dev_free(part);
     }
     return true;
 }
