@@ -16,6 +16,7 @@
 #include "dd.cuh"
 #include "fixacc.cuh"
 #include "l1.h"
+#include "limbmma.cuh"
 #include "runtime.h"
 
 namespace mw {
@@ -426,9 +427,9 @@ __global__ void k_iamax_final(int nparts, const AmaxKey *part, int64_t *out)
 
 // ---- DOT ---------------------------------------------------------------------
 // mdot.cpp:48-87 accumulates TwoProduct + Bailey three-limb sums on the FP64
-// pipe. Here the products are accumulated exactly (to 2^-126 of each product)
-// in per-thread integer fixed point (fixacc.cuh), the thread sums are added
-// as 128-bit extended floats in a fixed order (warp, block, then the grid's
+// pipe. Here the products are accumulated exactly (to 2^-116 of the largest
+// product of a warp) as limb products on the tensor cores, the warps' sums are
+// added as 128-bit extended floats in a fixed order (block, then the grid's
 // block partials), and the result is rounded once to double-double. The
 // result is deterministic for a given n and device and at least as accurate
 // as the reference's.
@@ -456,47 +457,205 @@ __device__ bool block_any(bool b)
     return __syncthreads_or(b ? 1 : 0) != 0;
 }
 
-__global__ void __launch_bounds__(kThreads, 4) k_mdot_partial(int64_t n, const double2 *__restrict__ x, int64_t incx,
+// The tensor-core form (limbmma.cuh): of a warp's 32 pairs (x_i, y_i), x_i is
+// aligned by the product's exponent to the warp's block, both are written as
+// 16 bytes to warp-private shared memory, and one ldmatrix of 16-bit units per
+// operand transposes them: lane (g, t) gets limbs 2g and 2g + 1 of elements
+// 2t, 2t + 1 of each eight, which two masks turn into fp16 subnormal pairs.
+// D[q][r] += sum_i X_iq Y_ir is then a 16 x 16 outer-product sum over K = 32 in
+// four MMAs (rows and columns in the order even limbs, odd limbs), all limb
+// products kept, and the dot product is sum D[q][r] 2^(8(q+r)).
+// Where the product is negative, X's limbs 0..14 are complemented, which
+// stands for 2^120 - 1 - X, and limb 15 is 1: D[15][r] sums the Y that
+// 2^120 - 1 has to be taken off for.
+// Two groups of 32 pairs per turn hide each other's latency; four turns of
+// pairs are in flight per lane (cp.async).
+//
+// Exactness: D grows by at most 255 * 255 per pair and stays below 2^24 units
+// for 4 turns of 64; then it moves to int32 sums, and after 64 of those (or
+// when a product above the block moves it up) to the warp's extended float.
+//
+// Bound: HBM (32 B per pair). Measured at n = 10^8: 867 -> 598 us (3.69 -> 5.35 TB/s); about 100
+// instructions per pair, where 19 IMAD.WIDE digit products and their digit
+// splits took 223.
+constexpr int kDotFlush = 4;            // turns of 64 pairs per move to the int32 sums
+constexpr int kDotFold = 64;            // moves per fold into the extended float
+constexpr int kDotStages = 4;           // turns in flight
+constexpr int kNoBlock = -(1 << 22);    // no nonzero product yet
+constexpr int kDotSmem = kDotStages * 4 * 16 * kThreads + 2 * 1024 * (kThreads / 32);
+
+__global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const double2 *__restrict__ x, int64_t incx,
                                                           const double2 *__restrict__ y, int64_t incy,
                                                           fx::XFPod *part)
 {
-    fx::Acc acc;
-    acc.reset();
-    fx::XF total;   // accumulators are folded in here every kMaxAdds products
-    total.zero = true; total.neg = false; total.m = 0; total.e = 0;
-    bool bad = false;
-    int cnt = 0;
-    auto fold = [&]() {
-        bad |= acc.bad;
-        total = xfp::xf_add(total, acc.finish());
-        acc.reset();
-        cnt = 0;
-    };
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (incx == 1 && incy == 1) {
-        // two elements in flight per thread; the column carries are
-        // propagated after each run of 2048 products, outside the inner loop
-        while (i + stride < n) {
-            const int64_t iend = i + 2 * stride * 1024;
-            for (; i + stride < n && i < iend; i += 2 * stride) {
-                const double2 x0 = __ldcs(x + i), y0 = __ldcs(y + i);
-                const double2 x1 = __ldcs(x + i + stride), y1 = __ldcs(y + i + stride);
-                acc.add_core(fx::decode(x0), fx::to_dig(fx::decode(y0)));
-                acc.add_core(fx::decode(x1), fx::to_dig(fx::decode(y1)));
-            }
-            acc.normalize();
-            if ((cnt += 2048) >= fx::kMaxAdds) fold();
+    // [stage][pair 0 x, y, pair 1 x, y][thread] 16 bytes, then per warp [pair][operand][element] 16 bytes
+    extern __shared__ __align__(16) unsigned char s_dot[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t nwarps = (int64_t)gridDim.x * (kThreads / 32), warp = (int64_t)blockIdx.x * (kThreads / 32) + wid;
+    const int64_t total = (n + 63) / 64;
+    const int64_t turns = warp < total ? (total - warp + nwarps - 1) / nwarps : 0;
+    // the lane's next pair (and the one 32 further), as addresses: either order
+    // of a BLAS increment is a start and a step
+    const int64_t i00 = warp * 64 + lane, sx = nwarps * 64 * incx, sy = nwarps * 64 * incy;
+    const double2 *px = x + vidx(i00, n, incx), *py = y + vidx(i00, n, incy);
+    int64_t room = n - i00;   // > 0: px, py are pairs of the vectors
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_dot) + threadIdx.x * 16u;
+    constexpr uint32_t kPlane = 16u * kThreads;
+    auto load = [&](int64_t turn) {   // turns in order; past the end nothing is read
+        const uint32_t d = ring + ((uint32_t)turn & (kDotStages - 1)) * (4 * kPlane);
+        if (room > 0) {
+            lmb::cp_async16(d, px);
+            lmb::cp_async16(d + kPlane, py);
         }
-    }
-    for (; i < n; i += stride) {
-        acc.add_prod(fx::decode(x[vidx(i, n, incx)]), fx::decode(y[vidx(i, n, incy)]));
-        if (++cnt >= fx::kMaxAdds) fold();
+        if (room > 32) {
+            lmb::cp_async16(d + 2 * kPlane, px + 32 * incx);
+            lmb::cp_async16(d + 3 * kPlane, py + 32 * incy);
+        }
+        px += sx;
+        py += sy;
+        room -= nwarps * 64;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int blk = kNoBlock;
+    bool bad = false;
+    float acc[2][4];
+    int sum[2][4];
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            acc[b][i] = 0.0f;
+            sum[b][i] = 0;
+        }
+    fx::XF tot;
+    tot.zero = true; tot.neg = false; tot.m = 0; tot.e = 0;
+    auto flush = [&]() {
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                sum[b][i] += __float2int_rn(acc[b][i] * 0x1p48f);
+                acc[b][i] = 0.0f;
+            }
+    };
+    // the warp's sums into its extended float (the same in every lane)
+    auto fold = [&]() {
+        flush();
+        // the lane's entries: limb 2g + a of x, 2(2t + c) + b of y
+        const int g = lane >> 2, t = lane & 3;
+        uint64_t W[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            int64_t p = 0;   // over the lane's limbs 4t .. 4t + 3 of y
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) p += (int64_t)sum[b][2 * a + c] << (8 * (2 * c + b));
+            const bool last = a == 1 && g == 7;   // limb 15: - (2^120 - 1)
+            lmb::add_at(W, last ? -p : p, 8 * (last ? 15 : 2 * g + a) + 32 * t);
+            lmb::add_at(W, last ? p : 0, 32 * t);
+        }
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sum[b][i] = 0;
+        lmb::lane_sum256(W, 32);
+        if (blk != kNoBlock) tot = xfp::xf_add(tot, fx::w256_to_xf(W, blk - 2 * lmb::kExpBias));
+    };
+
+    for (int u = 0; u < kDotStages - 1; ++u) load(u);
+    unsigned char *limbs = s_dot + kDotStages * 4 * kPlane + wid * 2048;
+    const uint32_t lrow = (uint32_t)__cvta_generic_to_shared(limbs) + lane * 16u;
+#pragma unroll 1
+    for (int64_t turn = 0; turn < turns; ++turn) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDotStages - 2) : "memory");
+        const unsigned char *cur = s_dot + ((uint32_t)turn & (kDotStages - 1)) * (4 * kPlane) + threadIdx.x * 16u;
+        uint32_t wx[2][4], wy[2][4], neg[2];
+        int sh[2];
+        bool fast = (warp + turn * nwarps) * 64 + 64 <= n;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const double2 vx = *reinterpret_cast<const double2 *>(cur + 2 * p * kPlane);
+            const double2 vy = *reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane);
+            int ehx, ehy;
+            const bool okx = lmb::split_fast(vx, wx[p], ehx), oky = lmb::split_fast(vy, wy[p], ehy);
+            sh[p] = blk - ehx - ehy;
+            fast = fast && okx && oky && (uint32_t)(sh[p] - 2) < 30u;
+            neg[p] = (uint32_t)((__double2hiint(vx.x) ^ __double2hiint(vy.x)) >> 31);
+        }
+        if (__all_sync(0xffffffffu, fast)) {
+#pragma unroll
+            for (int p = 0; p < 2; ++p) lmb::shr_short(wx[p], sh[p]);
+        } else {
+            // the end, zeros, operands off the straight-line path, long alignments, a larger block
+            const int64_t i0 = (warp + turn * nwarps) * 64 + lane;
+            int ep[2];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const fx::Op ox = fx::decode(*reinterpret_cast<const double2 *>(cur + 2 * p * kPlane));
+                const fx::Op oy = fx::decode(*reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane));
+                const bool no = ((ox.flags | oy.flags) & fx::kBad) != 0;
+                const bool in = i0 + 32 * p < n;   // else the stage holds an older pair or nothing
+                bad = bad || (no && in);
+                ep[p] = (no || !in || ((ox.flags | oy.flags) & fx::kZero))
+                            ? kNoBlock
+                            : ox.e + oy.e + 2 * lmb::kExpBias;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    wx[p][i] = ox.w[i];
+                    wy[p][i] = oy.w[i];
+                }
+            }
+            const int top = __reduce_max_sync(0xffffffffu, max(ep[0], ep[1]));
+            if (top != kNoBlock && top > blk - 2) {
+                if (blk != kNoBlock) fold();
+                blk = top + 4;
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                uint32_t sv[4];
+                fx::shr128(wx[p], ep[p] == kNoBlock ? 127 : min(blk - ep[p], 127), sv);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) wx[p][i] = ep[p] == kNoBlock ? 0u : sv[i];
+            }
+        }
+        load(turn + kDotStages - 1);   // into the stage read in the previous turn
+        __syncwarp();                  // the previous turn's limbs have been read
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            uint4 *st = reinterpret_cast<uint4 *>(limbs + 1024 * p) + lane;
+            st[0] = make_uint4(wx[p][0] ^ neg[p], wx[p][1] ^ neg[p], wx[p][2] ^ neg[p],
+                               (wx[p][3] ^ (neg[p] & 0xFFFFFFu)) | (neg[p] & 0x1000000u));
+            st[32] = make_uint4(wy[p][0], wy[p][1], wy[p][2], wy[p][3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            uint32_t a[4], b[4];   // elements 8j .. 8j + 7 in [j]
+            lmb::ldmatrix_x4_trans(a, lrow + 1024u * p);
+            lmb::ldmatrix_x4_trans(b, lrow + 1024u * p + 512u);
+#pragma unroll
+            for (int h = 0; h < 4; h += 2) {
+                const uint32_t a0 = a[h] & 0xFF00FFu, a1 = __byte_perm(a[h], 0u, 0x4341);
+                const uint32_t a2 = a[h + 1] & 0xFF00FFu, a3 = __byte_perm(a[h + 1], 0u, 0x4341);
+                lmb::mma16816(acc[0], a0, a1, a2, a3, b[h] & 0xFF00FFu, b[h + 1] & 0xFF00FFu);
+                lmb::mma16816(acc[1], a0, a1, a2, a3, __byte_perm(b[h], 0u, 0x4341), __byte_perm(b[h + 1], 0u, 0x4341));
+            }
+        }
+        if ((turn & (kDotFlush - 1)) == kDotFlush - 1) {
+            flush();
+            if ((turn & (kDotFlush * kDotFold - 1)) == kDotFlush * kDotFold - 1) fold();
+        }
     }
     fold();
     bad = block_any(bad);
-    fx::XF v = xf_block_sum(total);
-    if (threadIdx.x == 0) part[blockIdx.x] = fx::to_pod(v, bad);
+    __shared__ fx::XFPod sh_tot[kThreads / 32];
+    if (lane == 0) sh_tot[wid] = fx::to_pod(tot, false);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kThreads / 32; ++w) tot = xfp::xf_add(tot, fx::from_pod(sh_tot[w]));
+        part[blockIdx.x] = fx::to_pod(tot, bad);
+    }
 }
 
 __global__ void __launch_bounds__(kThreads) k_mdot_final(int nparts, const fx::XFPod *part, double2 *out)
@@ -605,13 +764,16 @@ bool launch_iamax(int64_t n, const void *x, int64_t inc, bool cplx, int64_t *res
 bool launch_mdot(int64_t n, const void *x, int64_t incx, const void *y, int64_t incy, dd_host *result_host,
                  const char *routine)
 {
-    int g = grid_for(n);
+    // one wave of resident blocks (two per SM), a turn of 64 pairs per warp at least
+    const int64_t wave = 2ll * device_sm_count(), need = (n + 2 * kThreads - 1) / (2 * kThreads);
+    const int g = (int)(need < wave ? need : wave);
     size_t bytes = (size_t)g * sizeof(fx::XFPod) + 256;
     char *buf = (char *)dev_alloc(bytes, routine);
     if (!buf) return false;
     fx::XFPod *part = (fx::XFPod *)buf;
     double2 *res = (double2 *)(buf + ((size_t)g * sizeof(fx::XFPod) + 15) / 16 * 16);
-    k_mdot_partial<<<g, kThreads, 0, stream()>>>(n, (const double2 *)x, incx, (const double2 *)y, incy, part);
+    cudaFuncSetAttribute(k_mdot_limb, cudaFuncAttributeMaxDynamicSharedMemorySize, kDotSmem);
+    k_mdot_limb<<<g, kThreads, kDotSmem, stream()>>>(n, (const double2 *)x, incx, (const double2 *)y, incy, part);
     k_mdot_final<<<1, kThreads, 0, stream()>>>(g, part, res);
     count_launch(2);
     double2 r;
