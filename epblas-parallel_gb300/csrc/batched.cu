@@ -45,7 +45,9 @@ namespace mw {
 
 namespace {
 
-constexpr int kNoExp = -30000;
+using fxg::exp_bound;
+using fxg::kNoExp;
+
 constexpr int GTHREADS = 256;  // 16 x 16 threads
 constexpr int GBK = 8;         // k-slab
 
@@ -63,13 +65,6 @@ struct GemmDesc {
     int64_t part_begin;   // first partial-tile slot: earlier split instances
                           // hold tiles * splitk slots each
 };
-
-__device__ __forceinline__ int exp_bound(double x)
-{
-    uint64_t b = (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull;
-    if (b == 0) return kNoExp;
-    return (int)(b >> 52) - 1023;
-}
 
 __device__ __forceinline__ double2 opA_at(const GemmDesc &d, int64_t i, int64_t p)
 {

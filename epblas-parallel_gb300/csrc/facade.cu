@@ -10,6 +10,7 @@
 // pointers) record an error and leave the outputs untouched.
 #include <atomic>
 #include <cctype>
+#include <cmath>
 #include <cstring>
 
 #include "gemm.h"
@@ -93,6 +94,17 @@ int pick_engine(const GemmArgs &g, bool cplx, int force_engine)
         // on the integer pipes and complex ones on the FP64 pipe.
         double work = (double)g.m * (double)g.n * (double)g.k;
         eng = (work >= 64.0 * 64.0 * 64.0 * 8.0 && g.k >= 32) ? MWBLAS_GEMM_OZAKI : MWBLAS_GEMM_FIXED;
+        if (eng == MWBLAS_GEMM_OZAKI && !cplx) {
+            // The real crossover: the scheme's six launches take about 58 us on
+            // the device however small the product is, and 40 more per 10^6
+            // outputs padded to its 256 x 256 tiles; the integer pipes' small
+            // tiles beat that up to about 200^3 (whole calls: 128^3 47 against
+            // 82 us, 200^3 75 against 85, 256^3 101 against 86; 16 x 8000 x 100
+            // 107 against 217).
+            const double fixed_us = gemm_fixed_small_us(g.m, g.n, g.k);
+            const double padded = std::ceil(g.m / 256.0) * std::ceil(g.n / 256.0) * 65536.0;
+            if (fixed_us >= 0.0 && fixed_us < 58.0 + 40e-6 * padded) eng = MWBLAS_GEMM_FIXED;
+        }
         if (eng == MWBLAS_GEMM_OZAKI && !ozaki_available()) eng = MWBLAS_GEMM_FIXED;
         if (eng == MWBLAS_GEMM_FIXED && cplx) eng = MWBLAS_GEMM_PLAIN;
     }

@@ -17,6 +17,16 @@ using fx::w256_to_xf;
 // Scaled operands are integers below 2^(FX_S + 1).
 constexpr int FX_S = 115;
 
+constexpr int kNoExp = -30000;   // row or column with no nonzero entry
+
+// |x| < 2^(e+1) with e = biased exponent - 1023 (1024: not finite)
+__device__ __forceinline__ int exp_bound(double x)
+{
+    const uint64_t b = (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull;
+    if (b == 0) return kNoExp;
+    return (int)(b >> 52) - 1023;
+}
+
 // v * 2^sh rounded to an integer (|v * 2^sh| < 2^116), as five balanced
 // 24-bit digits; bit operations only (fixacc.cuh's decode).
 __device__ __forceinline__ void dd_digits(double2 v, int sh, int d[5])

@@ -39,6 +39,8 @@ bool gemm_plain_cplx(const GemmArgs &g, const char *routine);
 
 // Fixed-point engine on the integer pipes (real only).
 bool gemm_fixed_real(const GemmArgs &g, const char *routine);
+// Estimated device time (us) of its small-tile path; < 0 where that does not apply.
+double gemm_fixed_small_us(int64_t m, int64_t n, int64_t k);
 
 // Integer-exact tensor-core engine (Ozaki scheme II). Returns false with an
 // error recorded on failure.

@@ -44,7 +44,6 @@ using namespace fxg;
 constexpr int FX_BM = 64, FX_BN = 64, FX_BK = 8;
 constexpr int FX_THREADS = 256;      // 16 x 16 threads, 4 x 4 outputs each
 constexpr int64_t FX_MAX_K = 16384;  // per launch (column-sum headroom)
-constexpr int kNoExpFx = -30000;
 
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(FX_THREADS, 1)
@@ -63,12 +62,12 @@ __global__ void __launch_bounds__(FX_THREADS, 1)
 
     if (tid < FX_BM) {
         const int64_t i = i0 + tid;
-        const int e = (i < m) ? ea[i] : kNoExpFx;
-        s_sa[tid] = (e <= kNoExpFx / 2) ? -100000 : FX_S - e;
+        const int e = (i < m) ? ea[i] : kNoExp;
+        s_sa[tid] = (e <= kNoExp / 2) ? -100000 : FX_S - e;
     } else if (tid < FX_BM + FX_BN) {
         const int64_t j = j0 + (tid - FX_BM);
-        const int e = (j < n) ? eb[j] : kNoExpFx;
-        s_sb[tid - FX_BM] = (e <= kNoExpFx / 2) ? -100000 : FX_S - e;
+        const int e = (j < n) ? eb[j] : kNoExp;
+        s_sb[tid - FX_BM] = (e <= kNoExp / 2) ? -100000 : FX_S - e;
     }
     __syncthreads();
 
@@ -169,7 +168,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1)
                 continue;
             }
             XF v;
-            if (ei <= kNoExpFx / 2 || ej <= kNoExpFx / 2) {
+            if (ei <= kNoExp / 2 || ej <= kNoExp / 2) {
                 v.zero = true; v.neg = false; v.m = 0; v.e = 0;
             } else {
                 v = sums_to_xf(acc[a][b], ei, ej);
@@ -179,7 +178,215 @@ __global__ void __launch_bounds__(FX_THREADS, 1)
     }
 }
 
+// Small products: tiles of T x T outputs (16 or 8), one output per thread
+// (T = 8: four threads, every fourth k each), and K in chunks of 64 over
+// grid.z, so that a product of a few thousand outputs spreads over the SMs.
+// A block holds its whole chunk, so it finds the row and column exponent bounds
+// itself: the elements are loaded once into registers, the bounds reduced in
+// shared memory, then the digits staged there. One chunk: C is updated here
+// (one launch, no scratch). Several: the chunks' sums go out as extended floats
+// and k_fixed_small_fold adds them in order; each chunk has its own bounds,
+// never above those of the whole rows, so nothing is lost against one scan.
+//
+// Bound: latency. 48 x 33 x 40 took 174 us as one 64 x 64 block behind two
+// exponent scans, now 8;
+// whole calls: 16^3 118 -> 27 us, 48 x 33 x 40 148 -> 27, 100^3 226 -> 46,
+// 16 x 16 x 8000 10.0 ms -> 55 us, 256^3 422 -> 100 us.
+constexpr int SM_KC = 64;
+
+template <int T, bool TA, bool TB>
+__global__ void __launch_bounds__(FX_THREADS)
+    k_gemm_fixed_small(int64_t m, int64_t n, int64_t k, const double2 *__restrict__ A, int64_t lda,
+                       const double2 *__restrict__ B, int64_t ldb, dd::real alpha, int alpha_one, dd::real beta,
+                       int beta_kind, double2 *C, int64_t ldc, int uplo, fx::XFPod *part)
+{
+    constexpr int G = FX_THREADS / (T * T);          // threads per output
+    constexpr int NU = T * SM_KC / FX_THREADS;       // elements per thread and operand
+    constexpr int S = 5 * T + 1;                     // digits of one k: odd stride for transposed staging
+    __shared__ __align__(8) int sA[SM_KC * S], sB[SM_KC * S];
+    __shared__ int s_ea[T], s_eb[T];
+    const int tid = threadIdx.x;
+    const int64_t i0 = (int64_t)blockIdx.x * T, j0 = (int64_t)blockIdx.y * T, k0 = (int64_t)blockIdx.z * SM_KC;
+    if ((uplo == 1 && i0 > j0 + T - 1) || (uplo == 2 && i0 + T - 1 < j0)) return;
+    const int kc = (int)min((int64_t)SM_KC, k - k0);
+    if (tid < T) s_ea[tid] = kNoExp;
+    else if (tid < 2 * T) s_eb[tid - T] = kNoExp;
+
+    double2 ra[NU], rb[NU];
+    int ia[NU], ib[NU];   // row (column) of the tile and k of each element
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+        const int idx = tid + u * FX_THREADS;
+        const int r = TA ? idx / SM_KC : idx % T, pa = TA ? idx % SM_KC : idx / T;
+        const int c = TB ? idx % T : idx / SM_KC, pb = TB ? idx / T : idx % SM_KC;
+        ia[u] = r | pa << 8;
+        ib[u] = c | pb << 8;
+        ra[u] = (i0 + r < m && pa < kc) ? (TA ? A[k0 + pa + (i0 + r) * lda] : A[i0 + r + (k0 + pa) * lda])
+                                        : make_double2(0.0, 0.0);
+        rb[u] = (j0 + c < n && pb < kc) ? (TB ? B[j0 + c + (k0 + pb) * ldb] : B[k0 + pb + (j0 + c) * ldb])
+                                        : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+        atomicMax(&s_ea[ia[u] & 255], exp_bound(ra[u].x));
+        atomicMax(&s_eb[ib[u] & 255], exp_bound(rb[u].x));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+        int d[5];
+        const int ea = s_ea[ia[u] & 255], eb = s_eb[ib[u] & 255];
+        dd_digits(ra[u], ea <= kNoExp / 2 ? -100000 : FX_S - ea, d);
+#pragma unroll
+        for (int t = 0; t < 5; ++t) sA[(ia[u] >> 8) * S + t * T + (ia[u] & 255)] = d[t];
+        dd_digits(rb[u], eb <= kNoExp / 2 ? -100000 : FX_S - eb, d);
+#pragma unroll
+        for (int t = 0; t < 5; ++t) sB[(ib[u] >> 8) * S + t * T + (ib[u] & 255)] = d[t];
+    }
+    __syncthreads();
+
+    const int r = tid % T, c = (tid / T) % T, kg = tid / (T * T);
+    long long acc[5] = {0, 0, 0, 0, 0};
+#pragma unroll 4
+    for (int p = kg; p < kc; p += G) {
+        int da[5], db[5];
+#pragma unroll
+        for (int t = 0; t < 5; ++t) {
+            da[t] = sA[p * S + t * T + r];
+            db[t] = sB[p * S + t * T + c];
+        }
+        mac_digits(acc, da, db);
+    }
+    if (G > 1) {   // the output's shares, exact integers, into its first thread
+        __syncthreads();
+        long long *red = reinterpret_cast<long long *>(sA);
+        if (kg > 0)
+#pragma unroll
+            for (int w = 0; w < 5; ++w) red[((kg - 1) * 5 + w) * (T * T) + tid % (T * T)] = acc[w];
+        __syncthreads();
+        if (kg > 0) return;
+#pragma unroll
+        for (int q = 0; q < G - 1; ++q)
+#pragma unroll
+            for (int w = 0; w < 5; ++w) acc[w] += red[(q * 5 + w) * (T * T) + tid];
+    }
+    const int64_t i = i0 + r, j = j0 + c;
+    if (i >= m || j >= n || (uplo == 1 && i > j) || (uplo == 2 && i < j)) return;
+    const int ei = s_ea[r], ej = s_eb[c];
+    const bool bad = ei >= 1024 || ej >= 1024;   // a non-finite entry in row i of op(A) or column j of op(B)
+    XF v;
+    if (bad || ei <= kNoExp / 2 || ej <= kNoExp / 2) {
+        v.zero = true; v.neg = false; v.m = 0; v.e = 0;
+    } else {
+        v = sums_to_xf(acc, ei, ej);
+    }
+    if (part) {
+        part[blockIdx.z * (m * n) + i + j * m] = fx::to_pod(v, bad);
+        return;
+    }
+    double2 *pc = C + i + j * ldc;
+    if (bad) {
+        const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+        *pc = make_double2(qnan, qnan);
+        return;
+    }
+    store_axpby(pc, v, xfp::xf_from_dd(alpha.hi, alpha.lo), alpha_one != 0, xfp::xf_from_dd(beta.hi, beta.lo), beta,
+                beta_kind);
+}
+
+// The chunks' sums of each output, eight lanes per output in a fixed order,
+// then C := alpha * sum + beta * C.
+__global__ void __launch_bounds__(256)
+    k_fixed_small_fold(int64_t m, int64_t n, int chunks, const fx::XFPod *__restrict__ part, dd::real alpha,
+                       int alpha_one, dd::real beta, int beta_kind, double2 *C, int64_t ldc, int uplo)
+{
+    const int sub = threadIdx.x & 7;
+    const int64_t o = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3), i = o % m, j = o / m;
+    const bool in = o < m * n && !(uplo == 1 && i > j) && !(uplo == 2 && i < j);
+    XF s;
+    s.zero = true; s.neg = false; s.m = 0; s.e = 0;
+    int bad = 0;
+    if (in) {
+        for (int c = sub; c < chunks; c += 8) {
+            const fx::XFPod p = part[(int64_t)c * (m * n) + o];
+            bad |= p.flags & 4;
+            s = xfp::xf_add(s, fx::from_pod(p));
+        }
+    }
+    for (int off = 4; off > 0; off >>= 1) {
+        s = xfp::xf_add(s, fx::xf_shfl_down(s, off));
+        bad |= __shfl_down_sync(0xffffffffu, bad, off);
+    }
+    if (sub != 0 || !in) return;
+    double2 *pc = C + i + j * ldc;
+    if (bad) {
+        const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+        *pc = make_double2(qnan, qnan);
+        return;
+    }
+    store_axpby(pc, s, xfp::xf_from_dd(alpha.hi, alpha.lo), alpha_one != 0, xfp::xf_from_dd(beta.hi, beta.lo), beta,
+                beta_kind);
+}
+
+// Device time of the small-tile path in us (fitted, +-20 %: 256^3 75, 500 x 500
+// x 8 20): blocks of 16 x 16 outputs x 64 k over the SMs, 6000 clocks each for
+// staging and epilogue and 236 per k for the products; < 0 where it does not
+// apply (grid and scratch limits).
+double small_us(int64_t m, int64_t n, int64_t k)
+{
+    const double chunks = std::ceil(k / (double)SM_KC);
+    if (n > 8 * 65535 || chunks > 65535.0 || chunks * (double)m * (double)n * sizeof(fx::XFPod) > 64.0 * 1048576.0)
+        return -1.0;
+    const double blocks = std::ceil(m / 16.0) * std::ceil(n / 16.0) * chunks;
+    return std::ceil(blocks / device_sm_count()) * (6000.0 + 236.0 * (k < SM_KC ? k : SM_KC)) / 1900.0;
+}
+
+// Whether the product goes to the small tiles: the 64 x 64 ones cost a wave of
+// 100,000 clocks (scans, the serial epilogue of 16 outputs per thread) and
+// 2363 per k, whether or not it fills the SMs.
+bool small_tiles(const GemmArgs &g)
+{
+    const double us = small_us(g.m, g.n, g.k);
+    const double waves = std::ceil(std::ceil(g.m / 64.0) * std::ceil(g.n / 64.0) / device_sm_count());
+    return us >= 0.0 && us < waves * (100000.0 + 2363.0 * g.k) / 1900.0;
+}
+
+template <int T>
+bool launch_small(const GemmArgs &g, const char *routine)
+{
+    const int64_t chunks = (g.k + SM_KC - 1) / SM_KC;
+    fx::XFPod *part = nullptr;
+    if (chunks > 1) {
+        part = (fx::XFPod *)dev_alloc(sizeof(fx::XFPod) * (size_t)(chunks * g.m * g.n), routine);
+        if (!part) return false;
+    }
+    const dim3 grid((unsigned)((g.m + T - 1) / T), (unsigned)((g.n + T - 1) / T), (unsigned)chunks);
+    const dd::real al = dd::make(g.alpha.hi, g.alpha.lo), be = dd::make(g.beta.hi, g.beta.lo);
+    const int alpha_one = (g.alpha.hi == 1.0 && g.alpha.lo == 0.0);
+#define MW_FXS(TA, TB)                                                                                             \
+    k_gemm_fixed_small<T, TA, TB><<<grid, FX_THREADS, 0, stream()>>>(g.m, g.n, g.k, (const double2 *)g.A, g.lda,   \
+                                                                     (const double2 *)g.B, g.ldb, al, alpha_one,  \
+                                                                     be, g.beta_kind, (double2 *)g.C, g.ldc,      \
+                                                                     g.uplo, part)
+    if (!g.ta && !g.tb) MW_FXS(false, false);
+    else if (!g.ta && g.tb) MW_FXS(false, true);
+    else if (g.ta && !g.tb) MW_FXS(true, false);
+    else MW_FXS(true, true);
+#undef MW_FXS
+    count_launch();
+    if (part) {
+        k_fixed_small_fold<<<(unsigned)((g.m * g.n + 31) / 32), 256, 0, stream()>>>(
+            g.m, g.n, (int)chunks, part, al, alpha_one, be, g.beta_kind, (double2 *)g.C, g.ldc, g.uplo);
+        count_launch();
+        dev_free(part);
+    }
+    return true;
+}
+
 }  // namespace
+
+double gemm_fixed_small_us(int64_t m, int64_t n, int64_t k) { return small_us(m, n, k); }
 
 bool gemm_fixed_real(const GemmArgs &g0, const char *routine)
 {
@@ -188,6 +395,11 @@ bool gemm_fixed_real(const GemmArgs &g0, const char *routine)
     if (g.k == 0) {
         launch_scale_matrix(g.m, g.n, g.beta, g.beta_kind, g.C, g.ldc, g.uplo);
         return true;
+    }
+    if (small_tiles(g)) {
+        // 8 x 8 tiles where 16 x 16 ones would still leave half of the SMs idle
+        const int64_t t16 = ((g.m + 15) / 16) * ((g.n + 15) / 16) * ((g.k + SM_KC - 1) / SM_KC);
+        return 2 * t16 <= device_sm_count() ? launch_small<8>(g, routine) : launch_small<16>(g, routine);
     }
     int *ex = (int *)dev_alloc(sizeof(int) * (size_t)(g.m + g.n), routine);
     if (!ex) return false;
