@@ -47,6 +47,44 @@ CRT_HD xw::XW to_xw(const xfp::XF &x)
 constexpr int kFL = 5;       // 32-bit limbs of the 160-bit fractions
 constexpr int kFLPad = 8;    // row stride (two 16-byte vectors)
 
+// T * M * 2^-S2 with T the signed 160-bit fraction of words x (changed), in
+// 32-bit words; Mx = M (times any folded scale factor).
+CRT_HD xw::XW fraction_xw(uint32_t x[kFL], const xw::XW &Mx, int S2)
+{
+    const uint32_t neg = x[kFL - 1] >> 31;
+    if (neg) {
+        uint32_t c = 1;
+        for (int t = 0; t < kFL; ++t) {
+            const uint32_t v = ~x[t] + c;
+            c = c & (x[t] == 0u);
+            x[t] = v;
+        }
+    }
+    // normalise |T| (bit 159 set), keep the top 128 bits
+    int sh = 0;
+    for (int k = 0; k < kFL - 1 && x[kFL - 1] == 0u; ++k) {
+        for (int t = kFL - 1; t > 0; --t) x[t] = x[t - 1];
+        x[0] = 0u;
+        sh += 32;
+    }
+    if (x[kFL - 1] == 0u) return xw::zero();
+    const int z = xw::clz32(x[kFL - 1]);
+    xw::XW r;
+    if (z) {
+        for (int t = kFL - 1; t > 0; --t) x[t] = xw::fshl(x[t - 1], x[t], z);
+        sh += z;
+    }
+    r.w[3] = x[4];
+    r.w[2] = x[3];
+    r.w[1] = x[2];
+    r.w[0] = x[1];
+    r.e = -128 - sh;
+    r.neg = neg;
+    r = xw::mul(r, Mx);
+    r.e -= S2;
+    return r;
+}
+
 struct Frac {
     uint64_t S[kFL];
 
@@ -115,38 +153,7 @@ struct Frac {
             x[t] = (uint32_t)v;
             carry = (uint32_t)(v >> 32);
         }
-        const uint32_t neg = x[kFL - 1] >> 31;
-        if (neg) {
-            uint32_t c = 1;
-            for (int t = 0; t < kFL; ++t) {
-                const uint32_t v = ~x[t] + c;
-                c = c & (x[t] == 0u);
-                x[t] = v;
-            }
-        }
-        // normalise |T| (bit 159 set), keep the top 128 bits
-        int sh = 0;
-        for (int k = 0; k < kFL - 1 && x[kFL - 1] == 0u; ++k) {
-            for (int t = kFL - 1; t > 0; --t) x[t] = x[t - 1];
-            x[0] = 0u;
-            sh += 32;
-        }
-        if (x[kFL - 1] == 0u) return xw::zero();
-        const int z = xw::clz32(x[kFL - 1]);
-        xw::XW r;
-        if (z) {
-            for (int t = kFL - 1; t > 0; --t) x[t] = xw::fshl(x[t - 1], x[t], z);
-            sh += z;
-        }
-        r.w[3] = x[4];
-        r.w[2] = x[3];
-        r.w[1] = x[2];
-        r.w[0] = x[1];
-        r.e = -128 - sh;
-        r.neg = neg;
-        r = xw::mul(r, Mx);
-        r.e -= S2;
-        return r;
+        return fraction_xw(x, Mx, S2);
     }
 };
 

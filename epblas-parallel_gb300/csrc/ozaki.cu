@@ -52,6 +52,8 @@
 #include "sm100.cuh"
 #include "crt.cuh"
 #include "fixacc.cuh"
+#include "fixround.cuh"
+#include "limbmma.cuh"
 #include "xfloat.cuh"
 
 namespace mw {
@@ -1524,18 +1526,147 @@ using xfp::xf_add;
 using xfp::xf_from_dd;
 using xfp::xf_mul;
 
-// Shared-memory copy of the CRT constants (broadcast reads; each row of F is
-// 32 bytes so a modulus' constants are two 16-byte loads).
-struct CrtSmem {
-    alignas(16) uint32_t F[kMaxMod][crt::kFLPad];
-    float pm[kMaxMod];
+// CRT sums on the tensor cores. The fraction sum_l c_l F_l mod 2^160 of an
+// element is a small matrix product, residues (K = moduli) times the 20 bytes
+// of every F_l: a warp takes 64 rows of a column of the residue planes. A
+// residue's 16-bit word is already the fp16 subnormal c * 2^-24, so the planes
+// go from memory to shared memory (cp.async) to MMA operands (ldmatrix) as they
+// are; the bytes of F sit in registers as fp16 integers. The FP32 sums start at
+// 0.5: below 361 * 255 * 40 < 2^22 units of 2^-24, they stay in [0.5, 1), whose
+// spacing is one unit, so they are exact and their words are 0x3F000000 + sum.
+// Pairs of columns are joined (16-bit spacing) and transposed through shared
+// memory so that every lane finishes whole elements; the words come out exactly
+// as the integer form (crt.cuh, Frac) gives them.
+//
+// Against that form (5 IMAD.WIDE per modulus and element, 140 of them at 28
+// moduli, issued at 26 lanes/clk/SM) an element costs 12 MMAs per 32 and about
+// 60 other instructions.
+constexpr int RC_ROWS = 64;                        // rows of a column per warp and turn
+constexpr int RC_TR = RC_ROWS * 12 * 4;            // bytes of the transpose buffer: 12 words per row
+__host__ __device__ constexpr int rc_planes(int ks) { return ks * 16 * RC_ROWS * 2; }
+
+template <int KS>
+struct CrtFrag {
+    uint32_t b[KS][3][2];
+    // this lane's share of the byte matrix (row l: modulus, column n: byte n of F_l)
+    __device__ __forceinline__ void fill(const OzCrtParams &K, int lane)
+    {
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int s = 0; s < KS; ++s)
+#pragma unroll
+            for (int v = 0; v < 3; ++v)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t w = 0;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int l = 16 * s + 8 * h + 2 * t + e, n = 8 * v + g;
+                        const uint32_t byte = l < K.nmod && n < 4 * crt::kFL ? (K.F[l][n >> 2] >> (8 * (n & 3))) & 0xFFu : 0u;
+                        w |= (uint32_t)__half_as_ushort(__uint2half_rn(byte)) << (16 * e);
+                    }
+                    b[s][v][h] = w;
+                }
+    }
 };
 
-__device__ __forceinline__ void crt_smem_fill(CrtSmem &sm, const OzCrtParams &K)
+// Zeros the plane rows nmod.. of a warp's buffer (their constants are zero, but
+// what the memory holds need not be a number).
+template <int KS>
+__device__ __forceinline__ void crt_clear(unsigned char *planes, int nmod, int lane)
 {
-    for (int i = threadIdx.x; i < K.nmod * crt::kFLPad; i += blockDim.x)
-        sm.F[i / crt::kFLPad][i % crt::kFLPad] = K.F[i / crt::kFLPad][i % crt::kFLPad];
-    for (int i = threadIdx.x; i < K.nmod; i += blockDim.x) sm.pm[i] = K.pm[i];
+    for (int i = nmod * 8 + lane; i < KS * 16 * 8; i += 32)
+        reinterpret_cast<uint4 *>(planes)[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Starts the copy of 64 rows (chunks of 8 rows below `chunks`) of one column of
+// nmod planes; q: the first row in plane 0, 16-byte aligned. 16-byte chunk c of
+// plane l goes to place c ^ (l % 8) of its 128 bytes, so that ldmatrix reads
+// eight planes without bank conflicts.
+__device__ __forceinline__ void crt_load(uint32_t planes, const uint16_t *q, int64_t plane, int nmod, int chunks,
+                                         int lane)
+{
+    const int c = lane & 7;
+    const uint16_t *p = q + (lane >> 3) * plane + 8 * c;
+    for (int l = lane >> 3; l < nmod; l += 4, p += 4 * plane)
+        if (c < chunks) lmb::cp_async16(planes + l * 128u + ((c ^ (l & 7)) << 4), p);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The column-pair sums of the warp's 64 rows into tr (12 words per row, 10 used).
+template <int KS>
+__device__ __forceinline__ void crt_sums(uint32_t planes, uint32_t *tr, const CrtFrag<KS> &f, int lane)
+{
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t row = planes + ((lane >> 4) * 8u + (lane & 7)) * 128u;
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+        float acc[3][4];
+#pragma unroll
+        for (int v = 0; v < 3; ++v)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[v][i] = 0.5f;
+        const uint32_t at = row + (((mt * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
+#pragma unroll
+        for (int s = 0; s < KS; ++s) {
+            uint32_t a[4];
+            lmb::ldmatrix_x4_trans(a, at + s * 2048u);
+#pragma unroll
+            for (int v = 0; v < 3; ++v)
+                lmb::mma16816(acc[v], a[0], a[1], a[2], a[3], f.b[s][v][0], f.b[s][v][1]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int v = 0; v < 3; ++v)
+                tr[(mt * 16 + g + 8 * h) * 12 + 4 * v + t] =
+                    __float_as_uint(acc[v][2 * h]) + (__float_as_uint(acc[v][2 * h + 1]) << 8);
+    }
+}
+
+__device__ __forceinline__ void add160(uint32_t a[crt::kFL], const uint32_t b[crt::kFL])
+{
+    asm("add.cc.u32 %0, %0, %5;\n\t"
+        "addc.cc.u32 %1, %1, %6;\n\t"
+        "addc.cc.u32 %2, %2, %7;\n\t"
+        "addc.cc.u32 %3, %3, %8;\n\t"
+        "addc.u32 %4, %4, %9;"
+        : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4])
+        : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]));
+}
+__device__ __forceinline__ void sub160(uint32_t a[crt::kFL], const uint32_t b[crt::kFL])
+{
+    asm("sub.cc.u32 %0, %0, %5;\n\t"
+        "subc.cc.u32 %1, %1, %6;\n\t"
+        "subc.cc.u32 %2, %2, %7;\n\t"
+        "subc.cc.u32 %3, %3, %8;\n\t"
+        "subc.u32 %4, %4, %9;"
+        : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4])
+        : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]));
+}
+
+// The 160-bit fraction sum of one row from its column pairs.
+__device__ __forceinline__ void crt_words(const uint32_t *tr, int row, uint32_t x[crt::kFL])
+{
+    const uint4 *p = reinterpret_cast<const uint4 *>(tr + row * 12);
+    const uint4 a = p[0], b = p[1];
+    const uint2 c = *reinterpret_cast<const uint2 *>(p + 2);
+    const uint64_t u0 = (uint64_t)a.y * 65536u + a.x, u1 = (uint64_t)a.w * 65536u + a.z;
+    const uint64_t u2 = (uint64_t)b.y * 65536u + b.x, u3 = (uint64_t)b.w * 65536u + b.z;
+    const uint64_t u4 = (uint64_t)c.y * 65536u + c.x;
+    asm("add.cc.u32 %1, %6, %10;\n\t"
+        "addc.cc.u32 %2, %7, %11;\n\t"
+        "addc.cc.u32 %3, %8, %12;\n\t"
+        "addc.u32 %4, %9, %13;\n\t"
+        // the 0x3F000000 of every column pair
+        "sub.cc.u32 %0, %5, 0x3F000000;\n\t"
+        "subc.cc.u32 %1, %1, 0x3F003F00;\n\t"
+        "subc.cc.u32 %2, %2, 0x3F003F00;\n\t"
+        "subc.cc.u32 %3, %3, 0x3F003F00;\n\t"
+        "subc.u32 %4, %4, 0x3F003F00;"
+        : "=&r"(x[0]), "=&r"(x[1]), "=&r"(x[2]), "=&r"(x[3]), "=&r"(x[4])
+        : "r"((uint32_t)u0), "r"((uint32_t)u1), "r"((uint32_t)u2), "r"((uint32_t)u3), "r"((uint32_t)u4),
+          "r"((uint32_t)(u0 >> 32)), "r"((uint32_t)(u1 >> 32)), "r"((uint32_t)(u2 >> 32)), "r"((uint32_t)(u3 >> 32)));
 }
 
 __device__ __forceinline__ dd::real xw_dd(const xw::XW &x)
@@ -1581,83 +1712,173 @@ __device__ __forceinline__ void tri_task(int uplo, int64_t t, int64_t slabs, int
     j = t - tri_prefix(uplo, x, n, S) + (uplo == 1 ? min(n, S * x) : 0);
 }
 
-// Output rows i0 and i0 + 1 (when `two`) of column j: the CRT sums of their
-// residues over the nmod planes (rcol points at row i0, column j of plane 0;
-// planes `plane` entries apart), then alpha M (folded into Mx), the power-of-
-// two scaling and beta C (beta as the extended float xb), one rounding to
-// double-double. pc points at C(i0, j).
-__device__ __forceinline__ void reconstruct_pair(const CrtSmem &sm, int nmod, const uint16_t *rcol, int64_t plane,
-                                                 int i0, bool two, int ea0, int ea1, int j, int ebj, int bsum,
-                                                 const xw::XW &Mx, const xw::XW &xb, dd::real beta, int beta_kind,
-                                                 double2 *pc, int uplo)
+// alpha M as four mantissa words at one exponent: for complex alpha both parts
+// (the smaller cut at 2^-128 of the larger).
+struct RecScale {
+    uint32_t re[4], im[4];
+    int e;
+    uint32_t neg_re, neg_im;
+    int has_im;
+};
+
+struct Words5 {
+    uint32_t x[crt::kFL];
+};
+
+// The signed 160-bit fraction of words x (changed) as magnitude and sign.
+__device__ __forceinline__ uint32_t frac_abs(uint32_t x[crt::kFL])
 {
-    // both rows outside the stored triangle: nothing to compute
-    if ((uplo == 1 && i0 > j) || (uplo == 2 && i0 + 1 < j)) return;
-    crt::Frac acc0, acc1;
-    acc0.reset();
-    acc1.reset();
-    const bool live0 = ea0 > kNoExp / 2 && ea0 < 1024 && ebj > kNoExp / 2 && ebj < 1024;
-    const bool live1 = two && ea1 > kNoExp / 2 && ea1 < 1024 && ebj > kNoExp / 2 && ebj < 1024;
-    if (live0 || live1) {
-        // residues of all moduli for both rows: the loads of 8 planes are
-        // issued together so that their latencies overlap
-        const uint32_t *q = reinterpret_cast<const uint32_t *>(rcol);
-        const int64_t qstep = plane / 2;
-        int l = 0;
-        for (; l + 8 <= nmod; l += 8) {
-            uint32_t c[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                c[u] = __ldcs(q);
-                q += qstep;
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                acc0.add(sm.F[l + u], c[u] & 0xFFFFu);
-                acc1.add(sm.F[l + u], c[u] >> 16);
-            }
-        }
-        for (; l < nmod; ++l, q += qstep) {
-            const uint32_t c = __ldcs(q);
-            acc0.add(sm.F[l], c & 0xFFFFu);
-            acc1.add(sm.F[l], c >> 16);
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int i = i0 + h;
-        if (h == 1 && !two) break;
-        if ((uplo == 1 && i > j) || (uplo == 2 && i < j)) continue;
-        const int eai = h ? ea1 : ea0;
-        double2 *pe = pc + h;
-        if (eai >= 1024 || ebj >= 1024) {   // a non-finite entry in row i of op(A) or column j of op(B)
-            const double qnan = __longlong_as_double(0x7ff8000000000000ll);
-            *pe = make_double2(qnan, qnan);
-            continue;
-        }
-        xw::XW v = xw::zero();
-        if (h ? live1 : live0) v = (h ? acc1 : acc0).finish_xw(Mx, bsum - 4 - eai - ebj);
-        if (beta_kind != 0) {
-            const double2 c0 = *pe;
-            if (!finite_hi(c0.x)) {
-                // non-finite C: the double-double operators propagate it
-                dd::real cv = dd::make(c0.x, c0.y);
-                if (beta_kind == 2) cv = dd::mul_exact(cv, beta);
-                dd::store(pe, dd::add_exact(cv, xw_dd(v)));
-                continue;
-            }
-            xw::XW xc = xw::from_dd(c0.x, c0.y);
-            if (beta_kind == 2) xc = xw::mul(xb, xc);
-            v = xw::add(v, xc);
-        }
-        dd::store(pe, xw_dd(v));
-    }
+    const uint32_t m = (uint32_t)((int)x[crt::kFL - 1] >> 31);
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %5, 0xFFFFFFFF;\n\t"   // the carry in: m & 1
+        "addc.cc.u32 %0, %6, 0;\n\t"
+        "addc.cc.u32 %1, %7, 0;\n\t"
+        "addc.cc.u32 %2, %8, 0;\n\t"
+        "addc.cc.u32 %3, %9, 0;\n\t"
+        "addc.u32 %4, %10, 0;\n\t}"
+        : "=&r"(x[0]), "=&r"(x[1]), "=&r"(x[2]), "=&r"(x[3]), "=&r"(x[4])
+        : "r"(m & 1u), "r"(x[0] ^ m), "r"(x[1] ^ m), "r"(x[2] ^ m), "r"(x[3] ^ m), "r"(x[4] ^ m));
+    return m & 1u;
 }
 
-// C(i, j) := alpha * X(i, j) * 2^-S2 + beta * C(i, j), real. Thread per pair
-// of rows, columns j = blockIdx.y, blockIdx.y + gridDim.y, ...; m and n below 2^31
-// (the host routes larger sizes elsewhere), so the per-element index work is
-// 32-bit or pointer increments.
+// a += (neg ? -1 : 1) * beta part b (b.w[3] != 0; kind 1: one) times the
+// double-double c; false where c needs the general path (a is unchanged then).
+__device__ __forceinline__ bool add_beta_c(fxr::Fix &a, double2 c, const xw::XW &b, bool one, uint32_t neg)
+{
+    const uint32_t hh = (uint32_t)__double2hiint(c.x);
+    if (((hh << 1) | (uint32_t)__double2loint(c.x)) == 0u)   // zero: nothing to add, unless lo is not finite
+        return ((__double2hiint(c.y) >> 20) & 0x7FF) != 0x7FF;
+    uint32_t w[4], q[5];
+    int eh;
+    if (!lmb::split_fast(c, w, eh)) return false;
+    int e = eh - lmb::kExpBias;
+    if (one) {
+        q[0] = w[0]; q[1] = w[1]; q[2] = w[2]; q[3] = w[3]; q[4] = 0u;
+    } else {
+        // W < 2^118 up to the top of its words first, so that the columns the
+        // product drops stay below 2^-123 of it
+        w[3] = __funnelshift_l(w[2], w[3], 10);
+        w[2] = __funnelshift_l(w[1], w[2], 10);
+        w[1] = __funnelshift_l(w[0], w[1], 10);
+        w[0] <<= 10;
+        fxr::mul44(w, b.w, q);
+        e += b.e + 86;
+        neg ^= b.neg;
+    }
+    fxr::add(a, q, e, neg ^ (hh >> 31));
+    return true;
+}
+
+// The general path of one output, in extended floats: rows or columns without
+// a nonzero entry, a non-finite C, C's elements off the straight-line decode.
+__device__ __noinline__ void reconstruct_slow(Words5 x, bool live, int S2, xw::XW Mx, xw::XW xb, dd::real beta,
+                                              int beta_kind, double2 c0, double2 *pe)
+{
+    xw::XW v = xw::zero();
+    if (live) v = crt::fraction_xw(x.x, Mx, S2);
+    if (beta_kind != 0) {
+        if (!finite_hi(c0.x)) {
+            // non-finite C: the double-double operators propagate it
+            dd::real cv = dd::make(c0.x, c0.y);
+            if (beta_kind == 2) cv = dd::mul_exact(cv, beta);
+            dd::store(pe, dd::add_exact(cv, xw_dd(v)));
+            return;
+        }
+        xw::XW xc = xw::from_dd(c0.x, c0.y);
+        if (beta_kind == 2) xc = xw::mul(xb, xc);
+        v = xw::add(v, xc);
+    }
+    dd::store(pe, xw_dd(v));
+}
+
+// One output: alpha M (folded into Mx) times the fraction of words x, the
+// power-of-two scaling and beta C (beta as the extended float xb; c0 = *pe where
+// beta_kind != 0), one rounding to double-double.
+__device__ __forceinline__ void reconstruct_one(uint32_t x[crt::kFL], int eai, int ebj, int bsum, const xw::XW &Mx,
+                                                const xw::XW &xb, dd::real beta, int beta_kind, double2 c0, double2 *pe)
+{
+    if (eai >= 1024 || ebj >= 1024) {   // a non-finite entry in row i of op(A) or column j of op(B)
+        const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+        *pe = make_double2(qnan, qnan);
+        return;
+    }
+    const bool live = eai > kNoExp / 2 && ebj > kNoExp / 2;
+    const int S2 = bsum - 4 - eai - ebj;
+    Words5 orig;
+#pragma unroll
+    for (int q = 0; q < crt::kFL; ++q) orig.x[q] = x[q];
+    fxr::Fix a;
+    a.neg = frac_abs(x) ^ Mx.neg;
+    fxr::mul54(x, Mx.w, a.w);
+    a.w[5] = 0u;
+    a.e = Mx.e - 32 - S2;
+    if (!live || (beta_kind != 0 && !add_beta_c(a, c0, xb, beta_kind == 1, 0u))) {
+        reconstruct_slow(orig, live, S2, Mx, xb, beta, beta_kind, c0, pe);
+        return;
+    }
+    double h, l;
+    fxr::to_dd(a, h, l);
+    *pe = make_double2(h, l);
+}
+
+// The (64-row slab of this warp, column) turns of a reconstruction. Full
+// output: the warp's own rows, columns blockIdx.y, + gridDim.y, ..; triangle:
+// the block's share of the task list, without the tasks whose rows of this warp
+// hold no stored entry.
+struct RecTurns {
+    int m, n, uplo, j;
+    int64_t i0, t, total, slabs, S, step;
+    // S rows per block (blockDim.x / 32 warps of 64)
+    __device__ __forceinline__ void begin(int m_, int n_, int uplo_)
+    {
+        m = m_;
+        n = n_;
+        uplo = uplo_;
+        S = 2 * (int64_t)blockDim.x;
+        if (uplo == 0) {
+            i0 = blockIdx.x * S + (threadIdx.x >> 5) * RC_ROWS;
+            j = i0 < m ? (int)blockIdx.y : n;
+            return;
+        }
+        slabs = (m + S - 1) / S;
+        total = tri_prefix(uplo, slabs, n, S);
+        t = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
+        step = (int64_t)gridDim.x * gridDim.y;
+        find();
+    }
+    __device__ __forceinline__ void find()
+    {
+        for (; t < total; t += step) {
+            int64_t x, jj;
+            tri_task(uplo, t, slabs, n, S, x, jj);
+            i0 = x * S + (threadIdx.x >> 5) * RC_ROWS;
+            j = (int)jj;
+            if (i0 < m && (uplo == 1 ? i0 <= jj : i0 + RC_ROWS > jj)) return;
+        }
+        j = n;
+    }
+    __device__ __forceinline__ bool more() const { return j < n; }
+    __device__ __forceinline__ void next()
+    {
+        if (uplo == 0) {
+            j = n - j > (int)gridDim.y ? j + (int)gridDim.y : n;
+            return;
+        }
+        t += step;
+        find();
+    }
+};
+
+// C(i, j) := alpha * X(i, j) * 2^-S2 + beta * C(i, j), real. A warp takes 64
+// rows of a column per turn, a lane rows lane and lane + 32 of them; the next
+// turn's residues are copied while this one's outputs are finished. m and n
+// below 2^31 (the host routes larger sizes elsewhere).
+//
+// Bound: instruction issue, 551 per output with a general beta (950 with the
+// sums as IMAD.WIDE and the update in extended floats; 830 with the sums on the
+// tensor cores alone). 4096^2: 0.62 -> 0.36 ms; the triangle of 8192^2: 1.44 ->
+// 0.90 ms; 1531 x 1277: 83 -> 58 us.
+template <int KS>
 __global__ void __launch_bounds__(256) k_oz_reconstruct(int m, int n, const uint16_t *__restrict__ R,
                                                         int64_t Mp, int64_t Np, const int *__restrict__ ea,
                                                         const int *__restrict__ eb, int bsum, OzCrtParams K,
@@ -1665,169 +1886,251 @@ __global__ void __launch_bounds__(256) k_oz_reconstruct(int m, int n, const uint
                                                         double2 *C, int64_t ldc, int uplo)
 {
     // Mx = alpha * M and xb = beta as extended floats (formed on the host).
-    // A thread takes rows i0, i0 + 1 (one 32-bit load per modulus serves both).
-    __shared__ CrtSmem sm;
-    crt_smem_fill(sm, K);
-    __syncthreads();
-    const int nmod = K.nmod;
+    extern __shared__ __align__(16) unsigned char s_rec[];
+    const int lane = threadIdx.x & 31;
+    unsigned char *mine = s_rec + (threadIdx.x >> 5) * (rc_planes(KS) + RC_TR);
+    const uint32_t planes = (uint32_t)__cvta_generic_to_shared(mine);
+    uint32_t *tr = reinterpret_cast<uint32_t *>(mine + rc_planes(KS));
+    CrtFrag<KS> f;
+    f.fill(K, lane);
+    crt_clear<KS>(mine, K.nmod, lane);
     const int64_t plane = Np * Mp;
-    if (uplo != 0) {
-        // a triangle: (512-row slab, column) tasks shared evenly by all blocks
-        const int64_t S = 2 * (int64_t)blockDim.x, slabs = (m + S - 1) / S, total = tri_prefix(uplo, slabs, n, S);
-        for (int64_t t = (int64_t)blockIdx.y * gridDim.x + blockIdx.x; t < total;
-             t += (int64_t)gridDim.x * gridDim.y) {
-            int64_t x, j;
-            tri_task(uplo, t, slabs, n, S, x, j);
-            const int i0 = (int)(x * S) + 2 * threadIdx.x;
-            if (i0 >= m) continue;
-            const bool two = i0 + 1 < m;
-            reconstruct_pair(sm, nmod, R + j * Mp + i0, plane, i0, two, ea[i0], two ? ea[i0 + 1] : kNoExp, (int)j,
-                             eb[j], bsum, Mx, xb, beta, beta_kind, C + i0 + j * ldc, uplo);
+    RecTurns T;
+    T.begin(m, n, uplo);
+    if (T.more()) crt_load(planes, R + T.j * Mp + T.i0, plane, K.nmod, 8, lane);
+    while (T.more()) {
+        const int i = (int)T.i0 + lane, j = T.j;
+        bool in[2];
+        double2 c0[2];
+        double2 *pe = C + i + j * ldc;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = i + 32 * h;
+            in[h] = r < m && !(uplo == 1 && r > j) && !(uplo == 2 && r < j);
+            c0[h] = in[h] && beta_kind != 0 ? pe[32 * h] : make_double2(0.0, 0.0);
         }
-        return;
+        const int ebj = eb[j];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        crt_sums<KS>(planes, tr, f, lane);
+        __syncwarp();
+        T.next();
+        if (T.more()) crt_load(planes, R + T.j * Mp + T.i0, plane, K.nmod, 8, lane);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!in[h]) continue;
+            uint32_t x[crt::kFL];
+            crt_words(tr, lane + 32 * h, x);
+            reconstruct_one(x, ea[i + 32 * h], ebj, bsum, Mx, xb, beta, beta_kind, c0[h], pe + 32 * h);
+        }
     }
-    const int i0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (i0 >= m) return;
-    const bool two = i0 + 1 < m;
-    const int ea0 = ea[i0], ea1 = two ? ea[i0 + 1] : kNoExp;
-    const int jstep = gridDim.y;
-    const uint16_t *rcol = R + (int64_t)blockIdx.y * Mp + i0;
-    double2 *pc = C + i0 + (int64_t)blockIdx.y * ldc;
-    const int64_t rstep = (int64_t)jstep * Mp, cstep = (int64_t)jstep * ldc;
-    for (int j = blockIdx.y; j < n; j += jstep, rcol += rstep, pc += cstep)
-        reconstruct_pair(sm, nmod, rcol, plane, i0, two, ea0, ea1, j, eb[j], bsum, Mx, xb, beta, beta_kind, pc, uplo);
+}
+
+// The general path of one complex output (see reconstruct_slow); diag: the
+// imaginary part is stored as zero.
+__device__ __noinline__ void reconstruct_c_slow(Words5 xr, Words5 xi, bool live, int S2, xw::XW Mx, xw::XW ar,
+                                                xw::XW ai, int alpha_one, dd::cplx beta, xw::XW br, xw::XW bi,
+                                                int beta_kind, int real_beta, bool diag, double2 *pc)
+{
+    xw::XW vr, vi;
+    vr = vi = xw::zero();
+    if (live) {
+        vr = crt::fraction_xw(xr.x, Mx, S2);
+        vi = crt::fraction_xw(xi.x, Mx, S2);
+    }
+    xw::XW rr = vr, ri = vi;
+    if (!alpha_one) {
+        xw::XW t = xw::mul(ai, vi);
+        t.neg ^= 1u;
+        rr = xw::add(xw::mul(ar, vr), t);
+        ri = xw::add(xw::mul(ar, vi), xw::mul(ai, vr));
+    }
+    if (beta_kind != 0) {
+        double2 c0r = pc[0], c0i = pc[1];
+        if (!finite_hi(c0r.x) || !finite_hi(c0i.x)) {
+            dd::cplx c0;
+            c0.re = dd::make(c0r.x, c0r.y);
+            c0.im = dd::make(c0i.x, c0i.y);
+            if (beta_kind == 2) {
+                if (real_beta) {
+                    c0.re = dd::mul_exact(beta.re, c0.re);
+                    c0.im = dd::mul_exact(beta.re, c0.im);
+                } else {
+                    c0 = dd::cmul_exact(c0, beta);
+                }
+            }
+            dd::cplx out;
+            out.re = dd::add_exact(c0.re, xw_dd(rr));
+            out.im = dd::add_exact(c0.im, xw_dd(ri));
+            if (diag) out.im = dd::make(0.0, 0.0);
+            dd::cstore(pc, out);
+            return;
+        }
+        xw::XW cr = xw::from_dd(c0r.x, c0r.y), ci = xw::from_dd(c0i.x, c0i.y);
+        if (beta_kind == 2) {
+            if (real_beta) {
+                cr = xw::mul(br, cr);
+                ci = xw::mul(br, ci);
+            } else {
+                xw::XW t = xw::mul(bi, ci);
+                t.neg ^= 1u;
+                xw::XW nr = xw::add(xw::mul(br, cr), t);
+                xw::XW ni = xw::add(xw::mul(br, ci), xw::mul(bi, cr));
+                cr = nr;
+                ci = ni;
+            }
+        }
+        rr = xw::add(rr, cr);
+        ri = xw::add(ri, ci);
+    }
+    dd::cplx out;
+    out.re = xw_dd(rr);
+    out.im = (diag) ? dd::make(0.0, 0.0) : xw_dd(ri);
+    dd::cstore(pc, out);
 }
 
 // Complex: R holds the residues of P1 = Ar*Br, P2 = Ai*Bi and
 // P3 = (Ar+Ai)*(Br+Bi) as components 0..2; Re = P1 - P2, Im = P3 - P1 - P2.
-__global__ void __launch_bounds__(256) k_oz_reconstruct_c(int m, int n, const uint16_t *__restrict__ R,
+// Warps and turns as in the real kernel, four warps per block (three components'
+// planes each); the sum is linear in the residues, so the components' fractions
+// are combined mod 2^160. 2049 x 1900: 0.54 -> 0.46 ms.
+template <int KS>
+__global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const uint16_t *__restrict__ R,
                                                           int64_t Mp, int64_t Np, const int *__restrict__ ea,
                                                           const int *__restrict__ eb, int bsum, OzCrtParams K,
                                                           xw::XW Mx, xw::XW ar, xw::XW ai, int alpha_one,
-                                                          dd::cplx beta, xw::XW br, xw::XW bi, int beta_kind,
+                                                          RecScale A, dd::cplx beta, xw::XW br, xw::XW bi, int beta_kind,
                                                           double2 *C, int64_t ldc, int uplo, int herm, int real_beta)
 {
     // Mx = M, (ar, ai) = alpha and (br, bi) = beta as extended floats (formed on the host)
-    __shared__ CrtSmem sm;
-    crt_smem_fill(sm, K);
-    __syncthreads();
-    const int nmod = K.nmod;
-    const int64_t cstride = (int64_t)nmod * Np * Mp;
-    // output (i, j)
-    auto one = [&](const int i, const int j) {
-        if ((uplo == 1 && i > j) || (uplo == 2 && i < j)) return;
+    extern __shared__ __align__(16) unsigned char s_rec[];
+    const int lane = threadIdx.x & 31;
+    unsigned char *mine = s_rec + (threadIdx.x >> 5) * (3 * rc_planes(KS) + RC_TR);
+    const uint32_t planes = (uint32_t)__cvta_generic_to_shared(mine);
+    uint32_t *tr = reinterpret_cast<uint32_t *>(mine + 3 * rc_planes(KS));
+    CrtFrag<KS> f;
+    f.fill(K, lane);
+    for (int z = 0; z < 3; ++z) crt_clear<KS>(mine + z * rc_planes(KS), K.nmod, lane);
+    const int64_t plane = Np * Mp, cstride = (int64_t)K.nmod * plane;
+    auto load = [&](int64_t i0, int j) {
+        for (int z = 0; z < 3; ++z)
+            crt_load(planes + z * rc_planes(KS), R + z * cstride + j * Mp + i0, plane, K.nmod, 8, lane);
+    };
+    // output (i, j) from the fractions of its real and imaginary parts
+    auto one = [&](const int i, const int j, uint32_t xr[crt::kFL], uint32_t xi[crt::kFL]) {
+        double2 *pc = C + 2 * (i + (int64_t)j * ldc);
         if (ea[i] >= 1024 || eb[j] >= 1024) {
             const double qnan = __longlong_as_double(0x7ff8000000000000ll);
-            double2 *pc = C + 2 * (i + (int64_t)j * ldc);
             pc[0] = make_double2(qnan, qnan);
             pc[1] = make_double2(qnan, qnan);
             return;
         }
-        xw::XW vr, vi;
-        vr = vi = xw::zero();
-        if (ea[i] > kNoExp / 2 && eb[j] > kNoExp / 2) {
-            crt::Frac accr, acci;
-            accr.reset();
-            acci.reset();
-            auto add_l = [&](int l, int p1, int p2, int p3) {
-                const int p = (int)sm.pm[l];
-                int re = p1 - p2;
-                if (re < 0) re += p;
-                int im = p3 - p1 - p2;
-                if (im < 0) im += p;
-                if (im < 0) im += p;
-                accr.add(sm.F[l], (uint32_t)re);
-                acci.add(sm.F[l], (uint32_t)im);
-            };
-            const uint16_t *rp = R + (int64_t)j * Mp + i;
-            const int64_t plane = Np * Mp;
-            int l = 0;
-            for (; l + 4 <= nmod; l += 4) {
-                int c[4][3];
+        const bool live = ea[i] > kNoExp / 2 && eb[j] > kNoExp / 2, diag = herm && i == j;
+        const int S2 = bsum - 4 - ea[i] - eb[j];
+        Words5 or_, oi_;
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int z = 0; z < 3; ++z) c[u][z] = __ldcs(rp + z * cstride + (int64_t)(l + u) * plane);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) add_l(l + u, c[u][0], c[u][1], c[u][2]);
-            }
-            for (; l < nmod; ++l) {
-                const uint16_t *q = rp + (int64_t)l * plane;
-                add_l(l, __ldcs(q), __ldcs(q + cstride), __ldcs(q + 2 * cstride));
-            }
-            const int S2 = bsum - 4 - ea[i] - eb[j];
-            vr = accr.finish_xw(Mx, S2);
-            vi = acci.finish_xw(Mx, S2);
+        for (int q = 0; q < crt::kFL; ++q) {
+            or_.x[q] = xr[q];
+            oi_.x[q] = xi[q];
         }
-        xw::XW rr = vr, ri = vi;
-        if (!alpha_one) {
-            xw::XW t = xw::mul(ai, vi);
-            t.neg ^= 1u;
-            rr = xw::add(xw::mul(ar, vr), t);
-            ri = xw::add(xw::mul(ar, vi), xw::mul(ai, vr));
+        // (re + i im) of alpha M: signed products in one frame
+        const uint32_t nr = frac_abs(xr), ni = frac_abs(xi);
+        fxr::Fix vr, vi;
+        fxr::mul54(xr, A.re, vr.w);
+        fxr::mul54(xi, A.re, vi.w);
+        vr.w[5] = vi.w[5] = 0u;
+        vr.neg = nr ^ A.neg_re;
+        vi.neg = ni ^ A.neg_re;
+        vr.e = vi.e = A.e - 32 - S2;
+        if (A.has_im) {
+            uint32_t p[5];
+            fxr::mul54(xi, A.im, p);
+            fxr::add(vr, p, vr.e, ni ^ A.neg_im ^ 1u);
+            fxr::mul54(xr, A.im, p);
+            fxr::add(vi, p, vi.e, nr ^ A.neg_im);
         }
-        double2 *pc = C + 2 * (i + (int64_t)j * ldc);
-        if (beta_kind != 0) {
-            double2 c0r = pc[0], c0i = pc[1];
-            if (!finite_hi(c0r.x) || !finite_hi(c0i.x)) {
-                dd::cplx c0;
-                c0.re = dd::make(c0r.x, c0r.y);
-                c0.im = dd::make(c0i.x, c0i.y);
-                if (beta_kind == 2) {
-                    if (real_beta) {
-                        c0.re = dd::mul_exact(beta.re, c0.re);
-                        c0.im = dd::mul_exact(beta.re, c0.im);
-                    } else {
-                        c0 = dd::cmul_exact(c0, beta);
-                    }
-                }
-                dd::cplx out;
-                out.re = dd::add_exact(c0.re, xw_dd(rr));
-                out.im = dd::add_exact(c0.im, xw_dd(ri));
-                if (herm && i == j) out.im = dd::make(0.0, 0.0);
-                dd::cstore(pc, out);
-                return;
-            }
-            xw::XW cr = xw::from_dd(c0r.x, c0r.y), ci = xw::from_dd(c0i.x, c0i.y);
-            if (beta_kind == 2) {
-                if (real_beta) {
-                    cr = xw::mul(br, cr);
-                    ci = xw::mul(br, ci);
-                } else {
-                    xw::XW t = xw::mul(bi, ci);
-                    t.neg ^= 1u;
-                    xw::XW nr = xw::add(xw::mul(br, cr), t);
-                    xw::XW ni = xw::add(xw::mul(br, ci), xw::mul(bi, cr));
-                    cr = nr;
-                    ci = ni;
-                }
-            }
-            rr = xw::add(rr, cr);
-            ri = xw::add(ri, ci);
+        bool fast = live;
+        if (beta_kind != 0 && live) {
+            const double2 cr = pc[0], ci = pc[1];
+            const bool b1 = beta_kind == 1;
+            fast = add_beta_c(vr, cr, br, b1, 0u) && add_beta_c(vi, ci, br, b1, 0u);
+            if (!b1 && !real_beta && bi.w[3] != 0u)
+                fast = fast && add_beta_c(vr, ci, bi, false, 1u) && add_beta_c(vi, cr, bi, false, 0u);
         }
-        dd::cplx out;
-        out.re = xw_dd(rr);
-        out.im = (herm && i == j) ? dd::make(0.0, 0.0) : xw_dd(ri);
-        dd::cstore(pc, out);
+        if (!fast) {
+            reconstruct_c_slow(or_, oi_, live, S2, Mx, ar, ai, alpha_one, beta, br, bi, beta_kind, real_beta, diag, pc);
+            return;
+        }
+        double h, l;
+        fxr::to_dd(vr, h, l);
+        pc[0] = make_double2(h, l);
+        fxr::to_dd(vi, h, l);
+        pc[1] = diag ? make_double2(0.0, 0.0) : make_double2(h, l);
     };
-    if (uplo != 0) {
-        // a triangle: (256-row slab, column) tasks shared evenly by all blocks
-        const int64_t S = blockDim.x, slabs = (m + S - 1) / S, total = tri_prefix(uplo, slabs, n, S);
-        for (int64_t t = (int64_t)blockIdx.y * gridDim.x + blockIdx.x; t < total;
-             t += (int64_t)gridDim.x * gridDim.y) {
-            int64_t x, j;
-            tri_task(uplo, t, slabs, n, S, x, j);
-            const int i = (int)(x * S) + threadIdx.x;
-            if (i < m) one(i, (int)j);
+    RecTurns T;
+    T.begin(m, n, uplo);
+    if (T.more()) load(T.i0, T.j);
+    while (T.more()) {
+        const int i = (int)T.i0 + lane, j = T.j;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        uint32_t xr[2][crt::kFL], xi[2][crt::kFL];
+#pragma unroll
+        for (int z = 0; z < 3; ++z) {
+            __syncwarp();   // the planes have landed; the previous component's words have been read
+            crt_sums<KS>(planes + z * rc_planes(KS), tr, f, lane);
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t x[crt::kFL];
+                crt_words(tr, lane + 32 * h, x);
+                // Re = P1 - P2, Im = P3 - P1 - P2
+                if (z == 0) {
+#pragma unroll
+                    for (int q = 0; q < crt::kFL; ++q) {
+                        xr[h][q] = x[q];
+                        xi[h][q] = 0u;
+                    }
+                    sub160(xi[h], x);
+                } else if (z == 1) {
+                    sub160(xr[h], x);
+                    sub160(xi[h], x);
+                } else {
+                    add160(xi[h], x);
+                }
+            }
         }
-        return;
+        __syncwarp();
+        T.next();
+        if (T.more()) load(T.i0, T.j);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = i + 32 * h;
+            if (r < m && !(uplo == 1 && r > j) && !(uplo == 2 && r < j)) one(r, j, xr[h], xi[h]);
+        }
     }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    for (int j = blockIdx.y; j < n; j += gridDim.y) one(i, j);
 }
 
 // ---- host ---------------------------------------------------------------------------------
+
+// alpha M for the complex reconstruction.
+RecScale rec_scale(const dd::cplx &alpha, bool one, const xw::XW &Mx)
+{
+    RecScale A;
+    const xw::XW r = one ? Mx : xw::mul(xw::from_dd(alpha.re.hi, alpha.re.lo), Mx);
+    const xw::XW i = one ? xw::zero() : xw::mul(xw::from_dd(alpha.im.hi, alpha.im.lo), Mx);
+    const bool rz = r.w[3] == 0u, iz = i.w[3] == 0u;
+    A.e = rz ? i.e : (iz ? r.e : std::max(r.e, i.e));
+    auto place = [&](const xw::XW &v, bool zero, uint32_t w[4]) {
+        w[0] = w[1] = w[2] = w[3] = 0u;
+        if (!zero && A.e - v.e < 128) xw::shr4(v.w, A.e - v.e, w);
+    };
+    place(r, rz, A.re);
+    place(i, iz, A.im);
+    A.neg_re = r.neg;
+    A.neg_im = i.neg;
+    A.has_im = iz ? 0 : 1;
+    return A;
+}
 
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 
@@ -2218,10 +2521,12 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             bool alpha_one = (g.alpha.hi == 1.0 && g.alpha.lo == 0.0);
             // alpha folded into M: alpha * X = T * (alpha M)
             const xw::XW aM = alpha_one ? Mx : xw::mul(xw::from_dd(g.alpha.hi, g.alpha.lo), Mx);
-            k_oz_reconstruct<<<grid, 256, 0, stream()>>>((int)m, (int)nn, Rj, Mp, Np, ea, eb + j0, bits_a + bits_b, cp, aM,
-                                                        xw::from_dd(g.beta.hi, g.beta.lo),
-                                                        dd::make(g.beta.hi, g.beta.lo), g.beta_kind, Cj, g.ldc,
-                                                        g.uplo);
+            auto kern = cp.nmod <= 32 ? k_oz_reconstruct<2> : k_oz_reconstruct<3>;
+            const int smem = 8 * (rc_planes(cp.nmod <= 32 ? 2 : 3) + RC_TR);
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            kern<<<grid, 256, smem, stream()>>>((int)m, (int)nn, Rj, Mp, Np, ea, eb + j0, bits_a + bits_b, cp, aM,
+                                                xw::from_dd(g.beta.hi, g.beta.lo), dd::make(g.beta.hi, g.beta.lo),
+                                                g.beta_kind, Cj, g.ldc, g.uplo);
         } else {
             dd::cplx al, be;
             al.re = dd::make(g.calpha.re.hi, g.calpha.re.lo);
@@ -2230,9 +2535,12 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             be.im = dd::make(g.cbeta.im.hi, g.cbeta.im.lo);
             bool alpha_one = (g.calpha.re.hi == 1.0 && g.calpha.re.lo == 0.0 && g.calpha.im.hi == 0.0 &&
                               g.calpha.im.lo == 0.0);
-            k_oz_reconstruct_c<<<grid, 256, 0, stream()>>>(
+            auto kern = cp.nmod <= 32 ? k_oz_reconstruct_c<2> : k_oz_reconstruct_c<3>;
+            const int smem = 4 * (3 * rc_planes(cp.nmod <= 32 ? 2 : 3) + RC_TR);
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            kern<<<grid, 128, smem, stream()>>>(
                 (int)m, (int)nn, Rj, Mp, Np, ea, eb + j0, bits_a + bits_b, cp, Mx, xw::from_dd(al.re.hi, al.re.lo),
-                xw::from_dd(al.im.hi, al.im.lo), alpha_one ? 1 : 0, be, xw::from_dd(be.re.hi, be.re.lo),
+                xw::from_dd(al.im.hi, al.im.lo), alpha_one ? 1 : 0, rec_scale(al, alpha_one, Mx), be, xw::from_dd(be.re.hi, be.re.lo),
                 xw::from_dd(be.im.hi, be.im.lo), g.beta_kind, Cj, g.ldc, g.uplo, g.herm ? 1 : 0, g.herm ? 1 : 0);
         }
         count_launch();
@@ -2568,30 +2876,75 @@ __global__ void __launch_bounds__(RT_THREADS, 4)
 }
 
 // alpha * X * 2^-S2 + beta C for every instance. A work item is 64 rows x 8
-// columns of one instance; thread t takes the row pair t % 32 of column t / 32
-// (the 32 threads of a column read consecutive residue words).
+// columns of one instance, a warp per column (crt_sums).
+template <int KS>
 __global__ void __launch_bounds__(256) k_grp_reconstruct(const OzGrpDesc *__restrict__ descs, int count,
                                                          int64_t items, const OzGrpClass *__restrict__ classes,
                                                          const int *__restrict__ ex, int bsum, OzCrtParams K)
 {
-    __shared__ CrtSmem sm;
-    crt_smem_fill(sm, K);
-    __syncthreads();
+    extern __shared__ __align__(16) unsigned char s_rec[];
+    const int lane = threadIdx.x & 31;
+    unsigned char *mine = s_rec + (threadIdx.x >> 5) * (rc_planes(KS) + RC_TR);
+    const uint32_t planes = (uint32_t)__cvta_generic_to_shared(mine);
+    uint32_t *tr = reinterpret_cast<uint32_t *>(mine + rc_planes(KS));
+    CrtFrag<KS> f;
+    f.fill(K, lane);
+    crt_clear<KS>(mine, K.nmod, lane);
     const int nmod = K.nmod;
-    for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
-        const OzGrpDesc &d = descs[grp_find(descs, count, w, 2)];
-        const OzGrpClass &c = classes[d.cls];
-        const int64_t t = w - d.rec_begin, ncg = (d.n + 7) / 8;
-        const int slab = (int)(t / ncg), j = (int)(t % ncg) * 8 + (threadIdx.x >> 5);
-        const int i0 = slab * 64 + 2 * (threadIdx.x & 31);
-        if (i0 >= d.m || j >= d.n) continue;
-        const bool two = i0 + 1 < d.m;
-        const int ea0 = ex[d.ea_off + i0], ea1 = two ? ex[d.ea_off + i0 + 1] : kNoExp;
+    // this warp's column of item w: false past the instance's columns
+    struct Turn {
+        const OzGrpDesc *d;
+        int i0, j;
+    };
+    auto locate = [&](int64_t w, Turn &t) -> bool {
+        t.d = &descs[grp_find(descs, count, w, 2)];
+        const int64_t q = w - t.d->rec_begin, ncg = (t.d->n + 7) / 8;
+        t.i0 = (int)(q / ncg) * RC_ROWS;
+        t.j = (int)(q % ncg) * 8 + (threadIdx.x >> 5);
+        return t.j < t.d->n;
+    };
+    auto load = [&](const Turn &t) {
+        const OzGrpClass &c = classes[t.d->cls];
         const int64_t plane = c.Np * c.Mp;
-        const uint16_t *R0 = c.R + (int64_t)d.slot * nmod * plane + d.r_off + i0;
+        // instances that share a slot start at multiples of 8 rows; nothing past the slot's rows is read
+        const int chunks = (int)min((int64_t)8, (c.Mp - t.d->r_off - t.i0) / 8);
+        crt_load(planes, c.R + (int64_t)t.d->slot * nmod * plane + t.d->r_off + t.i0 + (t.d->c_off + t.j) * c.Mp, plane,
+                 nmod, chunks, lane);
+    };
+    Turn cur{nullptr, 0, 0}, nxt{nullptr, 0, 0};
+    int64_t w = blockIdx.x;
+    auto advance = [&](Turn &t) -> bool {   // the warp's next column from item w on
+        for (; w < items; w += gridDim.x)
+            if (locate(w, t)) {
+                w += gridDim.x;
+                return true;
+            }
+        return false;
+    };
+    bool have = advance(cur);
+    if (have) load(cur);
+    while (have) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        crt_sums<KS>(planes, tr, f, lane);
+        __syncwarp();
+        const bool more = advance(nxt);
+        if (more) load(nxt);
+        const OzGrpDesc &d = *cur.d;
         const dd::real beta = dd::make(d.beta.x, d.beta.y);
-        reconstruct_pair(sm, nmod, R0 + (int64_t)(d.c_off + j) * c.Mp, plane, i0, two, ea0, ea1, j,
-                         ex[d.eb_off + j], bsum, d.aM, d.xb, beta, d.beta_kind, d.C + i0 + (int64_t)j * d.ldc, 0);
+        const int ebj = ex[d.eb_off + cur.j];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = cur.i0 + lane + 32 * h;
+            if (i >= d.m) continue;
+            uint32_t x[crt::kFL];
+            crt_words(tr, lane + 32 * h, x);
+            double2 *pe = d.C + i + (int64_t)cur.j * d.ldc;
+            reconstruct_one(x, ex[d.ea_off + i], ebj, bsum, d.aM, d.xb, beta, d.beta_kind,
+                            d.beta_kind != 0 ? *pe : make_double2(0.0, 0.0), pe);
+        }
+        cur = nxt;
+        have = more;
     }
 }
 
@@ -2828,7 +3181,10 @@ void ozgroup_launch(OzGroupPlan *pl, cudaStream_t s)
                                                              c.Mp, c.Np, pl->mp, c.R, device_status_word(), 0,
                                                              tiles_m2, tiles_n, nz, 0, 0, take_lost_load_injection(), L);
     }
-    k_grp_reconstruct<<<(unsigned)std::min<int64_t>(pl->items, (int64_t)sms * 8), 256, 0, s>>>(
+auto kern = pl->cp.nmod <= 32 ? k_grp_reconstruct<2> : k_grp_reconstruct<3>;
+    const int smem = 8 * (rc_planes(pl->cp.nmod <= 32 ? 2 : 3) + RC_TR);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        kern<<<(unsigned)std::min<int64_t>(pl->items, (int64_t)sms * 8), 256, smem, s>>>(
         pl->d_descs, count, pl->items, pl->d_classes, pl->d_ex, 2 * kGroupBits, pl->cp);
     count_launch(3 + (int64_t)pl->classes.size());
 }
