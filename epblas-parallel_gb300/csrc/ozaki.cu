@@ -469,21 +469,20 @@ void launch_residues(int64_t rows, int64_t kdim, const double2 *X, int64_t ld, c
 
 // ---- device: residues on the tensor cores -------------------------------------------------
 //
-// The limb dot products x_l = sum_q c_q * t_lq (c_q the 10-bit limbs of the
-// scaled integer, t_lq = 2^(10q) mod p_l, symmetric) are a small matrix
-// product, so they run as tcgen05 MMAs instead of FMAs per element and
-// modulus. Row i of the A operand (K = 64 fp16, 128-byte swizzled rows,
-// written by thread i) holds four consecutive elements of op(X), 16 halves
-// each: the limbs as s * (1024 + c_q) for q < 13 (fp16 0x6400 | c_q with the
-// element's sign bit: no conversion instruction), then -s * 1024 twice, then
-// a zero. B is block-diagonal: row v * 32 + l holds, at halves 16 v .. 16 v +
-// 15, t_l0 .. t_l12, then T1, T2 with T1 + T2 = sum_q t_lq (|T1|, |T2| <=
-// 1170, exact in fp16), then 0, so the offsets cancel exactly:
-//     x = s * sum_q (1024 + c_q) t_lq - s * 1024 (T1 + T2) = s * sum_q c_q t_lq.
-// Every partial sum is an integer below 13 * 2047 * 180 + 2 * 1024 * 1170 <
-// 2^23 (exact in fp32) and |x| <= 13 * 1023 * 180 < 2^22, so the symmetric
-// reduction of the FMA path (quotient estimate, no correction step) applies
-// and both paths store the same residues.
+// The limb dot products x_l = sum_q c_q * t_lq (c_q the bytes of the scaled
+// integer, t_lq = 2^(8q) mod p_l, symmetric) are a small matrix product, so they
+// run as tcgen05 MMAs instead of FMAs per element and modulus. Row i of the A
+// operand (K = 64 fp16, 128-byte swizzled rows, written by thread i) holds four
+// consecutive elements of op(X), their 16 signed bytes as fp16 integers. B is
+// block-diagonal: row v * 32 + l holds t_l0 .. t_l15 at halves 16 v .. 16 v + 15.
+// Every partial sum is an integer and |x| <= 16 * 255 * 180 < 2^20, so the
+// symmetric reduction of the FMA path (quotient estimate, no correction step)
+// applies and both paths store the same residues.
+//
+// A limb pair costs one PRMT (0x6400 | byte is 1024 + byte) and one HFMA2 (times
+// the sign, less 1024); the straight-line decode and a shift below a word serve
+// elements within 2^-20 of their row's bound. 4096^2 operand:
+// 365 -> about 320 instructions per element; 8192 x 2048 294 -> 264 us.
 //
 // Four MMAs of M = 128, N = 32, K = 16 (one per element slot v) leave x for
 // element v, modulus l in TMEM column v * 32 + l of lane i. A tile is 16 rows
@@ -498,7 +497,6 @@ constexpr int RT_TILE_BYTES = 128 * 128;   // 128 rows x 64 fp16
 // columns) share an SM.
 constexpr int RT_SMEM = 56 * 1024;
 constexpr int RT_MAX_MOD = 32;
-constexpr int RT_LIMBS = 13;   // 10-bit limbs of |F| < 2^121 (bits <= 120)
 
 // Chunk j (halves 8j .. 8j + 7) of a 128-byte operand row, 128-byte swizzle.
 __device__ __forceinline__ void st_row_chunk(uint8_t *tile, int row, int j, uint4 v)
@@ -533,22 +531,14 @@ __device__ __forceinline__ void scaled_int(double2 v, int sc, uint32_t (&y)[4], 
     }
 }
 
-// Halves 2w, 2w + 1 of an element's A row: limbs 2w, 2w + 1 as 0x6400 | c
-// with the sign bit s; past limb 12 the two offset corrections and a zero.
-template <int W>
-__device__ __forceinline__ uint32_t limb_word(const uint32_t (&y)[4], uint32_t s)
+// Limbs (bytes) 4q .. 4q + 3 of a word as signed fp16 integers: 0x6400 | byte is
+// 1024 + byte, times the sign, less 1024 times the sign.
+__device__ __forceinline__ uint2 limb_pairs(uint32_t word, __half2 sg, __half2 off)
 {
-    constexpr int b = 20 * W, wd = b >> 5, sh = b & 31;
-    const uint32_t corr = 0xE400u ^ (s & 0xFFFFu);   // -s * 1024
-    if (W < 6) {
-        const uint32_t g = __funnelshift_r(y[wd], wd + 1 < 4 ? y[wd + 1] : 0u, sh);   // bits b .. b + 31
-        return ((g & 0x3FFu) | ((g & 0xFFC00u) << 6) | 0x64006400u) ^ s;
-    } else if (W == 6) {
-        const uint32_t c12 = (__funnelshift_r(y[3], 0u, 120 - 96) & 0x3FFu);   // bits 120 .. 129
-        return ((c12 | 0x6400u) ^ (s & 0xFFFFu)) | (corr << 16);
-    } else {
-        return corr;
-    }
+    const uint32_t a = __byte_perm(word, 0x64646464u, 0x4140), b = __byte_perm(word, 0x64646464u, 0x4342);
+    const __half2 ha = __hfma2(*reinterpret_cast<const __half2 *>(&a), sg, off);
+    const __half2 hb = __hfma2(*reinterpret_cast<const __half2 *>(&b), sg, off);
+    return make_uint2(*reinterpret_cast<const uint32_t *>(&ha), *reinterpret_cast<const uint32_t *>(&hb));
 }
 
 // B of the tensor-core residue conversion, row tid = v * 32 + l (block-diagonal).
@@ -560,16 +550,12 @@ __device__ __forceinline__ void rt_constants(uint8_t *sB, const OzResParams &P, 
     for (int q = 0; q < 16; ++q) t[q] = 0.0f;
     if (l < P.nmod) {
         const int p = (int)P.p[l];
-        int pw = 1, sum = 0;
+        int pw = 1;
 #pragma unroll
-        for (int q = 0; q < RT_LIMBS; ++q) {
-            const int ts = pw > p / 2 ? pw - p : pw;
-            t[q] = (float)ts;
-            sum += ts;
-            pw = (pw * 1024) % p;
+        for (int q = 0; q < 16; ++q) {
+            t[q] = (float)(pw > p / 2 ? pw - p : pw);
+            pw = (pw * 256) % p;
         }
-        t[RT_LIMBS] = (float)(sum / 2);
-        t[RT_LIMBS + 1] = (float)(sum - sum / 2);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -585,20 +571,54 @@ __device__ __forceinline__ void rt_constants(uint8_t *sB, const OzResParams &P, 
 
 // A row tid: the limbs of four elements scaled by 2^(bits - 2 - e) (zeros
 // when the row has no live exponent).
-__device__ __forceinline__ void rt_limbs(uint8_t *a, int tid, const double2 (&cur)[4], int e, int bits)
+__device__ __forceinline__ void rt_limbs(uint8_t *tile, int tid, const double2 (&cur)[4], int e, int bits)
 {
     const bool live = e > kNoExp / 2;
     const int sc = bits - 2 - e;
+    // straight-line operands within 2^-20 or so of the row's bound (the shift
+    // below a word): the common case for all four
+    uint32_t y[4][4];
+    int r[4];
+    bool fast = live;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-        uint32_t y[4] = {0u, 0u, 0u, 0u};
-        bool ng = false;
-        if (live) scaled_int(cur[u], sc, y, ng);
-        const uint32_t s = ng ? 0x80008000u : 0u;
-        st_row_chunk(a, tid, 2 * u,
-                     make_uint4(limb_word<0>(y, s), limb_word<1>(y, s), limb_word<2>(y, s), limb_word<3>(y, s)));
-        st_row_chunk(a, tid, 2 * u + 1,
-                     make_uint4(limb_word<4>(y, s), limb_word<5>(y, s), limb_word<6>(y, s), limb_word<7>(y, s)));
+        int eh;
+        const bool ok = lmb::split_fast(cur[u], y[u], eh);
+        r[u] = lmb::kExpBias - sc - eh;
+        fast = fast && ok && (uint32_t)(r[u] - 1) < 31u;
+    }
+    if (fast) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t rb = (y[u][0] >> (r[u] - 1)) & 1u;
+            lmb::shr_short(y[u], r[u]);
+            asm("add.cc.u32 %0, %0, %4;\n\t"
+                "addc.cc.u32 %1, %1, 0;\n\t"
+                "addc.cc.u32 %2, %2, 0;\n\t"
+                "addc.u32 %3, %3, 0;"
+                : "+r"(y[u][0]), "+r"(y[u][1]), "+r"(y[u][2]), "+r"(y[u][3])
+                : "r"(rb));
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            bool ng;
+            if (live) {
+                scaled_int(cur[u], sc, y[u], ng);
+            } else {
+                y[u][0] = y[u][1] = y[u][2] = y[u][3] = 0u;
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint32_t s = (uint32_t)__double2hiint(cur[u].x) & 0x80000000u;
+        const uint32_t sgw = __byte_perm(0x3C003C00u ^ s, 0u, 0x3232), offw = __byte_perm(0xE400E400u ^ s, 0u, 0x3232);
+        const __half2 sg = *reinterpret_cast<const __half2 *>(&sgw), off = *reinterpret_cast<const __half2 *>(&offw);
+        const uint2 a = limb_pairs(y[u][0], sg, off), b = limb_pairs(y[u][1], sg, off);
+        const uint2 c = limb_pairs(y[u][2], sg, off), d = limb_pairs(y[u][3], sg, off);
+        st_row_chunk(tile, tid, 2 * u, make_uint4(a.x, a.y, b.x, b.y));
+        st_row_chunk(tile, tid, 2 * u + 1, make_uint4(c.x, c.y, d.x, d.y));
     }
 }
 
