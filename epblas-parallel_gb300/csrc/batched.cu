@@ -34,10 +34,15 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "dd.cuh"
 #include "fixgemm.cuh"
+#include "fixbeta.cuh"
+#include "fixround.cuh"
+#include "limbmma.cuh"
+#include "xword.cuh"
 #include "level3.h"
 #include "runtime.h"
 
@@ -64,7 +69,14 @@ struct GemmDesc {
     int64_t tile_begin;   // first tile counter (split instances only)
     int64_t part_begin;   // first partial-tile slot: earlier split instances
                           // hold tiles * splitk slots each
+    // tensor-core tiles only: the operands as limb bytes in the wave's scratch
+    int64_t conv_begin;   // first group of 32 lines (rows of op(A), then columns of op(B)) in the wave
+    int64_t a_off, b_off; // [line][kp] entries of 16 bytes
+    int64_t ea_off, eb_off;   // exponent bounds of the lines
+    int kp, pad;          // k rounded up to 16
+    xw::XW xa, xb;        // alpha, beta
 };
+static_assert(sizeof(xw::XW) == 24, "extended float size");
 
 __device__ __forceinline__ double2 opA_at(const GemmDesc &d, int64_t i, int64_t p)
 {
@@ -82,16 +94,359 @@ __device__ __forceinline__ void load_digits(const int *src, int (&dst)[R])
     if constexpr (R == 4) {
         const int4 v = *reinterpret_cast<const int4 *>(src);
         dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w;
-    } else if constexpr (R == 2) {
+    } else {
         const int2 v = *reinterpret_cast<const int2 *>(src);
         dst[0] = v.x; dst[1] = v.y;
-    } else {
-        dst[0] = *src;
     }
 }
 
-// GT x GT output tiles (GT = 16, 32 or 64; chosen per batch by the tuner),
-// 256 threads as 16 x 16, each with R x R outputs (R = GT / 16): rows R tx ..,
+// ---- 16 x 16 output tiles on the tensor cores (byte limbs) -----------------------------
+//
+// Operands are scaled to integers N below 2^116 of their row's (column's) bound,
+// as in the digit kernel below, and held as 16 bytes each in two's complement:
+// limbs 0..14 of N mod 2^120 and limb 15 = 1 where N < 0, of weight -2^120. A
+// first kernel writes them once per operand (k_grp_limbs), [line][k], so that
+// the tiles that share an operand do not convert it again (a batch of sizes
+// log-uniform in [8, 512] has four tiles per operand line on average; with the
+// conversion in the tiles the batch took as long as with the digit kernel).
+//
+// A warp takes two rows and 16 columns; for each output the 16 x 16 limb products
+// summed over k are two m16n8k16 MMAs per 16 k (rows and columns in the order
+// even limbs, odd limbs): one ldmatrix of 16-bit units per operand and 32 k,
+// whose masked halves are fp16 subnormals (limbmma.cuh). The FP32 sums start at
+// 2^-25 and stay, after 64 k at most 255 * 255 * 64 units of 2^-48 above it, in
+// [2^-25, 2^-24): exact, their words are 0x33000000 + sum. Each lane joins its
+// eight limb products of an output into one 64-bit integer (it holds limbs 2g,
+// 2g + 1 of the row and 4t .. 4t + 3 of the column) and adds it to the output's
+// row of 32 such sums in shared memory (64 chunks of 64 k at most per item). At
+// the end every lane takes one output: the 32 sums at weights 2^(16 (g + 2t)) are
+// one carry chain to a 256-bit integer, updated and rounded as in fixround.cuh.
+//
+// Bound: the legacy tensor path (1024 multiply-adds/clk/SM, 256 per limb-wise
+// multiply-add) against 15 IMAD.WIDE (26 lanes/clk/SM) in the digit kernels: 0.25
+// against 0.58 clk/SM; rows past m and columns past n cost nothing. Measured on
+// 4000 products of sizes log-uniform in [8, 512] (those with m or n below 128 or
+// k below 64): 9.8 ms and 0.84 for the limbs, 14.9 on 32 x 32 digit tiles; the
+// tensor pipe is a third busy, latency (16 warps per SM) takes the rest.
+constexpr int LT = 16;                              // tile edge
+constexpr int LT_KC = 64;                           // k per chunk
+constexpr int LT_OP = 2 * LT * LT_KC * 16;          // operand bytes of a chunk
+constexpr int LT_ROW = 33;                          // 64-bit sums per output (32 and a pad)
+constexpr int LT_SMEM = LT_OP + (GTHREADS / 32) * 32 * LT_ROW * 8;
+constexpr int64_t LT_WAVE = 1ll << 26;              // scratch entries (1 GiB) from which a batch is cut into waves
+
+// v * 2^sh (|.| < 2^116) rounded to an integer, as the 16 bytes described above.
+__device__ __forceinline__ uint4 limb_bytes(double2 v, int sh)
+{
+    uint32_t w[4];
+    int eh;
+    const bool ok = lmb::split_fast(v, w, eh);
+    const int r = lmb::kExpBias - sh - eh;
+    const uint32_t m = (uint32_t)(__double2hiint(v.x) >> 31);
+    uint32_t rb;
+    if (ok && (uint32_t)(r - 1) < 31u) {
+        rb = (w[0] >> (r - 1)) & 1u;
+        lmb::shr_short(w, r);
+    } else {
+        const fx::Op o = fx::decode(v);
+        const int q = -(o.e + sh);
+        w[0] = w[1] = w[2] = w[3] = rb = 0u;
+        if (!(o.flags & (fx::kZero | fx::kBad)) && q >= 1 && q < 118) {
+            uint32_t h[4];
+            fx::shr128(o.w, q, w);
+            fx::shr128(o.w, q - 1, h);   // rounding bit
+            rb = h[0] & 1u;
+        }
+    }
+    asm("add.cc.u32 %0, %0, %4;\n\t"
+        "addc.cc.u32 %1, %1, 0;\n\t"
+        "addc.cc.u32 %2, %2, 0;\n\t"
+        "addc.u32 %3, %3, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3])
+        : "r"(rb));
+    uint4 b;
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %4, 0xFFFFFFFF;\n\t"   // the carry in: m & 1
+        "addc.cc.u32 %0, %5, 0;\n\t"
+        "addc.cc.u32 %1, %6, 0;\n\t"
+        "addc.cc.u32 %2, %7, 0;\n\t"
+        "addc.u32 %3, %8, 0;\n\t}"
+        : "=&r"(b.x), "=&r"(b.y), "=&r"(b.z), "=&r"(b.w)
+        : "r"(m & 1u), "r"(w[0] ^ m), "r"(w[1] ^ m), "r"(w[2] ^ m), "r"(w[3] ^ m));
+    b.w &= 0x01FFFFFFu;
+    return b;
+}
+
+// The last descriptor whose `begin` is at most w.
+template <typename F>
+__device__ __forceinline__ int grp_search(int count, int64_t w, F begin)
+{
+    int lo = 0, hi = count - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (begin(mid) <= w) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Exponent bounds and limb bytes of 32 lines (rows of op(A) or columns of op(B))
+// of an instance per block; the second pass reads what the first left in the
+// caches.
+__global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restrict__ descs, int count, uint4 *out,
+                                                        int *ex)
+{
+    __shared__ int s_e[32];
+    const int tid = threadIdx.x;
+    const GemmDesc &d =
+        descs[grp_search(count, (int64_t)blockIdx.x, [&](int q) { return descs[q].conv_begin; })];
+    int grp = (int)((int64_t)blockIdx.x - d.conv_begin);
+    const int ga = (d.m + 31) / 32;
+    const bool isA = grp < ga;
+    if (!isA) grp -= ga;
+    const int line0 = grp * 32, nl = min(32, (isA ? d.m : d.n) - line0), k = d.k, kp = d.kp;
+    const bool along_k = isA ? d.ta != 0 : d.tb == 0;   // a line's entries are neighbours in memory
+    const int64_t ld = isA ? d.lda : d.ldb;
+    const double2 *X = (isA ? d.A : d.B) + (along_k ? line0 * ld : line0);
+    const int64_t sl = along_k ? ld : 1, sk = along_k ? 1 : ld;
+    if (tid < 32) s_e[tid] = kNoExp;
+    __syncthreads();
+    {
+        const int l = along_k ? tid >> 3 : tid & 31, q = along_k ? tid & 7 : tid >> 5;
+        if (l < nl) {
+            const double2 *x = X + l * sl + q * sk;
+            int e = kNoExp;
+#pragma unroll 4
+            for (int p = q; p < k; p += 8, x += 8 * sk) e = max(e, exp_bound(x->x));
+            atomicMax(&s_e[l], e);
+        }
+    }
+    __syncthreads();
+    if (tid < nl) ex[(isA ? d.ea_off : d.eb_off) + line0 + tid] = s_e[tid];
+    // 8 neighbours along k, or 8 lines x 4 k per warp: whole 64 bytes either way
+    const int l = along_k ? tid >> 3 : (tid & 7) + 8 * ((tid >> 5) & 3);
+    const int q = along_k ? tid & 7 : ((tid >> 3) & 3) + 4 * (tid >> 7);
+    if (l >= nl) return;
+    const int e = s_e[l];
+    const bool live = e > kNoExp / 2 && e < 1024;
+    const double2 *x = X + l * sl + q * sk;
+    uint4 *o = out + (isA ? d.a_off : d.b_off) + (int64_t)(line0 + l) * kp;
+#pragma unroll 2
+    for (int p = q; p < kp; p += 8, x += 8 * sk)
+        o[p] = live && p < k ? limb_bytes(*x, fxg::FX_S - e) : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Even and odd limbs of an ldmatrix word (16-bit units of two elements).
+__device__ __forceinline__ uint32_t limbs_even(uint32_t v) { return v & 0x00FF00FFu; }
+__device__ __forceinline__ uint32_t limbs_odd(uint32_t v) { return __byte_perm(v, 0u, 0x4341); }
+
+__global__ void __launch_bounds__(GTHREADS, 2) k_gemm_grouped_limb(const GemmDesc *__restrict__ descs, int count,
+                                                                  int total, unsigned long long *work_counter,
+                                                                  int *tile_counters, fx::XFPod *partials,
+                                                                  const uint4 *__restrict__ limbs,
+                                                                  const int *__restrict__ ex)
+{
+    extern __shared__ __align__(16) unsigned char s_dyn[];   // [operand row 0..31][64 k] 16 bytes, then the sums
+    __shared__ int s_item, s_last;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    unsigned long long *sums = reinterpret_cast<unsigned long long *>(s_dyn + LT_OP) + wid * (32 * LT_ROW);
+    const uint32_t op = (uint32_t)__cvta_generic_to_shared(s_dyn);
+    const uint32_t n15 = t == 3 ? 0u - 256u : 256u;
+    const int m15 = g == 7 ? -256 : 256;
+    // the 0x33000000 of each accumulator word (those times 256 vanish mod 2^32)
+    const unsigned long long off = (unsigned long long)(0x33000000ll * 65537 * (1 + m15));
+    for (;;) {
+        if (tid == 0) s_item = (int)min(atomicAdd(work_counter, 1ull), (unsigned long long)total);
+        __syncthreads();
+        const int w = s_item;
+        if (w >= total) return;
+        const GemmDesc &d = descs[grp_search(count, (int64_t)w, [&](int q) { return descs[q].work_begin; })];
+        const uint32_t local = (uint32_t)(w - d.work_begin), tile = local / (uint32_t)d.splitk;
+        const int split = (int)(local % (uint32_t)d.splitk);
+        const int i0 = (int)(tile % (uint32_t)d.tiles_m) * LT, j0 = (int)(tile / (uint32_t)d.tiles_m) * LT;
+        const int k0 = split * d.klen, kn = min(d.kp, k0 + d.klen) - k0;   // klen: multiples of 16 where split
+        const int mr = min(LT, d.m - i0), nc = min(LT, d.n - j0);
+        const uint4 *pA = limbs + d.a_off + (int64_t)i0 * d.kp + k0, *pB = limbs + d.b_off + (int64_t)j0 * d.kp + k0;
+        const bool rows = 2 * wid < mr;   // this warp has rows of the output
+        const uint32_t a_at = op + (2 * wid) * (LT_KC * 16);
+        const bool some = d.k > 0;
+        for (int c0 = 0; some && c0 < kn; c0 += LT_KC) {
+            if (c0 > 0) __syncthreads();   // the previous chunk's operands have been read
+            const int kc = min(LT_KC, kn - c0), p = tid & 63;
+            // rows 0..15 of op(A), 16..31 columns of op(B), four per turn; k goes to
+            // place k ^ (row % 8), so that ldmatrix is free of bank conflicts
+            if (p < kc) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int r = (tid >> 6) + 4 * (u & 3);
+                    const uint4 *src = (u < 4 ? pA : pB) + (int64_t)r * d.kp + c0 + p;
+                    if (r < (u < 4 ? mr : nc))
+                        lmb::cp_async16(op + ((((u < 4 ? 0 : LT) + r) * LT_KC + (p ^ (r & 7))) << 4), src);
+                }
+            }
+            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (!rows) continue;
+            const int nks = kc >> 4;   // steps of 16 k
+#pragma unroll 1
+            for (int r = 0; r < 2; ++r) {
+                uint32_t a[4][4];   // the row's operands of every step
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t x[4];
+                    lmb::ldmatrix_x4_trans(x, a_at + r * (LT_KC * 16) + (((32 * h + lane) ^ ((2 * wid + r) & 7)) << 4));
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        a[2 * h + q][0] = limbs_even(x[2 * q]);
+                        a[2 * h + q][1] = limbs_odd(x[2 * q]);
+                        a[2 * h + q][2] = limbs_even(x[2 * q + 1]);
+                        a[2 * h + q][3] = limbs_odd(x[2 * q + 1]);
+                    }
+                }
+                // four columns at a time, so that their products and sums overlap
+                auto columns = [&](int c, auto width) {
+                    constexpr int NC = decltype(width)::value;
+                    float acc[NC][2][4];
+                    uint32_t x[NC][4];
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        if (s >= nks) break;
+                        if ((s & 1) == 0)
+#pragma unroll
+                            for (int u = 0; u < NC; ++u)
+                                lmb::ldmatrix_x4_trans(x[u], op + (LT + c + u) * (LT_KC * 16) +
+                                                                 (((16 * s + lane) ^ ((c + u) & 7)) << 4));
+#pragma unroll
+                        for (int u = 0; u < NC; ++u) {
+                            const uint32_t x0 = x[u][2 * (s & 1)], x1 = x[u][2 * (s & 1) + 1];
+                            const uint32_t e0 = limbs_even(x0), e1 = limbs_even(x1);
+                            const uint32_t o0 = limbs_odd(x0), o1 = limbs_odd(x1);
+                            if (s == 0) {
+                                lmb::mma16816_from(acc[u][0], a[s][0], a[s][1], a[s][2], a[s][3], e0, e1, 0x1p-25f);
+                                lmb::mma16816_from(acc[u][1], a[s][0], a[s][1], a[s][2], a[s][3], o0, o1, 0x1p-25f);
+                            } else {
+                                lmb::mma16816(acc[u][0], a[s][0], a[s][1], a[s][2], a[s][3], e0, e1);
+                                lmb::mma16816(acc[u][1], a[s][0], a[s][1], a[s][2], a[s][3], o0, o1);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < NC; ++u) {
+                        // limbs 4t .. 4t + 3 of the column for each of the row's two limbs;
+                        // limb 15 (t = 3) and the row's limb 15 (g = 7) have negative weight
+                        auto word = [&](int b, int i) { return __float_as_uint(acc[u][b][i]); };
+                        const int lo0 = (int)(word(0, 0) + 256u * word(1, 0)), hi0 = (int)(word(0, 1) + n15 * word(1, 1));
+                        const int lo1 = (int)(word(0, 2) + 256u * word(1, 2)), hi1 = (int)(word(0, 3) + n15 * word(1, 3));
+                        const long long lo = (long long)lo1 * m15 + lo0, hi = (long long)hi1 * m15 + hi0;
+                        unsigned long long *at = sums + ((c + u) * 2 + r) * LT_ROW + lane;
+                        const unsigned long long q = (unsigned long long)(lo + hi * 65536) - off;
+                        *at = c0 == 0 ? q : *at + q;
+                    }
+                };
+                int c = 0;
+                for (; c + 4 <= nc; c += 4) columns(c, std::integral_constant<int, 4>{});
+                for (; c < nc; ++c) columns(c, std::integral_constant<int, 1>{});
+            }
+        }
+        __syncwarp();
+
+        // each lane one output: row 2 wid + (lane & 1), column lane / 2
+        const int orow = 2 * wid + (lane & 1), ocol = lane >> 1;
+        const bool in = orow < mr && ocol < nc;
+        const int ei = in && some ? ex[d.ea_off + i0 + orow] : kNoExp, ej = in && some ? ex[d.eb_off + j0 + ocol] : kNoExp;
+        bool bad = ei >= 1024 || ej >= 1024;
+        const bool live = !bad && ei > kNoExp / 2 && ej > kNoExp / 2;
+        double2 *pc = d.C + i0 + orow + (int64_t)(j0 + ocol) * d.ldc;
+        const double2 c_in = in && d.beta_kind != 0 && d.splitk == 1 ? *pc : make_double2(0.0, 0.0);
+        uint64_t W[4] = {0, 0, 0, 0};
+        if (live) {
+            const unsigned long long *at = sums + lane * LT_ROW;
+            long long carry = 0;   // sum at weight 2^(16 s), its low 16 bits to the result
+#pragma unroll
+            for (int s = 0; s < 14; ++s) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (s - 2 * q >= 0 && s - 2 * q < 8) carry += (long long)at[4 * (s - 2 * q) + q];
+                W[s >> 2] |= (uint64_t)((uint32_t)carry & 0xFFFFu) << (16 * (s & 3));
+                carry >>= 16;
+            }
+            W[3] |= (uint64_t)carry << 32;
+        }
+        const int e0 = ei + ej - 2 * fxg::FX_S;
+        bool done = false;
+        if (in && live && d.splitk == 1) {
+            // the top 160 bits of |W| (2^-134 of the largest product is cut), alpha, beta C, one rounding
+            const uint32_t m = (uint32_t)((int64_t)W[3] >> 63);
+            uint32_t x[8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                x[2 * q] = (uint32_t)W[q];
+                x[2 * q + 1] = (uint32_t)(W[q] >> 32);
+            }
+            fxr::cond_neg<8>(x, m);
+            fxr::Fix a;
+            a.neg = m & 1u;
+            if (d.alpha.x == 1.0 && d.alpha.y == 0.0) {
+#pragma unroll
+                for (int q = 0; q < 5; ++q) a.w[q] = x[3 + q];
+                a.e = e0 + 96;
+            } else {
+                fxr::mul54(x + 3, d.xa.w, a.w);
+                a.neg ^= d.xa.neg;
+                a.e = e0 + 96 + 128 + d.xa.e;
+            }
+            a.w[5] = 0u;
+            if (d.beta_kind == 0 || add_beta_c(a, c_in, d.xb, d.beta_kind == 1, 0u)) {
+                double h, l;
+                fxr::to_dd(a, h, l);
+                *pc = make_double2(h, l);
+                done = true;
+            }
+        }
+        xfp::XF v;
+        v.zero = true; v.neg = false; v.m = 0; v.e = 0;
+        if (live && !done) v = fx::w256_to_xf(W, e0);
+        if (d.splitk > 1) {
+            // this split's sums, then the last split of the tile finishes it
+            fx::XFPod *pt = partials + (d.part_begin + (int64_t)tile * d.splitk + split) * (LT * LT);
+            pt[ocol * LT + orow] = fx::to_pod(v, bad);
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(&tile_counters[d.tile_begin + tile], 1) == d.splitk - 1;
+            __syncthreads();
+            if (!s_last) continue;
+            __threadfence();
+            const fx::XFPod *base = partials + (d.part_begin + (int64_t)tile * d.splitk) * (LT * LT) + ocol * LT + orow;
+            v.zero = true; v.neg = false; v.m = 0; v.e = 0;
+            bad = false;
+            for (int s2 = 0; s2 < d.splitk; ++s2) {
+                // partials written by other CTAs: read through L2
+                const fx::XFPod *q = base + (int64_t)s2 * (LT * LT);
+                fx::XFPod pv;
+                pv.hi = __ldcg(&q->hi);
+                pv.lo = __ldcg(&q->lo);
+                pv.e = __ldcg(&q->e);
+                pv.flags = __ldcg(&q->flags);
+                bad |= (pv.flags & 4) != 0;
+                v = xfp::xf_add(v, fx::from_pod(pv));
+            }
+            if (tid == 0) tile_counters[d.tile_begin + tile] = 0;   // ready for the next replay
+        }
+        if (in && !done) {
+            if (bad) {
+                const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+                *pc = make_double2(qnan, qnan);
+            } else {
+                fxg::store_axpby(pc, v, xfp::xf_from_dd(d.alpha.x, d.alpha.y), d.alpha.x == 1.0 && d.alpha.y == 0.0,
+                                 xfp::xf_from_dd(d.beta.x, d.beta.y), dd::make(d.beta.x, d.beta.y), d.beta_kind);
+            }
+        }
+        __syncthreads();   // s_item and the operands are reused
+    }
+}
+
+// GT x GT output tiles (GT = 32 or 64) on the integer pipes, 256 threads as 16 x 16, each with R x R outputs (R = GT / 16): rows R tx ..,
 // columns R ty ...
 template <int GT>
 __global__ void __launch_bounds__(GTHREADS) k_gemm_grouped(const GemmDesc *__restrict__ descs, int count,
@@ -112,13 +467,7 @@ __global__ void __launch_bounds__(GTHREADS) k_gemm_grouped(const GemmDesc *__res
         __syncthreads();
         if (w >= total) return;
         // locate the instance (descs sorted by work_begin)
-        int lo = 0, hi = count - 1;
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (descs[mid].work_begin <= w) lo = mid;
-            else hi = mid - 1;
-        }
-        const GemmDesc d = descs[lo];
+        const GemmDesc d = descs[grp_search(count, w, [&](int q) { return descs[q].work_begin; })];
         const int64_t local = w - d.work_begin;
         const int split = (int)(local % d.splitk);
         const int64_t tile = local / d.splitk;
@@ -448,6 +797,13 @@ struct Plan {
     OzGroupPlan *oz = nullptr;
     int tile = 32;
     int64_t total = 0, split_tiles = 0, partial_elems = 0;
+    // tensor-core tiles: descriptors [first, first + count) share the limb scratch
+    struct Wave {
+        int first, count;
+        int64_t work, groups, entries, lines;
+    };
+    std::vector<Wave> waves;
+    int64_t wave_entries = 0, wave_lines = 0;   // largest of any wave
     // device state
     void *dev = nullptr;
     size_t dev_bytes = 0;
@@ -457,7 +813,7 @@ struct Plan {
 
 std::mutex g_batched_mu;
 std::map<uint64_t, Policy> g_policy_cache;   // shape class -> tuned policy
-Policy g_default_policy{512, 4, 32, 128, 0};
+Policy g_default_policy{512, 4, 16, 128, 0};
 thread_local int t_tuned_tile = 0;   // tile chosen by this thread's most recent tuning
 thread_local int t_tuned_oz = -1;    // tensor-core threshold chosen by it (0: none)
 std::atomic<int> g_forced_tile{0};   // mwblas_set_grouped_tile: 0 = tuned or default
@@ -503,9 +859,12 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
     const int GT = pol.tile;
     pl.tile = GT;
     int64_t work = 0, stiles = 0, pslots = 0;
+    pl.waves.clear();
+    pl.wave_entries = pl.wave_lines = 0;
     for (int64_t i = 0; i < count; ++i) {
         if (m[i] <= 0 || n[i] <= 0) continue;
-        GemmDesc d{};
+        GemmDesc d;
+        memset(&d, 0, sizeof(d));   // the plan key hashes the bytes, padding included
         d.A = (const double2 *)a[i];
         d.B = (const double2 *)b[i];
         d.C = (double2 *)c[i];
@@ -560,11 +919,41 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
         d.splitk = 1;
         if (pol.min_k_per_split > 0 && tiles <= pol.max_tiles_split && d.k >= 2 * pol.min_k_per_split)
             d.splitk = std::min(16, d.k / pol.min_k_per_split);
-        // the digit column sums hold at most 16384 multiply-adds per split
-        const int need_splits = (d.k + 16383) / 16384;
+        // the digit column sums hold at most 16384 multiply-adds per split, the
+        // limb sums 4096 (64 chunks below 2^54 each, four of them added)
+        const int kmax = GT == LT ? 4096 : 16384;
+        const int need_splits = (d.k + kmax - 1) / kmax;
         if (d.splitk < need_splits) d.splitk = need_splits;
-        d.klen = d.splitk > 1 ? ((d.k + d.splitk - 1) / d.splitk + GBK - 1) / GBK * GBK : std::max(d.k, 1);
+        d.kp = (d.k + 15) / 16 * 16;
+        const int kstep = GT == LT ? 16 : GBK;
+        d.klen = d.splitk > 1 ? ((d.k + d.splitk - 1) / d.splitk + kstep - 1) / kstep * kstep
+                              : std::max(GT == LT ? d.kp : d.k, 1);
         if (d.k == 0) d.klen = 1;
+        if (GT == LT) {
+            // splits past k would be empty: as many as klen needs
+            if (d.splitk > 1) d.splitk = (d.k + d.klen - 1) / d.klen;
+            d.xa = xw::from_dd(d.alpha.x, d.alpha.y);
+            d.xb = xw::from_dd(d.beta.x, d.beta.y);
+            const int64_t entries = ((int64_t)d.m + d.n) * d.kp, lines = d.k > 0 ? (int64_t)d.m + d.n : 0;
+            const int64_t tw = (int64_t)tiles * d.splitk;
+            if (pl.waves.empty() || pl.waves.back().entries + entries > LT_WAVE ||
+                pl.waves.back().work + tw > INT32_MAX)
+                pl.waves.push_back(Plan::Wave{(int)pl.descs.size(), 0, 0, 0, 0, 0});
+            Plan::Wave &wv = pl.waves.back();
+            work = wv.work;   // work items are numbered within the wave
+            d.conv_begin = wv.groups;
+            d.a_off = wv.entries;
+            d.b_off = wv.entries + (int64_t)d.m * d.kp;
+            d.ea_off = wv.lines;
+            d.eb_off = wv.lines + d.m;
+            wv.groups += d.k > 0 ? (d.m + 31) / 32 + (d.n + 31) / 32 : 0;
+            wv.entries += entries;
+            wv.lines += lines;
+            wv.work += tw;
+            wv.count++;
+            pl.wave_entries = std::max(pl.wave_entries, wv.entries);
+            pl.wave_lines = std::max(pl.wave_lines, wv.lines);
+        }
         d.work_begin = work;
         d.tile_begin = d.splitk > 1 ? stiles : 0;
         d.part_begin = d.splitk > 1 ? pslots : 0;
@@ -576,6 +965,7 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
         pl.descs.push_back(d);
     }
     pl.total = work;
+    for (const Plan::Wave &wv : pl.waves) pl.total = std::max(pl.total, wv.work);
     pl.split_tiles = stiles;
     pl.partial_elems = pslots * GT * GT;   // extended-float partials
 }
@@ -604,7 +994,8 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     const size_t d_bytes = pl.descs.size() * sizeof(GemmDesc);
     const size_t cnt_bytes = 256 + (size_t)(pl.split_tiles + 1) * sizeof(int);
     const size_t part_bytes = (size_t)pl.partial_elems * sizeof(fx::XFPod);
-    const size_t need = d_bytes + cnt_bytes + part_bytes + 512;
+    const size_t limb_bytes_ = (size_t)pl.wave_entries * 16, ex_bytes = (size_t)pl.wave_lines * sizeof(int);
+    const size_t need = d_bytes + cnt_bytes + part_bytes + limb_bytes_ + ex_bytes + 1024;
     const uint64_t key = plan_key(pl);
     cudaStream_t s = stream();
     if (pl.dev_bytes < need) {
@@ -617,7 +1008,8 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
         pl.dev_bytes = 0;
         if (!cuda_ok(cudaMalloc(&pl.dev, need), routine, "grouped plan buffer")) return false;
         pl.dev_bytes = need;
-        if (!cuda_ok(cudaMemset(pl.dev, 0, need), routine, "grouped plan clear")) return false;
+        // the tile counters start at zero (each replay leaves them so)
+        if (!cuda_ok(cudaMemset(pl.dev, 0, d_bytes + cnt_bytes + 512), routine, "grouped plan clear")) return false;
     }
     // layout: [descriptors][work counter (256 B) | tile counters][partials],
     // each region starting on a 256-byte boundary
@@ -628,6 +1020,9 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     unsigned long long *counter = (unsigned long long *)(base + cnt_off);
     int *tile_counters = (int *)(counter + 32);
     fx::XFPod *partials = (fx::XFPod *)(base + part_off);
+    const size_t limb_off = (part_off + part_bytes + 255) / 256 * 256;
+    uint4 *limbs = (uint4 *)(base + limb_off);
+    int *ex = (int *)(base + (limb_off + limb_bytes_ + 255) / 256 * 256);
     const int sms = device_sm_count();
     const int grid = (int)std::min<int64_t>(pl.total, (int64_t)sms * 16);
     if (pl.key != key) {
@@ -641,13 +1036,30 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
             if (!ozgroup_prepare(pl.oz, pl.oz_items, routine)) return false;
         }
     }
+    // the integer-pipe or limb-tile part on stream q; its counters start at zero
+    auto enqueue = [&](cudaStream_t q) {
+        cudaMemsetAsync(counter, 0, cnt_bytes, q);
+        if (pl.tile != LT) {
+            auto kern = pl.tile == 64 ? k_gemm_grouped<64> : k_gemm_grouped<32>;
+            kern<<<grid, GTHREADS, 0, q>>>(ddesc, (int)pl.descs.size(), pl.total, counter, tile_counters, partials);
+            return;
+        }
+        cudaFuncSetAttribute(k_gemm_grouped_limb, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
+        bool first = true;
+        for (const Plan::Wave &wv : pl.waves) {
+            if (!first) cudaMemsetAsync(counter, 0, sizeof(*counter), q);
+            first = false;
+            if (wv.groups > 0) k_grp_limbs<<<(unsigned)wv.groups, GTHREADS, 0, q>>>(ddesc + wv.first, wv.count, limbs, ex);
+            const int wgrid = (int)std::min<int64_t>(wv.work, (int64_t)sms * 2);
+            k_gemm_grouped_limb<<<wgrid, GTHREADS, LT_SMEM, q>>>(ddesc + wv.first, wv.count, (int)wv.work, counter,
+                                                                tile_counters, partials, limbs, ex);
+        }
+    };
     if (!use_graph) {
         pl.key = key;
         if (pl.total > 0) {
-            cudaMemsetAsync(counter, 0, cnt_bytes, s);
-            auto kern = pl.tile == 64 ? k_gemm_grouped<64> : (pl.tile == 16 ? k_gemm_grouped<16> : k_gemm_grouped<32>);
-            kern<<<grid, GTHREADS, 0, s>>>(ddesc, (int)pl.descs.size(), pl.total, counter, tile_counters, partials);
-            count_launch();
+            enqueue(s);
+            count_launch(pl.tile == LT ? 2 * (int64_t)pl.waves.size() : 1);
         }
         if (pl.oz && ozgroup_count(pl.oz) > 0) ozgroup_launch(pl.oz, s);
         return cuda_ok(cudaGetLastError(), routine, "grouped launch");
@@ -663,12 +1075,7 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
         bool ok = cuda_ok(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), routine, "begin capture");
         if (ok) {
             // counters start at zero on every replay
-            if (pl.total > 0) {
-                cudaMemsetAsync(counter, 0, cnt_bytes, cap);
-                auto kern = pl.tile == 64 ? k_gemm_grouped<64> : (pl.tile == 16 ? k_gemm_grouped<16> : k_gemm_grouped<32>);
-                kern<<<grid, GTHREADS, 0, cap>>>(ddesc, (int)pl.descs.size(), pl.total, counter, tile_counters,
-                                                 partials);
-            }
+            if (pl.total > 0) enqueue(cap);
             // the large instances on the tensor cores, in the same graph
             if (pl.oz && ozgroup_count(pl.oz) > 0) ozgroup_launch(pl.oz, cap);
             ok = cuda_ok(cudaStreamEndCapture(cap, &graph), routine, "end capture");
