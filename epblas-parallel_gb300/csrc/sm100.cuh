@@ -272,6 +272,15 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
+// The same without ordering the thread's earlier memory accesses: for barriers
+// that hand back tensor memory, whose accesses tcgen05.wait has completed and
+// tcgen05.fence::before_thread_sync orders. A release also waits for the thread's
+// stores to global memory.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr)
+{
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+
 // mbar_wait with acquire at cluster scope (arrivals made by the peer CTA).
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity)
 {

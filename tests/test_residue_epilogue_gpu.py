@@ -1,0 +1,26 @@
+"""The CTA-pair residue GEMM's epilogue against the CUDA-core residue kernel, bit
+for bit: column pairs cut by an odd edge, rows and columns past a tile, and both
+sides of the K at which the accumulator hand-back changes (2048)."""
+import numpy as np
+import pytest
+
+from conftest import mwb
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n", [(255, 129), (513, 257)])
+@pytest.mark.parametrize("k", [2048, 2049])
+def test_epilogue_bits(gpu, rng, m, n, k):
+    A, B = mwb.dd_matrix(rng, m, k), mwb.dd_matrix(rng, k, n)
+    outs = []
+    for kind in (1, 3):   # CUDA cores, CTA pairs
+        prev = gpu.lib.mwblas_set_ozaki_mma(kind)
+        try:
+            c = np.zeros((n, m, 2))
+            gpu.mgemm("N", "N", m, n, k, 1.0, A, m, B, k, 0.0, c, m, engine="ozaki")
+            assert gpu.last_error()[0] == 0, gpu.last_error()
+            outs.append(c)
+        finally:
+            gpu.lib.mwblas_set_ozaki_mma(prev)
+    np.testing.assert_array_equal(outs[0], outs[1])
