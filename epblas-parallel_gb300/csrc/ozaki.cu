@@ -1276,7 +1276,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
 // are faster with it: 8192 x 8192 x 4096 9000, 8800 and 8980, x 8192 17,370,
 // 17,140 and 18,720. Holding 96 to 128 columns in registers to hand the buffer
 // back sooner spills and loses a factor of 1.3 to 2.7.
-constexpr int64_t T2_RELAXED_K = 2048;
+constexpr int64_t T2_RELAXED_K = 3072;
 constexpr int T2_STAGES = 6;
 constexpr int T2_A_BYTES = 128 * TC_BK * 2;   // 16 KB
 constexpr int T2_B_BYTES = 128 * TC_BK * 2;   // 16 KB (half of the 256-row B tile)
@@ -2266,14 +2266,14 @@ bool read_widths(int64_t m, int64_t n, const int *ea, const int *eb, const int *
     const int ga = (int)std::min<int64_t>((m + 255) / 256, 4 * (int64_t)device_sm_count());
     const int gb = (int)std::min<int64_t>((n + 255) / 256, 4 * (int64_t)device_sm_count());
     k_width<<<ga, 256, 0, stream()>>>(m, ea, la, w);
-    k_width<<<gb, 256, 0, stream()>>>(n, eb, lb, w + 1);
-    count_launch(2);
+    if (eb != ea) k_width<<<gb, 256, 0, stream()>>>(n, eb, lb, w + 1);
+    count_launch(eb != ea ? 2 : 1);
     if (cudaMemcpyAsync(host, w, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream()) != cudaSuccess ||
         cudaStreamSynchronize(stream()) != cudaSuccess) {
         return false;   // the routine's own synchronisation reports the error
     }
     wa = host[0];
-    wb = host[1];
+    wb = eb != ea ? host[1] : wa;
     return true;
 }
 
@@ -2305,8 +2305,9 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
     }
     const int nc = cplx ? 3 : 1;
     // Real SYRK (op(B) = op(A)^T on the same array): op(B)'s residue rows are
-    // op(A)'s, so one conversion serves both operands; both then use the same
-    // per-modulus row padding.
+    // op(A)'s, so one exponent scan and one conversion serve both operands; both
+    // then use the same per-modulus row padding. (n = 8192, k = 2048: a scan is
+    // 70 us of 3900.)
     const bool shared_ops = !cplx && g.uplo != 0 && g.A == g.B && g.lda == g.ldb && g.ta != g.tb && m == n;
     const int64_t Np = (n + TC_BN - 1) / TC_BN * TC_BN;
     const int64_t Mp = shared_ops ? Np : (m + 255) / 256 * 256;   // the pair kernel's 256-row tiles
@@ -2339,8 +2340,9 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
                         (double)m * (double)n * (double)k >= kWidthMinWork;
     int *ex = (int *)dev_alloc(sizeof(int) * (size_t)(detect ? 2 * (m + n) + 4 : m + n + 2), routine);
     if (!ex) return false;
-    int *ea = ex, *eb = ex + m;
-    int *la = detect ? ex + m + n : nullptr, *lb = detect ? la + m : nullptr, *wbuf = detect ? lb + n : nullptr;
+    int *ea = ex, *eb = shared_ops ? ea : ex + m;
+    int *la = detect ? ex + m + n : nullptr, *lb = detect && !shared_ops ? la + m : la;
+    int *wbuf = detect ? la + m + n : nullptr;
     // Operands still arriving from the host: A's exponents and residues are
     // computed while B is copied, and C is waited for only by the
     // reconstruction, so its copy runs under the residue GEMMs.
@@ -2352,7 +2354,7 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
         return false;
     }
     if (!a_blocks) launch_exp_rows_of_op(g.A, g.ta ? k : m, g.ta ? m : k, g.lda, g.ta, E, ea, la);
-    if (!hs) launch_exp_cols_of_op(g.B, g.tb ? n : k, g.tb ? k : n, g.ldb, g.tb, E, eb, lb);
+    if (!hs && !shared_ops) launch_exp_cols_of_op(g.B, g.tb ? n : k, g.tb ? k : n, g.ldb, g.tb, E, eb, lb);
 
     // 2. precision and moduli. Rows of op(A) are scaled to bits_a bits and
     // columns of op(B) to bits_b: by default the 106 bits of a double-double,
@@ -2370,7 +2372,6 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             bits_b = std::max(8, std::min(bits, wb));
         }
     }
-    if (shared_ops) bits_a = bits_b = std::max(bits_a, bits_b);   // one conversion serves both operands
     const double need = (bits_a - 1) + (bits_b - 1) + std::log2((double)(k > 1 ? k : 1)) + 1.0 + 4.0 + (cplx ? 1.0 : 0.0);
     Moduli md = choose_moduli(need);
     g_last_moduli = md.n;
@@ -2460,7 +2461,7 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
     if (!blocked) {
         if (hs) {
             wait_event(hs->b_ready, routine);
-            exp_B(0, n);
+            if (!shared_ops) exp_B(0, n);
         }
         if (!shared_ops) convert_B(0, n, Np);
     }
