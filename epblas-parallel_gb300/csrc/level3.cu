@@ -105,13 +105,14 @@ __global__ void k_trsm_diag_right(int64_t c0, int nb, int64_t nrows, const doubl
 // fixed order (lanes 0 + 2, 1 + 3, then the two), rounded once; each row is
 // then multiplied by the double-double reciprocal of the diagonal, as the
 // reference's substitution does (mtrsm_serial.cpp:144).
-// Inv: block b at Inv + b*32*32, column-major with leading dimension 32.
+// Inv: the diagonal of order-nb blocks, block b at Inv + b*nb*nb, column-major with
+// leading dimension nb; the rest of each block is zero already.
 constexpr int kInvNB = 32;   // order of the directly inverted blocks (merged up to the leaf order)
 constexpr int kInvSplit = 4;  // threads per column
 
 __global__ void __launch_bounds__(kInvNB * kInvSplit) k_trsm_diag_inv(int64_t na, const double2 *__restrict__ A,
                                                                       int64_t lda, bool trans, bool lower, bool unit,
-                                                                      double2 *Inv)
+                                                                      double2 *Inv, int nbinv)
 {
     extern __shared__ fx::OpPod smem_inv[];
     fx::OpPod *sA = smem_inv;                    // [p][r]: sA[p * 32 + r] = -op(A)(o + r, o + p)
@@ -135,7 +136,8 @@ __global__ void __launch_bounds__(kInvNB * kInvSplit) k_trsm_diag_inv(int64_t na
     const int c = threadIdx.x / kInvSplit, part = threadIdx.x % kInvSplit;
     const bool active = c < nb;   // every lane stays for the shuffles
     const fx::Op one = fx::decode(make_double2(1.0, 0.0));
-    double2 *out = Inv + (int64_t)blockIdx.x * kInvNB * kInvNB + (int64_t)c * kInvNB;
+    const int64_t od = o % nbinv;   // the block's place in its order-nbinv block
+    double2 *out = Inv + (o - od) * nbinv + od + (od + c) * nbinv;
     for (int s = 0; s < nb; ++s) {
         const int r = lower ? s : nb - 1 - s;
         fx::Acc acc;
@@ -224,15 +226,17 @@ namespace {
 
 constexpr int64_t kTrsmLeaf = 64;
 
-// B[:, :] -= op(A)-block * X (side L) or X * op(A)-block (side R) through the
-// engine dispatch.
+bool is_one(dd_host v) { return v.hi == 1.0 && v.lo == 0.0; }
+
+// B[:, :] = alpha * B - op(A)-block * X (side L) or - X * op(A)-block (side R)
+// through the engine dispatch.
 bool trsm_update(bool left, int64_t m, int64_t n, int64_t k, const void *Ablk, int64_t lda, bool ta,
-                 const void *X, int64_t ldx, void *C, int64_t ldc, const char *routine)
+                 const void *X, int64_t ldx, dd_host alpha, void *C, int64_t ldc, const char *routine)
 {
     GemmArgs g;
     g.alpha = dd_host{-1.0, 0.0};
-    g.beta = dd_host{1.0, 0.0};
-    g.beta_kind = 1;
+    g.beta = alpha;
+    g.beta_kind = is_one(alpha) ? 1 : 2;
     g.m = m;
     g.n = n;
     g.k = k;
@@ -251,19 +255,19 @@ bool trsm_update(bool left, int64_t m, int64_t n, int64_t k, const void *Ablk, i
 // Recursive substitution on the na x na triangle of op(A) starting at (o, o).
 // Side L: B is na x nrhs (rows o..o+na of the caller's B). Side R: B is
 // nrhs x na (columns o..o+na). lower refers to op(A).
-// Leaf by explicit block inverse: X_blk = Inv_blk * B_blk (side L) or
-// B_blk * Inv_blk (side R) as one GEMM into T, copied back into B.
+// Leaf by explicit block inverse: X_blk = alpha * Inv_blk * B_blk (side L) or
+// alpha * B_blk * Inv_blk (side R) as one GEMM into T, copied back into B.
 struct TrsmInv {
     const double2 *inv = nullptr;   // inverses of the leaf diagonal blocks, block b at inv + b*nb*nb (ld nb)
     int64_t nb = kTrsmLeaf;         // leaf (and inverse block) order
     double2 *T = nullptr;           // nb x nrhs (or nrhs x nb) scratch
 };
 
-bool trsm_leaf_inv(bool left, int64_t o, int64_t na, int64_t nrhs, const TrsmInv &w, double2 *B, int64_t ldb,
-                   const char *routine)
+bool trsm_leaf_inv(bool left, int64_t o, int64_t na, int64_t nrhs, const TrsmInv &w, dd_host alpha, double2 *B,
+                   int64_t ldb, const char *routine)
 {
     GemmArgs g;
-    g.alpha = dd_host{1.0, 0.0};
+    g.alpha = alpha;
     g.beta = dd_host{0.0, 0.0};
     g.beta_kind = 0;
     const double2 *blk = w.inv + (o / w.nb) * w.nb * w.nb;
@@ -286,11 +290,13 @@ bool trsm_leaf_inv(bool left, int64_t o, int64_t na, int64_t nrhs, const TrsmInv
     return cuda_ok(st, routine, "trsm leaf copy");
 }
 
-bool trsm_rec(bool left, bool lower, bool trans, bool unit, int64_t o, int64_t na, int64_t nrhs, const void *A,
-              int64_t lda, double2 *B, int64_t ldb, const TrsmInv &w, const char *routine)
+// alpha scales B where it is first read: in the first solve below and in the
+// update's beta (1 where the leaves substitute, which do not scale).
+bool trsm_rec(bool left, bool lower, bool trans, bool unit, int64_t o, int64_t na, int64_t nrhs, dd_host alpha,
+              const void *A, int64_t lda, double2 *B, int64_t ldb, const TrsmInv &w, const char *routine)
 {
     const int64_t leaf = w.inv ? w.nb : kTrsmLeaf;
-    if (na <= leaf && w.inv) return trsm_leaf_inv(left, o, na, nrhs, w, B, ldb, routine);
+    if (na <= leaf && w.inv) return trsm_leaf_inv(left, o, na, nrhs, w, alpha, B, ldb, routine);
     if (na <= leaf) {
         if (left)
             k_trsm_diag_left<<<blocks_for(nrhs, 64), 64, 0, stream()>>>(o, (int)na, nrhs, (const double2 *)A, lda,
@@ -303,80 +309,56 @@ bool trsm_rec(bool left, bool lower, bool trans, bool unit, int64_t o, int64_t n
     }
     int64_t h = (na / 2 + leaf - 1) / leaf * leaf;
     if (h >= na) h = na - leaf;
+    const dd_host one{1.0, 0.0};
     const int64_t o1 = o, n1 = h, o2 = o + h, n2 = na - h;
     if (left) {
         // rows of B: first block B1 = rows o1.., second B2 = rows o2..
         if (lower) {
-            if (!trsm_rec(true, lower, trans, unit, o1, n1, nrhs, A, lda, B, ldb, w, routine)) return false;
-            // B2 -= op(A)[o2:, o1:o1+n1] * X1
-            if (!trsm_update(true, n2, nrhs, n1, op_block(A, lda, trans, o2, o1), lda, trans, B + o1, ldb, B + o2,
-                             ldb, routine))
+            if (!trsm_rec(true, lower, trans, unit, o1, n1, nrhs, alpha, A, lda, B, ldb, w, routine)) return false;
+            // B2 = alpha B2 - op(A)[o2:, o1:o1+n1] * X1
+            if (!trsm_update(true, n2, nrhs, n1, op_block(A, lda, trans, o2, o1), lda, trans, B + o1, ldb, alpha,
+                             B + o2, ldb, routine))
                 return false;
-            return trsm_rec(true, lower, trans, unit, o2, n2, nrhs, A, lda, B, ldb, w, routine);
+            return trsm_rec(true, lower, trans, unit, o2, n2, nrhs, one, A, lda, B, ldb, w, routine);
         }
-        if (!trsm_rec(true, lower, trans, unit, o2, n2, nrhs, A, lda, B, ldb, w, routine)) return false;
-        // B1 -= op(A)[o1:o1+n1, o2:] * X2
-        if (!trsm_update(true, n1, nrhs, n2, op_block(A, lda, trans, o1, o2), lda, trans, B + o2, ldb, B + o1, ldb,
-                         routine))
+        if (!trsm_rec(true, lower, trans, unit, o2, n2, nrhs, alpha, A, lda, B, ldb, w, routine)) return false;
+        // B1 = alpha B1 - op(A)[o1:o1+n1, o2:] * X2
+        if (!trsm_update(true, n1, nrhs, n2, op_block(A, lda, trans, o1, o2), lda, trans, B + o2, ldb, alpha,
+                         B + o1, ldb, routine))
             return false;
-        return trsm_rec(true, lower, trans, unit, o1, n1, nrhs, A, lda, B, ldb, w, routine);
+        return trsm_rec(true, lower, trans, unit, o1, n1, nrhs, one, A, lda, B, ldb, w, routine);
     }
     // side R: columns of B; op(A) upper -> left block first
     const bool upper = !lower;
     if (upper) {
-        if (!trsm_rec(false, lower, trans, unit, o1, n1, nrhs, A, lda, B, ldb, w, routine)) return false;
-        // B2 -= X1 * op(A)[o1:o1+n1, o2:]
-        if (!trsm_update(false, nrhs, n2, n1, op_block(A, lda, trans, o1, o2), lda, trans, B + o1 * ldb, ldb,
+        if (!trsm_rec(false, lower, trans, unit, o1, n1, nrhs, alpha, A, lda, B, ldb, w, routine)) return false;
+        // B2 = alpha B2 - X1 * op(A)[o1:o1+n1, o2:]
+        if (!trsm_update(false, nrhs, n2, n1, op_block(A, lda, trans, o1, o2), lda, trans, B + o1 * ldb, ldb, alpha,
                          B + o2 * ldb, ldb, routine))
             return false;
-        return trsm_rec(false, lower, trans, unit, o2, n2, nrhs, A, lda, B, ldb, w, routine);
+        return trsm_rec(false, lower, trans, unit, o2, n2, nrhs, one, A, lda, B, ldb, w, routine);
     }
-    if (!trsm_rec(false, lower, trans, unit, o2, n2, nrhs, A, lda, B, ldb, w, routine)) return false;
-    // B1 -= X2 * op(A)[o2:, o1:o1+n1]
-    if (!trsm_update(false, nrhs, n1, n2, op_block(A, lda, trans, o2, o1), lda, trans, B + o2 * ldb, ldb,
+    if (!trsm_rec(false, lower, trans, unit, o2, n2, nrhs, alpha, A, lda, B, ldb, w, routine)) return false;
+    // B1 = alpha B1 - X2 * op(A)[o2:, o1:o1+n1]
+    if (!trsm_update(false, nrhs, n1, n2, op_block(A, lda, trans, o2, o1), lda, trans, B + o2 * ldb, ldb, alpha,
                      B + o1 * ldb, ldb, routine))
         return false;
-    return trsm_rec(false, lower, trans, unit, o1, n1, nrhs, A, lda, B, ldb, w, routine);
-}
-
-// Copies the two half-block inverses into the diagonal of each merged block
-// and zeroes its off-diagonal triangle (upper right for lower, lower left for
-// upper). CTAs (merged block, 32-column group).
-__global__ void k_inv_merge_copy(int64_t na, int64_t S, const double2 *__restrict__ src, double2 *__restrict__ dst,
-                                 bool lower)
-{
-    const int64_t h = S / 2;
-    const int64_t o = (int64_t)blockIdx.x * S;
-    const int64_t n1 = min(h, na - o), n2 = max((int64_t)0, min(h, na - o - h));
-    const double2 *i1 = src + (2 * blockIdx.x) * h * h;
-    const double2 *i2 = src + (2 * blockIdx.x + 1) * h * h;
-    double2 *d = dst + (int64_t)blockIdx.x * S * S;
-    const int nt = (int)(n1 + n2), n1i = (int)n1, hi = (int)h, Si = (int)S;
-    // column per warp-strided loop, rows across the threads of a warp (coalesced)
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int cend = min(nt, (int)(blockIdx.y + 1) * 32);
-    for (int c = (int)blockIdx.y * 32 + wid; c < cend; c += nw) {
-        for (int r = lane; r < nt; r += 32) {
-            double2 v = make_double2(0.0, 0.0);
-            if (r < n1i && c < n1i) v = i1[r + c * hi];
-            else if (r >= n1i && c >= n1i) v = i2[(r - n1i) + (c - n1i) * hi];
-            d[r + c * Si] = v;   // the off-diagonal block is then written by the GEMMs
-        }
-    }
-    (void)lower;
+    return trsm_rec(false, lower, trans, unit, o1, n1, nrhs, one, A, lda, B, ldb, w, routine);
 }
 
 // Doubles the order of the diagonal-block inverses from h to 2h:
 //   lower: inv [L11 0; L21 L22] = [I1 0; -I2 L21 I1  I2]
 //   upper: inv [U11 U12; 0 U22] = [I1 -I1 U12 I2; 0  I2]
-// with two grouped GEMMs over all merged blocks.
-bool trsm_merge_inverses(int64_t na, int64_t h, const void *A, int64_t lda, bool trans, bool lower,
-                         const double2 *src, double2 *dst, double2 *tmp, const char *routine)
+// with two grouped GEMMs over all merged blocks. inv holds the order-nb blocks
+// the inverses grow in (block b at inv + b*nb*nb, leading dimension nb): every
+// level leaves I1 and I2 where they are and writes the block between them, and
+// the other triangle stays zero. Copying the halves into a second buffer of
+// twice the order at each level took 83 us for na = 4096, nb = 1024.
+bool trsm_merge_inverses(int64_t na, int64_t h, const void *A, int64_t lda, bool trans, bool lower, double2 *inv,
+                         int64_t nb, double2 *tmp, const char *routine)
 {
     const int64_t S = 2 * h;
     const int64_t nblk = (na + S - 1) / S;
-    k_inv_merge_copy<<<dim3((unsigned)nblk, (unsigned)((S + 31) / 32)), 256, 0, stream()>>>(na, S, src, dst, lower);
-    count_launch();
     std::vector<int64_t> m1, n1, k1, lda1, ldb1, ldc1, m2, n2, k2, lda2, ldb2, ldc2;
     std::vector<const mwblas_real64x2 *> a1, b1, a2, b2;
     std::vector<mwblas_real64x2 *> c1, c2;
@@ -385,33 +367,34 @@ bool trsm_merge_inverses(int64_t na, int64_t h, const void *A, int64_t lda, bool
         const int64_t o = b * S;
         const int64_t p1 = std::min(h, na - o), p2 = std::max((int64_t)0, std::min(h, na - o - h));
         if (p2 == 0) continue;
-        const double2 *I1 = src + (2 * b) * h * h, *I2 = src + (2 * b + 1) * h * h;
+        const int64_t od = o % nb;
+        double2 *D = inv + (o - od) * nb + od + od * nb;   // the merged block's first element
+        const double2 *I1 = D, *I2 = D + h + h * nb;
         double2 *T = tmp + b * h * h;
-        double2 *D = dst + b * S * S;
         if (lower) {
             // T = L21 * I1 (p2 x p1), off = -(I2 * T) into D[p1:, 0:p1]
             t1a.push_back(trans ? 'T' : 'N'); t1b.push_back('N');
             m1.push_back(p2); n1.push_back(p1); k1.push_back(p1);
             a1.push_back((const mwblas_real64x2 *)op_block(A, lda, trans, o + p1, o)); lda1.push_back(lda);
-            b1.push_back((const mwblas_real64x2 *)I1); ldb1.push_back(h);
+            b1.push_back((const mwblas_real64x2 *)I1); ldb1.push_back(nb);
             c1.push_back((mwblas_real64x2 *)T); ldc1.push_back(h);
             t2a.push_back('N'); t2b.push_back('N');
             m2.push_back(p2); n2.push_back(p1); k2.push_back(p2);
-            a2.push_back((const mwblas_real64x2 *)I2); lda2.push_back(h);
+            a2.push_back((const mwblas_real64x2 *)I2); lda2.push_back(nb);
             b2.push_back((const mwblas_real64x2 *)T); ldb2.push_back(h);
-            c2.push_back((mwblas_real64x2 *)(D + p1)); ldc2.push_back(S);
+            c2.push_back((mwblas_real64x2 *)(D + p1)); ldc2.push_back(nb);
         } else {
             // T = U12 * I2 (p1 x p2), off = -(I1 * T) into D[0:p1, p1:]
             t1a.push_back(trans ? 'T' : 'N'); t1b.push_back('N');
             m1.push_back(p1); n1.push_back(p2); k1.push_back(p2);
             a1.push_back((const mwblas_real64x2 *)op_block(A, lda, trans, o, o + p1)); lda1.push_back(lda);
-            b1.push_back((const mwblas_real64x2 *)I2); ldb1.push_back(h);
+            b1.push_back((const mwblas_real64x2 *)I2); ldb1.push_back(nb);
             c1.push_back((mwblas_real64x2 *)T); ldc1.push_back(h);
             t2a.push_back('N'); t2b.push_back('N');
             m2.push_back(p1); n2.push_back(p2); k2.push_back(p1);
-            a2.push_back((const mwblas_real64x2 *)I1); lda2.push_back(h);
+            a2.push_back((const mwblas_real64x2 *)I1); lda2.push_back(nb);
             b2.push_back((const mwblas_real64x2 *)T); ldb2.push_back(h);
-            c2.push_back((mwblas_real64x2 *)(D + p1 * S)); ldc2.push_back(S);
+            c2.push_back((mwblas_real64x2 *)(D + p1 * nb)); ldc2.push_back(nb);
         }
     }
     const int64_t cnt = (int64_t)m1.size();
@@ -439,10 +422,6 @@ bool trsm_device(char side, char uplo, char transa, char diag, int64_t m, int64_
     // op(A) is lower triangular iff (uplo == 'L') xor transposed.
     bool lower = ((uplo == 'L') != trans);
     double2 *b = (double2 *)B;
-    if (!(alpha.hi == 1.0 && alpha.lo == 0.0)) {
-        k_scale_fast<<<blocks_for(m * n, 256), 256, 0, stream()>>>(m, n, dd::make(alpha.hi, alpha.lo), b, ldb);
-        count_launch();
-    }
     const bool left = (side == 'L');
     const int64_t na = left ? m : n, nrhs = left ? n : m;
     // Many right-hand sides, or a large triangle: invert the diagonal blocks
@@ -452,7 +431,17 @@ bool trsm_device(char side, char uplo, char transa, char diag, int64_t m, int64_
     TrsmInv w;
     void *scratch = nullptr;
     bool ok = true;
-    if (nrhs >= 2 * kTrsmLeaf || na >= 128) {
+    const bool use_inv = nrhs >= 2 * kTrsmLeaf || na >= 128;
+    // With inverses alpha goes into the GEMMs that first read B (a pass over B is
+    // 61 us for 4096 x 1024). An alpha far from one scales B itself first, as an
+    // Inf or NaN does: the products before it could leave the range of a double.
+    const bool fold = use_inv && std::fabs(alpha.hi) > 0x1p-64 && std::fabs(alpha.hi) < 0x1p64;
+    if (!fold && !is_one(alpha)) {
+        k_scale_fast<<<blocks_for(m * n, 256), 256, 0, stream()>>>(m, n, dd::make(alpha.hi, alpha.lo), b, ldb);
+        count_launch();
+        alpha = dd_host{1.0, 0.0};
+    }
+    if (use_inv) {
         // leaf order 64, or 256 when the right-hand sides make the leaf GEMMs
         // worth it or there are only a few of them; the 32 x 32 inverses are
         // doubled up to it by merging with grouped GEMMs
@@ -466,7 +455,6 @@ bool trsm_device(char side, char uplo, char transa, char diag, int64_t m, int64_
                                                                                     : kTrsmLeaf;
         const int64_t nblk64 = (na + kInvNB - 1) / kInvNB;
         const int64_t nblk = (na + nb - 1) / nb;
-        const size_t inv64_bytes = (size_t)nblk64 * kInvNB * kInvNB * sizeof(double2);
         const size_t inv_bytes = (size_t)nblk * nb * nb * sizeof(double2);
         const size_t t_bytes = (size_t)nb * nrhs * sizeof(double2);
         // the merges' products: ceil(na / 2h) blocks of h x h at each level h
@@ -474,27 +462,24 @@ bool trsm_device(char side, char uplo, char transa, char diag, int64_t m, int64_
         for (int64_t h = kInvNB; h < nb; h *= 2)
             m_elems = std::max(m_elems, (size_t)((na + 2 * h - 1) / (2 * h)) * h * h);
         const size_t m_bytes = (m_elems * sizeof(double2) + 255) / 256 * 256;
-        // [inverse buffer A][inverse buffer B][merge products][T]: merges ping-pong between A and B
-        const size_t buf_bytes = (std::max(inv64_bytes, inv_bytes) + 255) / 256 * 256;
-        scratch = dev_alloc(2 * buf_bytes + m_bytes + t_bytes, routine);
+        // [inverses][merge products][T]
+        const size_t buf_bytes = (inv_bytes + 255) / 256 * 256;
+        scratch = dev_alloc(buf_bytes + m_bytes + t_bytes, routine);
         if (!scratch) return false;
-        double2 *bufA = (double2 *)scratch, *bufB = (double2 *)((char *)scratch + buf_bytes);
-        double2 *mtmp = (double2 *)((char *)scratch + 2 * buf_bytes);
-        w.T = (double2 *)((char *)scratch + 2 * buf_bytes + m_bytes);
+        double2 *inv = (double2 *)scratch, *mtmp = (double2 *)((char *)scratch + buf_bytes);
+        w.T = (double2 *)((char *)scratch + buf_bytes + m_bytes);
+        ok = cuda_ok(cudaMemsetAsync(inv, 0, inv_bytes, stream()), routine, "trsm inverse memset");
         const size_t smem = 2 * (size_t)kInvNB * kInvNB * sizeof(fx::OpPod);
         cudaFuncSetAttribute(k_trsm_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_trsm_diag_inv<<<(unsigned)nblk64, kInvNB * kInvSplit, smem, stream()>>>(na, (const double2 *)A, lda, trans, lower,
-                                                                     unit, bufA);
+                                                                     unit, inv, (int)nb);
         count_launch();
-        double2 *cur = bufA, *nxt = bufB;
-        for (int64_t h = kInvNB; h < nb && ok; h *= 2) {
-                ok = trsm_merge_inverses(na, h, A, lda, trans, lower, cur, nxt, mtmp, routine);
-            std::swap(cur, nxt);
-        }
-        w.inv = cur;
+        for (int64_t h = kInvNB; h < nb && ok; h *= 2)
+            ok = trsm_merge_inverses(na, h, A, lda, trans, lower, inv, nb, mtmp, routine);
+        w.inv = inv;
         w.nb = nb;
     }
-    if (ok) ok = trsm_rec(left, lower, trans, unit, 0, na, nrhs, A, lda, b, ldb, w, routine);
+    if (ok) ok = trsm_rec(left, lower, trans, unit, 0, na, nrhs, alpha, A, lda, b, ldb, w, routine);
     if (scratch) dev_free(scratch);
     return ok;
 }
