@@ -1307,19 +1307,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
     const int nsteps = (int)(Kp / TC_BK);
     const int kcs = kChunk / TC_BK;
     const int nch = (nsteps + kcs - 1) / kcs;
-    const int64_t units = (int64_t)nz * tiles_m2 * tiles_n;
-    auto unit_at = [&](int64_t u, int &tn, int &tm2, int &l) -> bool {
-        tn = tn0 + (int)(u % tiles_n);             // column tiles [tn0, tn0 + tiles_n)
-        tm2 = tm0 + (int)((u / tiles_n) % tiles_m2);   // row tile pairs [tm0, tm0 + tiles_m2)
-        l = (int)(u / ((int64_t)tiles_n * tiles_m2));
-        const int64_t i0 = (int64_t)tm2 * 256, j0 = (int64_t)tn * TC_BN;
-        return !((uplo == 1 && i0 > j0 + TC_BN - 1) || (uplo == 2 && i0 + 255 < j0));
+    // Units of one modulus: every tile, or a triangle's stored ones (m = n then),
+    // the longer index in the outer loop. Skipping the others in a walk over all
+    // tiles left the clusters with 175 to 213 units each of a triangle of 8192
+    // (k = 2048: 2509 us, now 2122).
+    const int64_t per = uplo ? (int64_t)tiles_n * (tiles_n + 1) / 2 : (int64_t)tiles_m2 * tiles_n;
+    const int64_t units = nz * per;
+    auto unit_at = [&](int64_t u, int &tn, int &tm2, int &l) {
+        l = (int)(u / per);
+        const int64_t t = u - l * per;
+        if (uplo) {
+            int64_t r = (int64_t)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+            while (r * (r + 1) / 2 > t) --r;
+            while ((r + 1) * (r + 2) / 2 <= t) ++r;
+            const int c = (int)(t - r * (r + 1) / 2);
+            tn = uplo == 1 ? (int)r : c;
+            tm2 = uplo == 1 ? c : (int)r;
+            return;
+        }
+        tm2 = (int)(t / tiles_n);
+        tn = tn0 + (int)(t - (int64_t)tm2 * tiles_n);   // column tiles [tn0, tn0 + tiles_n)
+        tm2 += tm0;                                     // row tile pairs [tm0, tm0 + tiles_m2)
     };
-    auto next_unit = [&](int64_t u) -> int64_t {
-        int tn, tm2, l;
-        while (u < units && !unit_at(u, tn, tm2, l)) u += ncl;
-        return u < units ? u : units;
-    };
+    auto next_unit = [&](int64_t u) -> int64_t { return u < units ? u : units; };
 
     if (warp == 0 && lane == 0) {
         for (int st = 0; st < T2_STAGES; ++st) {
@@ -1725,37 +1735,6 @@ __device__ __forceinline__ bool finite_hi(double x)
     return ((__double2hiint(x) >> 20) & 0x7FF) != 0x7FF;   // exponent field test, no FP64 compare
 }
 
-// Triangular outputs (uplo 1: i <= j, 2: i >= j) are walked as a list of
-// (row slab x, column j) tasks holding stored entries: slab x (rows
-// [S x, S x + S)) needs columns [S x, n) of an upper triangle and
-// [0, min(n, S x + S)) of a lower one. The blocks of a grid stride over that
-// list, so every block gets about the same share of the triangle (a slab per
-// block and all columns would leave the top slabs of an upper triangle with
-// 16 times the work of the bottom ones at n = 8192).
-__device__ __forceinline__ int64_t tri_prefix(int uplo, int64_t x, int64_t n, int64_t S)
-{
-    if (uplo == 1) {   // sum over x' < x of n - min(n, S x')
-        const int64_t q = min(x, (n + S - 1) / S);
-        return q * n - S * q * (q - 1) / 2;
-    }
-    const int64_t qf = n / S;   // sum over x' < x of min(n, S (x' + 1)); the first qf terms are S (x' + 1)
-    const int64_t q = min(x, qf);
-    return S * q * (q + 1) / 2 + max((int64_t)0, x - qf) * n;
-}
-
-__device__ __forceinline__ void tri_task(int uplo, int64_t t, int64_t slabs, int64_t n, int64_t S, int64_t &x,
-                                         int64_t &j)
-{
-    int64_t lo = 0, hi = slabs - 1;   // the first slab whose tasks extend past t
-    while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (tri_prefix(uplo, mid + 1, n, S) > t) hi = mid;
-        else lo = mid + 1;
-    }
-    x = lo;
-    j = t - tri_prefix(uplo, x, n, S) + (uplo == 1 ? min(n, S * x) : 0);
-}
-
 // alpha M as four mantissa words at one exponent: for complex alpha both parts
 // (the smaller cut at 2^-128 of the larger).
 struct RecScale {
@@ -1838,40 +1817,52 @@ __device__ __forceinline__ void reconstruct_one(uint32_t x[crt::kFL], int eai, i
 }
 
 // The (64-row slab of this warp, column) turns of a reconstruction. Full
-// output: the warp's own rows, columns blockIdx.y, + gridDim.y, ..; triangle:
-// the block's share of the task list, without the tasks whose rows of this warp
-// hold no stored entry.
+// output: the warp's own rows, columns blockIdx.y, + gridDim.y, .. Triangle
+// (uplo 1: i <= j, 2: i >= j): the blocks of the grid stride over the list of
+// (row slab x, column) tasks with stored entries, so that every block gets about
+// the same share: slab x (rows [S x, S x + S)) needs columns [S x, n) of an upper
+// triangle and [0, min(n, S x + S)) of a lower one. A block steps from slab to
+// slab as its tasks pass their ends (a search of the prefix sums for every task,
+// with its 64-bit divisions, took a fifth of the kernel); a warp skips tasks
+// whose rows of its own hold no stored entry.
 struct RecTurns {
-    int m, n, uplo, j;
-    int64_t i0, t, total, slabs, S, step;
+    int m, n, uplo, j, S, step;
+    int64_t i0, x, t;   // slab and task within it
     // S rows per block (blockDim.x / 32 warps of 64)
     __device__ __forceinline__ void begin(int m_, int n_, int uplo_)
     {
         m = m_;
         n = n_;
         uplo = uplo_;
-        S = 2 * (int64_t)blockDim.x;
+        S = 2 * (int)blockDim.x;
         if (uplo == 0) {
-            i0 = blockIdx.x * S + (threadIdx.x >> 5) * RC_ROWS;
+            i0 = (int64_t)blockIdx.x * S + (threadIdx.x >> 5) * RC_ROWS;
             j = i0 < m ? (int)blockIdx.y : n;
             return;
         }
-        slabs = (m + S - 1) / S;
-        total = tri_prefix(uplo, slabs, n, S);
-        t = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
-        step = (int64_t)gridDim.x * gridDim.y;
+        step = (int)(gridDim.x * gridDim.y);
+        x = 0;
+        t = (int)(blockIdx.y * gridDim.x + blockIdx.x);
         find();
     }
     __device__ __forceinline__ void find()
     {
-        for (; t < total; t += step) {
-            int64_t x, jj;
-            tri_task(uplo, t, slabs, n, S, x, jj);
+        for (;; t += step) {
+            for (;;) {   // the slab of task t
+                const int64_t r = x * S;
+                if (r >= m || (uplo == 1 && r >= n)) {
+                    j = n;
+                    return;
+                }
+                const int64_t tasks = uplo == 1 ? n - r : min((int64_t)n, r + S);
+                if (t < tasks) break;
+                t -= tasks;
+                ++x;
+            }
             i0 = x * S + (threadIdx.x >> 5) * RC_ROWS;
-            j = (int)jj;
-            if (i0 < m && (uplo == 1 ? i0 <= jj : i0 + RC_ROWS > jj)) return;
+            j = (int)(uplo == 1 ? x * S + t : t);
+            if (i0 < m && (uplo == 1 ? i0 <= j : i0 + RC_ROWS > j)) return;
         }
-        j = n;
     }
     __device__ __forceinline__ bool more() const { return j < n; }
     __device__ __forceinline__ void next()
@@ -1893,7 +1884,7 @@ struct RecTurns {
 // Bound: instruction issue, 551 per output with a general beta (950 with the
 // sums as IMAD.WIDE and the update in extended floats; 830 with the sums on the
 // tensor cores alone). 4096^2: 0.62 -> 0.36 ms; the triangle of 8192^2: 1.44 ->
-// 0.90 ms; 1531 x 1277: 83 -> 58 us.
+// 0.76 ms; 1531 x 1277: 83 -> 58 us.
 template <int KS>
 __global__ void __launch_bounds__(256) k_oz_reconstruct(int m, int n, const uint16_t *__restrict__ R,
                                                         int64_t Mp, int64_t Np, const int *__restrict__ ea,
@@ -2476,7 +2467,7 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
     auto pair_gemm = [&](int tn0, int ntn, int tm0 = 0, int ntm = 0) {
         cudaFuncSetAttribute(k_oz_gemm_tc_2sm, cudaFuncAttributeMaxDynamicSharedMemorySize, T2_SMEM);
         const int tiles_m2 = ntm > 0 ? ntm : (int)(Mp / 256);
-        const int64_t units = (int64_t)nz * tiles_m2 * ntn;
+        const int64_t units = (int64_t)nz * (g.uplo ? (int64_t)ntn * (ntn + 1) / 2 : (int64_t)tiles_m2 * ntn);
         const int64_t pairs = device_sm_count() / 2;
         const unsigned grid = 2u * (unsigned)(units < pairs ? units : pairs);
         k_oz_gemm_tc_2sm<<<grid, TCP_THREADS, T2_SMEM, stream()>>>(ma, mb, Mp, Np, Kp, m, n, mp, R,
