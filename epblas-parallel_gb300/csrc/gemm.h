@@ -81,12 +81,18 @@ void launch_scale_matrix_c(int64_t m, int64_t n, cdd_host beta, int beta_kind, v
                            bool herm = false);
 
 // Exponent bounds of the rows / columns of op(X) (X column-major
-// rows_x x cols_x; elem2 = 1 real, 2 complex); with `low`, also the binary
-// exponent of the lowest set bit in each row / column (0x3f3f3f3f when it
-// holds no nonzero finite entry).
+// rows_x x cols_x; elem2 = 1 real, 2 complex).
 void launch_exp_rows_of_op(const void *X, int64_t rows_x, int64_t cols_x, int64_t ld, bool trans, int elem2,
-                           int *out, int *low = nullptr);
+                           int *out);
 void launch_exp_cols_of_op(const void *X, int64_t rows_x, int64_t cols_x, int64_t ld, bool trans, int elem2,
-                           int *out, int *low = nullptr);
+                           int *out);
+
+// Both operands of g over depth k (A and B: g's, or where a chunk of the depth
+// starts) in one launch: op(A)'s row bounds to ex, op(B)'s column bounds to eb
+// (null: not scanned), and with la and lb the negated exponent of the lowest set
+// bit in each row / column (-0x3f3f3f3f and below: no nonzero finite entry). All
+// of these lie in ex[0, count), which is set to bytes of 0x80 first.
+void launch_exp_operands(const GemmArgs &g, int64_t k, const void *A, const void *B, int elem2, int *ex,
+                         int64_t count, int *eb, int *la, int *lb);
 
 }  // namespace mw

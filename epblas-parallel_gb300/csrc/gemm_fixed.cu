@@ -412,8 +412,7 @@ bool gemm_fixed_real(const GemmArgs &g0, const char *routine)
         const double2 *A = (const double2 *)g.A + (g.ta ? k0 : k0 * g.lda);
         const double2 *B = (const double2 *)g.B + (g.tb ? k0 * g.ldb : k0);
         // exponent bounds of this chunk's rows of op(A) and columns of op(B)
-        launch_exp_rows_of_op(A, g.ta ? kc : g.m, g.ta ? g.m : kc, g.lda, g.ta, 1, ea);
-        launch_exp_cols_of_op(B, g.tb ? g.n : kc, g.tb ? kc : g.n, g.ldb, g.tb, 1, eb);
+        launch_exp_operands(g, kc, A, B, 1, ex, g.m + g.n, eb, nullptr, nullptr);
         const dd::real be = (k0 == 0) ? dd::make(g.beta.hi, g.beta.lo) : dd::make(1.0, 0.0);
         const int bk = (k0 == 0) ? g.beta_kind : 1;
 #define MW_FX(TA, TB)                                                                                         \

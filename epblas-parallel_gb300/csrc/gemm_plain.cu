@@ -49,16 +49,15 @@ constexpr int kNoExp = -30000;   // row/column with no nonzero entry
 __device__ __forceinline__ int exp_bound(double x)
 {
     // |x| < 2^(e+1) with e = biased exponent - 1023 (subnormals use -1023).
-    uint64_t b = (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull;
-    if (b == 0) return kNoExp;
-    return (int)(b >> 52) - 1023;
+    const uint32_t w1 = (uint32_t)__double2hiint(x) & 0x7fffffffu, w0 = (uint32_t)__double2loint(x);
+    return (w1 | w0) == 0 ? kNoExp : (int)(w1 >> 20) - 1023;
 }
 
 // Binary exponent of the lowest set bit of the double-double value hi + lo
 // (kLowNone for zero). With |lo| <= ulp(hi)/2, lo's lowest bit lies below
 // hi's, so it is lo's when lo != 0. Non-finite values give kLowNone too (their
 // rows are NaN in the output whatever the width).
-constexpr int kLowNone = 0x3f3f3f3f;   // also the byte-wise memset value below
+constexpr int kLowNone = 0x3f3f3f3f;
 // A row holding one entry that alone spans >= 104 bits (hi's top bit to lo's
 // lowest) needs the full width whatever the rest holds: its low bound is set
 // to this, and its remaining entries are not examined.
@@ -78,79 +77,86 @@ __device__ __forceinline__ int low_bit(double2 v)
     return (bx ? (int)bx : 1) - 1075 + tz;
 }
 
-// Row exponent bound of a column-major matrix M (rows x cols, ld): out[i] =
-// max over j of exp_bound(M[i + j*ld].hi); with `low`, also low[i] = min over
-// j of low_bit(M[i + j*ld]). Thread per row, grid.y splits the columns;
-// combined with atomicMax / atomicMin.
-__global__ void k_exp_rows(int64_t rows, int64_t cols, const double2 *M, int64_t ld, int elem2, int *out,
-                           int64_t cols_per_y, int *low)
+// The scan of one operand: exponent bounds of the rows of op(X) (X stored
+// column-major, rows x cols), and with `low` the exponent of the lowest set bit
+// in each, negated. Both are combined by atomicMax onto values preset to bytes
+// of 0x80, below any that occurs.
+struct ExpScan {
+    const double2 *X;
+    int64_t rows, cols, ld;
+    int *out, *low;
+    int by_cols;             // op(X)'s rows are X's columns
+    int64_t per;             // columns (rows of X, by_cols) per block in y
+    uint32_t bx, blocks;     // blocks in x, and in all
+};
+
+template <bool LOW> __device__ __forceinline__ void scan_entry(double2 v, int &e, int &lb)
 {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= rows) return;
-    int64_t j0 = blockIdx.y * cols_per_y;
-    int64_t j1 = min(cols, j0 + cols_per_y);
-    int e = kNoExp, lb = kLowNone;
-    if (low) {
-#pragma unroll 4
-        for (int64_t j = j0; j < j1; ++j) {
-            const double2 *p = M + elem2 * (i + j * ld);
-            for (int w = 0; w < elem2; ++w) {
-                const double2 v = p[w];
-                const int ev = exp_bound(v.x);
-                e = max(e, ev);
-                if (lb != kLowFull) {
-                    const int lv = low_bit(v);
-                    lb = (lv != kLowNone && ev - lv >= 104) ? kLowFull : min(lb, lv);
-                }
-            }
-        }
-        atomicMin(low + i, lb);
-    } else {
-#pragma unroll 8
-        for (int64_t j = j0; j < j1; ++j) {
-            const double2 *p = M + elem2 * (i + j * ld);
-            for (int w = 0; w < elem2; ++w) e = max(e, exp_bound(p[w].x));
-        }
+    const int ev = exp_bound(v.x);
+    e = max(e, ev);
+    if (LOW && lb != kLowFull) {
+        const int lv = low_bit(v);
+        lb = (lv != kLowNone && ev - lv >= 104) ? kLowFull : min(lb, lv);
     }
-    atomicMax(out + i, e);
 }
 
-// Column exponent bound: out[j] = max over i of exp_bound(M[i + j*ld].hi)
-// (and low[j] = min of low_bit). Warp per column (or per rows_per-long piece
-// of a column along grid.y, combined with atomics), lanes stride down the
-// contiguous column.
-__global__ void k_exp_cols(int64_t rows, int64_t cols, const double2 *M, int64_t ld, int elem2, int *out, int *low,
-                           int64_t rows_per)
+// Both operands of a product in one launch: A's blocks, then B's. By rows a
+// thread takes a row of X over `per` columns, by columns a warp takes a column
+// over `per` rows; eight 16-byte loads are in flight per thread either way.
+// Bound by HBM for large operands and by its own latency for small ones, where
+// two scans, their presets and two width kernels in turn took most of the time:
+// scan and widths of 1024^3 63 -> 45 us, 2048^3 102 -> 69, 8192^3 503 -> 343.
+template <int E, bool LOW> __global__ void __launch_bounds__(256) k_exp_scan(ExpScan a, ExpScan b)
 {
-    int64_t j = blockIdx.x * (int64_t)(blockDim.x / 32) + threadIdx.x / 32;
-    int lane = threadIdx.x & 31;
-    if (j >= cols) return;
+    const bool first = blockIdx.x < a.blocks;
+    const ExpScan &q = first ? a : b;
+    const uint32_t id = first ? blockIdx.x : blockIdx.x - a.blocks;
+    const uint32_t y = id / q.bx, x = id - y * q.bx;
+    constexpr int U = 8 / E;   // entries per batch
     int e = kNoExp, lb = kLowNone;
-    const int64_t i1 = min(rows, (int64_t)(blockIdx.y + 1) * rows_per);
-    for (int64_t i = (int64_t)blockIdx.y * rows_per + lane; i < i1; i += 32) {
-        const double2 *p = M + elem2 * (i + j * ld);
-        for (int w = 0; w < elem2; ++w) {
-            const double2 v = p[w];
-            const int ev = exp_bound(v.x);
-            e = max(e, ev);
-            if (low && lb != kLowFull) {
-                const int lv = low_bit(v);
-                lb = (lv != kLowNone && ev - lv >= 104) ? kLowFull : min(lb, lv);
-            }
+    if (!q.by_cols) {
+        const int64_t i = (int64_t)x * 256 + threadIdx.x;
+        if (i >= q.rows) return;
+        const int64_t j0 = y * q.per, j1 = min(q.cols, j0 + q.per), step = E * q.ld;
+        const double2 *p = q.X + E * i + j0 * step;
+        int64_t left = j1 - j0;
+        for (; left >= U; left -= U) {
+            double2 v[U * E];
+#pragma unroll
+            for (int u = 0; u < U; ++u, p += step)
+#pragma unroll
+                for (int w = 0; w < E; ++w) v[u * E + w] = p[w];
+#pragma unroll
+            for (int u = 0; u < U * E; ++u) scan_entry<LOW>(v[u], e, lb);
         }
+        for (; left > 0; --left, p += step)
+            for (int w = 0; w < E; ++w) scan_entry<LOW>(p[w], e, lb);
+        atomicMax(q.out + i, e);
+        if (LOW) atomicMax(q.low + i, -lb);
+        return;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        e = max(e, __shfl_down_sync(0xffffffffu, e, off));
-        lb = min(lb, __shfl_down_sync(0xffffffffu, lb, off));
+    const int64_t j = (int64_t)x * 8 + threadIdx.x / 32;
+    const int lane = threadIdx.x & 31;
+    if (j >= q.cols) return;
+    const int64_t i0 = y * q.per, i1 = min(q.rows, i0 + q.per);
+    const double2 *p = q.X + E * (i0 + lane + j * q.ld);
+    int64_t left = i1 - i0 - lane;   // entries from this lane's on
+    for (; left > 32 * (U - 1); left -= 32 * U, p += 32 * U * E) {
+        double2 v[U * E];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int w = 0; w < E; ++w) v[u * E + w] = p[32 * u * E + w];
+#pragma unroll
+        for (int u = 0; u < U * E; ++u) scan_entry<LOW>(v[u], e, lb);
     }
+    for (; left > 0; left -= 32, p += 32 * E)
+        for (int w = 0; w < E; ++w) scan_entry<LOW>(p[w], e, lb);
+    e = __reduce_max_sync(0xffffffffu, e);
+    lb = __reduce_min_sync(0xffffffffu, lb);
     if (lane == 0) {
-        if (gridDim.y == 1) {
-            out[j] = e;
-            if (low) low[j] = lb;
-        } else {
-            atomicMax(out + j, e);
-            if (low) atomicMin(low + j, lb);
-        }
+        atomicMax(q.out + j, e);
+        if (LOW) atomicMax(q.low + j, -lb);
     }
 }
 
@@ -863,48 +869,75 @@ void launch_plain_c_conj(const GemmArgs &g, const int *ea, const int *eb)
 
 }  // namespace
 
-// Row exponents of op(X) where X is stored column-major (rows_x x cols_x) and
-// op(X) = X (trans=false) or X^T (trans=true). Produces one int per row of
-// op(X), and with `low` the exponent of the lowest set bit in that row.
-void launch_exp_rows_of_op(const void *X, int64_t rows_x, int64_t cols_x, int64_t ld, bool trans, int elem2,
-                           int *out, int *low)
+namespace {
+
+// The scan of the rows of op(X), X stored column-major (rows x cols) and op(X) =
+// X or, trans, X^T; blocks enough to cover the GPU a few times.
+ExpScan exp_scan(const void *X, int64_t rows, int64_t cols, int64_t ld, bool trans, int *out, int *low)
 {
+    ExpScan q;
+    q.X = (const double2 *)X;
+    q.rows = rows;
+    q.cols = cols;
+    q.ld = ld;
+    q.out = out;
+    q.low = low;
+    q.by_cols = trans;
+    int64_t bx, ys;
     if (!trans) {
-        // rows of X: thread per row, column range split over grid.y
-        // enough (rows, column-range) blocks to cover the GPU a few times
-        const int64_t rb = (rows_x + 255) / 256;
-        int64_t want_y = (4 * (int64_t)device_sm_count() + rb - 1) / rb;
-        int64_t per_y = (cols_x + want_y - 1) / want_y;
-        if (per_y < 16) per_y = 16;
-        if ((cols_x + per_y - 1) / per_y > 65535) per_y = (cols_x + 65534) / 65535;
-        dim3 grid((unsigned)rb, (unsigned)((cols_x + per_y - 1) / per_y));
-        cudaMemsetAsync(out, 0x80, sizeof(int) * rows_x, stream());
-        if (low) cudaMemsetAsync(low, 0x3f, sizeof(int) * rows_x, stream());   // kLowNone
-        k_exp_rows<<<grid, 256, 0, stream()>>>(rows_x, cols_x, (const double2 *)X, ld, elem2, out, per_y, low);
+        bx = (rows + 255) / 256;
+        ys = std::max<int64_t>(1, std::min((8 * (int64_t)device_sm_count() + bx - 1) / bx, (cols + 15) / 16));
+        q.per = std::max<int64_t>(1, (cols + ys - 1) / ys);
+        ys = std::max<int64_t>(1, (cols + q.per - 1) / q.per);
     } else {
-        // rows of X^T = columns of X: a warp per column, long columns cut into
-        // pieces of at least 256 rows when there are too few columns to cover
-        // the GPU a few times
-        const int64_t want = 32 * (int64_t)device_sm_count();
-        int64_t ys = (want + cols_x - 1) / cols_x;
-        ys = std::min<int64_t>(ys, (rows_x + 255) / 256);
-        ys = std::max<int64_t>(1, std::min<int64_t>(ys, 65535));
-        const int64_t rows_per = (rows_x + ys - 1) / ys;
-        if (ys > 1) {
-            cudaMemsetAsync(out, 0x80, sizeof(int) * cols_x, stream());
-            if (low) cudaMemsetAsync(low, 0x3f, sizeof(int) * cols_x, stream());   // kLowNone
-        }
-        dim3 grid((unsigned)((cols_x + 7) / 8), (unsigned)ys);
-        k_exp_cols<<<grid, 256, 0, stream()>>>(rows_x, cols_x, (const double2 *)X, ld, elem2, out, low, rows_per);
+        bx = (cols + 7) / 8;
+        ys = std::max<int64_t>(1, std::min((32 * (int64_t)device_sm_count() + cols - 1) / cols, (rows + 255) / 256));
+        q.per = std::max<int64_t>(1, (rows + ys - 1) / ys);
+        ys = std::max<int64_t>(1, (rows + q.per - 1) / q.per);
+    }
+    q.bx = (uint32_t)bx;
+    q.blocks = (uint32_t)(bx * ys);
+    return q;
+}
+
+void launch_exp_scan(const ExpScan &a, const ExpScan &b, int elem2)
+{
+    const unsigned grid = a.blocks + b.blocks;
+    const bool low = a.low != nullptr;
+    if (elem2 == 1) {
+        if (low) k_exp_scan<1, true><<<grid, 256, 0, stream()>>>(a, b);
+        else k_exp_scan<1, false><<<grid, 256, 0, stream()>>>(a, b);
+    } else {
+        if (low) k_exp_scan<2, true><<<grid, 256, 0, stream()>>>(a, b);
+        else k_exp_scan<2, false><<<grid, 256, 0, stream()>>>(a, b);
     }
     count_launch();
 }
 
+}  // namespace
+
+void launch_exp_operands(const GemmArgs &g, int64_t k, const void *A, const void *B, int elem2, int *ex,
+                         int64_t count, int *eb, int *la, int *lb)
+{
+    cudaMemsetAsync(ex, 0x80, sizeof(int) * count, stream());
+    const ExpScan a = exp_scan(A, g.ta ? k : g.m, g.ta ? g.m : k, g.lda, g.ta, ex, la);
+    ExpScan b = {};
+    if (eb) b = exp_scan(B, g.tb ? g.n : k, g.tb ? k : g.n, g.ldb, !g.tb, eb, lb);
+    launch_exp_scan(a, b, elem2);
+}
+
+void launch_exp_rows_of_op(const void *X, int64_t rows_x, int64_t cols_x, int64_t ld, bool trans, int elem2,
+                           int *out)
+{
+    cudaMemsetAsync(out, 0x80, sizeof(int) * (trans ? cols_x : rows_x), stream());
+    launch_exp_scan(exp_scan(X, rows_x, cols_x, ld, trans, out, nullptr), ExpScan{}, elem2);
+}
+
 // Column exponents of op(X): columns of X^T are rows of X and vice versa.
 void launch_exp_cols_of_op(const void *X, int64_t rows_x, int64_t cols_x, int64_t ld, bool trans, int elem2,
-                           int *out, int *low)
+                           int *out)
 {
-    launch_exp_rows_of_op(X, rows_x, cols_x, ld, !trans, elem2, out, low);
+    launch_exp_rows_of_op(X, rows_x, cols_x, ld, !trans, elem2, out);
 }
 
 void launch_scale_matrix(int64_t m, int64_t n, dd_host beta, int beta_kind, void *C, int64_t ldc, int uplo)
@@ -924,10 +957,7 @@ bool gemm_plain_real(const GemmArgs &g, const char *routine)
     int *ex = (int *)dev_alloc(sizeof(int) * (size_t)(g.m + g.n), routine);
     if (!ex) return false;
     int *ea = ex, *eb = ex + g.m;
-    // op(A) is m x k: A stored (ta ? k x m : m x k)
-    launch_exp_rows_of_op(g.A, g.ta ? g.k : g.m, g.ta ? g.m : g.k, g.lda, g.ta, 1, ea);
-    // op(B) is k x n: B stored (tb ? n x k : k x n)
-    launch_exp_cols_of_op(g.B, g.tb ? g.n : g.k, g.tb ? g.k : g.n, g.ldb, g.tb, 1, eb);
+    launch_exp_operands(g, g.k, g.A, g.B, 1, ex, g.m + g.n, eb, nullptr, nullptr);
     int64_t tiles64 = ((g.m + 63) / 64) * ((g.n + 63) / 64);
     const bool big = tiles64 >= 2 * (int64_t)device_sm_count();
     // TMA staging wants 16-byte aligned operands (always true of device
@@ -978,8 +1008,7 @@ bool gemm_plain_cplx(const GemmArgs &g, const char *routine)
     int *ex = (int *)dev_alloc(sizeof(int) * (size_t)(g.m + g.n), routine);
     if (!ex) return false;
     int *ea = ex, *eb = ex + g.m;
-    launch_exp_rows_of_op(g.A, g.ta ? g.k : g.m, g.ta ? g.m : g.k, g.lda, g.ta, 2, ea);
-    launch_exp_cols_of_op(g.B, g.tb ? g.n : g.k, g.tb ? g.k : g.n, g.ldb, g.tb, 2, eb);
+    launch_exp_operands(g, g.k, g.A, g.B, 2, ex, g.m + g.n, eb, nullptr, nullptr);
     if (!g.ta && !g.tb) launch_plain_c_conj<false, false>(g, ea, eb);
     else if (!g.ta && g.tb) launch_plain_c_conj<false, true>(g, ea, eb);
     else if (g.ta && !g.tb) launch_plain_c_conj<true, false>(g, ea, eb);

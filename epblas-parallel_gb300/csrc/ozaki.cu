@@ -2218,23 +2218,28 @@ int ozaki_last_bits(int operand) { return (operand == 0 || operand == 1) ? g_las
 
 namespace {
 
-// Significant width of op(X)'s rows (or op(B)'s columns): the largest
+// Significant width of op(A)'s rows and op(B)'s columns: the largest
 // e_i - low_i + 2 over rows that hold a nonzero finite entry, where e_i bounds
-// the row's binary exponents and low_i is the exponent of its lowest set bit.
-// Scaled to that many bits (A'_ip = a_ip * 2^(bits - 2 - e_i)), every entry of
-// such a row is an exact integer below 2^(bits - 1).
-constexpr int kLowNone = 0x3f3f3f3f;   // no nonzero finite entry (the scan's fill value)
-__global__ void k_width(int64_t rows, const int *__restrict__ e, const int *__restrict__ low, int *out)
+// the row's binary exponents and low_i is the exponent of its lowest set bit
+// (nl holds -low_i). Scaled to that many bits (A'_ip = a_ip * 2^(bits - 2 -
+// e_i)), every entry of such a row is an exact integer below 2^(bits - 1).
+// Rows [0, m) are op(A)'s, [m, total) op(B)'s; out[0] and out[1], preset below 0.
+constexpr int kNegLowNone = -0x3f3f3f3f;   // no nonzero finite entry
+__global__ void k_width(int64_t m, int64_t total, const int *__restrict__ e, const int *__restrict__ nl, int *out)
 {
-    int w = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
-        const int ei = e[i], li = low[i];
-        if (ei > kNoExp / 2 && ei < 1024 && li != kLowNone) w = max(w, ei - li + 2);
+    int w[2] = {0, 0};
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int ei = e[i], li = nl[i];
+        const int v = ei > kNoExp / 2 && ei < 1024 && li > kNegLowNone ? ei + li + 2 : 0;
+        if (i < m) w[0] = max(w[0], v);
+        else w[1] = max(w[1], v);
     }
-    for (int off = 16; off > 0; off >>= 1) w = max(w, __shfl_down_sync(0xffffffffu, w, off));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, w);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int v = __reduce_max_sync(0xffffffffu, w[q]);
+        if ((threadIdx.x & 31) == 0) atomicMax(out + q, v);
+    }
 }
-
 
 // Products at least this large (m n k) on device-resident operands size their
 // moduli from the operands' significant width; the readback of the two widths
@@ -2242,10 +2247,10 @@ __global__ void k_width(int64_t rows, const int *__restrict__ e, const int *__re
 // 1 % of a 1024^3 product).
 constexpr double kWidthMinWork = 1024.0 * 1024.0 * 1024.0;
 
-// The significant widths of op(A)'s rows and op(B)'s columns, read back to the
-// host; false when they could not be (the caller then keeps the full width).
-bool read_widths(int64_t m, int64_t n, const int *ea, const int *eb, const int *la, const int *lb, int *w,
-                 int &wa, int &wb)
+// The significant widths of op(A)'s rows and op(B)'s columns (none of its own:
+// op(A)'s), read back to the host; false when they could not be (the caller then
+// keeps the full width).
+bool read_widths(int64_t m, int64_t n, const int *e, const int *nl, int *w, int &wa, int &wb)
 {
     thread_local int *host = nullptr;
     if (!host && cudaHostAlloc((void **)&host, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
@@ -2253,18 +2258,15 @@ bool read_widths(int64_t m, int64_t n, const int *ea, const int *eb, const int *
         host = nullptr;
         return false;
     }
-    cudaMemsetAsync(w, 0, 2 * sizeof(int), stream());
-    const int ga = (int)std::min<int64_t>((m + 255) / 256, 4 * (int64_t)device_sm_count());
-    const int gb = (int)std::min<int64_t>((n + 255) / 256, 4 * (int64_t)device_sm_count());
-    k_width<<<ga, 256, 0, stream()>>>(m, ea, la, w);
-    if (eb != ea) k_width<<<gb, 256, 0, stream()>>>(n, eb, lb, w + 1);
-    count_launch(eb != ea ? 2 : 1);
+    const int grid = (int)std::min<int64_t>((m + n + 255) / 256, 4 * (int64_t)device_sm_count());
+    k_width<<<grid, 256, 0, stream()>>>(m, m + n, e, nl, w);
+    count_launch();
     if (cudaMemcpyAsync(host, w, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream()) != cudaSuccess ||
         cudaStreamSynchronize(stream()) != cudaSuccess) {
         return false;   // the routine's own synchronisation reports the error
     }
     wa = host[0];
-    wb = eb != ea ? host[1] : wa;
+    wb = n > 0 ? host[1] : wa;
     return true;
 }
 
@@ -2329,11 +2331,12 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
     }
     const bool detect = bits_req <= 0 && g.width && !g.hs && cap == cudaStreamCaptureStatusNone &&
                         (double)m * (double)n * (double)k >= kWidthMinWork;
-    int *ex = (int *)dev_alloc(sizeof(int) * (size_t)(detect ? 2 * (m + n) + 4 : m + n + 2), routine);
+    // [op(A)'s bounds][op(B)'s][op(A)'s lowest bits][op(B)'s][the two widths]
+    const int64_t nb = shared_ops ? 0 : n, ex_ints = detect ? 2 * (m + nb) + 2 : m + nb;
+    int *ex = (int *)dev_alloc(sizeof(int) * (size_t)ex_ints, routine);
     if (!ex) return false;
     int *ea = ex, *eb = shared_ops ? ea : ex + m;
-    int *la = detect ? ex + m + n : nullptr, *lb = detect && !shared_ops ? la + m : la;
-    int *wbuf = detect ? la + m + n : nullptr;
+    int *la = detect ? ex + m + nb : nullptr, *lb = detect ? la + m : nullptr;
     // Operands still arriving from the host: A's exponents and residues are
     // computed while B is copied, and C is waited for only by the
     // reconstruction, so its copy runs under the residue GEMMs.
@@ -2344,8 +2347,8 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
         dev_free(ex);
         return false;
     }
-    if (!a_blocks) launch_exp_rows_of_op(g.A, g.ta ? k : m, g.ta ? m : k, g.lda, g.ta, E, ea, la);
-    if (!hs && !shared_ops) launch_exp_cols_of_op(g.B, g.tb ? n : k, g.tb ? k : n, g.ldb, g.tb, E, eb, lb);
+    if (!hs) launch_exp_operands(g, k, g.A, g.B, E, ex, ex_ints, shared_ops ? nullptr : eb, la, lb);
+    else if (!a_blocks) launch_exp_rows_of_op(g.A, g.ta ? k : m, g.ta ? m : k, g.lda, g.ta, E, ea);
 
     // 2. precision and moduli. Rows of op(A) are scaled to bits_a bits and
     // columns of op(B) to bits_b: by default the 106 bits of a double-double,
@@ -2358,7 +2361,7 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
     int bits_a = bits, bits_b = bits;
     if (detect) {
         int wa = 0, wb = 0;
-        if (read_widths(m, n, ea, eb, la, lb, wbuf, wa, wb)) {
+        if (read_widths(m, nb, ea, la, la + m + nb, wa, wb)) {
             bits_a = std::max(8, std::min(bits, wa));
             bits_b = std::max(8, std::min(bits, wb));
         }
