@@ -34,7 +34,6 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <type_traits>
 #include <vector>
 
 #include "dd.cuh"
@@ -45,6 +44,7 @@
 #include "xword.cuh"
 #include "level3.h"
 #include "runtime.h"
+#include "sm100.cuh"
 
 namespace mw {
 
@@ -69,11 +69,11 @@ struct GemmDesc {
     int64_t tile_begin;   // first tile counter (split instances only)
     int64_t part_begin;   // first partial-tile slot: earlier split instances
                           // hold tiles * splitk slots each
-    // tensor-core tiles only: the operands as limb bytes in the wave's scratch
+    // tensor-core tiles only: the operands as limbs in the wave's scratch
     int64_t conv_begin;   // first group of 32 lines (rows of op(A), then columns of op(B)) in the wave
-    int64_t a_off, b_off; // [line][kp] entries of 16 bytes
+    int64_t a_off, b_off; // [64 k][line] blocks of LT_BLOCK bytes
     int64_t ea_off, eb_off;   // exponent bounds of the lines
-    int kp, pad;          // k rounded up to 16
+    int kp, kc;           // k rounded up to 16, blocks along k
     xw::XW xa, xb;        // alpha, beta
 };
 static_assert(sizeof(xw::XW) == 24, "extended float size");
@@ -100,42 +100,54 @@ __device__ __forceinline__ void load_digits(const int *src, int (&dst)[R])
     }
 }
 
-// ---- 16 x 16 output tiles on the tensor cores (byte limbs) -----------------------------
+// ---- 8 x 16 output tiles on the tensor cores (byte limbs) -------------------------------
 //
 // Operands are scaled to integers N below 2^116 of their row's (column's) bound,
-// as in the digit kernel below, and held as 16 bytes each in two's complement:
-// limbs 0..14 of N mod 2^120 and limb 15 = 1 where N < 0, of weight -2^120. A
-// first kernel writes them once per operand (k_grp_limbs), [line][k], so that
-// the tiles that share an operand do not convert it again (a batch of sizes
-// log-uniform in [8, 512] has four tiles per operand line on average; with the
-// conversion in the tiles the batch took as long as with the digit kernel).
+// as in the digit kernel below, and held as 15 digits d_i in [-128, 127] of base
+// 256, fp16 each, and a zero. A first kernel writes them once per operand
+// (k_grp_limbs) in blocks of 16 digits x 64 k per line, as the shared-memory image
+// of a K-major operand with 128-byte swizzle; the blocks of neighbouring lines are
+// neighbours, so the operands of a tile and 64 k are two bulk copies.
 //
-// A warp takes two rows and 16 columns; for each output the 16 x 16 limb products
-// summed over k are two m16n8k16 MMAs per 16 k (rows and columns in the order
-// even limbs, odd limbs): one ldmatrix of 16-bit units per operand and 32 k,
-// whose masked halves are fp16 subnormals (limbmma.cuh). The FP32 sums start at
-// 2^-25 and stay, after 64 k at most 255 * 255 * 64 units of 2^-48 above it, in
-// [2^-25, 2^-24): exact, their words are 0x33000000 + sum. Each lane joins its
-// eight limb products of an output into one 64-bit integer (it holds limbs 2g,
-// 2g + 1 of the row and 4t .. 4t + 3 of the column) and adds it to the output's
-// row of 32 such sums in shared memory (64 chunks of 64 k at most per item). At
-// the end every lane takes one output: the 32 sums at weights 2^(16 (g + 2t)) are
-// one carry chain to a 256-bit integer, updated and rounded as in fixround.cuh.
+// A tile is one tcgen05 accumulator: rows are the digits of 8 rows of op(A),
+// columns the digits of 16 columns of op(B), 128 x 256. Over 256 k its entries are
+// integers of at most 2^22, exact in FP32. Warps by role, one block per SM:
+//   0      finds the tiles' instances, 32 tiles at a time
+//   1      issues the MMAs; two accumulators, one filling while the other is read
+//   2..9   join the 256 digit products of an output to 32 64-bit sums at weights
+//          2^(16 (g + 2 t)) in shared memory: a lane holds one digit of a row and
+//          joins it with the 16 of a column (one tcgen05.ld) to words of 16, then
+//          32 bits, and with its neighbour's digit to its half of those
+//   10..17 two groups that take turns: a lane takes one output; the 32 sums are
+//          one carry chain to a 256-bit integer, updated and rounded as in
+//          fixround.cuh
+//   18     issues the tiles' copies, three stages ahead
 //
-// Bound: the legacy tensor path (1024 multiply-adds/clk/SM, 256 per limb-wise
-// multiply-add) against 15 IMAD.WIDE (26 lanes/clk/SM) in the digit kernels: 0.25
-// against 0.58 clk/SM; rows past m and columns past n cost nothing. Measured on
-// 4000 products of sizes log-uniform in [8, 512] (those with m or n below 128 or
-// k below 64): 9.8 ms and 0.84 for the limbs, 14.9 on 32 x 32 digit tiles; the
-// tensor pipe is a third busy, latency (16 warps per SM) takes the rest.
-constexpr int LT = 16;                              // tile edge
-constexpr int LT_KC = 64;                           // k per chunk
-constexpr int LT_OP = 2 * LT * LT_KC * 16;          // operand bytes of a chunk
+// Bound: the chain of its stages. On 1000 products of sizes log-uniform in [8, 512]
+// (those with m or n below 128 or k below 64) it takes 1.03 ms; the copies alone,
+// 7.7 GB from L2, take 0.46, with the MMAs 0.65, without the joining 0.78, without
+// the finishing 0.93; the tensor pipe is 20 % busy, issue 55 %. 16 joining or 12
+// finishing warps change nothing; with the search for a tile's instance in the
+// copying warp it took 1.2. On 4000 such products 9.8 ms on 16 x 16 tiles of the
+// legacy MMA (mma.sync, a third busy), 14.9 on 32 x 32 digit tiles, now 4.5, with
+// 1.2 for the digits (0.84 as bytes).
+constexpr int LT = 16;                              // the policy's name for these tiles
+constexpr int LT_M = 8, LT_N = 16;                  // rows and columns of a tile
+constexpr int LT_BLOCK = 16 * 64 * 2;               // bytes of a line's digits over 64 k
+constexpr int LT_A = LT_M * LT_BLOCK, LT_STAGE = (LT_M + LT_N) * LT_BLOCK, LT_STAGES = 3;
+constexpr int LT_ACC_K = 256;                       // k per accumulator
 constexpr int LT_ROW = 33;                          // 64-bit sums per output (32 and a pad)
-constexpr int LT_SMEM = LT_OP + (GTHREADS / 32) * 32 * LT_ROW * 8;
-constexpr int64_t LT_WAVE = 1ll << 26;              // scratch entries (1 GiB) from which a batch is cut into waves
+constexpr int LT_SUMS = LT_M * LT_N * LT_ROW;       // of a tile
+constexpr int LT_BATCH = 32;                        // tiles announced together, two batches at a time
+constexpr int LT_EXT = 8, LT_FIN = 8;              // extracting and finishing warps
+constexpr int LT_GROUPS = LT_FIN / 4;               // of finishing warps, taking turns
+constexpr int LT_EXTN = LT_N / (LT_EXT / 4);        // columns of an extracting warp
+constexpr int LT_THREADS = 32 * (3 + LT_EXT + LT_FIN);
+constexpr int LT_SMEM = 1024 + LT_STAGES * LT_STAGE + 2 * LT_SUMS * 8;
+constexpr int64_t LT_WAVE = 1ll << 19;              // blocks (1 GiB) from which a batch is cut into waves
 
-// v * 2^sh (|.| < 2^116) rounded to an integer, as the 16 bytes described above.
+// v * 2^sh (|.| < 2^116) rounded to an integer N, as the bytes of N + 128 (1 + 256 +
+// .. + 256^14): byte i holds d_i + 128.
 __device__ __forceinline__ uint4 limb_bytes(double2 v, int sh)
 {
     uint32_t w[4];
@@ -170,10 +182,13 @@ __device__ __forceinline__ uint4 limb_bytes(double2 v, int sh)
         "addc.cc.u32 %0, %5, 0;\n\t"
         "addc.cc.u32 %1, %6, 0;\n\t"
         "addc.cc.u32 %2, %7, 0;\n\t"
-        "addc.u32 %3, %8, 0;\n\t}"
+        "addc.u32 %3, %8, 0;\n\t"
+        "add.cc.u32 %0, %0, 0x80808080;\n\t"
+        "addc.cc.u32 %1, %1, 0x80808080;\n\t"
+        "addc.cc.u32 %2, %2, 0x80808080;\n\t"
+        "addc.u32 %3, %3, 0x00808080;\n\t}"
         : "=&r"(b.x), "=&r"(b.y), "=&r"(b.z), "=&r"(b.w)
         : "r"(m & 1u), "r"(w[0] ^ m), "r"(w[1] ^ m), "r"(w[2] ^ m), "r"(w[3] ^ m));
-    b.w &= 0x01FFFFFFu;
     return b;
 }
 
@@ -190,11 +205,11 @@ __device__ __forceinline__ int grp_search(int count, int64_t w, F begin)
     return lo;
 }
 
-// Exponent bounds and limb bytes of 32 lines (rows of op(A) or columns of op(B))
-// of an instance per block; the second pass reads what the first left in the
-// caches.
-__global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restrict__ descs, int count, uint4 *out,
-                                                        int *ex)
+// Exponent bounds and digits of 32 lines (rows of op(A) or columns of op(B)) of
+// an instance per block; the second pass reads what the first left in the
+// caches. A thread converts 8 k of a line: 16 bytes in each of the block's rows.
+__global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restrict__ descs, int count,
+                                                        unsigned char *out, int *ex)
 {
     __shared__ int s_e[32];
     const int tid = threadIdx.x;
@@ -229,220 +244,368 @@ __global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restri
     if (l >= nl) return;
     const int e = s_e[l];
     const bool live = e > kNoExp / 2 && e < 1024;
-    const double2 *x = X + l * sl + q * sk;
-    uint4 *o = out + (isA ? d.a_off : d.b_off) + (int64_t)(line0 + l) * kp;
-#pragma unroll 2
-    for (int p = q; p < kp; p += 8, x += 8 * sk)
-        o[p] = live && p < k ? limb_bytes(*x, fxg::FX_S - e) : make_uint4(0u, 0u, 0u, 0u);
-}
-
-// Even and odd limbs of an ldmatrix word (16-bit units of two elements).
-__device__ __forceinline__ uint32_t limbs_even(uint32_t v) { return v & 0x00FF00FFu; }
-__device__ __forceinline__ uint32_t limbs_odd(uint32_t v) { return __byte_perm(v, 0u, 0x4341); }
-
-__global__ void __launch_bounds__(GTHREADS, 2) k_gemm_grouped_limb(const GemmDesc *__restrict__ descs, int count,
-                                                                  int total, unsigned long long *work_counter,
-                                                                  int *tile_counters, fx::XFPod *partials,
-                                                                  const uint4 *__restrict__ limbs,
-                                                                  const int *__restrict__ ex)
-{
-    extern __shared__ __align__(16) unsigned char s_dyn[];   // [operand row 0..31][64 k] 16 bytes, then the sums
-    __shared__ int s_item, s_last;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    unsigned long long *sums = reinterpret_cast<unsigned long long *>(s_dyn + LT_OP) + wid * (32 * LT_ROW);
-    const uint32_t op = (uint32_t)__cvta_generic_to_shared(s_dyn);
-    const uint32_t n15 = t == 3 ? 0u - 256u : 256u;
-    const int m15 = g == 7 ? -256 : 256;
-    // the 0x33000000 of each accumulator word (those times 256 vanish mod 2^32)
-    const unsigned long long off = (unsigned long long)(0x33000000ll * 65537 * (1 + m15));
-    for (;;) {
-        if (tid == 0) s_item = (int)min(atomicAdd(work_counter, 1ull), (unsigned long long)total);
-        __syncthreads();
-        const int w = s_item;
-        if (w >= total) return;
-        const GemmDesc &d = descs[grp_search(count, (int64_t)w, [&](int q) { return descs[q].work_begin; })];
-        const uint32_t local = (uint32_t)(w - d.work_begin), tile = local / (uint32_t)d.splitk;
-        const int split = (int)(local % (uint32_t)d.splitk);
-        const int i0 = (int)(tile % (uint32_t)d.tiles_m) * LT, j0 = (int)(tile / (uint32_t)d.tiles_m) * LT;
-        const int k0 = split * d.klen, kn = min(d.kp, k0 + d.klen) - k0;   // klen: multiples of 16 where split
-        const int mr = min(LT, d.m - i0), nc = min(LT, d.n - j0);
-        const uint4 *pA = limbs + d.a_off + (int64_t)i0 * d.kp + k0, *pB = limbs + d.b_off + (int64_t)j0 * d.kp + k0;
-        const bool rows = 2 * wid < mr;   // this warp has rows of the output
-        const uint32_t a_at = op + (2 * wid) * (LT_KC * 16);
-        const bool some = d.k > 0;
-        for (int c0 = 0; some && c0 < kn; c0 += LT_KC) {
-            if (c0 > 0) __syncthreads();   // the previous chunk's operands have been read
-            const int kc = min(LT_KC, kn - c0), p = tid & 63;
-            // rows 0..15 of op(A), 16..31 columns of op(B), four per turn; k goes to
-            // place k ^ (row % 8), so that ldmatrix is free of bank conflicts
-            if (p < kc) {
+    const int lines = isA ? d.m : d.n;
+    const double2 *x = X + l * sl + (int64_t)(8 * q) * sk;
+    unsigned char *o = out + ((isA ? d.a_off : d.b_off) + line0 + l) * LT_BLOCK;
+    const int64_t next = (int64_t)lines * LT_BLOCK;
+    for (int p0 = 8 * q; p0 < kp; p0 += 64, x += 64 * sk, o += next) {
+        double2 v[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int r = (tid >> 6) + 4 * (u & 3);
-                    const uint4 *src = (u < 4 ? pA : pB) + (int64_t)r * d.kp + c0 + p;
-                    if (r < (u < 4 ? mr : nc))
-                        lmb::cp_async16(op + ((((u < 4 ? 0 : LT) + r) * LT_KC + (p ^ (r & 7))) << 4), src);
+        for (int u = 0; u < 8; ++u) v[u] = live && p0 + u < k ? x[u * sk] : make_double2(0.0, 0.0);
+        uint4 b[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            b[u] = live ? limb_bytes(v[u], fxg::FX_S - e)
+                        : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x808080u);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            uint32_t h[4] = {0u, 0u, 0u, 0u};
+            if (r < 15) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    auto word = [&](const uint4 &y) { return r < 4 ? y.x : r < 8 ? y.y : r < 12 ? y.z : y.w; };
+                    // 1024 + byte in both halves, less 1152
+                    const uint32_t t = __byte_perm(word(b[2 * u]), word(b[2 * u + 1]), (r & 3) | (4 + (r & 3)) << 8);
+                    asm("sub.f16x2 %0, %1, %2;" : "=r"(h[u]) : "r"((t & 0x00FF00FFu) | 0x64006400u), "r"(0x64806480u));
                 }
             }
-            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            if (!rows) continue;
-            const int nks = kc >> 4;   // steps of 16 k
-#pragma unroll 1
-            for (int r = 0; r < 2; ++r) {
-                uint32_t a[4][4];   // the row's operands of every step
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t x[4];
-                    lmb::ldmatrix_x4_trans(x, a_at + r * (LT_KC * 16) + (((32 * h + lane) ^ ((2 * wid + r) & 7)) << 4));
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        a[2 * h + q][0] = limbs_even(x[2 * q]);
-                        a[2 * h + q][1] = limbs_odd(x[2 * q]);
-                        a[2 * h + q][2] = limbs_even(x[2 * q + 1]);
-                        a[2 * h + q][3] = limbs_odd(x[2 * q + 1]);
-                    }
+            *reinterpret_cast<uint4 *>(o + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
+        }
+    }
+}
+
+// A tile as announced to the roles.
+struct LtItem {
+    int64_t a, b;                // first blocks of its operands
+    int desc, i0, j0, mr, nc, kn, tile, split;
+    int lines_a, lines_b;        // blocks from one 64 k to the next
+};
+
+__global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmDesc *__restrict__ descs, int count,
+                                                                    int total, int *tile_counters,
+                                                                    fx::XFPod *partials,
+                                                                    const unsigned char *__restrict__ limbs,
+                                                                    const int *__restrict__ ex, int *status)
+{
+    extern __shared__ unsigned char s_dyn[];   // stages, then the sums of two tiles
+    __shared__ uint64_t full[LT_STAGES], empty[LT_STAGES], accf[2], acce[2], sumf[LT_GROUPS], sume[2];
+    __shared__ uint64_t itemf[2], iteme[2], drain;
+    __shared__ LtItem items[2 * LT_BATCH];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_last[LT_GROUPS];
+    unsigned char *stages = (unsigned char *)(((uintptr_t)s_dyn + 1023) & ~(uintptr_t)1023);
+    unsigned long long *sums = reinterpret_cast<unsigned long long *>(stages + LT_STAGES * LT_STAGE);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_items = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < LT_STAGES; ++q) {
+            sm100::mbar_init(&full[q], 1);
+            sm100::mbar_init(&empty[q], 1);
+        }
+        for (int q = 0; q < 2; ++q) {
+            sm100::mbar_init(&accf[q], 1);
+            sm100::mbar_init(&acce[q], LT_EXT);
+            sm100::mbar_init(&sume[q], 4);
+        }
+        for (int q = 0; q < LT_GROUPS; ++q) sm100::mbar_init(&sumf[q], LT_EXT);
+        for (int q = 0; q < 2; ++q) {
+            sm100::mbar_init(&itemf[q], 1);
+            sm100::mbar_init(&iteme[q], 2 + LT_EXT + LT_FIN);
+        }
+        sm100::mbar_init(&drain, 1);
+        sm100::fence_mbar_init();
+    }
+    if (warp == 1) {
+        sm100::tmem_alloc(&s_tmem, 512);
+        sm100::tmem_relinquish();
+    }
+    sm100::tc_fence_before();
+    __syncthreads();
+    sm100::tc_fence_after();
+    const uint32_t tmem = s_tmem;
+
+    // Tile `it` of this block, once its batch is announced; `last` is the caller's
+    // previous tile (-1: none), whose batch it gives back with the step to another.
+    auto item = [&](int it, int last, int code) -> bool {
+        const int n = it / LT_BATCH;
+        if (last >= 0 && last / LT_BATCH == n) return true;
+        if (last >= 0) {
+            __syncwarp();
+            if (lane == 0) sm100::mbar_arrive(&iteme[(n - 1) & 1]);
+        }
+        return __all_sync(0xffffffffu, sm100::mbar_wait(&itemf[n & 1], (n >> 1) & 1, status, code));
+    };
+    if (warp == 0) {
+        for (int n = 0; n * LT_BATCH < n_items; ++n) {
+            if (n >= 2 &&
+                !__all_sync(0xffffffffu, sm100::mbar_wait(&iteme[n & 1], ((n >> 1) - 1) & 1, status, 1)))
+                break;
+            const int it = n * LT_BATCH + lane, w = (int)blockIdx.x + it * (int)gridDim.x;
+            if (it < n_items) {   // a lane's binary search beside the others'
+                LtItem x;
+                x.desc = grp_search(count, (int64_t)w, [&](int q) { return descs[q].work_begin; });
+                const GemmDesc &d = descs[x.desc];
+                const uint32_t local = (uint32_t)(w - d.work_begin), tile = local / (uint32_t)d.splitk;
+                x.tile = (int)tile;
+                x.split = (int)(local % (uint32_t)d.splitk);
+                x.i0 = (int)(tile % (uint32_t)d.tiles_m) * LT_M;
+                x.j0 = (int)(tile / (uint32_t)d.tiles_m) * LT_N;
+                const int k0 = x.split * d.klen;   // klen: multiples of 64 where split
+                x.kn = d.k > 0 ? min(d.kp, k0 + d.klen) - k0 : 0;
+                x.mr = min(LT_M, d.m - x.i0);
+                x.nc = min(LT_N, d.n - x.j0);
+                x.lines_a = d.m;
+                x.lines_b = d.n;
+                x.a = d.a_off + (int64_t)(k0 / 64) * d.m + x.i0;
+                x.b = d.b_off + (int64_t)(k0 / 64) * d.n + x.j0;
+                items[it % (2 * LT_BATCH)] = x;
+            }
+            __syncwarp();
+            if (lane == 0) sm100::mbar_arrive(&itemf[n & 1]);
+        }
+    } else if (warp == 2 + LT_EXT + LT_FIN) {
+        uint32_t gs = 0;   // stages filled
+        bool ok = true;
+        for (int it = 0; it < n_items && ok; ++it) {
+            if (!item(it, it - 1, 1)) break;
+            const LtItem &x = items[it % (2 * LT_BATCH)];
+            const unsigned char *pA = limbs + x.a * LT_BLOCK, *pB = limbs + x.b * LT_BLOCK;
+            for (int c0 = 0; c0 < x.kn; c0 += 64, ++gs) {
+                const int st = gs % LT_STAGES;
+                ok = gs < LT_STAGES ||
+                     __all_sync(0xffffffffu, sm100::mbar_wait(&empty[st], (gs / LT_STAGES - 1) & 1, status, 1));
+                if (!ok) break;
+                if (lane == 0) {
+                    unsigned char *at = stages + st * LT_STAGE;
+                    sm100::mbar_arrive_expect_tx(&full[st], (uint32_t)(x.mr + x.nc) * LT_BLOCK);
+                    sm100::bulk_load(at, pA, (uint32_t)x.mr * LT_BLOCK, &full[st]);
+                    sm100::bulk_load(at + LT_A, pB, (uint32_t)x.nc * LT_BLOCK, &full[st]);
                 }
-                // four columns at a time, so that their products and sums overlap
-                auto columns = [&](int c, auto width) {
-                    constexpr int NC = decltype(width)::value;
-                    float acc[NC][2][4];
-                    uint32_t x[NC][4];
+                pA += (int64_t)x.lines_a * LT_BLOCK;
+                pB += (int64_t)x.lines_b * LT_BLOCK;
+            }
+        }
+        // never leave with copies in flight: wait (bounded) for the last use of every stage
+        for (uint32_t t = gs > LT_STAGES ? gs - LT_STAGES : 0; t < gs; ++t)
+            sm100::mbar_wait(&full[t % LT_STAGES], (t / LT_STAGES) & 1, nullptr, 0);
+    } else if (warp == 1) {
+        uint32_t gs = 0, cg = 0;   // stages used, accumulators filled
+        bool ok = true;
+        for (int it = 0; it < n_items && ok; ++it) {
+            if (!item(it, it - 1, 2)) break;
+            const LtItem &x = items[it % (2 * LT_BATCH)];
+            const int kn = x.kn;
+            const uint32_t idesc = sm100::idesc_f16_f32(128, 16 * x.nc);
+            for (int c0 = 0; c0 < kn && ok; c0 += LT_ACC_K, ++cg) {
+                const int b = cg & 1;
+                if (cg >= 2) {
+                    ok = __all_sync(0xffffffffu, sm100::mbar_wait(&acce[b], (cg / 2 - 1) & 1, status, 2));
+                    if (!ok) break;
+                    sm100::tc_fence_after();
+                }
+                const int c1 = min(kn, c0 + LT_ACC_K);
+                for (int c = c0; c < c1; c += 64, ++gs) {
+                    const int st = gs % LT_STAGES;
+                    ok = __all_sync(0xffffffffu, sm100::mbar_wait(&full[st], (gs / LT_STAGES) & 1, status, 3));
+                    if (!ok) break;
+                    sm100::tc_fence_after();
+                    if (lane == 0) {
+                        const uint64_t ad = sm100::smem_desc_sw128(sm100::smem_u32(stages + st * LT_STAGE));
+                        const uint64_t bd = sm100::smem_desc_sw128(sm100::smem_u32(stages + st * LT_STAGE + LT_A));
+                        const int steps = min(4, (c1 - c) / 16);
+                        for (int q = 0; q < steps; ++q)
+                            sm100::mma_f16(tmem + b * 256, ad + 2 * q, bd + 2 * q, idesc, c > c0 || q > 0 ? 1u : 0u);
+                        sm100::mma_commit(&empty[st]);
+                        if (c + 64 >= c1) sm100::mma_commit(&accf[b]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        // no MMA may still be writing TMEM when it is freed
+        if (lane == 0) {
+            sm100::mma_commit(&drain);
+            sm100::mbar_wait(&drain, 0, nullptr, 0);
+        }
+    } else if (warp < 2 + LT_EXT) {
+        // rows 2 quad, 2 quad + 1 of the tile (lane: digit lane % 16 of one), columns LT_EXTN part ..
+        const int quad = warp & 3, part = (warp - 2) >> 2, odd = lane & 1;
+        const int row = 2 * quad + (lane >> 4);
+        const uint32_t at0 = tmem + ((uint32_t)(quad * 32) << 16) + part * (16 * LT_EXTN);
+        // weights of this lane's digit and its neighbour's
+        const uint32_t own = odd ? 256u : 1u, other = odd ? 1u : 256u;
+        const unsigned long long off = 0x8B400000ull * 257u * 65537u;
+        uint32_t cg = 0;
+        bool ok = true;
+        for (int it = 0; it < n_items && ok; ++it) {
+            const int sb = it & 1;
+            if (!item(it, it - 1, 4)) break;
+            const LtItem &x = items[it % (2 * LT_BATCH)];
+            const int nc = min(LT_EXTN, x.nc - LT_EXTN * part);
+            if (it >= 2) {
+                ok = __all_sync(0xffffffffu, sm100::mbar_wait(&sume[sb], (it / 2 - 1) & 1, status, 4));
+                if (!ok) break;
+            }
+            unsigned long long *to = sums + sb * LT_SUMS + ((LT_EXTN * part) * LT_M + row) * LT_ROW +
+                                     4 * ((lane & 15) >> 1) + 2 * odd;
+            for (int c0 = 0; c0 < x.kn; c0 += LT_ACC_K, ++cg) {
+                const int b = cg & 1;
+                ok = __all_sync(0xffffffffu, sm100::mbar_wait(&accf[b], (cg / 2) & 1, status, 4));
+                if (!ok) break;
+                sm100::tc_fence_after();
+                if (2 * quad < x.mr) {
+#pragma unroll 1
+                    for (int j = 0; j < nc; j += 2) {   // (a column past nc is stored too: nobody reads it)
+                        uint32_t r[32];
+                        sm100::tmem_ld32(at0 + b * 256 + j * 16, r);
+                        sm100::tmem_wait_ld();
 #pragma unroll
-                    for (int s = 0; s < 4; ++s) {
-                        if (s >= nks) break;
-                        if ((s & 1) == 0)
+                        for (int u = 0; u < 2; ++u) {
+                            uint32_t p[8];
 #pragma unroll
-                            for (int u = 0; u < NC; ++u)
-                                lmb::ldmatrix_x4_trans(x[u], op + (LT + c + u) * (LT_KC * 16) +
-                                                                 (((16 * s + lane) ^ ((c + u) & 7)) << 4));
+                            for (int q = 0; q < 8; ++q) {
+                                float2 f = make_float2(__uint_as_float(r[16 * u + 2 * q]),
+                                                       __uint_as_float(r[16 * u + 2 * q + 1]));
+                                f = __fadd2_rn(f, make_float2(12582912.0f, 12582912.0f));   // 0x4B400000 + integer
+                                p[q] = __float_as_uint(f.x) + 256u * __float_as_uint(f.y);   // 0x8B400000 + integer
+                            }
+                            uint32_t keep[4], got[4];
 #pragma unroll
-                        for (int u = 0; u < NC; ++u) {
-                            const uint32_t x0 = x[u][2 * (s & 1)], x1 = x[u][2 * (s & 1) + 1];
-                            const uint32_t e0 = limbs_even(x0), e1 = limbs_even(x1);
-                            const uint32_t o0 = limbs_odd(x0), o1 = limbs_odd(x1);
-                            if (s == 0) {
-                                lmb::mma16816_from(acc[u][0], a[s][0], a[s][1], a[s][2], a[s][3], e0, e1, 0x1p-25f);
-                                lmb::mma16816_from(acc[u][1], a[s][0], a[s][1], a[s][2], a[s][3], o0, o1, 0x1p-25f);
-                            } else {
-                                lmb::mma16816(acc[u][0], a[s][0], a[s][1], a[s][2], a[s][3], e0, e1);
-                                lmb::mma16816(acc[u][1], a[s][0], a[s][1], a[s][2], a[s][3], o0, o1);
+                            for (int q = 0; q < 4; ++q) {
+                                keep[q] = odd ? p[4 + q] : p[q];
+                                got[q] = __shfl_xor_sync(0xffffffffu, odd ? p[q] : p[4 + q], 1);
+                            }
+                            unsigned long long *dst = to + (j + u) * (LT_M * LT_ROW);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                unsigned long long y = (c0 == 0 ? 0ull : dst[h]) - off;
+                                y += (unsigned long long)keep[2 * h] * own;
+                                y += (unsigned long long)got[2 * h] * other;
+                                y += (unsigned long long)keep[2 * h + 1] * (own << 16);
+                                y += (unsigned long long)got[2 * h + 1] * (other << 16);
+                                dst[h] = y;
                             }
                         }
                     }
-#pragma unroll
-                    for (int u = 0; u < NC; ++u) {
-                        // limbs 4t .. 4t + 3 of the column for each of the row's two limbs;
-                        // limb 15 (t = 3) and the row's limb 15 (g = 7) have negative weight
-                        auto word = [&](int b, int i) { return __float_as_uint(acc[u][b][i]); };
-                        const int lo0 = (int)(word(0, 0) + 256u * word(1, 0)), hi0 = (int)(word(0, 1) + n15 * word(1, 1));
-                        const int lo1 = (int)(word(0, 2) + 256u * word(1, 2)), hi1 = (int)(word(0, 3) + n15 * word(1, 3));
-                        const long long lo = (long long)lo1 * m15 + lo0, hi = (long long)hi1 * m15 + hi0;
-                        unsigned long long *at = sums + ((c + u) * 2 + r) * LT_ROW + lane;
-                        const unsigned long long q = (unsigned long long)(lo + hi * 65536) - off;
-                        *at = c0 == 0 ? q : *at + q;
-                    }
-                };
-                int c = 0;
-                for (; c + 4 <= nc; c += 4) columns(c, std::integral_constant<int, 4>{});
-                for (; c < nc; ++c) columns(c, std::integral_constant<int, 1>{});
+                }
+                sm100::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) sm100::mbar_arrive(&acce[b]);
             }
+            __syncwarp();
+            if (ok && lane == 0) sm100::mbar_arrive(&sumf[it % LT_GROUPS]);
         }
-        __syncwarp();
-
-        // each lane one output: row 2 wid + (lane & 1), column lane / 2
-        const int orow = 2 * wid + (lane & 1), ocol = lane >> 1;
-        const bool in = orow < mr && ocol < nc;
-        const int ei = in && some ? ex[d.ea_off + i0 + orow] : kNoExp, ej = in && some ? ex[d.eb_off + j0 + ocol] : kNoExp;
-        bool bad = ei >= 1024 || ej >= 1024;
-        const bool live = !bad && ei > kNoExp / 2 && ej > kNoExp / 2;
-        double2 *pc = d.C + i0 + orow + (int64_t)(j0 + ocol) * d.ldc;
-        const double2 c_in = in && d.beta_kind != 0 && d.splitk == 1 ? *pc : make_double2(0.0, 0.0);
-        uint64_t W[4] = {0, 0, 0, 0};
-        if (live) {
-            const unsigned long long *at = sums + lane * LT_ROW;
-            long long carry = 0;   // sum at weight 2^(16 s), its low 16 bits to the result
+    } else {
+        const int group = (warp - 2 - LT_EXT) >> 2, part = (warp - 2 - LT_EXT) & 3;
+        const int orow = lane & 7, ocol = 4 * part + (lane >> 3), out = ocol * LT_M + orow;
+        for (int it = group; it < n_items; it += LT_GROUPS) {
+            const int sb = it & 1;
+            const unsigned long long *at = sums + sb * LT_SUMS + out * LT_ROW;
+            if (!item(it, it >= LT_GROUPS ? it - LT_GROUPS : -1, 5)) break;
+            const LtItem &x = items[it % (2 * LT_BATCH)];
+            const GemmDesc &d = descs[x.desc];
+            const bool in = orow < x.mr && ocol < x.nc, some = d.k > 0;
+            const int ei = in && some ? ex[d.ea_off + x.i0 + orow] : kNoExp;
+            const int ej = in && some ? ex[d.eb_off + x.j0 + ocol] : kNoExp;
+            bool bad = ei >= 1024 || ej >= 1024;
+            const bool live = !bad && ei > kNoExp / 2 && ej > kNoExp / 2;
+            double2 *pc = d.C + x.i0 + orow + (int64_t)(x.j0 + ocol) * d.ldc;
+            const double2 c_in = in && d.beta_kind != 0 && d.splitk == 1 ? *pc : make_double2(0.0, 0.0);
+            if (!__all_sync(0xffffffffu, sm100::mbar_wait(&sumf[group], (it / LT_GROUPS) & 1, status, 5))) break;
+            uint64_t W[4] = {0, 0, 0, 0};
+            if (live) {
+                long long carry = 0;   // sum at weight 2^(16 s), its low 16 bits to the result
 #pragma unroll
-            for (int s = 0; s < 14; ++s) {
+                for (int s = 0; s < 14; ++s) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (s - 2 * q >= 0 && s - 2 * q < 8) carry += (long long)at[4 * (s - 2 * q) + q];
-                W[s >> 2] |= (uint64_t)((uint32_t)carry & 0xFFFFu) << (16 * (s & 3));
-                carry >>= 16;
+                    for (int q = 0; q < 4; ++q)
+                        if (s - 2 * q >= 0 && s - 2 * q < 8) carry += (long long)at[4 * (s - 2 * q) + q];
+                    W[s >> 2] |= (uint64_t)((uint32_t)carry & 0xFFFFu) << (16 * (s & 3));
+                    carry >>= 16;
+                }
+                W[3] |= (uint64_t)carry << 32;
             }
-            W[3] |= (uint64_t)carry << 32;
-        }
-        const int e0 = ei + ej - 2 * fxg::FX_S;
-        bool done = false;
-        if (in && live && d.splitk == 1) {
-            // the top 160 bits of |W| (2^-134 of the largest product is cut), alpha, beta C, one rounding
-            const uint32_t m = (uint32_t)((int64_t)W[3] >> 63);
-            uint32_t x[8];
+            __syncwarp();
+            if (lane == 0) sm100::mbar_arrive(&sume[sb]);
+            const int e0 = ei + ej - 2 * fxg::FX_S;
+            bool done = false;
+            if (in && live && d.splitk == 1) {
+                // the top 160 bits of |W| (2^-134 of the largest product is cut), alpha, beta C, one rounding
+                const uint32_t m = (uint32_t)((int64_t)W[3] >> 63);
+                uint32_t x8[8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                x[2 * q] = (uint32_t)W[q];
-                x[2 * q + 1] = (uint32_t)(W[q] >> 32);
-            }
-            fxr::cond_neg<8>(x, m);
-            fxr::Fix a;
-            a.neg = m & 1u;
-            if (d.alpha.x == 1.0 && d.alpha.y == 0.0) {
+                for (int q = 0; q < 4; ++q) {
+                    x8[2 * q] = (uint32_t)W[q];
+                    x8[2 * q + 1] = (uint32_t)(W[q] >> 32);
+                }
+                fxr::cond_neg<8>(x8, m);
+                fxr::Fix a;
+                a.neg = m & 1u;
+                if (d.alpha.x == 1.0 && d.alpha.y == 0.0) {
 #pragma unroll
-                for (int q = 0; q < 5; ++q) a.w[q] = x[3 + q];
-                a.e = e0 + 96;
-            } else {
-                fxr::mul54(x + 3, d.xa.w, a.w);
-                a.neg ^= d.xa.neg;
-                a.e = e0 + 96 + 128 + d.xa.e;
+                    for (int q = 0; q < 5; ++q) a.w[q] = x8[3 + q];
+                    a.e = e0 + 96;
+                } else {
+                    fxr::mul54(x8 + 3, d.xa.w, a.w);
+                    a.neg ^= d.xa.neg;
+                    a.e = e0 + 96 + 128 + d.xa.e;
+                }
+                a.w[5] = 0u;
+                if (d.beta_kind == 0 || add_beta_c(a, c_in, d.xb, d.beta_kind == 1, 0u)) {
+                    double h, l;
+                    fxr::to_dd(a, h, l);
+                    *pc = make_double2(h, l);
+                    done = true;
+                }
             }
-            a.w[5] = 0u;
-            if (d.beta_kind == 0 || add_beta_c(a, c_in, d.xb, d.beta_kind == 1, 0u)) {
-                double h, l;
-                fxr::to_dd(a, h, l);
-                *pc = make_double2(h, l);
-                done = true;
-            }
-        }
-        xfp::XF v;
-        v.zero = true; v.neg = false; v.m = 0; v.e = 0;
-        if (live && !done) v = fx::w256_to_xf(W, e0);
-        if (d.splitk > 1) {
-            // this split's sums, then the last split of the tile finishes it
-            fx::XFPod *pt = partials + (d.part_begin + (int64_t)tile * d.splitk + split) * (LT * LT);
-            pt[ocol * LT + orow] = fx::to_pod(v, bad);
-            __threadfence();
-            __syncthreads();
-            if (tid == 0) s_last = atomicAdd(&tile_counters[d.tile_begin + tile], 1) == d.splitk - 1;
-            __syncthreads();
-            if (!s_last) continue;
-            __threadfence();
-            const fx::XFPod *base = partials + (d.part_begin + (int64_t)tile * d.splitk) * (LT * LT) + ocol * LT + orow;
+            xfp::XF v;
             v.zero = true; v.neg = false; v.m = 0; v.e = 0;
-            bad = false;
-            for (int s2 = 0; s2 < d.splitk; ++s2) {
-                // partials written by other CTAs: read through L2
-                const fx::XFPod *q = base + (int64_t)s2 * (LT * LT);
-                fx::XFPod pv;
-                pv.hi = __ldcg(&q->hi);
-                pv.lo = __ldcg(&q->lo);
-                pv.e = __ldcg(&q->e);
-                pv.flags = __ldcg(&q->flags);
-                bad |= (pv.flags & 4) != 0;
-                v = xfp::xf_add(v, fx::from_pod(pv));
+            if (live && !done) v = fx::w256_to_xf(W, e0);
+            if (d.splitk > 1) {
+                // this split's sums, then the last split of the tile finishes it
+                fx::XFPod *base = partials + (d.part_begin + (int64_t)x.tile * d.splitk) * (LT_M * LT_N) + out;
+                base[x.split * (LT_M * LT_N)] = fx::to_pod(v, bad);
+                __threadfence();
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(128) : "memory");
+                if (part == 0 && lane == 0)
+                    s_last[group] = atomicAdd(&tile_counters[d.tile_begin + x.tile], 1) == d.splitk - 1;
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(128) : "memory");
+                if (!s_last[group]) continue;
+                __threadfence();
+                v.zero = true; v.neg = false; v.m = 0; v.e = 0;
+                bad = false;
+                for (int s2 = 0; s2 < d.splitk; ++s2) {
+                    // partials written by other CTAs: read through L2
+                    const fx::XFPod *q = base + s2 * (LT_M * LT_N);
+                    fx::XFPod pv;
+                    pv.hi = __ldcg(&q->hi);
+                    pv.lo = __ldcg(&q->lo);
+                    pv.e = __ldcg(&q->e);
+                    pv.flags = __ldcg(&q->flags);
+                    bad |= (pv.flags & 4) != 0;
+                    v = xfp::xf_add(v, fx::from_pod(pv));
+                }
+                if (part == 0 && lane == 0) tile_counters[d.tile_begin + x.tile] = 0;   // ready for the next replay
             }
-            if (tid == 0) tile_counters[d.tile_begin + tile] = 0;   // ready for the next replay
-        }
-        if (in && !done) {
-            if (bad) {
-                const double qnan = __longlong_as_double(0x7ff8000000000000ll);
-                *pc = make_double2(qnan, qnan);
-            } else {
-                fxg::store_axpby(pc, v, xfp::xf_from_dd(d.alpha.x, d.alpha.y), d.alpha.x == 1.0 && d.alpha.y == 0.0,
-                                 xfp::xf_from_dd(d.beta.x, d.beta.y), dd::make(d.beta.x, d.beta.y), d.beta_kind);
+            if (in && !done) {
+                if (bad) {
+                    const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+                    *pc = make_double2(qnan, qnan);
+                } else {
+                    fxg::store_axpby(pc, v, xfp::xf_from_dd(d.alpha.x, d.alpha.y), d.alpha.x == 1.0 && d.alpha.y == 0.0,
+                                     xfp::xf_from_dd(d.beta.x, d.beta.y), dd::make(d.beta.x, d.beta.y), d.beta_kind);
+                }
             }
         }
-        __syncthreads();   // s_item and the operands are reused
+    }
+
+    sm100::tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        sm100::tc_fence_after();
+        sm100::tmem_dealloc(tmem, 512);
     }
 }
 
@@ -800,10 +963,10 @@ struct Plan {
     // tensor-core tiles: descriptors [first, first + count) share the limb scratch
     struct Wave {
         int first, count;
-        int64_t work, groups, entries, lines;
+        int64_t work, groups, blocks, lines;
     };
     std::vector<Wave> waves;
-    int64_t wave_entries = 0, wave_lines = 0;   // largest of any wave
+    int64_t wave_blocks = 0, wave_lines = 0;   // largest of any wave
     // device state
     void *dev = nullptr;
     size_t dev_bytes = 0;
@@ -860,7 +1023,7 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
     pl.tile = GT;
     int64_t work = 0, stiles = 0, pslots = 0;
     pl.waves.clear();
-    pl.wave_entries = pl.wave_lines = 0;
+    pl.wave_blocks = pl.wave_lines = 0;
     for (int64_t i = 0; i < count; ++i) {
         if (m[i] <= 0 || n[i] <= 0) continue;
         GemmDesc d;
@@ -913,19 +1076,20 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
             // only the beta pass: run as a k = 0 product (sigma irrelevant)
             d.k = 0;
         }
-        d.tiles_m = (d.m + GT - 1) / GT;
+        d.tiles_m = GT == LT ? (d.m + LT_M - 1) / LT_M : (d.m + GT - 1) / GT;
         d.tiles_n = (d.n + GT - 1) / GT;
         const int tiles = d.tiles_m * d.tiles_n;
         d.splitk = 1;
-        if (pol.min_k_per_split > 0 && tiles <= pol.max_tiles_split && d.k >= 2 * pol.min_k_per_split)
+        const int few = pol.max_tiles_split * (GT == LT ? LT / LT_M : 1);
+        if (pol.min_k_per_split > 0 && tiles <= few && d.k >= 2 * pol.min_k_per_split)
             d.splitk = std::min(16, d.k / pol.min_k_per_split);
         // the digit column sums hold at most 16384 multiply-adds per split, the
-        // limb sums 4096 (64 chunks below 2^54 each, four of them added)
+        // limb sums 4096 (16 accumulators' sums below 2^56 each, four of them added)
         const int kmax = GT == LT ? 4096 : 16384;
         const int need_splits = (d.k + kmax - 1) / kmax;
         if (d.splitk < need_splits) d.splitk = need_splits;
         d.kp = (d.k + 15) / 16 * 16;
-        const int kstep = GT == LT ? 16 : GBK;
+        const int kstep = GT == LT ? 64 : GBK;
         d.klen = d.splitk > 1 ? ((d.k + d.splitk - 1) / d.splitk + kstep - 1) / kstep * kstep
                               : std::max(GT == LT ? d.kp : d.k, 1);
         if (d.k == 0) d.klen = 1;
@@ -934,24 +1098,25 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
             if (d.splitk > 1) d.splitk = (d.k + d.klen - 1) / d.klen;
             d.xa = xw::from_dd(d.alpha.x, d.alpha.y);
             d.xb = xw::from_dd(d.beta.x, d.beta.y);
-            const int64_t entries = ((int64_t)d.m + d.n) * d.kp, lines = d.k > 0 ? (int64_t)d.m + d.n : 0;
+            d.kc = (d.k + 63) / 64;
+            const int64_t blocks = ((int64_t)d.m + d.n) * d.kc, lines = d.k > 0 ? (int64_t)d.m + d.n : 0;
             const int64_t tw = (int64_t)tiles * d.splitk;
-            if (pl.waves.empty() || pl.waves.back().entries + entries > LT_WAVE ||
+            if (pl.waves.empty() || pl.waves.back().blocks + blocks > LT_WAVE ||
                 pl.waves.back().work + tw > INT32_MAX)
                 pl.waves.push_back(Plan::Wave{(int)pl.descs.size(), 0, 0, 0, 0, 0});
             Plan::Wave &wv = pl.waves.back();
             work = wv.work;   // work items are numbered within the wave
             d.conv_begin = wv.groups;
-            d.a_off = wv.entries;
-            d.b_off = wv.entries + (int64_t)d.m * d.kp;
+            d.a_off = wv.blocks;
+            d.b_off = wv.blocks + (int64_t)d.m * d.kc;
             d.ea_off = wv.lines;
             d.eb_off = wv.lines + d.m;
             wv.groups += d.k > 0 ? (d.m + 31) / 32 + (d.n + 31) / 32 : 0;
-            wv.entries += entries;
+            wv.blocks += blocks;
             wv.lines += lines;
             wv.work += tw;
             wv.count++;
-            pl.wave_entries = std::max(pl.wave_entries, wv.entries);
+            pl.wave_blocks = std::max(pl.wave_blocks, wv.blocks);
             pl.wave_lines = std::max(pl.wave_lines, wv.lines);
         }
         d.work_begin = work;
@@ -967,7 +1132,7 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
     pl.total = work;
     for (const Plan::Wave &wv : pl.waves) pl.total = std::max(pl.total, wv.work);
     pl.split_tiles = stiles;
-    pl.partial_elems = pslots * GT * GT;   // extended-float partials
+    pl.partial_elems = pslots * (GT == LT ? LT_M * LT_N : GT * GT);   // extended-float partials
 }
 
 uint64_t plan_key(const Plan &pl)
@@ -994,7 +1159,7 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     const size_t d_bytes = pl.descs.size() * sizeof(GemmDesc);
     const size_t cnt_bytes = 256 + (size_t)(pl.split_tiles + 1) * sizeof(int);
     const size_t part_bytes = (size_t)pl.partial_elems * sizeof(fx::XFPod);
-    const size_t limb_bytes_ = (size_t)pl.wave_entries * 16, ex_bytes = (size_t)pl.wave_lines * sizeof(int);
+    const size_t limb_bytes_ = (size_t)pl.wave_blocks * LT_BLOCK, ex_bytes = (size_t)pl.wave_lines * sizeof(int);
     const size_t need = d_bytes + cnt_bytes + part_bytes + limb_bytes_ + ex_bytes + 1024;
     const uint64_t key = plan_key(pl);
     cudaStream_t s = stream();
@@ -1021,7 +1186,7 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     int *tile_counters = (int *)(counter + 32);
     fx::XFPod *partials = (fx::XFPod *)(base + part_off);
     const size_t limb_off = (part_off + part_bytes + 255) / 256 * 256;
-    uint4 *limbs = (uint4 *)(base + limb_off);
+    unsigned char *limbs = (unsigned char *)(base + limb_off);
     int *ex = (int *)(base + (limb_off + limb_bytes_ + 255) / 256 * 256);
     const int sms = device_sm_count();
     const int grid = (int)std::min<int64_t>(pl.total, (int64_t)sms * 16);
@@ -1045,14 +1210,13 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
             return;
         }
         cudaFuncSetAttribute(k_gemm_grouped_limb, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
-        bool first = true;
         for (const Plan::Wave &wv : pl.waves) {
-            if (!first) cudaMemsetAsync(counter, 0, sizeof(*counter), q);
-            first = false;
-            if (wv.groups > 0) k_grp_limbs<<<(unsigned)wv.groups, GTHREADS, 0, q>>>(ddesc + wv.first, wv.count, limbs, ex);
-            const int wgrid = (int)std::min<int64_t>(wv.work, (int64_t)sms * 2);
-            k_gemm_grouped_limb<<<wgrid, GTHREADS, LT_SMEM, q>>>(ddesc + wv.first, wv.count, (int)wv.work, counter,
-                                                                tile_counters, partials, limbs, ex);
+            if (wv.groups > 0)
+                k_grp_limbs<<<(unsigned)wv.groups, GTHREADS, 0, q>>>(ddesc + wv.first, wv.count, limbs, ex);
+            const int wgrid = (int)std::min<int64_t>(wv.work, sms);
+            k_gemm_grouped_limb<<<wgrid, LT_THREADS, LT_SMEM, q>>>(ddesc + wv.first, wv.count, (int)wv.work,
+                                                                  tile_counters, partials, limbs, ex,
+                                                                  device_status_word());
         }
     };
     if (!use_graph) {
@@ -1203,6 +1367,11 @@ bool grouped_validate(const char *routine, int64_t count, const char *ta, const 
 }
 
 }  // namespace
+
+void set_grouped_wait_limit(uint64_t ns)
+{
+    cudaMemcpyToSymbol(sm100::g_wait_limit_ns, &ns, sizeof(ns));
+}
 
 // Grouped GEMM for the library's own use (device arrays, arguments already
 // valid): its own plan, default split policy, stream-ordered (no sync).

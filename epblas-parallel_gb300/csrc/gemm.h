@@ -46,8 +46,10 @@ double gemm_fixed_small_us(int64_t m, int64_t n, int64_t k);
 // error recorded on failure.
 bool gemm_ozaki_real(const GemmArgs &g, int bits, const char *routine);
 bool gemm_ozaki_cplx(const GemmArgs &g, int bits, const char *routine);
-// Wait limit of the FP64 engine's TMA pipeline (its own copy of the device word).
+// Wait limits of the FP64 engine's TMA pipeline and of the grouped tiles (each its
+// own copy of the device word).
 void set_plain_wait_limit(uint64_t ns);
+void set_grouped_wait_limit(uint64_t ns);
 int ozaki_last_moduli();
 
 // Grouped products on the tensor cores (instances of mgemm_grouped):

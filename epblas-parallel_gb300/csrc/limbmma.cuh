@@ -95,16 +95,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t r[4], uint32_t addr)
                  : "memory");
 }
 
-// D = A * B + c in every entry
-__device__ __forceinline__ void mma16816_from(float d[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                              uint32_t b0, uint32_t b1, float c)
-{
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                 "{%10, %10, %10, %10};"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c));
-}
-
 // 256-bit two's complement helpers (four 64-bit words, least significant first)
 __device__ __forceinline__ void add256(uint64_t a[4], const uint64_t b[4])
 {

@@ -3227,7 +3227,10 @@ extern "C" uint64_t mwblas_set_wait_limit_ns(uint64_t ns)
     const uint64_t v = ns == 0 ? sm100::kWaitLimitNs : (ns < 1000000ull ? 1000000ull : ns);
     mw::clear_error();
     const cudaError_t st = cudaMemcpyToSymbol(sm100::g_wait_limit_ns, &v, sizeof(v));
-    if (st == cudaSuccess) mw::set_plain_wait_limit(v);
+    if (st == cudaSuccess) {
+        mw::set_plain_wait_limit(v);
+        mw::set_grouped_wait_limit(v);
+    }
     if (st != cudaSuccess) {
         mw::cuda_ok(st, "mwblas_set_wait_limit_ns", "cudaMemcpyToSymbol");
         return current.load();

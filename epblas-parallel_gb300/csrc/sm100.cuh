@@ -121,6 +121,16 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const void *desc, ui
         : "memory");
 }
 
+// Untiled bulk copy global -> shared, completion on `bar`; both addresses and the
+// size are multiples of 16 bytes.
+__device__ __forceinline__ void bulk_load(void *smem_dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(smem_dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 // ---- tcgen05: tensor memory ----------------------------------------------------
 
 // Allocates `ncols` TMEM columns (power of two >= 32); the TMEM address is

@@ -1,6 +1,6 @@
-"""The grouped GEMM's tensor-core tiles (16 x 16 outputs, two rows per warp, four
-columns at a time, k in steps of 16 and chunks of 64, splits from 4096) at their
-edges, against the binary128 oracle, in batches that mix every shape.
+"""The grouped GEMM's tensor-core tiles (8 x 16 outputs, two columns at a time, k in
+steps of 16, copies of 64, accumulators of 256, splits from 4096) at their edges,
+against the binary128 oracle, in batches that mix every shape.
 
 Operands are rounded to 116 bits of their row or column maximum and the rest is
 exact up to one rounding (16 2^-104 k |A| |B| allowed, as for the small tiles of
@@ -14,7 +14,7 @@ from conftest import mwb, orc
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1, 1), (2, 3, 15), (15, 16, 16), (16, 17, 17), (17, 5, 63), (33, 1, 64), (1, 33, 65), (16, 16, 128),
-          (31, 20, 129), (48, 47, 1), (5, 6, 4096), (3, 18, 4100), (9, 4, 9000), (20, 20, 0), (127, 40, 50)]
+          (31, 20, 129), (48, 47, 1), (8, 16, 256), (9, 17, 257), (7, 15, 513), (5, 6, 4096), (3, 18, 4100), (9, 4, 9000), (20, 20, 0), (127, 40, 50)]
 
 
 def batch(gpu, oracle, rng, kind, ta, tb):
