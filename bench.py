@@ -1127,7 +1127,7 @@ def run_workload(args):
                    "tile_chosen": int(lib.lib.mwblas_grouped_tuned_tile()),
                    "tensor_core_min_size_chosen": int(lib.lib.mwblas_grouped_tuned_tensor_min()),
                    "tensor_core_pack_depth_chosen": int(lib.lib.mwblas_grouped_tuned_tensor_pack()),
-                   "launch": "one CUDA graph per batch layout: the persistent integer-pipe kernel for the small "
+                   "launch": "one CUDA graph per batch layout: one kernel over the tiles of the small "
                              "instances, the grouped tensor-core residue GEMMs (one per padding class) for those "
                              "with m, n >= the chosen size and k >= 64"}
             if o:

@@ -3,17 +3,18 @@
 // instances calling mgemm_/mtrsm_, whose nested calls run serially,
 // mgemm_parallel.cpp:53-60).
 //
-// mgemm_grouped: one persistent kernel over all instances. The work list is
-// every (instance, 32x32 output tile, K split); CTAs of 256 threads pull items
-// from an atomic counter, so thousands of uneven instances keep all SMs busy.
-// Each item runs the fixed-point arithmetic of the integer-pipe engine
-// (gemm_fixed.cu, fixgemm.cuh): its A rows / B columns are scaled from an
-// exponent scan over the item's own K range (no pre-pass, no extra scratch),
-// converted to balanced 24-bit digits while staged, and multiplied with
-// exact 64-bit column sums. Items of a split instance write partial tiles as
-// extended floats; the CTA that completes a tile's last split sums the
-// partials in split order (deterministic) and applies alpha/beta with one
-// rounding. The per-call state (descriptors, work counter, split counters,
+// mgemm_grouped: the large instances go to the residue engine (ozaki.cu), the rest
+// to tiles of one kernel over all of them, so that thousands of uneven instances
+// keep all SMs busy. By default these are limb tiles on the tensor cores (their
+// section below); the forced 32 x 32 and 64 x 64 tiles run the fixed-point
+// arithmetic of the integer-pipe engine (gemm_fixed.cu, fixgemm.cuh): CTAs of 256
+// threads pull (instance, tile, K split) items from an atomic counter, and the
+// item's A rows / B columns are scaled from an exponent scan over its own K range
+// (no pre-pass, no extra scratch), converted to balanced 24-bit digits while
+// staged, and multiplied with exact 64-bit column sums. Items of a split instance
+// write partial tiles as extended floats; the CTA that completes a tile's last
+// split sums the partials in split order (deterministic) and applies alpha/beta
+// with one rounding. The per-call state (descriptors, work counter, split counters,
 // partial tiles) is uploaded and the kernel launched from a CUDA graph that is
 // captured once per batch layout and replayed.
 //

@@ -1,5 +1,6 @@
-// Integer fixed-point accumulation of double-double products, for the
-// bandwidth-bound reductions (DOT, GEMV) and the TRSM block inverses.
+// Integer fixed-point accumulation of double-double products, for the complex,
+// band and packed matrix-vector products, the grouped TRSM and the TRSM block
+// inverses (the real DOT and GEMV form theirs on the tensor cores, limbmma.cuh).
 //
 // On this part an FP64 instruction issues at ~1/40 of the integer rate, so a
 // double-double multiply-add on the FP64 pipe (12 instructions) cannot keep

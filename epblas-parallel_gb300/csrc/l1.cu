@@ -475,9 +475,9 @@ __device__ bool block_any(bool b)
 // for 4 turns of 64; then it moves to int32 sums, and after 64 of those (or
 // when a product above the block moves it up) to the warp's extended float.
 //
-// Bound: HBM (32 B per pair). Measured at n = 10^8: 867 -> 598 us (3.69 -> 5.35 TB/s); about 100
-// instructions per pair, where 19 IMAD.WIDE digit products and their digit
-// splits took 223.
+// Bound: HBM (32 B per pair) and instruction issue, both about two thirds busy.
+// Measured at n = 10^8: 867 -> 598 us (3.69 -> 5.35 TB/s); 149 instructions per
+// pair, where 19 IMAD.WIDE digit products and their digit splits took 223.
 constexpr int kDotFlush = 4;            // turns of 64 pairs per move to the int32 sums
 constexpr int kDotFold = 64;            // moves per fold into the extended float
 constexpr int kDotStages = 4;           // turns in flight

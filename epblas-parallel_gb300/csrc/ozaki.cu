@@ -21,13 +21,10 @@
 //     (512 * 180^2 + 361 < 2^24) and after each chunk the accumulator is
 //     reduced modulo p in place; two accumulators alternate so the MMA pipe
 //     keeps running while the epilogue reduces the other one.
-//  4. CRT reconstruction (integer only): X = sum_l c_l * W_l - q * M with
-//     W_l = (M/p_l) * ((M/p_l)^-1 mod p_l) and q = round(sum_l c_l u_l / p_l)
-//     estimated in fp32 (exact because |X| << M by construction), then the
-//     top 106 bits of X become the double-double (hi, lo) with exponents
-//     built directly, scaled back by 2^-(sA_i + sB_j); the alpha/beta update
-//     runs in double-double on the FP64 pipe, which the scheme otherwise
-//     does not touch.
+//  4. CRT reconstruction (integer only): X / M = frac(sum_l c_l u_l / p_l) with
+//     u_l = (M/p_l)^-1 mod p_l, as a 160-bit fraction whose sum over l runs on
+//     the tensor cores; times alpha M, plus beta C, in fixed point and rounded
+//     once to the double-double (hi, lo). The FP64 pipe is not used.
 //
 // A modulus count L of ~27 (8192^3, bits = 106) replaces the 18 FP64
 // instructions per multiply-add of the reference's kernel by 27 fp16
@@ -483,7 +480,7 @@ void launch_residues(int64_t rows, int64_t kdim, const double2 *X, int64_t ld, c
 // A limb pair costs one PRMT (0x6400 | byte is 1024 + byte) and one HFMA2 (times
 // the sign, less 1024); the straight-line decode and a shift below a word serve
 // elements within 2^-20 of their row's bound. 4096^2 operand:
-// 365 -> about 320 instructions per element; 8192 x 2048 294 -> 264 us.
+// 346 -> 281 instructions per element; 8192 x 2048 294 -> 264 us.
 //
 // Four MMAs of M = 128, N = 32, K = 16 (one per element slot v) leave x for
 // element v, modulus l in TMEM column v * 32 + l of lane i. A tile is 16 rows
@@ -1267,15 +1264,16 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
 // and both CTAs' epilogue warps release accumulators on the even CTA's barrier.
 // With long K the tensor pipe bounds it, below K = 2048 the epilogue, which stores
 // 2 bytes per column and row: it packs two columns' residues in 16-bit halves
-// (three instructions a column instead of six) and, up to K = 2048, hands a
+// (three instructions a column instead of six) and, up to K = 3072, hands a
 // buffer back without waiting for its stores, as a cluster-scope release does.
 // 28 moduli, us before, packed, and packed without the wait: 4096 x 4096 x 512
 // 461, 386 and 358; x 1024 692, 621 and 608; x 2048 1179, 1112 and 1105; 1024 x
-// 1024 x 512 42, 39 and 35; 8192 x 8192 x 2048 4728, 4440 and 4397. From K = 4096
-// on the wait costs nothing and the large products, which run at the power cap,
-// are faster with it: 8192 x 8192 x 4096 9000, 8800 and 8980, x 8192 17,370,
-// 17,140 and 18,720. Holding 96 to 128 columns in registers to hand the buffer
-// back sooner spills and loses a factor of 1.3 to 2.7.
+// 1024 x 512 42, 39 and 35; 8192 x 8192 x 2048 4728, 4440 and 4397, x 3072 6450
+// packed and 6365 without the wait. From K = 4096 on the wait costs nothing, and
+// the large products, which run at the power cap, are faster with it: 8192 x 8192
+// x 4096 9000, 8800 and 8980, x 8192 17,370, 17,140 and 18,720. Holding 96 to 128
+// columns in registers to hand the buffer back sooner spills and loses a factor
+// of 1.3 to 2.7.
 constexpr int64_t T2_RELAXED_K = 3072;
 constexpr int T2_STAGES = 6;
 constexpr int T2_A_BYTES = 128 * TC_BK * 2;   // 16 KB

@@ -471,35 +471,37 @@ void mgemm_ozaki_64_(const char *transa, const char *transb, const int64_t *m,
  * flags transa[i]/transb[i], sizes and leading dimensions. The matrix pointers
  * must be 16-byte aligned device (or managed) memory; the per-instance arrays
  * are host arrays.
- * One persistent kernel runs every instance, launched from a CUDA graph that is
- * reused while the batch layout is unchanged. Returns 0 or an error code. */
+ * Runs from a CUDA graph that is reused while the batch layout is unchanged.
+ * Returns 0 or an error code. */
 int mgemm_grouped(int64_t count, const char *transa, const char *transb, const int64_t *m, const int64_t *n,
                   const int64_t *k, const MWBLAS_R *alpha, const MWBLAS_R *const *a, const int64_t *lda,
                   const MWBLAS_R *const *b, const int64_t *ldb, const MWBLAS_R *beta, MWBLAS_R *const *c,
                   const int64_t *ldc);
-/* Autotuner for mgemm_grouped: times the output tile edge (16, 32, 64) and
- * then the split-K policies on this batch (results go to scratch copies; C is
+/* Autotuner for mgemm_grouped: times the tensor-core size and packing depth, the
+ * tiles of the rest (16, 32, 64) and their split-K policies on this batch (results go to scratch copies; C is
  * not modified) and keeps the fastest for batches of the same shape class.
- * *chosen = minimum K per split (0 = none); the tile edge is returned by
+ * *chosen = minimum K per split (0 = none); the tiles are returned by
  * mwblas_grouped_tuned_tile(). */
 int mgemm_grouped_tune(int64_t count, const char *transa, const char *transb, const int64_t *m,
                        const int64_t *n, const int64_t *k, const MWBLAS_R *alpha, const MWBLAS_R *const *a,
                        const int64_t *lda, const MWBLAS_R *const *b, const int64_t *ldb, const MWBLAS_R *beta,
                        MWBLAS_R *const *c, const int64_t *ldc, int *chosen);
-/* Tile edge (16, 32 or 64) chosen by this thread's most recent
+/* Tiles (16, 32 or 64, below) chosen by this thread's most recent
  * mgemm_grouped_tune call (0 before any). No counterpart in the reference. */
 int mwblas_grouped_tuned_tile(void);
-/* Forces mgemm_grouped's tile edge (16, 32 or 64; anything else = 0 = the
- * tuned or default choice). All give results within the same bound. Returns
- * the previous setting. */
+/* Forces mgemm_grouped's tiles for the instances outside the residue engine: 16 =
+ * limb tiles on the tensor cores (8 x 16 outputs; the default; scratch of 32 bytes
+ * per operand entry, at most 1 GiB and one instance), 32 or 64 = square tiles on
+ * the integer pipes; anything else = 0 = the tuned or default choice. All give
+ * results within the same bound. Returns the previous setting. */
 int mwblas_set_grouped_tile(int tile);
 /* mgemm_grouped runs instances with m, n >= size and 64 <= k <= 16384 on the
  * tensor cores (Ozaki scheme, full 106-bit width, padded to classes of
  * 256-row/column and 64..512-deep tiles, one residue GEMM per class) and the
- * rest on the integer pipes; 0 = none, -1 = the tuned or default choice
+ * rest on the tiles above; 0 = none, -1 = the tuned or default choice
  * (default 128). Returns the previous setting. mwblas_grouped_tuned_tensor_min
  * returns the size this thread's most recent mgemm_grouped_tune chose (0 =
- * integer pipes only). No counterpart in the reference. */
+ * tiles only). No counterpart in the reference. */
 int mwblas_set_grouped_tensor_min(int size);
 int mwblas_grouped_tuned_tensor_min(void);
 /* mgemm_grouped packs the remaining instances with k >= kmin several to a
