@@ -96,19 +96,23 @@ __global__ void k_trsm_diag_right(int64_t c0, int nb, int64_t nrows, const doubl
 }
 
 // Inverses of the 32 x 32 diagonal blocks of op(A) (the last block may be
-// shorter), one CTA per block, four threads per column c of the inverse:
-// solve op(A)_blk x = e_c by substitution over all rows (x is zero above c
-// for a lower triangle, so every thread walks the same rows and the block
-// entries are shared-memory broadcasts). The four threads of a column split
-// each sum sum_p L(r,p) x(p) by p mod 4, accumulate their shares in integer
-// fixed point (fixacc.cuh) and add the four results as extended floats in a
-// fixed order (lanes 0 + 2, 1 + 3, then the two), rounded once; each row is
-// then multiplied by the double-double reciprocal of the diagonal, as the
-// reference's substitution does (mtrsm_serial.cpp:144).
+// shorter), one CTA per block: the two 16 x 16 halves of its diagonal at the same
+// time, four threads per column c of each inverse, then the block between them as
+// two products. A half solves op(A)_half x = e_c by substitution over all rows (x
+// is zero above c for a lower triangle, so every thread walks the same rows and
+// the block entries are shared-memory broadcasts). The four threads of a column
+// split each sum sum_p L(r,p) x(p) by p mod 4, accumulate their shares in integer
+// fixed point (fixacc.cuh) and add the four results as extended floats in a fixed
+// order (lanes 0 + 2, 1 + 3, then the two), rounded once; each row is then
+// multiplied by the double-double reciprocal of the diagonal, as the reference's
+// substitution does (mtrsm_serial.cpp:144).
+// Bound: the latency of the rows in turn, about 4 us each: 128 blocks 124 us with
+// 32 rows in turn, now 78.
 // Inv: the diagonal of order-nb blocks, block b at Inv + b*nb*nb, column-major with
 // leading dimension nb; the rest of each block is zero already.
-constexpr int kInvNB = 32;   // order of the directly inverted blocks (merged up to the leaf order)
-constexpr int kInvSplit = 4;  // threads per column
+constexpr int kInvNB = 32;          // order of the blocks (merged up to the leaf order)
+constexpr int kInvH = kInvNB / 2;   // order of the halves
+constexpr int kInvSplit = 4;        // threads per column
 
 __global__ void __launch_bounds__(kInvNB * kInvSplit) k_trsm_diag_inv(int64_t na, const double2 *__restrict__ A,
                                                                       int64_t lda, bool trans, bool lower, bool unit,
@@ -133,32 +137,70 @@ __global__ void __launch_bounds__(kInvNB * kInvSplit) k_trsm_diag_inv(int64_t na
         sInvDiag[r] = make_double2(iv.hi, iv.lo);
     }
     __syncthreads();
-    const int c = threadIdx.x / kInvSplit, part = threadIdx.x % kInvSplit;
-    const bool active = c < nb;   // every lane stays for the shuffles
     const fx::Op one = fx::decode(make_double2(1.0, 0.0));
     const int64_t od = o % nbinv;   // the block's place in its order-nbinv block
-    double2 *out = Inv + (o - od) * nbinv + od + (od + c) * nbinv;
-    for (int s = 0; s < nb; ++s) {
-        const int r = lower ? s : nb - 1 - s;
+    double2 *out = Inv + (o - od) * nbinv + od + od * nbinv;
+    auto put = [&](int r, int c, double h, double l) { out[r + (int64_t)c * nbinv] = make_double2(h, l); };
+    {
+        // the two halves' inverses, 64 threads each
+        const int base = threadIdx.x < 64 ? 0 : kInvH, nh = max(0, min(kInvH, nb - base));
+        const int c = (threadIdx.x & 63) / kInvSplit, part = threadIdx.x % kInvSplit;
+        const bool active = c < nh;   // every lane stays for the shuffles
+        for (int s = 0; s < nh; ++s) {
+            const int r = lower ? s : nh - 1 - s;
+            fx::Acc acc;
+            acc.reset();
+            if (active) {
+                if (r == c && part == 0) acc.add_prod(one, one);
+                const int p0 = lower ? 0 : r + 1, p1 = lower ? r : nh;
+                for (int p = p0 + part; p < p1; p += kInvSplit)
+                    acc.add_prod(fx::from_pod(sA[(base + p) * kInvNB + base + r]),
+                                 fx::from_pod(sX[(base + p) * kInvNB + base + c]));
+            }
+            xfp::XF v = acc.finish();
+            v = xfp::xf_add(v, fx::xf_shfl_down(v, 2));   // parts 0 + 2, 1 + 3
+            v = xfp::xf_add(v, fx::xf_shfl_down(v, 1));   // (0 + 2) + (1 + 3)
+            if (active && part == 0) {
+                double h, l;
+                xfp::xf_to_dd(v, h, l);
+                const dd::real x = dd::mul_fast(dd::make(h, l), dd::load(&sInvDiag[base + r]));
+                sX[(base + r) * kInvNB + base + c] = fx::to_pod(fx::decode(make_double2(x.hi, x.lo)));
+                put(base + r, base + c, x.hi, x.lo);
+            }
+            __syncwarp();   // x_c(r) is read by the column's other three threads (same warp) from the next row on
+        }
+    }
+    if (nb <= kInvH) return;
+    __syncthreads();
+    // The block between them, as in trsm_merge_inverses (sA holds -op(A)): T = -L21 I1
+    // or -U12 I2, kept in sX's other triangle, then I2 T or I1 T.
+    const int n2 = nb - kInvH, rows = lower ? n2 : kInvH, cols = lower ? kInvH : n2;
+    const int tr = lower ? 0 : kInvH, tc = lower ? kInvH : 0;   // where T is kept
+    for (int idx = threadIdx.x; idx < rows * cols; idx += blockDim.x) {
+        const int i = idx % rows, c = idx / rows;
         fx::Acc acc;
         acc.reset();
-        if (active) {
-            if (r == c && part == 0) acc.add_prod(one, one);
-            const int p0 = lower ? 0 : r + 1, p1 = lower ? r : nb;
-            for (int p = p0 + part; p < p1; p += kInvSplit)
-                acc.add_prod(fx::from_pod(sA[p * kInvNB + r]), fx::from_pod(sX[p * kInvNB + c]));
-        }
-        xfp::XF v = acc.finish();
-        v = xfp::xf_add(v, fx::xf_shfl_down(v, 2));   // parts 0 + 2, 1 + 3
-        v = xfp::xf_add(v, fx::xf_shfl_down(v, 1));   // (0 + 2) + (1 + 3)
-        if (active && part == 0) {
-            double h, l;
-            xfp::xf_to_dd(v, h, l);
-            const dd::real x = dd::mul_fast(dd::make(h, l), dd::load(&sInvDiag[r]));
-            sX[r * kInvNB + c] = fx::to_pod(fx::decode(make_double2(x.hi, x.lo)));
-            out[r] = make_double2(x.hi, x.lo);
-        }
-        __syncwarp();   // x_c(r) is read by the column's other three threads (same warp) from the next row on
+        const int p0 = lower ? c : 0, p1 = lower ? kInvH : c + 1;
+        for (int p = p0; p < p1; ++p)
+            acc.add_prod(fx::from_pod(lower ? sA[p * kInvNB + kInvH + i] : sA[(kInvH + p) * kInvNB + i]),
+                         fx::from_pod(lower ? sX[p * kInvNB + c] : sX[(kInvH + p) * kInvNB + kInvH + c]));
+        double h, l;
+        xfp::xf_to_dd(acc.finish(), h, l);
+        sX[(tr + i) * kInvNB + tc + c] = fx::to_pod(fx::decode(make_double2(h, l)));
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < rows * cols; idx += blockDim.x) {
+        const int i = idx % rows, c = idx / rows;
+        fx::Acc acc;
+        acc.reset();
+        const int p0 = lower ? 0 : i, p1 = lower ? i + 1 : kInvH;
+        for (int p = p0; p < p1; ++p)
+            acc.add_prod(fx::from_pod(lower ? sX[(kInvH + i) * kInvNB + kInvH + p] : sX[i * kInvNB + p]),
+                         fx::from_pod(sX[(tr + p) * kInvNB + tc + c]));
+        double h, l;
+        xfp::xf_to_dd(acc.finish(), h, l);
+        if (lower) put(kInvH + i, c, h, l);
+        else put(i, kInvH + c, h, l);
     }
 }
 
