@@ -752,11 +752,26 @@ __device__ __forceinline__ void rt_finish(const RtCta &c, const OzResParams &P, 
     }
 }
 
-template <bool ROWC>
+// An operand of the conversion: row r and place c along k of op(X) lie at
+// X[r + c ld] (rowc) or X[c + r ld]; out[l][r][c] with plane_rows rows a plane,
+// rows_pad of them written.
+struct ResOp {
+    const double2 *X;
+    const int *rexp;
+    __half *out;
+    int64_t ld, plane_rows, rows, rows_pad;
+    int bits, rowc;
+};
+
+// WHAT 0, 1: operand a alone, of that rowc. 2: both in one launch, the row tiles of
+// a, then b's: two launches in turn leave the SMs idle at the end of the first, and
+// small operands fill them once. us for both operands, apart and in one: 512^2 30
+// and 20, 1024^2 51 and 40, 2048^2 143 and 138, 4096^2 521 and 520, 8192^2 2138 and
+// 2240; TRSM of order 4096, with seven such products, 2113 and 2050.
+constexpr int64_t RT_BOTH = 1 << 25;   // entries of both up to which they share a launch
+template <int WHAT>
 __global__ void __launch_bounds__(RT_THREADS, 4)
-    k_oz_residues_tc(int64_t rows, int64_t kdim, const double2 *__restrict__ X, int64_t ld,
-                     const int *__restrict__ rexp, int bits, OzResParams P, __half *__restrict__ out, int64_t rows_pad,
-                     int64_t kpad, int64_t plane_rows, int *status)
+    k_oz_residues_tc(const ResOp a, const ResOp b, int kdim, OzResParams P, int64_t kpad, int *status)
 {
     extern __shared__ uint8_t rt_raw[];
     const RtCta cta = rt_setup(rt_raw, P);
@@ -764,46 +779,52 @@ __global__ void __launch_bounds__(RT_THREADS, 4)
     // tiles t = blockIdx.x + i * gridDim.x as (row, column) tile pairs, stepped
     // without divisions (32-bit: fewer than 2^31 tiles)
     const int nct = (int)(kpad / RT_COLS);
-    const int ntr = (int)((rows_pad + RT_ROWS - 1) / RT_ROWS);
+    const int ntra = (int)((a.rows_pad + RT_ROWS - 1) / RT_ROWS);
+    const int ntr = WHAT == 2 ? ntra + (int)((b.rows_pad + RT_ROWS - 1) / RT_ROWS) : ntra;
     const int rl = tid >> 3, cq = (tid & 7) * 4;
-    const int64_t plane = plane_rows * kpad;
     const int step_r = (int)(gridDim.x / (unsigned)nct), step_c = (int)(gridDim.x % (unsigned)nct);
 
     auto fetch = [&](int tr, int tc, double2 (&v)[4]) {
-        const int r = tr * RT_ROWS + rl, c = tc * RT_COLS + cq;
-        const bool rok = r < rows;
-        const double2 *x = ROWC ? X + r + (int64_t)c * ld : X + c + (int64_t)r * ld;
+        const bool first = WHAT != 2 || tr < ntra, rowc = WHAT == 2 ? (first ? a.rowc : b.rowc) != 0 : WHAT == 1;
+        const ResOp &q = first ? a : b;
+        const int r = (first ? tr : tr - ntra) * RT_ROWS + rl, c = tc * RT_COLS + cq;
+        const bool rok = r < q.rows;
+        const double2 *x = rowc ? q.X + r + (int64_t)c * q.ld : q.X + c + (int64_t)r * q.ld;
+        const int64_t step = rowc ? q.ld : 1;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            v[u] = (rok && c + u < kdim) ? x[ROWC ? u * ld : u] : make_double2(0.0, 0.0);
+        for (int u = 0; u < 4; ++u, x += step) v[u] = (rok && c + u < kdim) ? *x : make_double2(0.0, 0.0);
     };
 
     double2 cur[4];
     int tr = (int)(blockIdx.x / (unsigned)nct), tc = (int)(blockIdx.x % (unsigned)nct);
     if (tr < ntr) fetch(tr, tc, cur);
     __half *po = nullptr;   // the previous tile (its sums in TMEM): this thread's output
+    int64_t pplane = 0;
     bool pok = false, have_prev = false;
     int it = 0, failed = 0;
     for (; tr < ntr; ++it) {
-        const int b = it & 1;
-        const int r = tr * RT_ROWS + rl;
-        rt_limbs(cta.sA + b * RT_TILE_BYTES, tid, cur, r < rows ? rexp[r] : kNoExp, bits);
-        __half *o = out + (int64_t)r * kpad + tc * RT_COLS + cq;
-        const bool ok = r < rows_pad;
-        int tr2 = tr + step_r, tc2 = tc + step_c;
-        if (tc2 >= nct) {
-            tc2 -= nct;
-            tr2 += 1;
+        const int buf = it & 1;
+        const bool first = WHAT != 2 || tr < ntra;
+        const ResOp &q = first ? a : b;
+        const int r = (first ? tr : tr - ntra) * RT_ROWS + rl;
+        rt_limbs(cta.sA + buf * RT_TILE_BYTES, tid, cur, r < q.rows ? q.rexp[r] : kNoExp, q.bits);
+        __half *o = q.out + (int64_t)r * kpad + tc * RT_COLS + cq;
+        const int64_t plane = q.plane_rows * kpad;
+        const bool ok = r < q.rows_pad;
+        tr += step_r;
+        tc += step_c;
+        if (tc >= nct) {
+            tc -= nct;
+            tr += 1;
         }
-        if (tr2 < ntr) fetch(tr2, tc2, cur);   // in flight during the epilogue and the MMA below
-        if (!rt_step(cta, P, b, it, have_prev, po, plane, pok, status, failed)) break;
+        if (tr < ntr) fetch(tr, tc, cur);   // in flight during the epilogue and the MMA below
+        if (!rt_step(cta, P, buf, it, have_prev, po, pplane, pok, status, failed)) break;
         po = o;
+        pplane = plane;
         pok = ok;
         have_prev = true;
-        tr = tr2;
-        tc = tc2;
     }
-    rt_finish(cta, P, it, have_prev, po, plane, pok, status, failed);
+    rt_finish(cta, P, it, have_prev, po, pplane, pok, status, failed);
     rt_teardown(cta);
 }
 
@@ -811,25 +832,18 @@ std::atomic<int> g_res_tc{1};   // mwblas_set_residue_tc
 
 // Real operands on the tensor-core path when the layout allows it (k padded
 // to the tile width, at most 32 moduli); false: the caller uses the FMA path.
-template <bool ROWC>
-bool launch_residues_tc(int64_t rows, int64_t kdim, const double2 *X, int64_t ld, const int *rexp, int bits,
-                        const OzResParams &rp, __half *out, int64_t rows_pad, int64_t kpad, int64_t plane_rows)
+bool launch_residues_tc(const ResOp &a, const ResOp &b, int64_t kdim, const OzResParams &rp, int64_t kpad)
 {
-    if (g_res_tc.load() == 0 || rp.nmod > RT_MAX_MOD || kpad % RT_COLS != 0 || rows_pad <= 0 || !ozaki_available())
+    if (g_res_tc.load() == 0 || rp.nmod > RT_MAX_MOD || kpad % RT_COLS != 0 || a.rows_pad <= 0 || !ozaki_available())
         return false;
-    static int attr_set[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!attr_set[dev & 63]) {
-        cudaFuncSetAttribute(k_oz_residues_tc<ROWC>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM);
-        attr_set[dev & 63] = 1;
-    }
-    const int64_t ntiles = ((rows_pad + RT_ROWS - 1) / RT_ROWS) * (kpad / RT_COLS);
-    if (ntiles >= ((int64_t)1 << 31) || rows_pad >= ((int64_t)1 << 31)) return false;
+    const int64_t ntr = (a.rows_pad + RT_ROWS - 1) / RT_ROWS + (b.rows_pad + RT_ROWS - 1) / RT_ROWS;
+    const int64_t ntiles = ntr * (kpad / RT_COLS);
+    if (ntiles >= ((int64_t)1 << 31) || std::max(a.rows_pad, b.rows_pad) >= ((int64_t)1 << 31)) return false;
     int64_t grid = 4 * (int64_t)device_sm_count();
     if (grid > ntiles) grid = ntiles;
-    k_oz_residues_tc<ROWC><<<(unsigned)grid, RT_THREADS, RT_SMEM, stream()>>>(
-        rows, kdim, X, ld, rexp, bits, rp, out, rows_pad, kpad, plane_rows, device_status_word());
+    auto kern = b.rows_pad > 0 ? k_oz_residues_tc<2> : a.rowc ? k_oz_residues_tc<1> : k_oz_residues_tc<0>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM);
+    kern<<<(unsigned)grid, RT_THREADS, RT_SMEM, stream()>>>(a, b, (int)kdim, rp, kpad, device_status_word());
     count_launch();
     return true;
 }
@@ -2402,6 +2416,9 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
     // Rows [i0, i0 + ni) of op(A), with their exponent bounds, go to residue
     // rows [i0, i0 + rpad) of every plane (zeros past m).
     auto a_rows_at = [&](int64_t i0) { return (const double2 *)g.A + (int64_t)E * (g.ta ? i0 * g.lda : i0); };
+    auto res_a = [&](int64_t i0, int64_t ni, int64_t rpad) {
+        return ResOp{a_rows_at(i0), ea + i0, Ares + i0 * Kp, g.lda, Mp, ni, rpad, bits_a, g.ta ? 0 : 1};
+    };
     auto convert_A = [&](int64_t i0, int64_t ni, int64_t rpad) {
         const double2 *Ai = a_rows_at(i0);
         __half *Ao = Ares + i0 * Kp;
@@ -2409,9 +2426,7 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             if (!g.ta) launch_residues<true, true>(ni, k, Ai, g.lda, ea + i0, bits_a, rp, Ao, rpad, Kp, g.ca, Mp);
             else launch_residues<false, true>(ni, k, Ai, g.lda, ea + i0, bits_a, rp, Ao, rpad, Kp, g.ca, Mp);
         } else {
-            const bool tc = !g.ta ? launch_residues_tc<true>(ni, k, Ai, g.lda, ea + i0, bits_a, rp, Ao, rpad, Kp, Mp)
-                                  : launch_residues_tc<false>(ni, k, Ai, g.lda, ea + i0, bits_a, rp, Ao, rpad, Kp, Mp);
-            if (tc) return;
+            if (launch_residues_tc(res_a(i0, ni, rpad), ResOp{}, k, rp, Kp)) return;
             if (!g.ta) launch_residues<true, false>(ni, k, Ai, g.lda, ea + i0, bits_a, rp, Ao, rpad, Kp, 0, Mp);
             else launch_residues<false, false>(ni, k, Ai, g.lda, ea + i0, bits_a, rp, Ao, rpad, Kp, 0, Mp);
         }
@@ -2424,9 +2439,10 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
         convert_A(i0, ni, i0 + h >= m ? Mp - i0 : ni);
     };
     const int64_t n_ablocks = a_blocks ? (m + hs->a_rows - 1) / hs->a_rows : 0;
-    if (!a_blocks) {
+    const bool at_once = !hs && !cplx && !shared_ops && (m + n) * k <= RT_BOTH;   // both are here, and small
+    if (!a_blocks && !at_once) {
         convert_A(0, m, Mp);
-    } else if (!blocked) {
+    } else if (a_blocks && !blocked) {
         for (int64_t ib = 0; ib < n_ablocks; ++ib) a_block(ib);
     }
     // op(B)(p, j) = B[p + j*ldb] is contiguous along k; op(B) = B^T along the
@@ -2436,6 +2452,9 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
     auto exp_B = [&](int64_t j0, int64_t nn) {
         launch_exp_cols_of_op(b_cols(j0), g.tb ? nn : k, g.tb ? k : nn, g.ldb, g.tb, E, eb + j0);
     };
+    auto res_b = [&](int64_t j0, int64_t nn, int64_t rpad) {
+        return ResOp{b_cols(j0), eb + j0, Bres + j0 * Kp, g.ldb, Np, nn, rpad, bits_b, g.tb ? 1 : 0};
+    };
     auto convert_B = [&](int64_t j0, int64_t nn, int64_t rpad) {
         const double2 *Bj = b_cols(j0);
         __half *Bo = Bres + j0 * Kp;
@@ -2443,9 +2462,7 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             if (!g.tb) launch_residues<false, true>(nn, k, Bj, g.ldb, eb + j0, bits_b, rp, Bo, rpad, Kp, g.cb, Np);
             else launch_residues<true, true>(nn, k, Bj, g.ldb, eb + j0, bits_b, rp, Bo, rpad, Kp, g.cb, Np);
         } else {
-            const bool tc = !g.tb ? launch_residues_tc<false>(nn, k, Bj, g.ldb, eb + j0, bits_b, rp, Bo, rpad, Kp, Np)
-                                  : launch_residues_tc<true>(nn, k, Bj, g.ldb, eb + j0, bits_b, rp, Bo, rpad, Kp, Np);
-            if (tc) return;
+            if (launch_residues_tc(res_b(j0, nn, rpad), ResOp{}, k, rp, Kp)) return;
             if (!g.tb) launch_residues<false, false>(nn, k, Bj, g.ldb, eb + j0, bits_b, rp, Bo, rpad, Kp, 0, Np);
             else launch_residues<true, false>(nn, k, Bj, g.ldb, eb + j0, bits_b, rp, Bo, rpad, Kp, 0, Np);
         }
@@ -2455,7 +2472,12 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             wait_event(hs->b_ready, routine);
             if (!shared_ops) exp_B(0, n);
         }
-        if (!shared_ops) convert_B(0, n, Np);
+        if (at_once && !launch_residues_tc(res_a(0, m, Mp), res_b(0, n, Np), k, rp, Kp)) {
+            convert_A(0, m, Mp);
+            convert_B(0, n, Np);
+        } else if (!at_once && !shared_ops) {
+            convert_B(0, n, Np);
+        }
     }
 
     // 4. residue GEMMs, one batch entry per (component, modulus)
