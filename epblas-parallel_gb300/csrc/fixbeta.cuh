@@ -6,7 +6,7 @@
 
 namespace mw {
 
-// a += (neg ? -1 : 1) * beta part b (b.w[3] != 0; kind 1: one) times the
+// a += (neg ? -1 : 1) * beta part b (which may be zero; kind 1: one) times the
 // double-double c; false where c needs the general path (a is unchanged then).
 __device__ __forceinline__ bool add_beta_c(fxr::Fix &a, double2 c, const xw::XW &b, bool one, uint32_t neg)
 {
@@ -30,7 +30,7 @@ __device__ __forceinline__ bool add_beta_c(fxr::Fix &a, double2 c, const xw::XW 
         e += b.e + 86;
         neg ^= b.neg;
     }
-    fxr::add(a, q, e, neg ^ (hh >> 31));
+    fxr::add_term(a, q, e, neg ^ (hh >> 31));
     return true;
 }
 

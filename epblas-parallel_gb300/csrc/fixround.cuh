@@ -214,7 +214,8 @@ XW_HD void shr6(uint32_t w[6], int d)
 XW_HD bool is_zero(const Fix &a) { return (a.w[0] | a.w[1] | a.w[2] | a.w[3] | a.w[4] | a.w[5]) == 0u; }
 
 // a += (neg ? -q : q) * 2^eq, cut below the unit of the coarser operand
-// (a zero a takes q's frame).
+// (a zero a takes q's frame). q's frame counts even where q is zero: sums
+// whose terms can be zero use add_term.
 XW_HD void add(Fix &a, const uint32_t q[5], int eq, uint32_t neg)
 {
     const int d = is_zero(a) ? -192 : a.e - eq;
@@ -236,6 +237,14 @@ XW_HD void add(Fix &a, const uint32_t q[5], int eq, uint32_t neg)
     for (int t = 0; t < 6; ++t) a.w[t] = k[t];
     a.e = sq ? a.e : eq;
     a.neg = nk ^ (m & 1u);
+}
+
+// add for a term that may be zero: a zero has no frame, so a stays as it is
+// (beta = (0, b) on a complex C: a zero product of exponent -31 would cut the
+// sum, held to 2^-139, at 2^-31).
+XW_HD void add_term(Fix &a, const uint32_t q[5], int eq, uint32_t neg)
+{
+    if ((q[0] | q[1] | q[2] | q[3] | q[4]) != 0u) add(a, q, eq, neg);
 }
 
 // Round to double-double as xword.cuh's to_dd: hi the top 53 bits, rounded half

@@ -2064,9 +2064,9 @@ __global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const ui
         if (A.has_im) {
             uint32_t p[5];
             fxr::mul54(xi, A.im, p);
-            fxr::add(vr, p, vr.e, ni ^ A.neg_im ^ 1u);
+            fxr::add_term(vr, p, vr.e, ni ^ A.neg_im ^ 1u);
             fxr::mul54(xr, A.im, p);
-            fxr::add(vi, p, vi.e, nr ^ A.neg_im);
+            fxr::add_term(vi, p, vi.e, nr ^ A.neg_im);
         }
         bool fast = live;
         if (beta_kind != 0 && live) {
