@@ -286,11 +286,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
                                                                     int total, int *tile_counters,
                                                                     fx::XFPod *partials,
                                                                     const unsigned char *__restrict__ limbs,
-                                                                    const int *__restrict__ ex, int *status)
+                                                                    const int *__restrict__ ex, int *status,
+                                                                    int lose_loads)
 {
     extern __shared__ unsigned char s_dyn[];   // stages, then the sums of two tiles
     __shared__ uint64_t full[LT_STAGES], empty[LT_STAGES], accf[2], acce[2], sumf[LT_GROUPS], sume[2];
     __shared__ uint64_t itemf[2], iteme[2], drain;
+    __shared__ uint64_t partf[LT_GROUPS], lastf[LT_GROUPS];   // a group's partial sums are out; s_last is set
     __shared__ LtItem items[2 * LT_BATCH];
     __shared__ uint32_t s_tmem;
     __shared__ int s_last[LT_GROUPS];
@@ -309,7 +311,11 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
             sm100::mbar_init(&acce[q], LT_EXT);
             sm100::mbar_init(&sume[q], 4);
         }
-        for (int q = 0; q < LT_GROUPS; ++q) sm100::mbar_init(&sumf[q], LT_EXT);
+        for (int q = 0; q < LT_GROUPS; ++q) {
+            sm100::mbar_init(&sumf[q], LT_EXT);
+            sm100::mbar_init(&partf[q], 4);
+            sm100::mbar_init(&lastf[q], 1);
+        }
         for (int q = 0; q < 2; ++q) {
             sm100::mbar_init(&itemf[q], 1);
             sm100::mbar_init(&iteme[q], 2 + LT_EXT + LT_FIN);
@@ -368,7 +374,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
     } else if (warp == 2 + LT_EXT + LT_FIN) {
         uint32_t gs = 0;   // stages filled
         bool ok = true;
-        for (int it = 0; it < n_items && ok; ++it) {
+        // lose_loads (a failure-injection hook): no copy at all, so that nothing is in
+        // flight and the MMA warp's first wait runs out
+        for (int it = 0; it < n_items && ok && !lose_loads; ++it) {
             if (!item(it, it - 1, 1)) break;
             const LtItem &x = items[it % (2 * LT_BATCH)];
             const unsigned char *pA = limbs + x.a * LT_BLOCK, *pB = limbs + x.b * LT_BLOCK;
@@ -500,6 +508,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
     } else {
         const int group = (warp - 2 - LT_EXT) >> 2, part = (warp - 2 - LT_EXT) & 3;
         const int orow = lane & 7, ocol = 4 * part + (lane >> 3), out = ocol * LT_M + orow;
+        uint32_t splits = 0;   // split tiles of this group so far
         for (int it = group; it < n_items; it += LT_GROUPS) {
             const int sb = it & 1;
             const unsigned long long *at = sums + sb * LT_SUMS + out * LT_ROW;
@@ -568,11 +577,22 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
                 fx::XFPod *base = partials + (d.part_begin + (int64_t)x.tile * d.splitk) * (LT_M * LT_N) + out;
                 base[x.split * (LT_M * LT_N)] = fx::to_pod(v, bad);
                 __threadfence();
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(128) : "memory");
-                if (part == 0 && lane == 0)
-                    s_last[group] = atomicAdd(&tile_counters[d.tile_begin + x.tile], 1) == d.splitk - 1;
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(128) : "memory");
-                if (!s_last[group]) continue;
+                __syncwarp();
+                // the group's warps meet at barriers with a limit (not at a named barrier): one
+                // of them may have left after a wait that gave up
+                const uint32_t phase = splits++ & 1;
+                if (lane == 0) sm100::mbar_arrive(&partf[group]);
+                if (part == 0) {
+                    if (!__all_sync(0xffffffffu, sm100::mbar_wait(&partf[group], phase, status, 6))) break;
+                    if (lane == 0) {
+                        s_last[group] = atomicAdd(&tile_counters[d.tile_begin + x.tile], 1) == d.splitk - 1;
+                        sm100::mbar_arrive(&lastf[group]);
+                    }
+                }
+                if (!__all_sync(0xffffffffu, sm100::mbar_wait(&lastf[group], phase, status, 6))) break;
+                const bool finish = s_last[group] != 0;
+                __syncwarp();
+                if (!finish) continue;
                 __threadfence();
                 v.zero = true; v.neg = false; v.m = 0; v.e = 0;
                 bad = false;
@@ -1202,6 +1222,9 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
             if (!ozgroup_prepare(pl.oz, pl.oz_items, routine)) return false;
         }
     }
+    // a launch with lost copies (test hook) is not kept in a graph
+    const int lose = pl.tile == LT && pl.total > 0 ? take_lost_load_injection() : 0;
+    if (lose) use_graph = false;
     // the integer-pipe or limb-tile part on stream q; its counters start at zero
     auto enqueue = [&](cudaStream_t q) {
         cudaMemsetAsync(counter, 0, cnt_bytes, q);
@@ -1217,11 +1240,11 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
             const int wgrid = (int)std::min<int64_t>(wv.work, sms);
             k_gemm_grouped_limb<<<wgrid, LT_THREADS, LT_SMEM, q>>>(ddesc + wv.first, wv.count, (int)wv.work,
                                                                   tile_counters, partials, limbs, ex,
-                                                                  device_status_word());
+                                                                  device_status_word(), lose);
         }
     };
     if (!use_graph) {
-        pl.key = key;
+        pl.key = lose ? 0 : key;
         if (pl.total > 0) {
             enqueue(s);
             count_launch(pl.tile == LT ? 2 * (int64_t)pl.waves.size() : 1);

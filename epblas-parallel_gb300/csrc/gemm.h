@@ -51,6 +51,8 @@ bool gemm_ozaki_cplx(const GemmArgs &g, int bits, const char *routine);
 void set_plain_wait_limit(uint64_t ns);
 void set_grouped_wait_limit(uint64_t ns);
 int ozaki_last_moduli();
+// Whether the next tensor-core launch is to lose its operand loads (test hook).
+int take_lost_load_injection();
 
 // Grouped products on the tensor cores (instances of mgemm_grouped):
 // ozgroup_prepare allocates and uploads everything for a list of real

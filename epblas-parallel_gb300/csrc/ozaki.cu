@@ -113,8 +113,12 @@ int g_last_bits[2] = {0, 0};   // bits of op(A), op(B) in the most recent call
 int g_mma_kind = -1;   // 0 tcgen05 per tile, 1 SIMT cross-check, 2 tcgen05 persistent, 3 CTA pairs (default)
 
 // Failure injection for the bounded-wait path: the next g_lose_loads launches
-// of the CTA-pair residue GEMM issue no operand loads (see k_oz_gemm_tc_2sm).
+// of the CTA-pair residue GEMM (k_oz_gemm_tc_2sm) or of the grouped limb tiles
+// issue no operand loads.
 std::atomic<int> g_lose_loads{0};
+
+}  // namespace
+
 int take_lost_load_injection()
 {
     int v = g_lose_loads.load();
@@ -122,6 +126,8 @@ int take_lost_load_injection()
     }
     return v > 0 ? 1 : 0;
 }
+
+namespace {
 
 // Optional per-phase timing with CUDA events on the library stream.
 enum { PH_EXP = 0, PH_RES, PH_GEMM, PH_REC, PH_N };

@@ -629,8 +629,8 @@ void mwblas_debug_fail_alloc_after(int64_t count);
  * Returns the previous limit. No counterpart in the reference. */
 uint64_t mwblas_set_wait_limit_ns(uint64_t ns);
 
-/* Test hook: the next `count` launches of the CTA-pair residue GEMM issue no
- * operand loads, so their first wait for a landed operand stage runs out (with
+/* Test hook: the next `count` launches of the CTA-pair residue GEMM or of the
+ * grouped limb tiles issue no operand loads, so their first wait for a landed operand stage runs out (with
  * nothing in flight) and the call reports MWBLAS_ERR_TIMEOUT. Exercises the
  * timeout path without a GPU fault. */
 void mwblas_debug_lose_operand_loads(int count);
