@@ -1184,6 +1184,11 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     const size_t need = d_bytes + cnt_bytes + part_bytes + limb_bytes_ + ex_bytes + 1024;
     const uint64_t key = plan_key(pl);
     cudaStream_t s = stream();
+    // The key names the layout whose descriptors the buffers hold: none from here
+    // until every step for a new one has succeeded, so that a call that fails half
+    // way cannot leave the old key over memory that is gone or rewritten.
+    const bool same = pl.key == key && pl.dev_bytes >= need;
+    if (!same) pl.key = 0;
     if (pl.dev_bytes < need) {
         if (pl.exec) {
             cudaGraphExecDestroy(pl.exec);
@@ -1192,7 +1197,7 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
         if (pl.dev) cudaFree(pl.dev);
         pl.dev = nullptr;
         pl.dev_bytes = 0;
-        if (!cuda_ok(cudaMalloc(&pl.dev, need), routine, "grouped plan buffer")) return false;
+        if (!(pl.dev = plan_alloc(need, routine))) return false;
         pl.dev_bytes = need;
         // the tile counters start at zero (each replay leaves them so)
         if (!cuda_ok(cudaMemset(pl.dev, 0, d_bytes + cnt_bytes + 512), routine, "grouped plan clear")) return false;
@@ -1211,7 +1216,7 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     int *ex = (int *)(base + (limb_off + limb_bytes_ + 255) / 256 * 256);
     const int sms = device_sm_count();
     const int grid = (int)std::min<int64_t>(pl.total, (int64_t)sms * 16);
-    if (pl.key != key) {
+    if (!same) {
         // descriptors change only with the batch layout; upload outside the graph
         if (!pl.descs.empty() &&
             !cuda_ok(cudaMemcpyAsync(ddesc, pl.descs.data(), d_bytes, cudaMemcpyHostToDevice, s), routine,
@@ -1252,7 +1257,7 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
         if (pl.oz && ozgroup_count(pl.oz) > 0) ozgroup_launch(pl.oz, s);
         return cuda_ok(cudaGetLastError(), routine, "grouped launch");
     }
-    if (!pl.exec || pl.key != key) {
+    if (!pl.exec || !same) {
         if (pl.exec) {
             cudaGraphExecDestroy(pl.exec);
             pl.exec = nullptr;
@@ -1314,7 +1319,7 @@ bool trsm_prepare_and_launch(TrsmPlan &pl, const char *routine)
         pl.dev = nullptr;
         pl.dev_bytes = 0;
         pl.key = 0;
-        if (!cuda_ok(cudaMalloc(&pl.dev, need), routine, "grouped TRSM plan buffer")) return false;
+        if (!(pl.dev = plan_alloc(need, routine))) return false;
         pl.dev_bytes = need;
     }
     // layout: [descriptors][work counter (256 B)][decoded solutions]
@@ -1322,6 +1327,7 @@ bool trsm_prepare_and_launch(TrsmPlan &pl, const char *routine)
     unsigned long long *counter = (unsigned long long *)((char *)pl.dev + d_bytes);
     fx::Op *xops = (fx::Op *)((char *)pl.dev + d_bytes + 256);
     if (pl.key != key) {
+        pl.key = 0;   // until the new layout's steps have all succeeded
         if (pl.exec) {
             cudaGraphExecDestroy(pl.exec);
             pl.exec = nullptr;

@@ -3181,7 +3181,7 @@ bool ozgroup_prepare(OzGroupPlan *pl, const std::vector<OzGroupItem> &items, con
         if (pl->dev) cudaFree(pl->dev);
         pl->dev = nullptr;
         pl->dev_bytes = 0;
-        if (!cuda_ok(cudaMalloc(&pl->dev, need), routine, "grouped tensor-core plan buffer")) return false;
+        if (!(pl->dev = plan_alloc(need, routine))) return false;
         pl->dev_bytes = need;
     }
     char *base = (char *)pl->dev;

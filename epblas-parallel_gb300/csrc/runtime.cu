@@ -161,27 +161,47 @@ bool check_device_status(const char *routine)
     return false;
 }
 
+namespace {
+
+// The allocation-failure test hook: true when this allocation is to fail.
+bool fail_injected(const char *routine)
+{
+    int64_t left = g_fail_alloc_after.load();
+    if (left < 0) return false;
+    g_fail_alloc_after.store(left - 1);   // 0 becomes -1: off
+    if (left > 0) return false;
+    set_error(routine, MWBLAS_ERR_ALLOC, "device allocation failed (injected by test hook)");
+    return true;
+}
+
+// The pointer, or nullptr with the error recorded and cleared from the runtime
+// (left there, it would fail the next call's launch check).
+void *checked_alloc(cudaError_t st, void *p, size_t bytes, const char *routine)
+{
+    if (st == cudaSuccess) return p;
+    cudaGetLastError();
+    set_error(routine, MWBLAS_ERR_ALLOC,
+              "device allocation of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(st));
+    return nullptr;
+}
+
+}  // namespace
+
 void *dev_alloc(size_t bytes, const char *routine)
 {
     if (bytes == 0) bytes = 16;
-    int64_t left = g_fail_alloc_after.load();
-    if (left >= 0) {
-        if (left == 0) {
-            g_fail_alloc_after.store(-1);
-            set_error(routine, MWBLAS_ERR_ALLOC, "device allocation failed (injected by test hook)");
-            return nullptr;
-        }
-        g_fail_alloc_after.store(left - 1);
-    }
+    if (fail_injected(routine)) return nullptr;
     void *p = nullptr;
-    cudaError_t st = cudaMallocAsync(&p, bytes, stream());
-    if (st != cudaSuccess) {
-        cudaGetLastError();
-        set_error(routine, MWBLAS_ERR_ALLOC,
-                  "device allocation of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(st));
-        return nullptr;
-    }
-    return p;
+    const cudaError_t st = cudaMallocAsync(&p, bytes, stream());
+    return checked_alloc(st, p, bytes, routine);
+}
+
+void *plan_alloc(size_t bytes, const char *routine)
+{
+    if (fail_injected(routine)) return nullptr;
+    void *p = nullptr;
+    const cudaError_t st = cudaMalloc(&p, bytes);
+    return checked_alloc(st, p, bytes, routine);
 }
 
 void dev_free(void *p)

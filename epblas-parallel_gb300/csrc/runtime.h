@@ -49,6 +49,8 @@ bool ensure_device(const char *routine);
 // test hook fires).
 void *dev_alloc(size_t bytes, const char *routine);
 void dev_free(void *p);
+// The same for a buffer that a plan keeps between calls (cudaMalloc; cudaFree frees it).
+void *plan_alloc(size_t bytes, const char *routine);
 
 // True when the pointer is device or managed memory that kernels may use.
 bool is_device_pointer(const void *p);
