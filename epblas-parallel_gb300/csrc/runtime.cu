@@ -1,5 +1,6 @@
 // Host runtime: errors, streams, device scratch and host<->device staging.
 #include "runtime.h"
+#include "statusmirror.h"
 
 #include <algorithm>
 #include <atomic>
@@ -28,6 +29,7 @@ struct ThreadErr {
 thread_local ThreadErr t_err;
 thread_local cudaStream_t t_stream = nullptr;   // nullptr = cudaStreamPerThread
 thread_local bool t_sync = true;
+thread_local StatusWatch t_watch[64];   // per device
 
 std::atomic<mwblas_error_hook> g_hook{nullptr};
 std::atomic<int64_t> g_fail_alloc_after{-1};
@@ -38,7 +40,7 @@ struct DeviceState {
     bool ready = false;
     int sm_count = 0;
     int *status = nullptr;   // device word for bounded-wait timeouts, then the address of its mirror
-    int *status_host = nullptr;   // the mirror: mapped host memory
+    uint64_t *status_host = nullptr;   // the mirror: mapped host memory (statusmirror.h)
 };
 std::mutex g_dev_mu;
 DeviceState g_dev[64];
@@ -86,9 +88,15 @@ bool ensure_device(const char *routine)
         return false;
     }
     DeviceState &ds = g_dev[dev];
-    if (ds.ready) return true;
+    if (ds.ready) {
+        t_watch[dev].begin(__atomic_load_n(ds.status_host, __ATOMIC_ACQUIRE));
+        return true;
+    }
     std::lock_guard<std::mutex> lk(g_dev_mu);
-    if (ds.ready) return true;
+    if (ds.ready) {
+        t_watch[dev].begin(__atomic_load_n(ds.status_host, __ATOMIC_ACQUIRE));
+        return true;
+    }
     cudaDeviceProp prop;
     if (!cuda_ok(cudaGetDeviceProperties(&prop, dev), routine, "cudaGetDeviceProperties")) return false;
     if (prop.major < 10) {
@@ -105,10 +113,10 @@ bool ensure_device(const char *routine)
     }
     // [code, 0, mapped address of the host's mirror]
     void *mirror = nullptr, *mirror_dev = nullptr;
-    if (!cuda_ok(cudaHostAlloc(&mirror, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), routine,
+    if (!cuda_ok(cudaHostAlloc(&mirror, sizeof(uint64_t), cudaHostAllocMapped | cudaHostAllocPortable), routine,
                  "cudaHostAlloc(status)"))
         return false;
-    *(int *)mirror = 0;
+    *(uint64_t *)mirror = 0;
     struct {
         int code, pad;
         void *mirror;
@@ -125,7 +133,8 @@ bool ensure_device(const char *routine)
         cudaFreeHost(mirror);
         return false;
     }
-    ds.status_host = (int *)mirror;
+    ds.status_host = (uint64_t *)mirror;
+    t_watch[dev].begin(0);
     ds.ready = true;
     return true;
 }
@@ -152,9 +161,9 @@ bool check_device_status(const char *routine)
 {
     int dev = 0;
     cudaGetDevice(&dev);
-    int *h = g_dev[dev].status_host;
-    if (!h || __atomic_load_n(h, __ATOMIC_ACQUIRE) == 0) return true;
-    const int v = __atomic_exchange_n(h, 0, __ATOMIC_ACQ_REL);
+    uint64_t *h = g_dev[dev].status_host;
+    if (!h) return true;
+    const int v = t_watch[dev].check(__atomic_load_n(h, __ATOMIC_ACQUIRE));
     if (v == 0) return true;
     cudaMemsetAsync(g_dev[dev].status, 0, sizeof(int), stream());
     set_error(routine, MWBLAS_ERR_TIMEOUT, "a bounded device wait gave up (status " + std::to_string(v) + ")");

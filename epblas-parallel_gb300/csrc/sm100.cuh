@@ -33,15 +33,18 @@ __device__ __forceinline__ uint64_t globaltimer_ns()
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Records a wait that gave up: `code` in the device word (first writer wins),
-// which the kernels' own waits poll, and in the host's mirror of it, whose
+// Records a wait that gave up. `seen`: what the caller read in the device word;
+// where that is zero, `code` goes there (first writer wins), for the other waits
+// to poll. Either way a stamp (time and code) goes to the host's mirror, whose
 // mapped address lies behind the device word (runtime.cu), so that the host
-// learns of it at its stream synchronisation without a copy.
-__device__ __forceinline__ void report_timeout(int *status, int code)
+// learns of it at its stream synchronisation without a copy: a kernel that only
+// follows the device word stamps too, as its own thread may have read the
+// earlier stamp already (statusmirror.h).
+__device__ __forceinline__ void report_timeout(int *status, int seen, int code)
 {
-    if (atomicCAS(status, 0, code) != 0) return;
-    int *host = *(int *volatile *)(status + 2);
-    *(volatile int *)host = code;
+    if (seen == 0) atomicCAS(status, 0, code);
+    unsigned long long *host = *(unsigned long long *volatile *)(status + 2);
+    *(volatile unsigned long long *)host = globaltimer_ns() << 8 | (unsigned)((seen ? seen : code) & 0xFF);
     __threadfence_system();
 }
 
@@ -95,9 +98,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *s
     while (true) {
         for (int i = 0; i < 32; ++i)
             if (mbar_try_wait(bar, parity)) return true;
-        if (status && *(volatile int *)status != 0) return false;
-        if (globaltimer_ns() - t0 > limit) {
-            if (status) report_timeout(status, code);
+        const int seen = status ? *(volatile int *)status : 0;
+        if (seen != 0 || globaltimer_ns() - t0 > limit) {
+            if (status) report_timeout(status, seen, code);
             return false;
         }
     }
@@ -312,9 +315,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
     while (true) {
         for (int i = 0; i < 32; ++i)
             if (mbar_try_wait_cluster(bar, parity)) return true;
-        if (status && *(volatile int *)status != 0) return false;
-        if (globaltimer_ns() - t0 > limit) {
-            if (status) report_timeout(status, code);
+        const int seen = status ? *(volatile int *)status : 0;
+        if (seen != 0 || globaltimer_ns() - t0 > limit) {
+            if (status) report_timeout(status, seen, code);
             return false;
         }
     }
