@@ -427,12 +427,12 @@ __global__ void k_iamax_final(int nparts, const AmaxKey *part, int64_t *out)
 
 // ---- DOT ---------------------------------------------------------------------
 // mdot.cpp:48-87 accumulates TwoProduct + Bailey three-limb sums on the FP64
-// pipe. Here the products are accumulated exactly (to 2^-116 of the largest
-// product of a warp) as limb products on the tensor cores, the warps' sums are
-// added as 128-bit extended floats in a fixed order (block, then the grid's
-// block partials), and the result is rounded once to double-double. The
-// result is deterministic for a given n and device and at least as accurate
-// as the reference's.
+// pipe. Here each product, one factor rounded to 2^-115 of the largest of its
+// warp's block of at most 4096 products, is accumulated exactly as limb products
+// on the tensor cores, the warps' sums are added as 128-bit extended floats in a
+// fixed order (block, then the grid's block partials), and the result is rounded
+// once to double-double. It is deterministic for a given n and device, and off by
+// at most 2^-104 sum |x y| beyond that rounding.
 
 __device__ fx::XF xf_block_sum(fx::XF v)
 {
@@ -472,14 +472,22 @@ __device__ bool block_any(bool b)
 // pairs are in flight per lane (cp.async).
 //
 // Exactness: D grows by at most 255 * 255 per pair and stays below 2^24 units
-// for 4 turns of 64; then it moves to int32 sums, and after 64 of those (or
+// for 4 turns of 64; then it moves to int32 sums, and after 16 of those (or
 // when a product above the block moves it up) to the warp's extended float.
 //
+// Accuracy: x_i is rounded where its alignment cuts it (for free: the half unit
+// enters the decode's carry chain), and every 4096 pairs the warp starts from
+// the block of the next products again. Cut to one block for the whole run with
+// three bits more of margin, a dominating product among equal-signed small ones
+// made it 8 units of 2^-104 sum |x y| off at n = 10^7 and 80 at 10^8 (per-thread
+// blocks of some 330 products: 0.1 and 0.7); now below 0.1 at any n.
+//
 // Bound: HBM (32 B per pair) and instruction issue, both about two thirds busy.
-// Measured at n = 10^8: 867 -> 598 us (3.69 -> 5.35 TB/s); 149 instructions per
-// pair, where 19 IMAD.WIDE digit products and their digit splits took 223.
+// Measured at n = 10^8: 867 -> 598 us (3.69 -> 5.35 TB/s) before the rounding and
+// the restarts, which take 10 us; 149 instructions per pair, where 19 IMAD.WIDE
+// digit products and their digit splits took 223.
 constexpr int kDotFlush = 4;            // turns of 64 pairs per move to the int32 sums
-constexpr int kDotFold = 64;            // moves per fold into the extended float
+constexpr int kDotFold = 16;            // moves per fold into the extended float
 constexpr int kDotStages = 4;           // turns in flight
 constexpr int kNoBlock = -(1 << 22);    // no nonzero product yet
 constexpr int kDotSmem = kDotStages * 4 * 16 * kThreads + 2 * 1024 * (kThreads / 32);
@@ -578,9 +586,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
             const double2 vx = *reinterpret_cast<const double2 *>(cur + 2 * p * kPlane);
             const double2 vy = *reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane);
             int ehx, ehy;
-            const bool okx = lmb::split_fast(vx, wx[p], ehx), oky = lmb::split_fast(vy, wy[p], ehy);
-            sh[p] = blk - ehx - ehy;
-            fast = fast && okx && oky && (uint32_t)(sh[p] - 2) < 30u;
+            const bool oky = lmb::split_fast(vy, wy[p], ehy);
+            sh[p] = blk - lmb::hi_exp(vx) - ehy;
+            const bool okx = lmb::split_fast(vx, wx[p], ehx, lmb::half_unit(sh[p]));
+            fast = fast && okx && oky && (uint32_t)sh[p] < 32u;
             neg[p] = (uint32_t)((__double2hiint(vx.x) ^ __double2hiint(vy.x)) >> 31);
         }
         if (__all_sync(0xffffffffu, fast)) {
@@ -589,7 +598,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
         } else {
             // the end, zeros, operands off the straight-line path, long alignments, a larger block
             const int64_t i0 = (warp + turn * nwarps) * 64 + lane;
-            int ep[2];
+            int ep[2], top = kNoBlock;
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
                 const fx::Op ox = fx::decode(*reinterpret_cast<const double2 *>(cur + 2 * p * kPlane));
@@ -600,21 +609,23 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
                 ep[p] = (no || !in || ((ox.flags | oy.flags) & fx::kZero))
                             ? kNoBlock
                             : ox.e + oy.e + 2 * lmb::kExpBias;
+                // (an x that is not normalised may have more than 118 bits)
+                if (ep[p] != kNoBlock) top = max(top, ep[p] + max(0, 10 - __clz((int)ox.w[3])));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     wx[p][i] = ox.w[i];
                     wy[p][i] = oy.w[i];
                 }
             }
-            const int top = __reduce_max_sync(0xffffffffu, max(ep[0], ep[1]));
-            if (top != kNoBlock && top > blk - 2) {
+            top = __reduce_max_sync(0xffffffffu, top);
+            if (top != kNoBlock && top > blk) {
                 if (blk != kNoBlock) fold();
-                blk = top + 4;
+                blk = top + 1;
             }
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
                 uint32_t sv[4];
-                fx::shr128(wx[p], ep[p] == kNoBlock ? 127 : min(blk - ep[p], 127), sv);
+                lmb::shr_round(wx[p], ep[p] == kNoBlock ? 127 : min(blk - ep[p], 127), sv);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) wx[p][i] = ep[p] == kNoBlock ? 0u : sv[i];
             }
@@ -644,7 +655,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
         }
         if ((turn & (kDotFlush - 1)) == kDotFlush - 1) {
             flush();
-            if ((turn & (kDotFlush * kDotFold - 1)) == kDotFlush * kDotFold - 1) fold();
+            if ((turn & (kDotFlush * kDotFold - 1)) == kDotFlush * kDotFold - 1) {
+                fold();
+                blk = kNoBlock;   // the next products find their own block
+            }
         }
     }
     fold();

@@ -31,7 +31,9 @@ using fx::XF;
 // normalised). A zero or subnormal lo needs no test: its biased exponent 0
 // makes the shift at least 75, which leaves nothing of it (a subnormal lo is
 // then below 2^-127 of hi).
-__device__ __forceinline__ bool split_fast(double2 v, uint32_t w[4], int &eh)
+// `half`: added to W's lowest word, 2^(sh - 1) for a W that is then shifted right
+// by sh, which rounds it to nearest.
+__device__ __forceinline__ bool split_fast(double2 v, uint32_t w[4], int &eh, uint32_t half = 0u)
 {
     const uint32_t hl = (uint32_t)__double2loint(v.x), hh = (uint32_t)__double2hiint(v.x);
     const uint32_t ll = (uint32_t)__double2loint(v.y), lh = (uint32_t)__double2hiint(v.y);
@@ -47,13 +49,34 @@ __device__ __forceinline__ bool split_fast(double2 v, uint32_t w[4], int &eh)
         "addc.cc.u32 %2, %6, %9;\n\t"
         "addc.u32 %3, %7, %9;"
         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
-        : "r"(t0 ^ mask), "r"(t1 ^ mask), "r"(hl), "r"((hh & 0xFFFFFu) | 0x100000u), "r"(mask & 1u), "r"(mask));
+        : "r"(t0 ^ mask), "r"(t1 ^ mask), "r"(hl), "r"((hh & 0xFFFFFu) | 0x100000u), "r"(half - mask), "r"(mask));
     eh = (int)uh;
     return (uh - 128u) < 0x77Fu && (int)r >= 0;
 }
 
 // fixacc.cuh's exponent (v = +-W * 2^e) of a biased hi exponent
 constexpr int kExpBias = 1139;
+
+// split_fast's eh
+__device__ __forceinline__ int hi_exp(double2 v) { return (int)(((uint32_t)__double2hiint(v.x) << 1) >> 21); }
+
+// 2^(sh - 1) for 0 < sh < 32, 0 for sh = 0
+__device__ __forceinline__ uint32_t half_unit(int sh) { return __funnelshift_l(0x80000000u, 0u, sh); }
+
+// W / 2^sh rounded to nearest, 0 <= sh < 128
+__device__ __forceinline__ void shr_round(const uint32_t w[4], int sh, uint32_t y[4])
+{
+    uint32_t t[4];
+    fx::shr128(w, sh > 0 ? sh - 1 : 0, t);
+    const uint32_t one = sh > 0 ? 1u : 0u;
+    asm("add.cc.u32 %0, %0, %4;\n\t"
+        "addc.cc.u32 %1, %1, 0;\n\t"
+        "addc.cc.u32 %2, %2, 0;\n\t"
+        "addc.u32 %3, %3, 0;"
+        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3])
+        : "r"(one));
+    fx::shr128(t, (int)one, y);
+}
 
 // W >> sh for 0 <= sh < 32
 __device__ __forceinline__ void shr_short(uint32_t w[4], int sh)
