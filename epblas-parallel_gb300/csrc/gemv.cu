@@ -98,17 +98,25 @@ __global__ void k_gemv_n_final(int64_t m, int nchunks, const double2 *part, dd::
 // depends only on g: they are laid out once per window of 32 indices in shared
 // memory and read with three 16-byte loads.
 //
-// Exactness: x's limbs are balanced (|.| <= 128), A's are bytes, 15 limbs
-// each, so a column grows by at most 15 * 255 * 128 per index and stays below
+// Exactness: x's limbs are balanced (|.| <= 128), 15 of them, A's are bytes, at
+// most 16, so a column grows by at most 16 * 255 * 128 per index and stays below
 // 2^24 units for a window's 32; then it moves to an int32 (at most 64 windows
 // per block). Each output keeps a block exponent: a product of exponent ep is
-// aligned by B - ep >= 0 bits, rounded to nearest; one above the block folds the
-// sums into an extended float in shared memory and moves B to three bits above
-// that product (rare after the first groups; with one bit of margin the moves
+// aligned by B - ep bits, rounded to nearest where that cuts it. The first one
+// above the block folds the sums into an extended float in shared memory and
+// moves B to three bits above that product (with one bit of margin the moves
 // cost 8 % on uniform and 50 % on normally distributed entries). So a product is
 // off by at most half of 2^-113 of the largest of its output and chunk. Cut to
 // four bits of margin, one dominating product among 2000 equal-signed ones made
 // it 1.1 units of 2^-104 sum |a x|, now 0.1, at the same speed.
+//
+// Zeros, alignments beyond a word and products up to nine bits above their block
+// go through a loop of their own, which shifts any way (the block moves at the
+// window's end), and groups of zeros leave it early. 8192^2 N, us, with the
+// general decode for each such group, as the digit form was, and now: 1 % zeros
+// 538, 729 and 485; 90 % 755, 569 and 530; every fourth x zero 567, 492 and 488;
+// a triangle 535, 383 and 335; exponents over 2^40 876, 519 and 540; dense 301,
+// 493 and 301.
 //
 // Bound: HBM (16 B per element) in principle, instruction issue in practice:
 // about 80 per element, where the 24-bit digit form with 19 IMAD.WIDE per
@@ -127,6 +135,7 @@ constexpr int kColWords = 104;            // B entry of one index: 8 x 12 words,
 constexpr int kR = 2, kE = 2 * kR;        // 16-output tiles per warp, elements per lane and group
 constexpr int kStages = 4;                // groups of four indices in flight per thread (cp.async)
 constexpr int kZeroE = -(1 << 20), kBadE = 1 << 20;   // exponent marks: zero (or past the end), non-finite
+constexpr int kOver = 9;                  // bits a product may lie above its block
 constexpr int kNoBlock = -(1 << 22);                  // an output that has seen no nonzero product yet
 
 struct GemvArgs {
@@ -302,11 +311,12 @@ __global__ void __launch_bounds__(256, 2) k_gemv_limb(const GemvArgs g)
                     acc[h][v][i] = 0.0f;
                 }
     };
-    // the column sums into the outputs' extended floats (all outputs of the warp)
-    auto fold = [&]() {
+    // the column sums into the outputs' extended floats: outputs r0 + g + 8e of the set bits e
+    auto fold = [&](uint32_t which) {
         flush();
 #pragma unroll
         for (int e = 0; e < kE; ++e) {
+            if (!(which >> e & 1u)) continue;
             uint64_t W[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
@@ -323,97 +333,187 @@ __global__ void __launch_bounds__(256, 2) k_gemv_limb(const GemvArgs g)
         __syncwarp();
     };
 
+    // += the aligned elements' limbs times x's
+    auto products = [&](const uint32_t (&w)[kE][4], const uint32_t (&sgn)[kE], const uint32_t *sb) {
+        uint32_t f[12];
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(sb + lg * 12 + 4 * v);
+            f[4 * v] = q.x; f[4 * v + 1] = q.y; f[4 * v + 2] = q.z; f[4 * v + 3] = q.w;
+        }
+#pragma unroll
+        for (int h = 0; h < kR; ++h)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t a0 = lmb::limbs_lo(w[2 * h][u], sgn[2 * h]);
+                const uint32_t a1 = lmb::limbs_lo(w[2 * h + 1][u], sgn[2 * h + 1]);
+                const uint32_t a2 = lmb::limbs_hi(w[2 * h][u], sgn[2 * h]);
+                const uint32_t a3 = lmb::limbs_hi(w[2 * h + 1][u], sgn[2 * h + 1]);
+#pragma unroll
+                for (int v = 0; v < 3; ++v) {
+                    if (v == 2 && u < 2) continue;        // limbs 16 and up of x: zero
+                    const int b = 2 * (2 - (2 * v - u));   // pair of window 2v - u
+                    lmb::mma16816(acc[h][v], a0, a1, a2, a3, f[b], f[b + 1]);
+                }
+            }
+    };
+
     if (active)
         for (int it = 0; it < kStages - 1; ++it) load_a(it);
+    bool any_shift = false, idle = false, far = false;
+    uint32_t over = 0u;   // byte e: bits by which output r0 + g + 8e has gone above its block in this window
     for (int win = 0; win < nwin; ++win) {
         if (win + 1 < nwin) expand(win + 1);
         if (win + 2 < nwin && wid == (win + 2) % nw) split_x(win + 2);
         if (active) {
             const uint32_t *sb = s_b[win & 1] + lt * kColWords;
             const int it1 = min(8 * win + 8, nit);
+            int it = 8 * win;
+            while (it < it1) {
+                // groups whose elements are all on the straight line, within a word of their block
 #pragma unroll 1
-            for (int it = 8 * win; it < it1; ++it, sb += 4 * kColWords) {
-                asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
-                const unsigned char *cur = s_stage + slot + (size_t)(it & (kStages - 1)) * kE * st_e;
-                uint32_t w[kE][4], sgn[kE];
-                int sh[kE];
-                const int xe = (int)sb[96];
-                bool fast = true;
+                for (; it < it1 && !any_shift; ++it, sb += 4 * kColWords) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+                    const unsigned char *cur = s_stage + slot + (size_t)(it & (kStages - 1)) * kE * st_e;
+                    uint32_t w[kE][4], sgn[kE];
+                    int sh[kE];
+                    const int xe = (int)sb[96];
+                    bool fast = true;
 #pragma unroll
-                for (int e = 0; e < kE; ++e) {
-                    const double2 v = *reinterpret_cast<const double2 *>(cur + e * st_e);
-                    int eh;
-                    sh[e] = blk[e] - xe - lmb::hi_exp(v);
-                    const bool ok = lmb::split_fast(v, w[e], eh, lmb::half_unit(sh[e]));
-                    fast = fast && ok && (uint32_t)sh[e] < 32u;
-                    sgn[e] = (uint32_t)__double2hiint(v.x) & 0x80000000u;
-                }
-                if (__all_sync(0xffffffffu, fast)) {
+                    for (int e = 0; e < kE; ++e) {
+                        const double2 v = *reinterpret_cast<const double2 *>(cur + e * st_e);
+                        int eh;
+                        sh[e] = blk[e] - xe - lmb::hi_exp(v);
+                        const bool ok = lmb::split_fast(v, w[e], eh, lmb::half_unit(sh[e]));
+                        fast = fast && ok && (uint32_t)sh[e] < 32u;
+                        sgn[e] = (uint32_t)__double2hiint(v.x) & 0x80000000u;
+                    }
+                    if (!__all_sync(0xffffffffu, fast)) {
+                        any_shift = true;
+                        break;
+                    }
 #pragma unroll
                     for (int e = 0; e < kE; ++e) lmb::shr_short(w[e], sh[e]);
-                } else {
-                    // zeros, operands off the straight-line path, long alignments, a larger block
-                    int ep[kE], top[kE];
-                    bool raise = false;
-#pragma unroll
-                    for (int e = 0; e < kE; ++e) {
-                        const fx::Op o = fx::decode(*reinterpret_cast<const double2 *>(cur + e * st_e));
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) w[e][i] = o.w[i];
-                        const bool no = xe == kBadE || (o.flags & fx::kBad);
-                        if (no) bad |= 1u << e;
-                        ep[e] = (no || xe == kZeroE || (o.flags & fx::kZero)) ? kNoBlock : o.e + lmb::kExpBias + xe;
-                        top[e] = max(ep[e], __shfl_xor_sync(0xffffffffu, ep[e], 1));
-                        top[e] = max(top[e], __shfl_xor_sync(0xffffffffu, top[e], 2));
-                        raise = raise || (top[e] != kNoBlock && top[e] > blk[e]);
-                    }
-                    if (__any_sync(0xffffffffu, raise)) {
-                        int seen = blk[0];
-#pragma unroll
-                        for (int e = 1; e < kE; ++e) seen = max(seen, blk[e]);
-                        if (__any_sync(0xffffffffu, seen != kNoBlock)) fold();
-#pragma unroll
-                        for (int e = 0; e < kE; ++e)
-                            if (top[e] != kNoBlock && top[e] > blk[e]) blk[e] = top[e] + 3;
-                    }
-#pragma unroll
-                    for (int e = 0; e < kE; ++e) {
-                        const int d = ep[e] == kNoBlock ? 127 : min(blk[e] - ep[e], 127);
-                        uint32_t sv[4];
-                        lmb::shr_round(w[e], d, sv);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) w[e][i] = ep[e] == kNoBlock ? 0u : sv[i];
-                    }
+                    load_a(it + kStages - 1);   // into the stage read in the previous turn
+                    products(w, sgn, sb);
                 }
-                load_a(it + kStages - 1);   // into the stage read in the previous turn
-                uint32_t f[12];
+                // the others, in a loop of their own (in the same one they cost it 5 to 15 %), until
+                // a group that the first loop takes
+#pragma unroll 1
+                for (; it < it1 && any_shift; ++it, sb += 4 * kColWords) {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+                    const unsigned char *cur = s_stage + slot + (size_t)(it & (kStages - 1)) * kE * st_e;
+                    uint32_t w[kE][4], sgn[kE];
+                    int sh[kE];
+                    const int xe = (int)sb[96];
+                    if (idle) {   // after a group of zeros, another one costs a look
+                        bool dead = xe != kBadE;
 #pragma unroll
-                for (int v = 0; v < 3; ++v) {
-                    const uint4 q = *reinterpret_cast<const uint4 *>(sb + lg * 12 + 4 * v);
-                    f[4 * v] = q.x; f[4 * v + 1] = q.y; f[4 * v + 2] = q.z; f[4 * v + 3] = q.w;
-                }
-#pragma unroll
-                for (int h = 0; h < kR; ++h)
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint32_t a0 = lmb::limbs_lo(w[2 * h][u], sgn[2 * h]);
-                        const uint32_t a1 = lmb::limbs_lo(w[2 * h + 1][u], sgn[2 * h + 1]);
-                        const uint32_t a2 = lmb::limbs_hi(w[2 * h][u], sgn[2 * h]);
-                        const uint32_t a3 = lmb::limbs_hi(w[2 * h + 1][u], sgn[2 * h + 1]);
-#pragma unroll
-                        for (int v = 0; v < 3; ++v) {
-                            if (v == 2 && u < 2) continue;        // limbs 16 and up of x: zero
-                            const int b = 2 * (2 - (2 * v - u));   // pair of window 2v - u
-                            lmb::mma16816(acc[h][v], a0, a1, a2, a3, f[b], f[b + 1]);
+                        for (int e = 0; e < kE; ++e) {
+                            const double2 v = *reinterpret_cast<const double2 *>(cur + e * st_e);
+                            dead = dead && (lmb::all_zero(v) || (xe == kZeroE && lmb::is_fast(v)));
+                        }
+                        if (__all_sync(0xffffffffu, dead)) {
+                            load_a(it + kStages - 1);
+                            continue;
                         }
                     }
+                    // zeros, long alignments and products up to 2^kOver above their block (A's 16
+                    // limbs hold 128 bits, W has 118; the block moves at the end of the window):
+                    // the same decode, any shift
+                    bool plain = xe != kBadE, live = false, fast = true, near = true;
+                    uint32_t above = 0u;
+#pragma unroll
+                    for (int e = 0; e < kE; ++e) {
+                        const double2 v = *reinterpret_cast<const double2 *>(cur + e * st_e);
+                        int eh;
+                        const bool ok = lmb::split_fast(v, w[e], eh), zero = lmb::all_zero(v);
+                        const bool none = zero || xe == kZeroE;
+                        sh[e] = blk[e] - xe - eh;
+                        fast = fast && ok && (uint32_t)sh[e] < 32u;
+                        near = near && ok && sh[e] < 32;
+                        plain = plain && (ok || zero) && (sh[e] >= -kOver || none);
+                        live = live || !none;
+                        if (sh[e] < 0 && !none) above |= (uint32_t)min(-sh[e], kOver) << (8 * e);
+                        sh[e] = none ? 127 : min(sh[e] + kOver, 127);   // at 127 nothing is left of a zero's W
+                        sgn[e] = (uint32_t)__double2hiint(v.x) & 0x80000000u;
+                    }
+                    any_shift = !__all_sync(0xffffffffu, fast);
+                    if (__all_sync(0xffffffffu, plain)) {
+                        over = __vmaxu4(over, above);
+                        idle = !__any_sync(0xffffffffu, live);
+                        far = !__all_sync(0xffffffffu, near);
+#pragma unroll
+                        for (int e = 0; e < kE; ++e) {
+                            uint32_t sv[4];
+#pragma unroll
+                            for (int i = 3; i > 0; --i) w[e][i] = __funnelshift_l(w[e][i - 1], w[e][i], kOver);
+                            w[e][0] <<= kOver;
+                            lmb::shr_round(w[e], sh[e], sv);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) w[e][i] = sv[i];
+                        }
+                    } else {
+                        // operands off the straight-line path, a larger block
+                        idle = false;
+                        int ep[kE], top[kE];
+                        uint32_t raise = 0u, move = 0u;   // blocks that go up, those of them with sums to fold
+#pragma unroll
+                        for (int e = 0; e < kE; ++e) {
+                            const fx::Op o = fx::decode(*reinterpret_cast<const double2 *>(cur + e * st_e));
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) w[e][i] = o.w[i];
+                            const bool no = xe == kBadE || (o.flags & fx::kBad);
+                            if (no) bad |= 1u << e;
+                            ep[e] = (no || xe == kZeroE || (o.flags & fx::kZero)) ? kNoBlock : o.e + lmb::kExpBias + xe;
+                            const int o8 = (int)(over >> (8 * e)) & 255;
+                            top[e] = max(ep[e], o8 ? blk[e] + o8 : kNoBlock);
+                            top[e] = max(top[e], __shfl_xor_sync(0xffffffffu, top[e], 1));
+                            top[e] = max(top[e], __shfl_xor_sync(0xffffffffu, top[e], 2));
+                            if (top[e] != kNoBlock && top[e] > blk[e]) {
+                                raise |= 1u << e;
+                                if (blk[e] != kNoBlock) move |= 1u << e;
+                            }
+                        }
+                        over = 0u;
+                        move = __reduce_or_sync(0xffffffffu, move);
+                        if (move) fold(move);
+#pragma unroll
+                        for (int e = 0; e < kE; ++e) {
+                            if (raise >> e & 1u) blk[e] = top[e] + 3;
+                            const int d = ep[e] == kNoBlock ? 127 : min(blk[e] - ep[e], 127);
+                            uint32_t sv[4];
+                            lmb::shr_round(w[e], d, sv);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) w[e][i] = ep[e] == kNoBlock ? 0u : sv[i];
+                        }
+                    }
+                    load_a(it + kStages - 1);   // into the stage read in the previous turn
+                    if (!idle) products(w, sgn, sb);
+                }
             }
             flush();
+            // blocks that products went above go up, three bits above those, where that is what keeps
+            // the groups in the second loop
+            if (!far && __any_sync(0xffffffffu, over != 0u)) {
+                over = __vmaxu4(over, __shfl_xor_sync(0xffffffffu, over, 1));
+                over = __vmaxu4(over, __shfl_xor_sync(0xffffffffu, over, 2));
+                uint32_t move = 0u;
+#pragma unroll
+                for (int e = 0; e < kE; ++e) move |= (over >> (8 * e) & 255u) ? 1u << e : 0u;
+                fold(__reduce_or_sync(0xffffffffu, move));
+#pragma unroll
+                for (int e = 0; e < kE; ++e) {
+                    const int o8 = (int)(over >> (8 * e)) & 255;
+                    if (o8) blk[e] += o8 + 3;
+                }
+                over = 0u;
+            }
         }
         __syncthreads();
     }
     if (!active) return;
-    fold();
+    fold((1u << kE) - 1u);
     uint32_t mine = 0;   // lane r: whether output r saw a non-finite operand
 #pragma unroll
     for (int e = 0; e < kE; ++e) {

@@ -484,8 +484,13 @@ __device__ bool block_any(bool b)
 //
 // Bound: HBM (32 B per pair) and instruction issue, both about two thirds busy.
 // Measured at n = 10^8: 867 -> 598 us (3.69 -> 5.35 TB/s) before the rounding and
-// the restarts, which take 10 us; 149 instructions per pair, where 19 IMAD.WIDE
-// digit products and their digit splits took 223.
+// the restarts; 149 instructions per pair, where 19 IMAD.WIDE
+// digit products and their digit splits took 223. Turns with zeros or alignments
+// beyond a word have a loop of their own, which shifts any way, and pass without
+// products where all are zero: whole call at n = 10^8, with the general decode for
+// each such turn, as the digit form was, and now: a zero in 64 1268, 949 and 850 us;
+// the second half zero 897, 691 and 676; exponents over 2^40 1245, 957 and 872;
+// dense 642, 907 and 648.
 constexpr int kDotFlush = 4;            // turns of 64 pairs per move to the int32 sums
 constexpr int kDotFold = 16;            // moves per fold into the extended float
 constexpr int kDotStages = 4;           // turns in flight
@@ -574,83 +579,33 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
     for (int u = 0; u < kDotStages - 1; ++u) load(u);
     unsigned char *limbs = s_dot + kDotStages * 4 * kPlane + wid * 2048;
     const uint32_t lrow = (uint32_t)__cvta_generic_to_shared(limbs) + lane * 16u;
-#pragma unroll 1
-    for (int64_t turn = 0; turn < turns; ++turn) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kDotStages - 2) : "memory");
-        const unsigned char *cur = s_dot + ((uint32_t)turn & (kDotStages - 1)) * (4 * kPlane) + threadIdx.x * 16u;
-        uint32_t wx[2][4], wy[2][4], neg[2];
-        int sh[2];
-        bool fast = (warp + turn * nwarps) * 64 + 64 <= n;
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const double2 vx = *reinterpret_cast<const double2 *>(cur + 2 * p * kPlane);
-            const double2 vy = *reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane);
-            int ehx, ehy;
-            const bool oky = lmb::split_fast(vy, wy[p], ehy);
-            sh[p] = blk - lmb::hi_exp(vx) - ehy;
-            const bool okx = lmb::split_fast(vx, wx[p], ehx, lmb::half_unit(sh[p]));
-            fast = fast && okx && oky && (uint32_t)sh[p] < 32u;
-            neg[p] = (uint32_t)((__double2hiint(vx.x) ^ __double2hiint(vy.x)) >> 31);
-        }
-        if (__all_sync(0xffffffffu, fast)) {
-#pragma unroll
-            for (int p = 0; p < 2; ++p) lmb::shr_short(wx[p], sh[p]);
-        } else {
-            // the end, zeros, operands off the straight-line path, long alignments, a larger block
-            const int64_t i0 = (warp + turn * nwarps) * 64 + lane;
-            int ep[2], top = kNoBlock;
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const fx::Op ox = fx::decode(*reinterpret_cast<const double2 *>(cur + 2 * p * kPlane));
-                const fx::Op oy = fx::decode(*reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane));
-                const bool no = ((ox.flags | oy.flags) & fx::kBad) != 0;
-                const bool in = i0 + 32 * p < n;   // else the stage holds an older pair or nothing
-                bad = bad || (no && in);
-                ep[p] = (no || !in || ((ox.flags | oy.flags) & fx::kZero))
-                            ? kNoBlock
-                            : ox.e + oy.e + 2 * lmb::kExpBias;
-                // (an x that is not normalised may have more than 118 bits)
-                if (ep[p] != kNoBlock) top = max(top, ep[p] + max(0, 10 - __clz((int)ox.w[3])));
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    wx[p][i] = ox.w[i];
-                    wy[p][i] = oy.w[i];
-                }
-            }
-            top = __reduce_max_sync(0xffffffffu, top);
-            if (top != kNoBlock && top > blk) {
-                if (blk != kNoBlock) fold();
-                blk = top + 1;
-            }
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                uint32_t sv[4];
-                lmb::shr_round(wx[p], ep[p] == kNoBlock ? 127 : min(blk - ep[p], 127), sv);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) wx[p][i] = ep[p] == kNoBlock ? 0u : sv[i];
-            }
-        }
+    // the turn's aligned limbs into the sums, and what is due after it
+    auto products = [&](int64_t turn, const uint32_t (&wx)[2][4], const uint32_t (&wy)[2][4], const uint32_t (&neg)[2],
+                        bool go) {
         load(turn + kDotStages - 1);   // into the stage read in the previous turn
-        __syncwarp();                  // the previous turn's limbs have been read
+        if (go) {
+            __syncwarp();   // the previous turn's limbs have been read
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            uint4 *st = reinterpret_cast<uint4 *>(limbs + 1024 * p) + lane;
-            st[0] = make_uint4(wx[p][0] ^ neg[p], wx[p][1] ^ neg[p], wx[p][2] ^ neg[p],
-                               (wx[p][3] ^ (neg[p] & 0xFFFFFFu)) | (neg[p] & 0x1000000u));
-            st[32] = make_uint4(wy[p][0], wy[p][1], wy[p][2], wy[p][3]);
-        }
-        __syncwarp();
+            for (int p = 0; p < 2; ++p) {
+                uint4 *st = reinterpret_cast<uint4 *>(limbs + 1024 * p) + lane;
+                st[0] = make_uint4(wx[p][0] ^ neg[p], wx[p][1] ^ neg[p], wx[p][2] ^ neg[p],
+                                   (wx[p][3] ^ (neg[p] & 0xFFFFFFu)) | (neg[p] & 0x1000000u));
+                st[32] = make_uint4(wy[p][0], wy[p][1], wy[p][2], wy[p][3]);
+            }
+            __syncwarp();
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            uint32_t a[4], b[4];   // elements 8j .. 8j + 7 in [j]
-            lmb::ldmatrix_x4_trans(a, lrow + 1024u * p);
-            lmb::ldmatrix_x4_trans(b, lrow + 1024u * p + 512u);
+            for (int p = 0; p < 2; ++p) {
+                uint32_t a[4], b[4];   // elements 8j .. 8j + 7 in [j]
+                lmb::ldmatrix_x4_trans(a, lrow + 1024u * p);
+                lmb::ldmatrix_x4_trans(b, lrow + 1024u * p + 512u);
 #pragma unroll
-            for (int h = 0; h < 4; h += 2) {
-                const uint32_t a0 = a[h] & 0xFF00FFu, a1 = __byte_perm(a[h], 0u, 0x4341);
-                const uint32_t a2 = a[h + 1] & 0xFF00FFu, a3 = __byte_perm(a[h + 1], 0u, 0x4341);
-                lmb::mma16816(acc[0], a0, a1, a2, a3, b[h] & 0xFF00FFu, b[h + 1] & 0xFF00FFu);
-                lmb::mma16816(acc[1], a0, a1, a2, a3, __byte_perm(b[h], 0u, 0x4341), __byte_perm(b[h + 1], 0u, 0x4341));
+                for (int h = 0; h < 4; h += 2) {
+                    const uint32_t a0 = a[h] & 0xFF00FFu, a1 = __byte_perm(a[h], 0u, 0x4341);
+                    const uint32_t a2 = a[h + 1] & 0xFF00FFu, a3 = __byte_perm(a[h + 1], 0u, 0x4341);
+                    lmb::mma16816(acc[0], a0, a1, a2, a3, b[h] & 0xFF00FFu, b[h + 1] & 0xFF00FFu);
+                    lmb::mma16816(acc[1], a0, a1, a2, a3, __byte_perm(b[h], 0u, 0x4341),
+                                  __byte_perm(b[h + 1], 0u, 0x4341));
+                }
             }
         }
         if ((turn & (kDotFlush - 1)) == kDotFlush - 1) {
@@ -659,6 +614,109 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
                 fold();
                 blk = kNoBlock;   // the next products find their own block
             }
+        }
+    };
+    int64_t turn = 0;
+    bool any_shift = true;
+    while (turn < turns) {
+        // turns whose operands are all on the straight line, within a word of the block
+#pragma unroll 1
+        for (; turn < turns && !any_shift; ++turn) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kDotStages - 2) : "memory");
+            const unsigned char *cur = s_dot + ((uint32_t)turn & (kDotStages - 1)) * (4 * kPlane) + threadIdx.x * 16u;
+            uint32_t wx[2][4], wy[2][4], neg[2];
+            int sh[2];
+            bool fast = (warp + turn * nwarps) * 64 + 64 <= n;
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const double2 vx = *reinterpret_cast<const double2 *>(cur + 2 * p * kPlane);
+                const double2 vy = *reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane);
+                int ehx, ehy;
+                const bool oky = lmb::split_fast(vy, wy[p], ehy);
+                sh[p] = blk - lmb::hi_exp(vx) - ehy;
+                const bool okx = lmb::split_fast(vx, wx[p], ehx, lmb::half_unit(sh[p]));
+                fast = fast && okx && oky && (uint32_t)sh[p] < 32u;
+                neg[p] = (uint32_t)((__double2hiint(vx.x) ^ __double2hiint(vy.x)) >> 31);
+            }
+            if (!__all_sync(0xffffffffu, fast)) {
+                any_shift = true;
+                break;
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p) lmb::shr_short(wx[p], sh[p]);
+            products(turn, wx, wy, neg, true);
+        }
+        // the others, in a loop of their own (in the same one they cost it 2 to 5 %), until a turn
+        // that the first loop takes
+#pragma unroll 1
+        for (; turn < turns && any_shift; ++turn) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kDotStages - 2) : "memory");
+            const unsigned char *cur = s_dot + ((uint32_t)turn & (kDotStages - 1)) * (4 * kPlane) + threadIdx.x * 16u;
+            const int64_t i0 = (warp + turn * nwarps) * 64;
+            uint32_t wx[2][4], wy[2][4], neg[2];
+            int sh[2];
+            // zeros and long alignments at the block there is: the same decode, any shift
+            bool plain = i0 + 64 <= n, live = false, fast = plain;
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const double2 vx = *reinterpret_cast<const double2 *>(cur + 2 * p * kPlane);
+                const double2 vy = *reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane);
+                int ehx, ehy;
+                const bool okx = lmb::split_fast(vx, wx[p], ehx), oky = lmb::split_fast(vy, wy[p], ehy);
+                const bool zx = lmb::all_zero(vx), zy = lmb::all_zero(vy), none = zx || zy;
+                sh[p] = blk - ehx - ehy;
+                fast = fast && okx && oky && (uint32_t)sh[p] < 32u;
+                plain = plain && (okx || zx) && (oky || zy) && (sh[p] >= 0 || none);
+                live = live || !none;
+                sh[p] = none ? 127 : min(sh[p], 127);   // W < 2^118: nothing is left of it at 127
+                neg[p] = (uint32_t)((__double2hiint(vx.x) ^ __double2hiint(vy.x)) >> 31);
+            }
+            any_shift = !__all_sync(0xffffffffu, fast);
+            bool go = true;
+            if (__all_sync(0xffffffffu, plain)) {
+                go = __any_sync(0xffffffffu, live);
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    uint32_t sv[4];
+                    lmb::shr_round(wx[p], sh[p], sv);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) wx[p][i] = sv[i];
+                }
+            } else {
+                // the end, operands off the straight-line path, a larger block
+                int ep[2], top = kNoBlock;
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const fx::Op ox = fx::decode(*reinterpret_cast<const double2 *>(cur + 2 * p * kPlane));
+                    const fx::Op oy = fx::decode(*reinterpret_cast<const double2 *>(cur + (2 * p + 1) * kPlane));
+                    const bool no = ((ox.flags | oy.flags) & fx::kBad) != 0;
+                    const bool in = i0 + lane + 32 * p < n;   // else the stage holds an older pair or nothing
+                    bad = bad || (no && in);
+                    ep[p] = (no || !in || ((ox.flags | oy.flags) & fx::kZero))
+                                ? kNoBlock
+                                : ox.e + oy.e + 2 * lmb::kExpBias;
+                    // (an x that is not normalised may have more than 118 bits)
+                    if (ep[p] != kNoBlock) top = max(top, ep[p] + max(0, 10 - __clz((int)ox.w[3])));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        wx[p][i] = ox.w[i];
+                        wy[p][i] = oy.w[i];
+                    }
+                }
+                top = __reduce_max_sync(0xffffffffu, top);
+                if (top != kNoBlock && top > blk) {
+                    if (blk != kNoBlock) fold();
+                    blk = top + 1;
+                }
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    uint32_t sv[4];
+                    lmb::shr_round(wx[p], ep[p] == kNoBlock ? 127 : min(blk - ep[p], 127), sv);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) wx[p][i] = ep[p] == kNoBlock ? 0u : sv[i];
+                }
+            }
+            products(turn, wx, wy, neg, go);
         }
     }
     fold();

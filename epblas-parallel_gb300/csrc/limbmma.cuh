@@ -33,6 +33,11 @@ using fx::XF;
 // then below 2^-127 of hi).
 // `half`: added to W's lowest word, 2^(sh - 1) for a W that is then shifted right
 // by sh, which rounds it to nearest.
+__device__ __forceinline__ bool is_fast(double2 v)
+{
+    const uint32_t uh = ((uint32_t)__double2hiint(v.x) << 1) >> 21, ul = ((uint32_t)__double2hiint(v.y) << 1) >> 21;
+    return (uh - 128u) < 0x77Fu && (int)(uh - ul - 53u) >= 0;
+}
 __device__ __forceinline__ bool split_fast(double2 v, uint32_t w[4], int &eh, uint32_t half = 0u)
 {
     const uint32_t hl = (uint32_t)__double2loint(v.x), hh = (uint32_t)__double2hiint(v.x);
@@ -51,7 +56,7 @@ __device__ __forceinline__ bool split_fast(double2 v, uint32_t w[4], int &eh, ui
         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
         : "r"(t0 ^ mask), "r"(t1 ^ mask), "r"(hl), "r"((hh & 0xFFFFFu) | 0x100000u), "r"(half - mask), "r"(mask));
     eh = (int)uh;
-    return (uh - 128u) < 0x77Fu && (int)r >= 0;
+    return is_fast(v);
 }
 
 // fixacc.cuh's exponent (v = +-W * 2^e) of a biased hi exponent
@@ -59,6 +64,13 @@ constexpr int kExpBias = 1139;
 
 // split_fast's eh
 __device__ __forceinline__ int hi_exp(double2 v) { return (int)(((uint32_t)__double2hiint(v.x) << 1) >> 21); }
+
+// hi and lo both zero, of either sign (split_fast's W is 2^116 then)
+__device__ __forceinline__ bool all_zero(double2 v)
+{
+    return ((((uint32_t)__double2hiint(v.x) | (uint32_t)__double2hiint(v.y)) << 1) | (uint32_t)__double2loint(v.x) |
+            (uint32_t)__double2loint(v.y)) == 0u;
+}
 
 // 2^(sh - 1) for 0 < sh < 32, 0 for sh = 0
 __device__ __forceinline__ uint32_t half_unit(int sh) { return __funnelshift_l(0x80000000u, 0u, sh); }
@@ -75,7 +87,10 @@ __device__ __forceinline__ void shr_round(const uint32_t w[4], int sh, uint32_t 
         "addc.u32 %3, %3, 0;"
         : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3])
         : "r"(one));
-    fx::shr128(t, (int)one, y);
+    y[0] = __funnelshift_r(t[0], t[1], one);
+    y[1] = __funnelshift_r(t[1], t[2], one);
+    y[2] = __funnelshift_r(t[2], t[3], one);
+    y[3] = t[3] >> one;
 }
 
 // W >> sh for 0 <= sh < 32
