@@ -1753,12 +1753,9 @@ __device__ __forceinline__ bool finite_hi(double x)
     return ((__double2hiint(x) >> 20) & 0x7FF) != 0x7FF;   // exponent field test, no FP64 compare
 }
 
-// alpha M as four mantissa words at one exponent: for complex alpha both parts
-// (the smaller cut at 2^-128 of the larger).
+// alpha M for complex alpha: both parts, 128 bits each.
 struct RecScale {
-    uint32_t re[4], im[4];
-    int e;
-    uint32_t neg_re, neg_im;
+    xw::XW re, im;
     int has_im;
 };
 
@@ -2058,21 +2055,22 @@ __global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const ui
             or_.x[q] = xr[q];
             oi_.x[q] = xi[q];
         }
-        // (re + i im) of alpha M: signed products in one frame
+        // (re + i im) of alpha M: signed products, each part's in its own frame
         const uint32_t nr = frac_abs(xr), ni = frac_abs(xi);
         fxr::Fix vr, vi;
-        fxr::mul54(xr, A.re, vr.w);
-        fxr::mul54(xi, A.re, vi.w);
+        fxr::mul54(xr, A.re.w, vr.w);
+        fxr::mul54(xi, A.re.w, vi.w);
         vr.w[5] = vi.w[5] = 0u;
-        vr.neg = nr ^ A.neg_re;
-        vi.neg = ni ^ A.neg_re;
-        vr.e = vi.e = A.e - 32 - S2;
+        vr.neg = nr ^ A.re.neg;
+        vi.neg = ni ^ A.re.neg;
+        vr.e = vi.e = A.re.e - 32 - S2;
         if (A.has_im) {
             uint32_t p[5];
-            fxr::mul54(xi, A.im, p);
-            fxr::add_term(vr, p, vr.e, ni ^ A.neg_im ^ 1u);
-            fxr::mul54(xr, A.im, p);
-            fxr::add_term(vi, p, vi.e, nr ^ A.neg_im);
+            const int e = A.im.e - 32 - S2;
+            fxr::mul54(xi, A.im.w, p);
+            fxr::add_term(vr, p, e, ni ^ A.im.neg ^ 1u);
+            fxr::mul54(xr, A.im.w, p);
+            fxr::add_term(vi, p, e, nr ^ A.im.neg);
         }
         bool fast = live;
         if (beta_kind != 0 && live) {
@@ -2141,19 +2139,9 @@ __global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const ui
 RecScale rec_scale(const dd::cplx &alpha, bool one, const xw::XW &Mx)
 {
     RecScale A;
-    const xw::XW r = one ? Mx : xw::mul(xw::from_dd(alpha.re.hi, alpha.re.lo), Mx);
-    const xw::XW i = one ? xw::zero() : xw::mul(xw::from_dd(alpha.im.hi, alpha.im.lo), Mx);
-    const bool rz = r.w[3] == 0u, iz = i.w[3] == 0u;
-    A.e = rz ? i.e : (iz ? r.e : std::max(r.e, i.e));
-    auto place = [&](const xw::XW &v, bool zero, uint32_t w[4]) {
-        w[0] = w[1] = w[2] = w[3] = 0u;
-        if (!zero && A.e - v.e < 128) xw::shr4(v.w, A.e - v.e, w);
-    };
-    place(r, rz, A.re);
-    place(i, iz, A.im);
-    A.neg_re = r.neg;
-    A.neg_im = i.neg;
-    A.has_im = iz ? 0 : 1;
+    A.re = one ? Mx : xw::mul(xw::from_dd(alpha.re.hi, alpha.re.lo), Mx);
+    A.im = one ? xw::zero() : xw::mul(xw::from_dd(alpha.im.hi, alpha.im.lo), Mx);
+    A.has_im = A.im.w[3] != 0u;
     return A;
 }
 
