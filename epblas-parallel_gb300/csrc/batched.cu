@@ -73,7 +73,7 @@ struct GemmDesc {
     // tensor-core tiles only: the operands as limbs in the wave's scratch
     int64_t conv_begin;   // first group of 32 lines (rows of op(A), then columns of op(B)) in the wave
     int64_t a_off, b_off; // [64 k][line] blocks of LT_BLOCK bytes
-    int64_t ea_off, eb_off;   // exponent bounds of the lines
+    int64_t ea_off, eb_off;   // exponent bounds of the lines, split after split
     int kp, kc;           // k rounded up to 16, blocks along k
     xw::XW xa, xb;        // alpha, beta
 };
@@ -207,8 +207,9 @@ __device__ __forceinline__ int grp_search(int count, int64_t w, F begin)
 }
 
 // Exponent bounds and digits of 32 lines (rows of op(A) or columns of op(B)) of
-// an instance per block; the second pass reads what the first left in the
-// caches. A thread converts 8 k of a line: 16 bytes in each of the block's rows.
+// an instance per block, one bound per K split; the second pass reads what the
+// first left in the caches. A thread converts 8 k of a line: 16 bytes in each of
+// the block's rows.
 __global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restrict__ descs, int count,
                                                         unsigned char *out, int *ex)
 {
@@ -225,52 +226,61 @@ __global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restri
     const int64_t ld = isA ? d.lda : d.ldb;
     const double2 *X = (isA ? d.A : d.B) + (along_k ? line0 * ld : line0);
     const int64_t sl = along_k ? ld : 1, sk = along_k ? 1 : ld;
-    if (tid < 32) s_e[tid] = kNoExp;
-    __syncthreads();
-    {
-        const int l = along_k ? tid >> 3 : tid & 31, q = along_k ? tid & 7 : tid >> 5;
-        if (l < nl) {
-            const double2 *x = X + l * sl + q * sk;
-            int e = kNoExp;
-#pragma unroll 4
-            for (int p = q; p < k; p += 8, x += 8 * sk) e = max(e, exp_bound(x->x));
-            atomicMax(&s_e[l], e);
-        }
-    }
-    __syncthreads();
-    if (tid < nl) ex[(isA ? d.ea_off : d.eb_off) + line0 + tid] = s_e[tid];
-    // 8 neighbours along k, or 8 lines x 4 k per warp: whole 64 bytes either way
+    // the scan's line and place along k, and the conversion's: 8 neighbours along k, or
+    // 8 lines x 4 k per warp (whole 64 bytes either way)
+    const int ls = along_k ? tid >> 3 : tid & 31, qs = along_k ? tid & 7 : tid >> 5;
     const int l = along_k ? tid >> 3 : (tid & 7) + 8 * ((tid >> 5) & 3);
     const int q = along_k ? tid & 7 : ((tid >> 3) & 3) + 4 * (tid >> 7);
-    if (l >= nl) return;
-    const int e = s_e[l];
-    const bool live = e > kNoExp / 2 && e < 1024;
     const int lines = isA ? d.m : d.n;
-    const double2 *x = X + l * sl + (int64_t)(8 * q) * sk;
-    unsigned char *o = out + ((isA ? d.a_off : d.b_off) + line0 + l) * LT_BLOCK;
     const int64_t next = (int64_t)lines * LT_BLOCK;
-    for (int p0 = 8 * q; p0 < kp; p0 += 64, x += 64 * sk, o += next) {
-        double2 v[8];
+    const int klen = d.klen;
+    const double2 *xs = X + ls * sl + (int64_t)qs * sk, *x = X + l * sl + (int64_t)(8 * q) * sk;
+    unsigned char *o = out + ((isA ? d.a_off : d.b_off) + line0 + l) * LT_BLOCK;
+    int *pe = ex + (isA ? d.ea_off : d.eb_off) + line0 + tid;
+    int ps = qs, p0 = 8 * q;
+#pragma unroll 1
+    for (int sp = 0, k1 = klen; sp < d.splitk; ++sp, k1 += klen, pe += lines) {
+        const int ke = min(k, k1), kp1 = min(kp, k1);
+        if (sp > 0) __syncthreads();   // the last split's bounds have been read
+        if (tid < 32) s_e[tid] = kNoExp;
+        __syncthreads();
+        if (ls < nl) {
+            int e = kNoExp;
+#pragma unroll 4
+            for (; ps < ke; ps += 8, xs += 8 * sk) e = max(e, exp_bound(xs->x));
+            atomicMax(&s_e[ls], e);
+        }
+        __syncthreads();
+        if (tid < nl) *pe = s_e[tid];
+        if (l >= nl) continue;
+        const int e = s_e[l];
+        const bool live = e > kNoExp / 2 && e < 1024;
+        for (; p0 < kp1; p0 += 64, x += 64 * sk, o += next) {
+            double2 v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = live && p0 + u < k ? x[u * sk] : make_double2(0.0, 0.0);
-        uint4 b[8];
+            for (int u = 0; u < 8; ++u) v[u] = live && p0 + u < k ? x[u * sk] : make_double2(0.0, 0.0);
+            uint4 b[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            b[u] = live ? limb_bytes(v[u], fxg::FX_S - e)
-                        : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x808080u);
+            for (int u = 0; u < 8; ++u)
+                b[u] = live ? limb_bytes(v[u], fxg::FX_S - e)
+                            : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x808080u);
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            uint32_t h[4] = {0u, 0u, 0u, 0u};
-            if (r < 15) {
+            for (int r = 0; r < 16; ++r) {
+                uint32_t h[4] = {0u, 0u, 0u, 0u};
+                if (r < 15) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    auto word = [&](const uint4 &y) { return r < 4 ? y.x : r < 8 ? y.y : r < 12 ? y.z : y.w; };
-                    // 1024 + byte in both halves, less 1152
-                    const uint32_t t = __byte_perm(word(b[2 * u]), word(b[2 * u + 1]), (r & 3) | (4 + (r & 3)) << 8);
-                    asm("sub.f16x2 %0, %1, %2;" : "=r"(h[u]) : "r"((t & 0x00FF00FFu) | 0x64006400u), "r"(0x64806480u));
+                    for (int u = 0; u < 4; ++u) {
+                        auto word = [&](const uint4 &y) { return r < 4 ? y.x : r < 8 ? y.y : r < 12 ? y.z : y.w; };
+                        // 1024 + byte in both halves, less 1152
+                        const uint32_t t =
+                            __byte_perm(word(b[2 * u]), word(b[2 * u + 1]), (r & 3) | (4 + (r & 3)) << 8);
+                        asm("sub.f16x2 %0, %1, %2;"
+                            : "=r"(h[u])
+                            : "r"((t & 0x00FF00FFu) | 0x64006400u), "r"(0x64806480u));
+                    }
                 }
+                *reinterpret_cast<uint4 *>(o + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
             }
-            *reinterpret_cast<uint4 *>(o + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
         }
     }
 }
@@ -516,8 +526,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
             const LtItem &x = items[it % (2 * LT_BATCH)];
             const GemmDesc &d = descs[x.desc];
             const bool in = orow < x.mr && ocol < x.nc, some = d.k > 0;
-            const int ei = in && some ? ex[d.ea_off + x.i0 + orow] : kNoExp;
-            const int ej = in && some ? ex[d.eb_off + x.j0 + ocol] : kNoExp;
+            const int ei = in && some ? ex[d.ea_off + (int64_t)x.split * d.m + x.i0 + orow] : kNoExp;
+            const int ej = in && some ? ex[d.eb_off + (int64_t)x.split * d.n + x.j0 + ocol] : kNoExp;
             bool bad = ei >= 1024 || ej >= 1024;
             const bool live = !bad && ei > kNoExp / 2 && ej > kNoExp / 2;
             double2 *pc = d.C + x.i0 + orow + (int64_t)(x.j0 + ocol) * d.ldc;
@@ -1101,8 +1111,9 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
         d.tiles_n = (d.n + GT - 1) / GT;
         const int tiles = d.tiles_m * d.tiles_n;
         d.splitk = 1;
-        const int few = pol.max_tiles_split * (GT == LT ? LT / LT_M : 1);
-        if (pol.min_k_per_split > 0 && tiles <= few && d.k >= 2 * pol.min_k_per_split)
+        // (limb tiles: counted as 32 x 32 ones, so that the same products split)
+        const int64_t count_as = GT == LT ? ((int64_t)d.m + 31) / 32 * (((int64_t)d.n + 31) / 32) : tiles;
+        if (pol.min_k_per_split > 0 && count_as <= pol.max_tiles_split && d.k >= 2 * pol.min_k_per_split)
             d.splitk = std::min(16, d.k / pol.min_k_per_split);
         // the digit column sums hold at most 16384 multiply-adds per split, the
         // limb sums 4096 (16 accumulators' sums below 2^56 each, four of them added)
@@ -1120,7 +1131,8 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
             d.xa = xw::from_dd(d.alpha.x, d.alpha.y);
             d.xb = xw::from_dd(d.beta.x, d.beta.y);
             d.kc = (d.k + 63) / 64;
-            const int64_t blocks = ((int64_t)d.m + d.n) * d.kc, lines = d.k > 0 ? (int64_t)d.m + d.n : 0;
+            const int64_t blocks = ((int64_t)d.m + d.n) * d.kc;
+            const int64_t lines = d.k > 0 ? ((int64_t)d.m + d.n) * d.splitk : 0;   // bounds: one per line and split
             const int64_t tw = (int64_t)tiles * d.splitk;
             if (pl.waves.empty() || pl.waves.back().blocks + blocks > LT_WAVE ||
                 pl.waves.back().work + tw > INT32_MAX)
@@ -1131,7 +1143,7 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
             d.a_off = wv.blocks;
             d.b_off = wv.blocks + (int64_t)d.m * d.kc;
             d.ea_off = wv.lines;
-            d.eb_off = wv.lines + d.m;
+            d.eb_off = wv.lines + (int64_t)d.m * d.splitk;
             wv.groups += d.k > 0 ? (d.m + 31) / 32 + (d.n + 31) / 32 : 0;
             wv.blocks += blocks;
             wv.lines += lines;
