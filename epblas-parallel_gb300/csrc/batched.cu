@@ -145,7 +145,7 @@ constexpr int LT_GROUPS = LT_FIN / 4;               // of finishing warps, takin
 constexpr int LT_EXTN = LT_N / (LT_EXT / 4);        // columns of an extracting warp
 constexpr int LT_THREADS = 32 * (3 + LT_EXT + LT_FIN);
 constexpr int LT_SMEM = 1024 + LT_STAGES * LT_STAGE + 2 * LT_SUMS * 8;
-constexpr int64_t LT_WAVE = 1ll << 19;              // blocks (1 GiB) from which a batch is cut into waves
+constexpr int64_t LT_WAVE = 1ll << 19;              // blocks (1 GiB) of a wave at most
 
 // v * 2^sh (|.| < 2^116) rounded to an integer N, as the bytes of N + 128 (1 + 256 +
 // .. + 256^14): byte i holds d_i + 128.
@@ -990,8 +990,11 @@ struct Plan {
     std::vector<OzGroupItem> oz_items;   // instances routed to the tensor-core engine
     OzGroupPlan *oz = nullptr;
     int tile = 32;
-    int64_t total = 0, split_tiles = 0, partial_elems = 0;
-    // tensor-core tiles: descriptors [first, first + count) share the limb scratch
+    int64_t split_tiles = 0, partial_elems = 0;
+    // square tiles: the descriptors from `square` on, their work items and the place of
+    // their partial tiles
+    int64_t square = 0, square_work = 0, square_partials = 0;
+    // limb tiles: descriptors [first, first + count) share the limb scratch
     struct Wave {
         int first, count;
         int64_t work, groups, blocks, lines;
@@ -1003,6 +1006,16 @@ struct Plan {
     size_t dev_bytes = 0;
     cudaGraphExec_t exec = nullptr;
     uint64_t key = 0;
+
+    Plan() = default;
+    Plan(const Plan &) = delete;
+    Plan &operator=(const Plan &) = delete;
+    ~Plan()   // at the end of its thread (or of a tuner call)
+    {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (dev) cudaFree(dev);
+        ozgroup_destroy(oz);
+    }
 };
 
 std::mutex g_batched_mu;
@@ -1050,11 +1063,69 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
     pl.oz_items.clear();
     const int oz_min = (pol.oz_min > 0 && ozaki_available()) ? pol.oz_min : 0;
     const int pack_k = (pol.pack_k > 0 && ozaki_available()) ? pol.pack_k : 0;
-    const int GT = pol.tile;
-    pl.tile = GT;
-    int64_t work = 0, stiles = 0, pslots = 0;
+    pl.tile = pol.tile;
+    std::vector<GemmDesc> squares;
+    int64_t stiles = 0, pslots = 0, sq_work = 0, sq_pslots = 0;
     pl.waves.clear();
     pl.wave_blocks = pl.wave_lines = 0;
+    // d on tiles of GT: its tiles, splits and places
+    auto place = [&](GemmDesc &d, const int GT) {
+        d.tiles_m = GT == LT ? (d.m + LT_M - 1) / LT_M : (d.m + GT - 1) / GT;
+        d.tiles_n = (d.n + GT - 1) / GT;
+        const int tiles = d.tiles_m * d.tiles_n;
+        d.splitk = 1;
+        // (limb tiles: counted as 32 x 32 ones, so that the same products split)
+        const int64_t count_as = GT == LT ? ((int64_t)d.m + 31) / 32 * (((int64_t)d.n + 31) / 32) : tiles;
+        if (pol.min_k_per_split > 0 && count_as <= pol.max_tiles_split && d.k >= 2 * pol.min_k_per_split)
+            d.splitk = std::min(16, d.k / pol.min_k_per_split);
+        // the digit column sums hold at most 16384 multiply-adds per split, the
+        // limb sums 4096 (16 accumulators' sums below 2^56 each, four of them added)
+        const int kmax = GT == LT ? 4096 : 16384;
+        const int need_splits = (d.k + kmax - 1) / kmax;
+        if (d.splitk < need_splits) d.splitk = need_splits;
+        d.kp = (d.k + 15) / 16 * 16;
+        const int kstep = GT == LT ? 64 : GBK;
+        d.klen = d.splitk > 1 ? ((d.k + d.splitk - 1) / d.splitk + kstep - 1) / kstep * kstep
+                              : std::max(GT == LT ? d.kp : d.k, 1);
+        if (d.k == 0) d.klen = 1;
+        int64_t *work = &sq_work, *slots = &sq_pslots;
+        if (GT == LT) {
+            // splits past k would be empty: as many as klen needs
+            if (d.splitk > 1) d.splitk = (d.k + d.klen - 1) / d.klen;
+            d.xa = xw::from_dd(d.alpha.x, d.alpha.y);
+            d.xb = xw::from_dd(d.beta.x, d.beta.y);
+            d.kc = (d.k + 63) / 64;
+            const int64_t blocks = ((int64_t)d.m + d.n) * d.kc;
+            const int64_t lines = d.k > 0 ? ((int64_t)d.m + d.n) * d.splitk : 0;   // bounds: one per line and split
+            const int64_t tw = (int64_t)tiles * d.splitk;
+            if (pl.waves.empty() || pl.waves.back().blocks + blocks > LT_WAVE ||
+                pl.waves.back().work + tw > INT32_MAX)
+                pl.waves.push_back(Plan::Wave{(int)pl.descs.size(), 0, 0, 0, 0, 0});
+            Plan::Wave &wv = pl.waves.back();
+            d.conv_begin = wv.groups;
+            d.a_off = wv.blocks;
+            d.b_off = wv.blocks + (int64_t)d.m * d.kc;
+            d.ea_off = wv.lines;
+            d.eb_off = wv.lines + (int64_t)d.m * d.splitk;
+            wv.groups += d.k > 0 ? (d.m + 31) / 32 + (d.n + 31) / 32 : 0;
+            wv.blocks += blocks;
+            wv.lines += lines;
+            wv.count++;
+            pl.wave_blocks = std::max(pl.wave_blocks, wv.blocks);
+            pl.wave_lines = std::max(pl.wave_lines, wv.lines);
+            work = &wv.work;   // work items are numbered within the wave
+            slots = &pslots;
+        }
+        d.work_begin = *work;
+        d.tile_begin = d.splitk > 1 ? stiles : 0;
+        d.part_begin = d.splitk > 1 ? *slots : 0;
+        if (d.splitk > 1) {
+            stiles += tiles;
+            *slots += (int64_t)tiles * d.splitk;
+        }
+        *work += (int64_t)tiles * d.splitk;
+        (GT == LT ? pl.descs : squares).push_back(d);
+    };
     for (int64_t i = 0; i < count; ++i) {
         if (m[i] <= 0 || n[i] <= 0) continue;
         GemmDesc d;
@@ -1107,65 +1178,46 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
             // only the beta pass: run as a k = 0 product (sigma irrelevant)
             d.k = 0;
         }
-        d.tiles_m = GT == LT ? (d.m + LT_M - 1) / LT_M : (d.m + GT - 1) / GT;
-        d.tiles_n = (d.n + GT - 1) / GT;
-        const int tiles = d.tiles_m * d.tiles_n;
-        d.splitk = 1;
-        // (limb tiles: counted as 32 x 32 ones, so that the same products split)
-        const int64_t count_as = GT == LT ? ((int64_t)d.m + 31) / 32 * (((int64_t)d.n + 31) / 32) : tiles;
-        if (pol.min_k_per_split > 0 && count_as <= pol.max_tiles_split && d.k >= 2 * pol.min_k_per_split)
-            d.splitk = std::min(16, d.k / pol.min_k_per_split);
-        // the digit column sums hold at most 16384 multiply-adds per split, the
-        // limb sums 4096 (16 accumulators' sums below 2^56 each, four of them added)
-        const int kmax = GT == LT ? 4096 : 16384;
-        const int need_splits = (d.k + kmax - 1) / kmax;
-        if (d.splitk < need_splits) d.splitk = need_splits;
-        d.kp = (d.k + 15) / 16 * 16;
-        const int kstep = GT == LT ? 64 : GBK;
-        d.klen = d.splitk > 1 ? ((d.k + d.splitk - 1) / d.splitk + kstep - 1) / kstep * kstep
-                              : std::max(GT == LT ? d.kp : d.k, 1);
-        if (d.k == 0) d.klen = 1;
-        if (GT == LT) {
-            // splits past k would be empty: as many as klen needs
-            if (d.splitk > 1) d.splitk = (d.k + d.klen - 1) / d.klen;
-            d.xa = xw::from_dd(d.alpha.x, d.alpha.y);
-            d.xb = xw::from_dd(d.beta.x, d.beta.y);
-            d.kc = (d.k + 63) / 64;
-            const int64_t blocks = ((int64_t)d.m + d.n) * d.kc;
-            const int64_t lines = d.k > 0 ? ((int64_t)d.m + d.n) * d.splitk : 0;   // bounds: one per line and split
-            const int64_t tw = (int64_t)tiles * d.splitk;
-            if (pl.waves.empty() || pl.waves.back().blocks + blocks > LT_WAVE ||
-                pl.waves.back().work + tw > INT32_MAX)
-                pl.waves.push_back(Plan::Wave{(int)pl.descs.size(), 0, 0, 0, 0, 0});
-            Plan::Wave &wv = pl.waves.back();
-            work = wv.work;   // work items are numbered within the wave
-            d.conv_begin = wv.groups;
-            d.a_off = wv.blocks;
-            d.b_off = wv.blocks + (int64_t)d.m * d.kc;
-            d.ea_off = wv.lines;
-            d.eb_off = wv.lines + (int64_t)d.m * d.splitk;
-            wv.groups += d.k > 0 ? (d.m + 31) / 32 + (d.n + 31) / 32 : 0;
-            wv.blocks += blocks;
-            wv.lines += lines;
-            wv.work += tw;
-            wv.count++;
-            pl.wave_blocks = std::max(pl.wave_blocks, wv.blocks);
-            pl.wave_lines = std::max(pl.wave_lines, wv.lines);
+        // An instance of many lines goes in pieces that a wave holds. On the square tiles,
+        // which need no scratch: one with a k so long that its pieces would be thin, and one
+        // whose splits (every 4096 k here, 16384 there) would leave partial tiles of more than
+        // a wave and an eighth of its operands.
+        const int64_t kc = std::max<int64_t>(1, ((int64_t)d.k + 63) / 64), lines = LT_WAVE / kc;
+        const double partial = d.k > 4096 ? 32.0 * d.m * d.n * ((d.k + 4095) / 4096) : 0.0;
+        if (pol.tile != LT) {
+            place(d, pol.tile);
+        } else if (((int64_t)d.m + d.n > lines && lines < 512) ||
+                   (partial > (double)LT_WAVE * LT_BLOCK && partial > 2.0 * ((double)d.m + d.n) * d.k)) {
+            place(d, 32);
+        } else {
+            if ((int64_t)d.m + d.n <= lines) {
+                place(d, LT);
+                continue;
+            }
+            const int half = (int)(lines / 2 / 16 * 16);
+            const int pm = d.m <= half ? d.m : (d.n <= half ? (int)((lines - d.n) / 16 * 16) : half);
+            const int pn = d.n <= half ? d.n : (d.m <= half ? (int)((lines - d.m) / 16 * 16) : half);
+            for (int r0 = 0; r0 < d.m; r0 += pm) {
+                for (int c0 = 0; c0 < d.n; c0 += pn) {
+                    GemmDesc q = d;
+                    q.A = d.A + (d.ta ? (int64_t)r0 * d.lda : r0);
+                    q.B = d.B + (d.tb ? c0 : (int64_t)c0 * d.ldb);
+                    q.C = d.C + r0 + (int64_t)c0 * d.ldc;
+                    q.m = std::min(pm, d.m - r0);
+                    q.n = std::min(pn, d.n - c0);
+                    place(q, LT);
+                }
+            }
         }
-        d.work_begin = work;
-        d.tile_begin = d.splitk > 1 ? stiles : 0;
-        d.part_begin = d.splitk > 1 ? pslots : 0;
-        if (d.splitk > 1) {
-            stiles += tiles;
-            pslots += (int64_t)tiles * d.splitk;
-        }
-        work += (int64_t)tiles * d.splitk;
-        pl.descs.push_back(d);
     }
-    pl.total = work;
-    for (const Plan::Wave &wv : pl.waves) pl.total = std::max(pl.total, wv.work);
+    pl.square = (int64_t)pl.descs.size();
+    pl.square_work = sq_work;
+    pl.descs.insert(pl.descs.end(), squares.begin(), squares.end());
     pl.split_tiles = stiles;
-    pl.partial_elems = pslots * (GT == LT ? LT_M * LT_N : GT * GT);   // extended-float partials
+    // extended-float partials
+    const int sq = pl.tile == LT ? 32 : pl.tile;
+    pl.square_partials = pslots * (LT_M * LT_N);
+    pl.partial_elems = pl.square_partials + sq_pslots * sq * sq;
 }
 
 uint64_t plan_key(const Plan &pl)
@@ -1180,7 +1232,7 @@ uint64_t plan_key(const Plan &pl)
     const uint64_t *q = (const uint64_t *)pl.oz_items.data();
     const size_t nq = pl.oz_items.size() * sizeof(OzGroupItem) / 8;
     for (size_t i = 0; i < nq; ++i) h = (h ^ q[i]) * 1099511628211ull;
-    return mix(mix(h, (uint64_t)pl.tile), (uint64_t)pl.oz_items.size());
+    return mix(mix(mix(h, (uint64_t)pl.tile), (uint64_t)pl.square), (uint64_t)pl.oz_items.size());
 }
 
 // (Re)creates the device buffers and the graph when the batch layout changed.
@@ -1188,7 +1240,7 @@ uint64_t plan_key(const Plan &pl)
 // to call): the kernels are enqueued directly instead of capturing a graph.
 bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
 {
-    if ((pl.descs.empty() || pl.total == 0) && pl.oz_items.empty()) return true;
+    if (pl.descs.empty() && pl.oz_items.empty()) return true;
     const size_t d_bytes = pl.descs.size() * sizeof(GemmDesc);
     const size_t cnt_bytes = 256 + (size_t)(pl.split_tiles + 1) * sizeof(int);
     const size_t part_bytes = (size_t)pl.partial_elems * sizeof(fx::XFPod);
@@ -1227,7 +1279,6 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     unsigned char *limbs = (unsigned char *)(base + limb_off);
     int *ex = (int *)(base + (limb_off + limb_bytes_ + 255) / 256 * 256);
     const int sms = device_sm_count();
-    const int grid = (int)std::min<int64_t>(pl.total, (int64_t)sms * 16);
     if (!same) {
         // descriptors change only with the batch layout; upload outside the graph
         if (!pl.descs.empty() &&
@@ -1240,16 +1291,19 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
         }
     }
     // a launch with lost copies (test hook) is not kept in a graph
-    const int lose = pl.tile == LT && pl.total > 0 ? take_lost_load_injection() : 0;
+    const int lose = !pl.waves.empty() ? take_lost_load_injection() : 0;
     if (lose) use_graph = false;
-    // the integer-pipe or limb-tile part on stream q; its counters start at zero
+    // the square-tile and limb-tile parts on stream q; the counters start at zero
     auto enqueue = [&](cudaStream_t q) {
+        if (pl.descs.empty()) return;
         cudaMemsetAsync(counter, 0, cnt_bytes, q);
-        if (pl.tile != LT) {
+        if (pl.square_work > 0) {
             auto kern = pl.tile == 64 ? k_gemm_grouped<64> : k_gemm_grouped<32>;
-            kern<<<grid, GTHREADS, 0, q>>>(ddesc, (int)pl.descs.size(), pl.total, counter, tile_counters, partials);
-            return;
+            const int grid = (int)std::min<int64_t>(pl.square_work, (int64_t)sms * 16);
+            kern<<<grid, GTHREADS, 0, q>>>(ddesc + pl.square, (int)((int64_t)pl.descs.size() - pl.square),
+                                           pl.square_work, counter, tile_counters, partials + pl.square_partials);
         }
+        if (pl.waves.empty()) return;
         cudaFuncSetAttribute(k_gemm_grouped_limb, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
         for (const Plan::Wave &wv : pl.waves) {
             if (wv.groups > 0)
@@ -1262,10 +1316,8 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
     };
     if (!use_graph) {
         pl.key = lose ? 0 : key;
-        if (pl.total > 0) {
-            enqueue(s);
-            count_launch(pl.tile == LT ? 2 * (int64_t)pl.waves.size() : 1);
-        }
+        enqueue(s);
+        count_launch(2 * (int64_t)pl.waves.size() + (pl.square_work > 0 ? 1 : 0));
         if (pl.oz && ozgroup_count(pl.oz) > 0) ozgroup_launch(pl.oz, s);
         return cuda_ok(cudaGetLastError(), routine, "grouped launch");
     }
@@ -1280,7 +1332,7 @@ bool prepare_and_launch(Plan &pl, const char *routine, bool use_graph = true)
         bool ok = cuda_ok(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), routine, "begin capture");
         if (ok) {
             // counters start at zero on every replay
-            if (pl.total > 0) enqueue(cap);
+            enqueue(cap);
             // the large instances on the tensor cores, in the same graph
             if (pl.oz && ozgroup_count(pl.oz) > 0) ozgroup_launch(pl.oz, cap);
             ok = cuda_ok(cudaStreamEndCapture(cap, &graph), routine, "end capture");
@@ -1565,9 +1617,6 @@ extern "C" int mgemm_grouped_tune(int64_t count, const char *transa, const char 
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (pl.exec) cudaGraphExecDestroy(pl.exec);
-    if (pl.dev) cudaFree(pl.dev);
-    ozgroup_destroy(pl.oz);
     cudaFree(scratch);
     {
         std::lock_guard<std::mutex> lk(g_batched_mu);

@@ -490,10 +490,11 @@ int mgemm_grouped_tune(int64_t count, const char *transa, const char *transb, co
  * mgemm_grouped_tune call (0 before any). No counterpart in the reference. */
 int mwblas_grouped_tuned_tile(void);
 /* Forces mgemm_grouped's tiles for the instances outside the residue engine: 16 =
- * limb tiles on the tensor cores (8 x 16 outputs; the default; scratch of 32 bytes
- * per operand entry, at most 1 GiB and one instance), 32 or 64 = square tiles on
- * the integer pipes; anything else = 0 = the tuned or default choice. All give
- * results within the same bound. Returns the previous setting. */
+ * limb tiles on the tensor cores (8 x 16 outputs; scratch of 2 KiB per row of op(A)
+ * and column of op(B) for every 64 of k begun, at most 1 GiB at a time: batches in
+ * waves, large instances in pieces), 32 or 64 = square tiles on the integer pipes;
+ * anything else = 0 = the tuned or default choice. All give results within the
+ * same bound. Returns the previous setting. */
 int mwblas_set_grouped_tile(int tile);
 /* mgemm_grouped runs instances with m, n >= size and 64 <= k <= 16384 on the
  * tensor cores (Ozaki scheme, full 106-bit width, padded to classes of
