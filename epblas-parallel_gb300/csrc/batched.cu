@@ -983,6 +983,7 @@ struct Policy {
     int tile = 32;             // output tile edge: 16, 32 or 64
     int oz_min = 0;            // instances with m, n >= oz_min and k >= 64 run on the tensor cores (0: none)
     int pack_k = 0;            // the other instances with k >= pack_k share tensor-core slots, in pieces of <= 256 x 256 (0: none)
+    bool by_cost = true;       // limb tiles: not for a short k that the 32 x 32 tiles finish sooner
 };
 
 struct Plan {
@@ -1017,6 +1018,19 @@ struct Plan {
         ozgroup_destroy(oz);
     }
 };
+
+// Device time of an m x n x k product on the limb and on the 32 x 32 digit tiles, in
+// ns of a full GPU. The limb tiles' digit products are joined whatever k is (us of
+// 2000 products, limb and digit tiles: 127 x 127 x 8 3650 and 2625, x 16 3660 and
+// 3210, x 32 3700 and 4400; 48 x 48 x 8 1155 and 1080, x 16 1160 and 1250).
+double limb_ns(int64_t m, int64_t n, int64_t k)
+{
+    return (double)((m + LT_M - 1) / LT_M) * (double)((n + LT_N - 1) / LT_N) * (12.0 + 0.085 * (k > 64 ? k - 64 : 0));
+}
+double digit_ns(int64_t m, int64_t n, int64_t k)
+{
+    return (double)((m + 31) / 32) * (double)((n + 31) / 32) * (50.0 + 19.0 * (k <= 8 ? 0 : (k - 1) / 8));
+}
 
 std::mutex g_batched_mu;
 std::map<uint64_t, Policy> g_policy_cache;   // shape class -> tuned policy
@@ -1068,6 +1082,20 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
     int64_t stiles = 0, pslots = 0, sq_work = 0, sq_pslots = 0;
     pl.waves.clear();
     pl.wave_blocks = pl.wave_lines = 0;
+    // Instances with a short k on the digit tiles, in a launch of their own, where that
+    // saves a sixth of the limb tiles' time (4000 products in [8, 512], a quarter of them
+    // of k <= 24: 40 us slower with two launches; 127 x 127 x 8: a quarter faster).
+    bool short_k = false;
+    if (pol.tile == LT && pol.by_cost) {
+        double all = 0.0, saved = 0.0;
+        for (int64_t i = 0; i < count; ++i) {
+            if (m[i] <= 0 || n[i] <= 0) continue;
+            const double l = limb_ns(m[i], n[i], k[i]);
+            if (!(oz_min > 0 && m[i] >= oz_min && n[i] >= oz_min && k[i] >= 64)) all += l;
+            if (k[i] <= 24) saved += std::max(0.0, l - digit_ns(m[i], n[i], k[i]));
+        }
+        short_k = saved > all / 6.0;
+    }
     // d on tiles of GT: its tiles, splits and places
     auto place = [&](GemmDesc &d, const int GT) {
         d.tiles_m = GT == LT ? (d.m + LT_M - 1) / LT_M : (d.m + GT - 1) / GT;
@@ -1186,7 +1214,7 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
         const double partial = d.k > 4096 ? 32.0 * d.m * d.n * ((d.k + 4095) / 4096) : 0.0;
         if (pol.tile != LT) {
             place(d, pol.tile);
-        } else if (((int64_t)d.m + d.n > lines && lines < 512) ||
+        } else if ((short_k && digit_ns(d.m, d.n, d.k) < limb_ns(d.m, d.n, d.k)) || ((int64_t)d.m + d.n > lines && lines < 512) ||
                    (partial > (double)LT_WAVE * LT_BLOCK && partial > 2.0 * ((double)d.m + d.n) * d.k)) {
             place(d, 32);
         } else {
@@ -1507,7 +1535,10 @@ extern "C" int mgemm_grouped(int64_t count, const char *transa, const char *tran
         auto it = g_policy_cache.find(shape_class(count, m, n, k));
         if (it != g_policy_cache.end()) pol = it->second;
     }
-    if (g_forced_tile.load() > 0) pol.tile = g_forced_tile.load();
+    if (g_forced_tile.load() > 0) {
+        pol.tile = g_forced_tile.load();
+        pol.by_cost = false;
+    }
     if (g_forced_oz.load() >= 0) pol.oz_min = g_forced_oz.load();
     if (g_forced_pack.load() >= 0) pol.pack_k = g_forced_pack.load();
     Plan &pl = t_plan;

@@ -493,8 +493,9 @@ int mwblas_grouped_tuned_tile(void);
  * limb tiles on the tensor cores (8 x 16 outputs; scratch of 2 KiB per row of op(A)
  * and column of op(B) for every 64 of k begun, at most 1 GiB at a time: batches in
  * waves, large instances in pieces), 32 or 64 = square tiles on the integer pipes;
- * anything else = 0 = the tuned or default choice. All give results within the
- * same bound. Returns the previous setting. */
+ * anything else = 0 = the tuned or default choice (16, and the square tiles of 32
+ * for instances with a short k). All give results within the same bound. Returns
+ * the previous setting. */
 int mwblas_set_grouped_tile(int tile);
 /* mgemm_grouped runs instances with m, n >= size and 64 <= k <= 16384 on the
  * tensor cores (Ozaki scheme, full 106-bit width, padded to classes of

@@ -1,6 +1,6 @@
 """Grouped products at the lines between the limb tiles, their waves and pieces, and
-the square tiles: instances of more lines than a wave holds (rows, columns), and a k
-so long that a wave holds few lines. Against the binary128
+the square tiles: short k, instances of more lines than a wave holds (rows,
+columns, both), and a k so long that a wave holds few lines. Against the binary128
 oracle (16 units of 2^-104 k |A| |B|, as for the tiles alone); the scratch that a
 call keeps stays below a wave (1 GiB) and what the square tiles' partials take.
 """
@@ -31,6 +31,28 @@ def on_thread(body):
     t.join()
     if failures:
         raise failures[0]
+
+
+@pytest.mark.parametrize("ta,tb", [("N", "N"), ("T", "T")])
+def test_short_k(gpu, oracle, rng, ta, tb):
+    import torch
+    shapes = [(m, n, k) for m, n in ((1, 1), (8, 16), (40, 48), (64, 64), (127, 130), (300, 40))
+              for k in (0, 1, 7, 8, 9, 16, 17, 24, 25, 32)]
+    al, be = mwb.random_dd(rng, ()) + np.array([1.5, 0.0]), mwb.random_dd(rng, ())
+    inst = [(m, n, k, mwb.dd_matrix(rng, *((m, k) if ta == "N" else (k, m))),
+             mwb.dd_matrix(rng, *((k, n) if tb == "N" else (n, k))), mwb.dd_matrix(rng, m, n)) for m, n, k in shapes]
+    dev = [[torch.from_numpy(np.ascontiguousarray(x) if x.size else np.zeros((1, 1, 2))).cuda() for x in t[3:]]
+           for t in inst]
+    col, ptr, count = (lambda i: [t[i] for t in inst]), (lambda i: [d[i].data_ptr() for d in dev]), len(inst)
+    lda = [max(1, m if ta == "N" else k) for m, n, k in shapes]
+    ldb = [max(1, k if tb == "N" else n) for m, n, k in shapes]
+    assert gpu.mgemm_grouped([ta] * count, [tb] * count, col(0), col(1), col(2), [al] * count, ptr(0), lda, ptr(1), ldb,
+                             [be] * count, ptr(2), col(0)) == 0, gpu.last_error()
+    for (m, n, k, A, B, C0), d, la, lb in zip(inst, dev, lda, ldb):
+        want = oracle.qgemm(ta, tb, m, n, k, al, A, la, B, lb, be, C0.copy(), m)
+        op = orc.dd_abs(al) * (k * orc.dd_absmax(A) * orc.dd_absmax(B) if k else 0.0)
+        op += orc.dd_abs(be) * orc.dd_absmax(C0)
+        assert orc.normwise_error(d[2].cpu().numpy(), want, op) <= 16 * orc.EPS_DD, (m, n, k)
 
 
 @pytest.mark.parametrize("m,n,k", [(20, WAVE + 100000, 32), (WAVE + 3, 8, 40), (24, 140000, 300), (60, 1000000, 1),
