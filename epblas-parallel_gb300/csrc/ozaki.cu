@@ -215,6 +215,16 @@ __device__ __forceinline__ float u11_to_float(uint32_t c)
     return __int_as_float(0x4B000000 | c) - 8388608.0f;   // exact for c < 2^23
 }
 
+// W << -r for -8 < r <= 0: the top binade of a row scaled to more than 117 bits
+// (W has 118), where the image is exact.
+__device__ __forceinline__ void scale_up(const uint32_t w[4], int r, uint32_t y[4])
+{
+    y[3] = __funnelshift_l(w[2], w[3], -r);
+    y[2] = __funnelshift_l(w[1], w[2], -r);
+    y[1] = __funnelshift_l(w[0], w[1], -r);
+    y[0] = w[0] << -r;
+}
+
 // op(X) is rows x kdim; element (r, c) lives at X[r + c*ld] (ROWC) or
 // X[c + r*ld]. Writes out[l][r][c] (fp16, row stride kpad) for the padded
 // ranges r < rows_pad, c < kpad (zeros outside op(X)).
@@ -238,6 +248,8 @@ __device__ __forceinline__ void to_limbs(double2 v, int sc, float (&fl)[kResLimb
             "addc.u32 %3, %3, 0;"
             : "+r"(y[0]), "+r"(y[1]), "+r"(y[2]), "+r"(y[3])
             : "r"((word >> (rb & 31)) & 1u));
+    } else if (!(o.flags & (fx::kZero | fx::kBad)) && r <= 0 && r > -8) {
+        scale_up(o.w, r, y);
     }
     // 11-bit limbs: bits [11q, 11q + 11) of the 128-bit F
 #pragma unroll
@@ -532,6 +544,8 @@ __device__ __forceinline__ void scaled_int(double2 v, int sc, uint32_t (&y)[4], 
             "addc.u32 %3, %3, 0;"
             : "+r"(y[0]), "+r"(y[1]), "+r"(y[2]), "+r"(y[3])
             : "r"((word >> (rb & 31)) & 1u));
+    } else if (!(o.flags & (fx::kZero | fx::kBad)) && r <= 0 && r > -8) {
+        scale_up(o.w, r, y);
     }
 }
 
