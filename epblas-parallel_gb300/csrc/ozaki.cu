@@ -58,7 +58,8 @@ namespace mw {
 
 namespace {
 
-constexpr int kMaxMod = 40;
+// Two operands of 120 bits over 65,536 k and a complex sum need 260 bits: 32 moduli from 361 down.
+constexpr int kMaxMod = 32;
 constexpr int kResLimbs = 11;   // 11-bit limbs of |A'| (bits <= 120)
 constexpr int kNoExp = -30000;
 constexpr int kMaxP = 361;      // largest modulus: residues |r| <= 180 are exact in fp16
@@ -85,7 +86,6 @@ struct OzModParams {
 struct OzCrtParams {
     int nmod;
     uint32_t F[kMaxMod][crt::kFLPad];   // 160-bit fractions u_l / p_l
-    float pm[kMaxMod];
     uint64_t Mhi, Mlo;                  // M = (Mhi:Mlo) * 2^Me, truncated
     int Me;
 };
@@ -93,7 +93,7 @@ struct OzCrtParams {
 int gcd(int a, int b) { return b ? gcd(b, a % b) : a; }
 
 // The largest pairwise-coprime moduli <= kMaxP (greedy from the top), enough
-// of them for `need_bits` bits of product.
+// of them for `need_bits` bits of product; none where kMaxMod do not reach it.
 Moduli choose_moduli(double need_bits)
 {
     Moduli md;
@@ -105,6 +105,7 @@ Moduli choose_moduli(double need_bits)
         md.p[md.n++] = c;
         have += std::log2((double)c);
     }
+    if (have < need_bits) md.n = 0;
     return md;
 }
 
@@ -512,7 +513,6 @@ constexpr int RT_TILE_BYTES = 128 * 128;   // 128 rows x 64 fp16
 // Two A tiles and B, barriers; sized so that at most four CTAs (4 x 128 TMEM
 // columns) share an SM.
 constexpr int RT_SMEM = 56 * 1024;
-constexpr int RT_MAX_MOD = 32;
 
 // Chunk j (halves 8j .. 8j + 7) of a 128-byte operand row, 128-byte swizzle.
 __device__ __forceinline__ void st_row_chunk(uint8_t *tile, int row, int j, uint4 v)
@@ -660,7 +660,7 @@ __device__ __forceinline__ void rt_store(uint32_t lane_base, const OzResParams &
 {
     const int nmod = P.nmod;
 #pragma unroll
-    for (int l0 = 0; l0 < RT_MAX_MOD; l0 += 16) {
+    for (int l0 = 0; l0 < kMaxMod; l0 += 16) {
         if (l0 >= nmod) break;   // uniform
         uint32_t x[4][16];
 #pragma unroll
@@ -854,7 +854,7 @@ std::atomic<int> g_res_tc{1};   // mwblas_set_residue_tc
 // to the tile width, at most 32 moduli); false: the caller uses the FMA path.
 bool launch_residues_tc(const ResOp &a, const ResOp &b, int64_t kdim, const OzResParams &rp, int64_t kpad)
 {
-    if (g_res_tc.load() == 0 || rp.nmod > RT_MAX_MOD || kpad % RT_COLS != 0 || a.rows_pad <= 0 || !ozaki_available())
+    if (g_res_tc.load() == 0 || kpad % RT_COLS != 0 || a.rows_pad <= 0 || !ozaki_available())
         return false;
     const int64_t ntr = (a.rows_pad + RT_ROWS - 1) / RT_ROWS + (b.rows_pad + RT_ROWS - 1) / RT_ROWS;
     const int64_t ntiles = ntr * (kpad / RT_COLS);
@@ -1361,7 +1361,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
         tn = tn0 + (int)(t - (int64_t)tm2 * tiles_n);   // column tiles [tn0, tn0 + tiles_n)
         tm2 += tm0;                                     // row tile pairs [tm0, tm0 + tiles_m2)
     };
-    auto next_unit = [&](int64_t u) -> int64_t { return u < units ? u : units; };
 
     if (warp == 0 && lane == 0) {
         for (int st = 0; st < T2_STAGES; ++st) {
@@ -1394,8 +1393,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             // lose_loads (a failure-injection hook): issue no operand load at
             // all, so that the MMA issuer's first wait for a landed stage runs
             // out with nothing in flight anywhere in the pair
-            for (int64_t ua = lose_loads ? units : next_unit(cid); ua < units && ok;) {
-                const int64_t ub = next_unit(ua + ncl);
+            for (int64_t ua = lose_loads ? units : (int64_t)cid; ua < units && ok;) {
+                const int64_t ub = ua + ncl;
                 const int nu = ub < units ? 2 : 1;
                 int32_t ya[2], yb[2];
                 for (int v = 0; v < nu; ++v) {
@@ -1419,7 +1418,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                         }
                     }
                 }
-                ua = nu == 2 ? next_unit(ub + ncl) : units;
+                ua = nu == 2 ? ub + ncl : units;
             }
             // Never leave with copies in flight. A stage is released (empty, in
             // both CTAs) only after the MMAs that read it retired, i.e. after
@@ -1440,8 +1439,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
             uint32_t gs = 0;
             uint32_t uses[2] = {0, 0};
             bool ok = true;
-            for (int64_t ua = next_unit(cid); ua < units && ok;) {
-                const int64_t ub = next_unit(ua + ncl);
+            for (int64_t ua = (int64_t)cid; ua < units && ok;) {
+                const int64_t ub = ua + ncl;
                 const int nu = ub < units ? 2 : 1;
                 for (int c = 0; c < nch && ok; ++c) {
                     const int s0 = c * kcs, s1 = min(nsteps, s0 + kcs);
@@ -1469,7 +1468,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                         ++uses[b];
                     }
                 }
-                ua = nu == 2 ? next_unit(ub + ncl) : units;
+                ua = nu == 2 ? ub + ncl : units;
             }
             sm100::mma_commit_pair(drain, 1);
             sm100::mbar_wait(drain, 0, nullptr, 0);
@@ -1484,8 +1483,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
         const uint32_t acce_lead[2] = {sm100::mapa(&acce[0], 0), sm100::mapa(&acce[1], 0)};
         uint32_t fcnt[2] = {0, 0};
         bool ok = true;
-        for (int64_t ua = next_unit(cid); ua < units && ok;) {
-            const int64_t ub = next_unit(ua + ncl);
+        for (int64_t ua = (int64_t)cid; ua < units && ok;) {
+            const int64_t ub = ua + ncl;
             const int nu = ub < units ? 2 : 1;
             for (int c = 0; c < nch && ok; ++c) {
                 for (int b = 0; b < nu; ++b) {
@@ -1557,7 +1556,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCP_THREADS, 1)
                     }
                 }
             }
-            ua = nu == 2 ? next_unit(ub + ncl) : units;
+            ua = nu == 2 ? ub + ncl : units;
         }
     }
 
@@ -1618,7 +1617,7 @@ using xfp::xf_mul;
 // residue's 16-bit word is already the fp16 subnormal c * 2^-24, so the planes
 // go from memory to shared memory (cp.async) to MMA operands (ldmatrix) as they
 // are; the bytes of F sit in registers as fp16 integers. The FP32 sums start at
-// 0.5: below 361 * 255 * 40 < 2^22 units of 2^-24, they stay in [0.5, 1), whose
+// 0.5: below 361 * 255 * 32 < 2^22 units of 2^-24, they stay in [0.5, 1), whose
 // spacing is one unit, so they are exact and their words are 0x3F000000 + sum.
 // Pairs of columns are joined (16-bit spacing) and transposed through shared
 // memory so that every lane finishes whole elements; the words come out exactly
@@ -1628,10 +1627,10 @@ using xfp::xf_mul;
 // moduli, issued at 26 lanes/clk/SM) an element costs 12 MMAs per 32 and about
 // 60 other instructions.
 constexpr int RC_ROWS = 64;                        // rows of a column per warp and turn
+constexpr int KS = kMaxMod / 16;                   // steps of 16 moduli
 constexpr int RC_TR = RC_ROWS * 12 * 4;            // bytes of the transpose buffer: 12 words per row
 __host__ __device__ constexpr int rc_planes(int ks) { return ks * 16 * RC_ROWS * 2; }
 
-template <int KS>
 struct CrtFrag {
     uint32_t b[KS][3][2];
     // this lane's share of the byte matrix (row l: modulus, column n: byte n of F_l)
@@ -1658,7 +1657,6 @@ struct CrtFrag {
 
 // Zeros the plane rows nmod.. of a warp's buffer (their constants are zero, but
 // what the memory holds need not be a number).
-template <int KS>
 __device__ __forceinline__ void crt_clear(unsigned char *planes, int nmod, int lane)
 {
     for (int i = nmod * 8 + lane; i < KS * 16 * 8; i += 32)
@@ -1680,8 +1678,7 @@ __device__ __forceinline__ void crt_load(uint32_t planes, const uint16_t *q, int
 }
 
 // The column-pair sums of the warp's 64 rows into tr (12 words per row, 10 used).
-template <int KS>
-__device__ __forceinline__ void crt_sums(uint32_t planes, uint32_t *tr, const CrtFrag<KS> &f, int lane)
+__device__ __forceinline__ void crt_sums(uint32_t planes, uint32_t *tr, const CrtFrag &f, int lane)
 {
     const int g = lane >> 2, t = lane & 3;
     const uint32_t row = planes + ((lane >> 4) * 8u + (lane & 7)) * 128u;
@@ -1914,7 +1911,6 @@ struct RecTurns {
 // sums as IMAD.WIDE and the update in extended floats; 830 with the sums on the
 // tensor cores alone). 4096^2: 0.62 -> 0.36 ms; the triangle of 8192^2: 1.44 ->
 // 0.76 ms; 1531 x 1277: 83 -> 58 us.
-template <int KS>
 __global__ void __launch_bounds__(256) k_oz_reconstruct(int m, int n, const uint16_t *__restrict__ R,
                                                         int64_t Mp, int64_t Np, const int *__restrict__ ea,
                                                         const int *__restrict__ eb, int bsum, OzCrtParams K,
@@ -1927,9 +1923,9 @@ __global__ void __launch_bounds__(256) k_oz_reconstruct(int m, int n, const uint
     unsigned char *mine = s_rec + (threadIdx.x >> 5) * (rc_planes(KS) + RC_TR);
     const uint32_t planes = (uint32_t)__cvta_generic_to_shared(mine);
     uint32_t *tr = reinterpret_cast<uint32_t *>(mine + rc_planes(KS));
-    CrtFrag<KS> f;
+    CrtFrag f;
     f.fill(K, lane);
-    crt_clear<KS>(mine, K.nmod, lane);
+    crt_clear(mine, K.nmod, lane);
     const int64_t plane = Np * Mp;
     RecTurns T;
     T.begin(m, n, uplo);
@@ -1948,7 +1944,7 @@ __global__ void __launch_bounds__(256) k_oz_reconstruct(int m, int n, const uint
         const int ebj = eb[j];
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncwarp();
-        crt_sums<KS>(planes, tr, f, lane);
+        crt_sums(planes, tr, f, lane);
         __syncwarp();
         T.next();
         if (T.more()) crt_load(planes, R + T.j * Mp + T.i0, plane, K.nmod, 8, lane);
@@ -2030,7 +2026,6 @@ __device__ __noinline__ void reconstruct_c_slow(Words5 xr, Words5 xi, bool live,
 // Warps and turns as in the real kernel, four warps per block (three components'
 // planes each); the sum is linear in the residues, so the components' fractions
 // are combined mod 2^160. 2049 x 1900: 0.54 -> 0.46 ms.
-template <int KS>
 __global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const uint16_t *__restrict__ R,
                                                           int64_t Mp, int64_t Np, const int *__restrict__ ea,
                                                           const int *__restrict__ eb, int bsum, OzCrtParams K,
@@ -2044,9 +2039,9 @@ __global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const ui
     unsigned char *mine = s_rec + (threadIdx.x >> 5) * (3 * rc_planes(KS) + RC_TR);
     const uint32_t planes = (uint32_t)__cvta_generic_to_shared(mine);
     uint32_t *tr = reinterpret_cast<uint32_t *>(mine + 3 * rc_planes(KS));
-    CrtFrag<KS> f;
+    CrtFrag f;
     f.fill(K, lane);
-    for (int z = 0; z < 3; ++z) crt_clear<KS>(mine + z * rc_planes(KS), K.nmod, lane);
+    for (int z = 0; z < 3; ++z) crt_clear(mine + z * rc_planes(KS), K.nmod, lane);
     const int64_t plane = Np * Mp, cstride = (int64_t)K.nmod * plane;
     auto load = [&](int64_t i0, int j) {
         for (int z = 0; z < 3; ++z)
@@ -2114,7 +2109,7 @@ __global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const ui
 #pragma unroll
         for (int z = 0; z < 3; ++z) {
             __syncwarp();   // the planes have landed; the previous component's words have been read
-            crt_sums<KS>(planes + z * rc_planes(KS), tr, f, lane);
+            crt_sums(planes + z * rc_planes(KS), tr, f, lane);
             __syncwarp();
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -2207,7 +2202,6 @@ void fill_crt_params(const Moduli &md, OzCrtParams &cp)
     cp.nmod = md.n;
     xfp::XF Mx;
     crt::constants(md.p, md.n, cp.F, Mx);
-    for (int l = 0; l < md.n; ++l) cp.pm[l] = (float)md.p[l];
     cp.Mhi = (uint64_t)(Mx.m >> 64);
     cp.Mlo = (uint64_t)Mx.m;
     cp.Me = Mx.e;
@@ -2387,7 +2381,12 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
         }
     }
     const double need = (bits_a - 1) + (bits_b - 1) + std::log2((double)(k > 1 ? k : 1)) + 1.0 + 4.0 + (cplx ? 1.0 : 0.0);
-    Moduli md = choose_moduli(need);
+    const Moduli md = choose_moduli(need);
+    if (md.n == 0) {
+        set_error(routine, MWBLAS_ERR_UNSUPPORTED, "operands too wide for the tensor-core engine's moduli");
+        dev_free(ex);
+        return false;
+    }
     g_last_moduli = md.n;
     g_last_bits[0] = bits_a;
     g_last_bits[1] = bits_b;
@@ -2560,12 +2559,11 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             bool alpha_one = (g.alpha.hi == 1.0 && g.alpha.lo == 0.0);
             // alpha folded into M: alpha * X = T * (alpha M)
             const xw::XW aM = alpha_one ? Mx : xw::mul(xw::from_dd(g.alpha.hi, g.alpha.lo), Mx);
-            auto kern = cp.nmod <= 32 ? k_oz_reconstruct<2> : k_oz_reconstruct<3>;
-            const int smem = 8 * (rc_planes(cp.nmod <= 32 ? 2 : 3) + RC_TR);
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            kern<<<grid, 256, smem, stream()>>>((int)m, (int)nn, Rj, Mp, Np, ea, eb + j0, bits_a + bits_b, cp, aM,
-                                                xw::from_dd(g.beta.hi, g.beta.lo), dd::make(g.beta.hi, g.beta.lo),
-                                                g.beta_kind, Cj, g.ldc, g.uplo);
+            const int smem = 8 * (rc_planes(KS) + RC_TR);
+            cudaFuncSetAttribute(k_oz_reconstruct, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            k_oz_reconstruct<<<grid, 256, smem, stream()>>>(
+                (int)m, (int)nn, Rj, Mp, Np, ea, eb + j0, bits_a + bits_b, cp, aM, xw::from_dd(g.beta.hi, g.beta.lo),
+                dd::make(g.beta.hi, g.beta.lo), g.beta_kind, Cj, g.ldc, g.uplo);
         } else {
             dd::cplx al, be;
             al.re = dd::make(g.calpha.re.hi, g.calpha.re.lo);
@@ -2574,10 +2572,9 @@ bool gemm_ozaki(const GemmArgs &g0, bool cplx, int bits_req, const char *routine
             be.im = dd::make(g.cbeta.im.hi, g.cbeta.im.lo);
             bool alpha_one = (g.calpha.re.hi == 1.0 && g.calpha.re.lo == 0.0 && g.calpha.im.hi == 0.0 &&
                               g.calpha.im.lo == 0.0);
-            auto kern = cp.nmod <= 32 ? k_oz_reconstruct_c<2> : k_oz_reconstruct_c<3>;
-            const int smem = 4 * (3 * rc_planes(cp.nmod <= 32 ? 2 : 3) + RC_TR);
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            kern<<<grid, 128, smem, stream()>>>(
+            const int smem = 4 * (3 * rc_planes(KS) + RC_TR);
+            cudaFuncSetAttribute(k_oz_reconstruct_c, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            k_oz_reconstruct_c<<<grid, 128, smem, stream()>>>(
                 (int)m, (int)nn, Rj, Mp, Np, ea, eb + j0, bits_a + bits_b, cp, Mx, xw::from_dd(al.re.hi, al.re.lo),
                 xw::from_dd(al.im.hi, al.im.lo), alpha_one ? 1 : 0, rec_scale(al, alpha_one, Mx), be, xw::from_dd(be.re.hi, be.re.lo),
                 xw::from_dd(be.im.hi, be.im.lo), g.beta_kind, Cj, g.ldc, g.uplo, g.herm ? 1 : 0, g.herm ? 1 : 0);
@@ -2940,7 +2937,6 @@ __global__ void __launch_bounds__(256) k_grp_clear_tails(const OzGrpDesc *__rest
 
 // alpha * X * 2^-S2 + beta C for every instance. A work item is 64 rows x 8
 // columns of one instance, a warp per column (crt_sums).
-template <int KS>
 __global__ void __launch_bounds__(256) k_grp_reconstruct(const OzGrpDesc *__restrict__ descs, int count,
                                                          int64_t items, const OzGrpClass *__restrict__ classes,
                                                          const int *__restrict__ ex, int bsum, OzCrtParams K)
@@ -2950,9 +2946,9 @@ __global__ void __launch_bounds__(256) k_grp_reconstruct(const OzGrpDesc *__rest
     unsigned char *mine = s_rec + (threadIdx.x >> 5) * (rc_planes(KS) + RC_TR);
     const uint32_t planes = (uint32_t)__cvta_generic_to_shared(mine);
     uint32_t *tr = reinterpret_cast<uint32_t *>(mine + rc_planes(KS));
-    CrtFrag<KS> f;
+    CrtFrag f;
     f.fill(K, lane);
-    crt_clear<KS>(mine, K.nmod, lane);
+    crt_clear(mine, K.nmod, lane);
     const int nmod = K.nmod;
     // this warp's column of item w: false past the instance's columns
     struct Turn {
@@ -2989,7 +2985,7 @@ __global__ void __launch_bounds__(256) k_grp_reconstruct(const OzGrpDesc *__rest
     while (have) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncwarp();
-        crt_sums<KS>(planes, tr, f, lane);
+        crt_sums(planes, tr, f, lane);
         __syncwarp();
         const bool more = advance(nxt);
         if (more) load(nxt);
@@ -3073,7 +3069,11 @@ bool ozgroup_prepare(OzGroupPlan *pl, const std::vector<OzGroupItem> &items, con
     int64_t kmax = 1;
     for (const OzGroupItem &it : items) kmax = std::max<int64_t>(kmax, it.k);
     pl->md = choose_moduli(2.0 * (kGroupBits - 1) + std::log2((double)kmax) + 1.0 + 4.0);
-    pl->res_tc = g_res_tc.load() != 0 && pl->md.n <= RT_MAX_MOD;
+    if (pl->md.n == 0) {
+        set_error(routine, MWBLAS_ERR_UNSUPPORTED, "k too long for the tensor-core engine's moduli");
+        return false;
+    }
+    pl->res_tc = g_res_tc.load() != 0;
     const int trows = pl->res_tc ? RT_ROWS : 32;   // conversion tile rows
     fill_res_params(pl->md, pl->rp, pl->mp);
     fill_crt_params(pl->md, pl->cp);
@@ -3246,17 +3246,12 @@ void ozgroup_launch(OzGroupPlan *pl, cudaStream_t s)
                                                              c.Mp, c.Np, pl->mp, c.R, device_status_word(), 0,
                                                              tiles_m2, tiles_n, nz, 0, 0, take_lost_load_injection(), L);
     }
-    auto kern = pl->cp.nmod <= 32 ? k_grp_reconstruct<2> : k_grp_reconstruct<3>;
-    const int smem = 8 * (rc_planes(pl->cp.nmod <= 32 ? 2 : 3) + RC_TR);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    kern<<<(unsigned)std::min<int64_t>(pl->items, (int64_t)sms * 8), 256, smem, s>>>(
+    const int smem = 8 * (rc_planes(KS) + RC_TR);
+    cudaFuncSetAttribute(k_grp_reconstruct, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_grp_reconstruct<<<(unsigned)std::min<int64_t>(pl->items, (int64_t)sms * 8), 256, smem, s>>>(
         pl->d_descs, count, pl->items, pl->d_classes, pl->d_ex, 2 * kGroupBits, pl->cp);
     count_launch(3 + (int64_t)pl->classes.size());
 }
-
-namespace {
-
-}  // namespace
 
 bool gemm_ozaki_real(const GemmArgs &g, int bits, const char *routine) { return gemm_ozaki(g, false, bits, routine); }
 bool gemm_ozaki_cplx(const GemmArgs &g, int bits, const char *routine) { return gemm_ozaki(g, true, bits, routine); }
