@@ -14,6 +14,7 @@
 // in mdot.cpp:60-64) so that its partial sums fit its fixed scratch array.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "dd.cuh"
@@ -128,6 +129,7 @@ __global__ void k_gemv_n_final(int64_t m, int nchunks, const double2 *part, dd::
 // 1.11 ms (more shared-memory reads and set-up per element), loads into
 // registers one group ahead in place of the cp.async ring 1.29 ms.
 
+constexpr int kShort = 32;                // reductions up to this take a thread per output
 constexpr int kWin = 32;                  // reduction indices per window
 constexpr int kMaxChunk = 64 * kWin;      // per block: int32 column sums stay below 2^30
 constexpr int kColWords = 104;            // B entry of one index: 8 x 12 words, its exponent, pad (8 mod 32 words:
@@ -532,6 +534,53 @@ __global__ void __launch_bounds__(256, 2) k_gemv_limb(const GemvArgs g)
     }
 }
 
+// Short reductions (len <= kShort): a thread per output, its products added in fixed
+// point (fixacc.cuh) against x's digits in shared memory, y updated in the same
+// launch. The limb kernel works in windows of 32 indices and sets up shared memory
+// per 256 outputs. Whole call, us, limb kernel and this one: 2,000,000 outputs N,
+// len 1 329 and 99, 8 369 and 187, 24 456 and 365, 32 577 and 459, 48 606 and 635;
+// 5000 outputs, len 4 38 and 34, 24 41 and 39, 32 42 and 44.
+__global__ void __launch_bounds__(256) k_gemv_short(const GemvArgs g)
+{
+    __shared__ fx::Dig s_d[kShort];
+    bool mine = true;   // x holds neither zeros nor non-finite values
+    if (threadIdx.x < (unsigned)g.len) {
+        s_d[threadIdx.x] = fx::to_dig(fx::decode(g.x[vidx(threadIdx.x, g.len, g.incx)]));
+        mine = (s_d[threadIdx.x].flags & (fx::kZero | fx::kBad)) == 0;
+    }
+    const bool plain = __syncthreads_and(mine) != 0;
+    const xfp::XF xa = xfp::xf_from_dd(g.alpha.hi, g.alpha.lo);
+    for (int64_t r = blockIdx.x * 256ll + threadIdx.x; r < g.rows; r += gridDim.x * 256ll) {
+        const double2 *a = g.A + r * g.rs;
+        fx::Acc acc;
+        acc.reset();
+        int c = 0;
+        for (; c + 4 <= (int)g.len; c += 4) {   // four in flight, one block-exponent test for normal operands
+            double2 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u, a += g.cs) v[u] = __ldcs(a);
+            if (fx::decode_is_fast(v[0]) && fx::decode_is_fast(v[1]) && fx::decode_is_fast(v[2]) &&
+                fx::decode_is_fast(v[3]) && plain) {
+                fx::Op o[4];
+                int e[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    o[u] = fx::decode_fast(v[u]);
+                    e[u] = o[u].e + s_d[c + u].e;
+                }
+                acc.admit(max(max(e[0], e[1]), max(e[2], e[3])));
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc.mul_fast(o[u], s_d[c + u], acc.B - e[u]);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc.add_core(fx::decode(v[u]), s_d[c + u]);
+            }
+        }
+        for (; c < (int)g.len; ++c, a += g.cs) acc.add_core(fx::decode(__ldcs(a)), s_d[c]);
+        gemv_store(g, r, xa, acc.finish(), acc.bad);
+    }
+}
+
 // The chunks' sums of each output, LANES lanes per output in a fixed order,
 // then the update of y.
 template <int LANES>
@@ -587,6 +636,13 @@ bool gemv_device(bool trans, int64_t m, int64_t n, dd_host alpha, const void *A,
     g.alpha = dd::make(alpha.hi, alpha.lo);
     g.beta = be;
     g.beta_kind = beta_kind;
+    if (len <= kShort) {
+        const int64_t blocks = std::min<int64_t>((rows + 255) / 256, 8ll * sms);
+        g.part = nullptr;
+        k_gemv_short<<<(unsigned)blocks, 256, 0, stream()>>>(g);
+        count_launch();
+        return true;
+    }
     // 16 kR outputs per warp, up to eight warps per block: fewer where eight
     // would leave SMs without a block (a small product is bound by the latency
     // of its windows in turn, about 2 us each), and four where the last block
