@@ -71,7 +71,7 @@ struct GemmDesc {
     int64_t part_begin;   // first partial-tile slot: earlier split instances
                           // hold tiles * splitk slots each
     // tensor-core tiles only: the operands as limbs in the wave's scratch
-    int64_t conv_begin;   // first group of 32 lines (rows of op(A), then columns of op(B)) in the wave
+    int64_t conv_begin;   // first (32 lines of op(A), then op(B); K split) of the conversion in the wave
     int64_t a_off, b_off; // [64 k][line] blocks of LT_BLOCK bytes
     int64_t ea_off, eb_off;   // exponent bounds of the lines, split after split
     int kp, kc;           // k rounded up to 16, blocks along k
@@ -207,9 +207,10 @@ __device__ __forceinline__ int grp_search(int count, int64_t w, F begin)
 }
 
 // Exponent bounds and digits of 32 lines (rows of op(A) or columns of op(B)) of
-// an instance per block, one bound per K split; the second pass reads what the
-// first left in the caches. A thread converts 8 k of a line: 16 bytes in each of
-// the block's rows.
+// one K split of an instance per block; the second pass reads what the first left
+// in the caches. A thread converts 8 k of a line: 16 bytes in each of the block's
+// rows. (A block per 32 lines for all of k left 3 products of 64 x 64 x 16384 to 12
+// blocks: 1039 us the call, now 244.)
 __global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restrict__ descs, int count,
                                                         unsigned char *out, int *ex)
 {
@@ -217,70 +218,63 @@ __global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restri
     const int tid = threadIdx.x;
     const GemmDesc &d =
         descs[grp_search(count, (int64_t)blockIdx.x, [&](int q) { return descs[q].conv_begin; })];
-    int grp = (int)((int64_t)blockIdx.x - d.conv_begin);
+    const uint32_t at = (uint32_t)((int64_t)blockIdx.x - d.conv_begin);
+    int grp = (int)(at / (uint32_t)d.splitk);
+    const int sp = (int)(at - (uint32_t)grp * (uint32_t)d.splitk), k0 = sp * d.klen;
     const int ga = (d.m + 31) / 32;
     const bool isA = grp < ga;
     if (!isA) grp -= ga;
-    const int line0 = grp * 32, nl = min(32, (isA ? d.m : d.n) - line0), k = d.k, kp = d.kp;
+    const int lines = isA ? d.m : d.n, line0 = grp * 32, nl = min(32, lines - line0);
+    const int k = min(d.k - k0, d.klen), kp = min(d.kp - k0, d.klen);
     const bool along_k = isA ? d.ta != 0 : d.tb == 0;   // a line's entries are neighbours in memory
     const int64_t ld = isA ? d.lda : d.ldb;
-    const double2 *X = (isA ? d.A : d.B) + (along_k ? line0 * ld : line0);
     const int64_t sl = along_k ? ld : 1, sk = along_k ? 1 : ld;
-    // the scan's line and place along k, and the conversion's: 8 neighbours along k, or
-    // 8 lines x 4 k per warp (whole 64 bytes either way)
-    const int ls = along_k ? tid >> 3 : tid & 31, qs = along_k ? tid & 7 : tid >> 5;
-    const int l = along_k ? tid >> 3 : (tid & 7) + 8 * ((tid >> 5) & 3);
-    const int q = along_k ? tid & 7 : ((tid >> 3) & 3) + 4 * (tid >> 7);
-    const int lines = isA ? d.m : d.n;
-    const int64_t next = (int64_t)lines * LT_BLOCK;
-    const int klen = d.klen;
-    const double2 *xs = X + ls * sl + (int64_t)qs * sk, *x = X + l * sl + (int64_t)(8 * q) * sk;
-    unsigned char *o = out + ((isA ? d.a_off : d.b_off) + line0 + l) * LT_BLOCK;
-    int *pe = ex + (isA ? d.ea_off : d.eb_off) + line0 + tid;
-    int ps = qs, p0 = 8 * q;
-#pragma unroll 1
-    for (int sp = 0, k1 = klen; sp < d.splitk; ++sp, k1 += klen, pe += lines) {
-        const int ke = min(k, k1), kp1 = min(kp, k1);
-        if (sp > 0) __syncthreads();   // the last split's bounds have been read
-        if (tid < 32) s_e[tid] = kNoExp;
-        __syncthreads();
-        if (ls < nl) {
+    const double2 *X = (isA ? d.A : d.B) + line0 * sl + k0 * sk;
+    if (tid < 32) s_e[tid] = kNoExp;
+    __syncthreads();
+    {
+        const int l = along_k ? tid >> 3 : tid & 31, q = along_k ? tid & 7 : tid >> 5;
+        if (l < nl) {
+            const double2 *x = X + l * sl + q * sk;
             int e = kNoExp;
 #pragma unroll 4
-            for (; ps < ke; ps += 8, xs += 8 * sk) e = max(e, exp_bound(xs->x));
-            atomicMax(&s_e[ls], e);
+            for (int p = q; p < k; p += 8, x += 8 * sk) e = max(e, exp_bound(x->x));
+            atomicMax(&s_e[l], e);
         }
-        __syncthreads();
-        if (tid < nl) *pe = s_e[tid];
-        if (l >= nl) continue;
-        const int e = s_e[l];
-        const bool live = e > kNoExp / 2 && e < 1024;
-        for (; p0 < kp1; p0 += 64, x += 64 * sk, o += next) {
-            double2 v[8];
+    }
+    __syncthreads();
+    if (tid < nl) ex[(isA ? d.ea_off : d.eb_off) + (int64_t)sp * lines + line0 + tid] = s_e[tid];
+    // 8 neighbours along k, or 8 lines x 4 k per warp: whole 64 bytes either way
+    const int l = along_k ? tid >> 3 : (tid & 7) + 8 * ((tid >> 5) & 3);
+    const int q = along_k ? tid & 7 : ((tid >> 3) & 3) + 4 * (tid >> 7);
+    if (l >= nl) return;
+    const int e = s_e[l];
+    const bool live = e > kNoExp / 2 && e < 1024;
+    const double2 *x = X + l * sl + (int64_t)(8 * q) * sk;
+    unsigned char *o = out + ((isA ? d.a_off : d.b_off) + (int64_t)(k0 / 64) * lines + line0 + l) * LT_BLOCK;
+    const int64_t next = (int64_t)lines * LT_BLOCK;
+    for (int p0 = 8 * q; p0 < kp; p0 += 64, x += 64 * sk, o += next) {
+        double2 v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = live && p0 + u < k ? x[u * sk] : make_double2(0.0, 0.0);
-            uint4 b[8];
+        for (int u = 0; u < 8; ++u) v[u] = live && p0 + u < k ? x[u * sk] : make_double2(0.0, 0.0);
+        uint4 b[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                b[u] = live ? limb_bytes(v[u], fxg::FX_S - e)
-                            : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x808080u);
+        for (int u = 0; u < 8; ++u)
+            b[u] = live ? limb_bytes(v[u], fxg::FX_S - e)
+                        : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x808080u);
 #pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                uint32_t h[4] = {0u, 0u, 0u, 0u};
-                if (r < 15) {
+        for (int r = 0; r < 16; ++r) {
+            uint32_t h[4] = {0u, 0u, 0u, 0u};
+            if (r < 15) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        auto word = [&](const uint4 &y) { return r < 4 ? y.x : r < 8 ? y.y : r < 12 ? y.z : y.w; };
-                        // 1024 + byte in both halves, less 1152
-                        const uint32_t t =
-                            __byte_perm(word(b[2 * u]), word(b[2 * u + 1]), (r & 3) | (4 + (r & 3)) << 8);
-                        asm("sub.f16x2 %0, %1, %2;"
-                            : "=r"(h[u])
-                            : "r"((t & 0x00FF00FFu) | 0x64006400u), "r"(0x64806480u));
-                    }
+                for (int u = 0; u < 4; ++u) {
+                    auto word = [&](const uint4 &y) { return r < 4 ? y.x : r < 8 ? y.y : r < 12 ? y.z : y.w; };
+                    // 1024 + byte in both halves, less 1152
+                    const uint32_t t = __byte_perm(word(b[2 * u]), word(b[2 * u + 1]), (r & 3) | (4 + (r & 3)) << 8);
+                    asm("sub.f16x2 %0, %1, %2;" : "=r"(h[u]) : "r"((t & 0x00FF00FFu) | 0x64006400u), "r"(0x64806480u));
                 }
-                *reinterpret_cast<uint4 *>(o + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
             }
+            *reinterpret_cast<uint4 *>(o + r * 128 + ((q ^ (r & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
         }
     }
 }
@@ -1135,7 +1129,7 @@ void build_descs(Plan &pl, int64_t count, const char *ta, const char *tb, const 
             d.b_off = wv.blocks + (int64_t)d.m * d.kc;
             d.ea_off = wv.lines;
             d.eb_off = wv.lines + (int64_t)d.m * d.splitk;
-            wv.groups += d.k > 0 ? (d.m + 31) / 32 + (d.n + 31) / 32 : 0;
+            wv.groups += d.k > 0 ? ((int64_t)(d.m + 31) / 32 + (d.n + 31) / 32) * d.splitk : 0;
             wv.blocks += blocks;
             wv.lines += lines;
             wv.count++;
