@@ -2085,9 +2085,16 @@ __global__ void __launch_bounds__(128) k_oz_reconstruct_c(int m, int n, const ui
         if (beta_kind != 0 && live) {
             const double2 cr = pc[0], ci = pc[1];
             const bool b1 = beta_kind == 1;
-            fast = add_beta_c(vr, cr, br, b1, 0u) && add_beta_c(vi, ci, br, b1, 0u);
-            if (!b1 && !real_beta && bi.w[3] != 0u)
-                fast = fast && add_beta_c(vr, ci, bi, false, 1u) && add_beta_c(vi, cr, bi, false, 0u);
+            ImageC re, im;
+            fast = image_c(cr.x, cr.y, re) && image_c(ci.x, ci.y, im);
+            if (fast) {
+                add_image(vr, re, br, b1, 0u);
+                add_image(vi, im, br, b1, 0u);
+                if (!b1 && !real_beta && bi.w[3] != 0u) {
+                    add_image(vr, im, bi, false, 1u);
+                    add_image(vi, re, bi, false, 0u);
+                }
+            }
         }
         if (!fast) {
             reconstruct_c_slow(or_, oi_, live, S2, Mx, ar, ai, alpha_one, beta, br, bi, beta_kind, real_beta, diag, pc);
