@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restri
     const GemmDesc &d =
         descs[grp_search(count, (int64_t)blockIdx.x, [&](int q) { return descs[q].conv_begin; })];
     const uint32_t at = (uint32_t)((int64_t)blockIdx.x - d.conv_begin);
-    int grp = (int)(at / (uint32_t)d.splitk);
+    int grp = (int)(d.splitk == 1 ? at : at / (uint32_t)d.splitk);
     const int sp = (int)(at - (uint32_t)grp * (uint32_t)d.splitk), k0 = sp * d.klen;
     const int ga = (d.m + 31) / 32;
     const bool isA = grp < ga;
@@ -520,8 +520,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
             const LtItem &x = items[it % (2 * LT_BATCH)];
             const GemmDesc &d = descs[x.desc];
             const bool in = orow < x.mr && ocol < x.nc, some = d.k > 0;
-            const int ei = in && some ? ex[d.ea_off + (int64_t)x.split * d.m + x.i0 + orow] : kNoExp;
-            const int ej = in && some ? ex[d.eb_off + (int64_t)x.split * d.n + x.j0 + ocol] : kNoExp;
+            const int ei = in && some ? ex[d.ea_off + (int64_t)x.split * x.lines_a + x.i0 + orow] : kNoExp;
+            const int ej = in && some ? ex[d.eb_off + (int64_t)x.split * x.lines_b + x.j0 + ocol] : kNoExp;
             bool bad = ei >= 1024 || ej >= 1024;
             const bool live = !bad && ei > kNoExp / 2 && ej > kNoExp / 2;
             double2 *pc = d.C + x.i0 + orow + (int64_t)(x.j0 + ocol) * d.ldc;
