@@ -6,7 +6,8 @@
 // mgemm_grouped: the large instances go to the residue engine (ozaki.cu), the rest
 // to tiles of one kernel over all of them, so that thousands of uneven instances
 // keep all SMs busy. By default these are limb tiles on the tensor cores (their
-// section below); the forced 32 x 32 and 64 x 64 tiles run the fixed-point
+// section below). Square tiles (32 x 32 beside the limb tiles where build_descs says
+// so, 32 x 32 or 64 x 64 for all where forced or tuned) run the fixed-point
 // arithmetic of the integer-pipe engine (gemm_fixed.cu, fixgemm.cuh): CTAs of 256
 // threads pull (instance, tile, K split) items from an atomic counter, and the
 // item's A rows / B columns are scaled from an exponent scan over its own K range
@@ -103,8 +104,8 @@ __device__ __forceinline__ void load_digits(const int *src, int (&dst)[R])
 
 // ---- 8 x 16 output tiles on the tensor cores (byte limbs) -------------------------------
 //
-// Operands are scaled to integers N below 2^116 of their row's (column's) bound,
-// as in the digit kernel below, and held as 15 digits d_i in [-128, 127] of base
+// Operands are scaled to integers N below 2^116 of their row's (column's) bound over
+// the tile's K split, as in the digit kernel below, and held as 15 digits d_i in [-128, 127] of base
 // 256, fp16 each, and a zero. A first kernel writes them once per operand
 // (k_grp_limbs) in blocks of 16 digits x 64 k per line, as the shared-memory image
 // of a K-major operand with 128-byte swizzle; the blocks of neighbouring lines are
@@ -130,8 +131,8 @@ __device__ __forceinline__ void load_digits(const int *src, int (&dst)[R])
 // the finishing 0.93; the tensor pipe is 20 % busy, issue 55 %. 16 joining or 12
 // finishing warps change nothing; with the search for a tile's instance in the
 // copying warp it took 1.2. On 4000 such products 9.8 ms on 16 x 16 tiles of the
-// legacy MMA (mma.sync, a third busy), 14.9 on 32 x 32 digit tiles, now 4.5, with
-// 1.2 for the digits (0.84 as bytes).
+// legacy MMA (mma.sync, a third busy), 14.9 on 32 x 32 digit tiles, now 4.6, with
+// 1.26 for the digits (0.84 as bytes).
 constexpr int LT = 16;                              // the policy's name for these tiles
 constexpr int LT_M = 8, LT_N = 16;                  // rows and columns of a tile
 constexpr int LT_BLOCK = 16 * 64 * 2;               // bytes of a line's digits over 64 k

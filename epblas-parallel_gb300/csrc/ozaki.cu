@@ -1907,9 +1907,9 @@ struct RecTurns {
 // turn's residues are copied while this one's outputs are finished. m and n
 // below 2^31 (the host routes larger sizes elsewhere).
 //
-// Bound: instruction issue, 551 per output with a general beta (950 with the
+// Bound: instruction issue, 563 per output with a general beta (950 with the
 // sums as IMAD.WIDE and the update in extended floats; 830 with the sums on the
-// tensor cores alone). 4096^2: 0.62 -> 0.36 ms; the triangle of 8192^2: 1.44 ->
+// tensor cores alone). 4096^2: 0.62 -> 0.37 ms; the triangle of 8192^2: 1.44 ->
 // 0.76 ms; 1531 x 1277: 83 -> 58 us.
 __global__ void __launch_bounds__(256) k_oz_reconstruct(int m, int n, const uint16_t *__restrict__ R,
                                                         int64_t Mp, int64_t Np, const int *__restrict__ ea,
