@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(GTHREADS) k_grp_limbs(const GemmDesc *__restri
 // A tile as announced to the roles.
 struct LtItem {
     int64_t a, b;                // first blocks of its operands
+    int64_t ea, eb;              // first of its lines' exponent bounds
     int desc, i0, j0, mr, nc, kn, tile, split;
     int lines_a, lines_b;        // blocks from one 64 k to the next
 };
@@ -371,6 +372,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
                 x.lines_b = d.n;
                 x.a = d.a_off + (int64_t)(k0 / 64) * d.m + x.i0;
                 x.b = d.b_off + (int64_t)(k0 / 64) * d.n + x.j0;
+                x.ea = d.ea_off + (int64_t)x.split * d.m + x.i0;
+                x.eb = d.eb_off + (int64_t)x.split * d.n + x.j0;
                 items[it % (2 * LT_BATCH)] = x;
             }
             __syncwarp();
@@ -521,8 +524,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) k_gemm_grouped_limb(const GemmD
             const LtItem &x = items[it % (2 * LT_BATCH)];
             const GemmDesc &d = descs[x.desc];
             const bool in = orow < x.mr && ocol < x.nc, some = d.k > 0;
-            const int ei = in && some ? ex[d.ea_off + (int64_t)x.split * x.lines_a + x.i0 + orow] : kNoExp;
-            const int ej = in && some ? ex[d.eb_off + (int64_t)x.split * x.lines_b + x.j0 + ocol] : kNoExp;
+            const int ei = in && some ? ex[x.ea + orow] : kNoExp;
+            const int ej = in && some ? ex[x.eb + ocol] : kNoExp;
             bool bad = ei >= 1024 || ej >= 1024;
             const bool live = !bad && ei > kNoExp / 2 && ej > kNoExp / 2;
             double2 *pc = d.C + x.i0 + orow + (int64_t)(x.j0 + ocol) * d.ldc;

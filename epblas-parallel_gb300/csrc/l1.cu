@@ -488,9 +488,9 @@ __device__ bool block_any(bool b)
 // digit products and their digit splits took 223. Turns with zeros or alignments
 // beyond a word have a loop of their own, which shifts any way, and pass without
 // products where all are zero: whole call at n = 10^8, with the general decode for
-// each such turn, as the digit form was, and now: a zero in 64 1268, 949 and 850 us;
-// the second half zero 897, 691 and 676; exponents over 2^40 1245, 957 and 872;
-// dense 642, 907 and 648.
+// each such turn, as the digit form was, and now: a zero in 64 1268, 949 and 866 us;
+// the second half zero 897, 691 and 675; exponents over 2^40 1245, 957 and 888;
+// dense 642, 907 and 641.
 constexpr int kDotFlush = 4;            // turns of 64 pairs per move to the int32 sums
 constexpr int kDotFold = 16;            // moves per fold into the extended float
 constexpr int kDotStages = 4;           // turns in flight
@@ -579,6 +579,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
     for (int u = 0; u < kDotStages - 1; ++u) load(u);
     unsigned char *limbs = s_dot + kDotStages * 4 * kPlane + wid * 2048;
     const uint32_t lrow = (uint32_t)__cvta_generic_to_shared(limbs) + lane * 16u;
+    bool any_shift = true;   // (the first turn has no block)
     // the turn's aligned limbs into the sums, and what is due after it
     auto products = [&](int64_t turn, const uint32_t (&wx)[2][4], const uint32_t (&wy)[2][4], const uint32_t (&neg)[2],
                         bool go) {
@@ -613,11 +614,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
             if ((turn & (kDotFlush * kDotFold - 1)) == kDotFlush * kDotFold - 1) {
                 fold();
                 blk = kNoBlock;   // the next products find their own block
+                any_shift = true;
             }
         }
     };
     int64_t turn = 0;
-    bool any_shift = true;
     while (turn < turns) {
         // turns whose operands are all on the straight line, within a word of the block
 #pragma unroll 1
@@ -684,6 +685,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_mdot_limb(int64_t n, const doub
                 }
             } else {
                 // the end, operands off the straight-line path, a larger block
+                any_shift = false;   // the next turn may well be dense
                 int ep[2], top = kNoBlock;
 #pragma unroll
                 for (int p = 0; p < 2; ++p) {
